@@ -113,12 +113,14 @@ size_t solve_bytes(const ot2d_params& p, int precision) {
 
 bool batch_fits(int precision, bool precon, int kd_max, int jd_max) {
   if (kd_max < 3 || jd_max < 3 || kd_max - 2 > 1024) return false;
-  const int nw = lu_nband(kd_max);
-  size_t lu;
-  if (precision == OT2D_FP32_MIXED)
-    lu = precon ? lu_smem_bytes<float, true>(nw, 1, jd_max) : lu_smem_bytes<float, false>(nw, 1, jd_max);
-  else
-    lu = precon ? lu_smem_bytes<double, true>(nw, 1, jd_max) : lu_smem_bytes<double, false>(nw, 1, jd_max);
+  // the mesh limit: in bands of 32 rows, the single-copy record ring (28 f32 /
+  // 26 FP64 elements per cell, 36 / 34 preconditioned), the cross-band ring
+  // and counters of every band, and one row of halo contributions, within
+  // one CTA's shared memory (the sweeps, spread over a cluster, need less)
+  const size_t es = precision == OT2D_FP32_MIXED ? sizeof(float) : sizeof(double);
+  const size_t ls = precision == OT2D_FP32_MIXED ? (precon ? 36 : 28) : (precon ? 34 : 26);
+  const size_t nb = (size_t)lu_nband(kd_max, 32);
+  const size_t lu = nb * (2 * 32 * ls * es + 16 + 128 * 4 * es + 4) + 16 + 4 * (size_t)jd_max * es;
   return lu <= (size_t)SMEM_OPTIN_MAX && sizeof(double) * 3 * (size_t)jd_max <= (size_t)SMEM_OPTIN_MAX;
 }
 
@@ -422,7 +424,7 @@ int DevBatch<R>::build(const std::vector<Slice<R>>& sl, cudaStream_t st) {
   // six prefix tables of n+1 entries: cell blocks, k-lines, j-lines, LU
   // record blocks, 32-line groups, residual tiles
   std::vector<int32_t> idx(6 * (n + 1));
-  int cells = 0, jl = 0, kl = 0, lub = 0, grp = 0, tiles = 0, maxw = 1, maxwall = 1, maxkd = 1, moving = 0, precon = 0;
+  int cells = 0, jl = 0, kl = 0, lub = 0, grp = 0, tiles = 0, maxwall = 1, maxkd = 1, moving = 0, precon = 0;
   int maxnbc = 0, limmask = 0;
   int tj = 16, tk = 16;
   rt_shape_dims(rt_shape, tj, tk);
@@ -437,10 +439,11 @@ int DevBatch<R>::build(const std::vector<Slice<R>>& sl, cudaStream_t st) {
     cells += (jd * kd + CELL_BS - 1) / CELL_BS;
     jl += kd - 2;   // k-lines solved along j
     kl += jd - 2;   // j-lines solved along k
-    lub += (lu_nband(kd) * lu_nstep(jd) * 32 + LU_PREP_BS - 1) / LU_PREP_BS;
-    grp += lu_nband(kd);
+    // record blocks: enough for the plain and the preconditioned band layout
+    auto rec_blocks = [&](int rb) { return (lu_nband(kd, rb) * lu_nstep(jd, rb) * rb + lu_prep_bs<R>() - 1) / lu_prep_bs<R>(); };
+    lub += std::max(rec_blocks(LuSplit<R, false>::RB), rec_blocks(LuSplit<R, true>::RB));
+    grp += (kd - 2 + 31) / 32;
     tiles += ((jd - 2 + tj - 1) / tj) * ((kd - 2 + tk - 1) / tk);
-    maxw = std::max(maxw, lu_nband(kd));
     maxwall = std::max(maxwall, jd);
     maxkd = std::max(maxkd, kd);
   }
@@ -470,7 +473,6 @@ int DevBatch<R>::build(const std::vector<Slice<R>>& sl, cudaStream_t st) {
   b.moving = moving;
   b.precon = precon;
   b.cell_blocks = cells;
-  b.max_lu_warps = maxw;
   b.max_wall = maxwall;
   b.max_kd = maxkd;
   b.max_nbc = maxnbc;

@@ -7,85 +7,97 @@
 //     sweeps need from it -- its scaled residual, tscale/2, the diagonal d
 //     and the primitive / metric / spectral-radius factors of its outgoing
 //     contributions (lhs.f:524-563, :626-653) -- and stores them in a
-//     "skewed band" record: rows are grouped in bands of 32 (one warp, one
-//     row per lane) and the record of step t of a band holds, for every
-//     lane l, the cell at column t-l.  One wavefront step of a warp is then
-//     one contiguous chunk (24 fields x 32 lanes).
+//     "skewed band" record: rows are grouped in bands of RB rows (one warp,
+//     32 / RB lanes per row) and the record of step t of a band holds, for
+//     every row r of the band, the cell at column t-r.  One wavefront step of
+//     a warp is then one contiguous chunk (24 fields x RB cells).
 //  2. k_lu_edges: point-Jacobi scaling of the halo residuals (lhs.f:567-598),
 //     their contributions to the first/last interior row and column, and
 //     (FP64) the reference's conservative->primitive->conservative round trip
 //     of q (lhs.f:524-531, :805-811).
-//  3. k_lu_sweep<FWD> (one CTA per slice, warp w = band w): the warps
-//     advance in a skewed lockstep; each warp streams its chunks into a
-//     shared-memory ring with cp.async.bulk (TMA) completing on mbarriers,
-//     the (j-1,k) contribution stays in registers, the (j,k-1) one arrives
-//     from the neighbouring lane by shuffle and across bands through a
-//     double-buffered shared slot.  Every cell sees exactly the operands of
+//  3. k_lu_sweep<FWD> (a cluster of 1..8 CTAs per slice, one warp per band):
+//     the warps advance in a skewed lockstep; each warp streams its chunks
+//     into a shared-memory ring with cp.async.bulk (TMA) completing on
+//     mbarriers.  The lanes of a cell share its arithmetic (LuSplit), the
+//     contribution to the next row arrives by shuffle, across bands through a
+//     shared-memory ring and across the CTAs of the cluster through the next
+//     CTA's shared memory (st.async).  Every cell sees exactly the operands of
 //     the reference's hyperplane order, so the sweep equals the sequential
 //     one operation for operation.
 #pragma once
+#include <type_traits>
 #include "dev_common.cuh"
 
 namespace ot2d {
 
-// A (band, step) chunk holds the records of the band's 32 lanes one after
-// another (lane-major): lane l's 24 fields are contiguous, so a lane reads
-// four consecutive fields with one (f32) or two (f64) 16-byte shared loads.
-// Each record is padded to LS elements so that the eight lanes of a load
-// phase hit disjoint banks (f32: 112-byte stride, f64: 208-byte stride).
-// (Interleaving 16-byte field groups over the lanes instead was measured
-// slower in the backward sweep.)  With Turkel preconditioning (PRE, the
+// Lanes per cell and rows per band of the sweeps.  A sweep is a chain of
+// ncol + nrow steps, so its time is the time of one step.  Two lanes per cell
+// (both form the cell's correction, the even one its xi contribution, the odd
+// one its eta contribution) leave an f32 step 70 instructions instead of 127
+// and ~290 cycles; one lane per cell (bands of 32 rows) took 315.  FP64: the
+// pipe takes a warp instruction every 64 cycles per SM sub-partition whatever
+// the lanes do, so a step is the number of FP64 operations of a lane: 78 with
+// one lane per cell (5900 cycles a step), 47 with two, 21 with four, one per
+// variable (1930 cycles; the exchange between the lanes is the rest).  The
+// preconditioned FP64 operator, whose preconditioner couples the four
+// variables once more, stays at two.  Both sweeps and their records, 257x65
+// FP64: 1710 -> 765 us; 385x97: 2658 -> 1220; FP32-mixed 769x193: 485 -> 301.
+template <class R, bool PRE = false>
+struct LuSplit {
+  static constexpr int LP = (sizeof(R) == 8 && !PRE) ? 4 : 2;   // lanes per cell
+  static constexpr int RB = 32 / LP;                            // rows per band
+};
+
+// A (band, step) chunk holds the records of the band's RB cells one after
+// another (row-major): a cell's 24 fields are contiguous, so a lane reads
+// several consecutive fields with 16-byte shared loads.  The record stride LS
+// puts the rows of a load phase on disjoint banks: f32 24 elements (four rows
+// and both directions' groups of a 16-byte phase cover the 32 banks), FP64 28
+// (four rows x four 8-byte fields).  With Turkel preconditioning (PRE, the
 // preilu2d operator of lhs.f:2-467) a record carries 8 more fields: the
 // chk*qq products of both sweeps and the preconditioner factor.
 template <class R, bool PRE = false>
 struct LuLay {
   static constexpr int NF = PRE ? 32 : 24;                                   // fields per record
-  static constexpr int LS = sizeof(R) == 4 ? (PRE ? 36 : 28) : (PRE ? 34 : 26);   // elements per lane record
-  static constexpr int CH = 32 * LS;                                         // elements per chunk
+  static constexpr int LS = sizeof(R) == 4 ? (PRE ? 36 : 24) : (PRE ? 34 : 28);   // elements per cell record
+  static constexpr int RB = LuSplit<R, PRE>::RB;
+  static constexpr int CH = RB * LS;                                         // elements per chunk
 };
-// record fields
+// record fields; each group of four is one 16-byte (f32) access
 enum {
   LF_S = 0,    // 0..3: residual (forward input, then forward result)
-  LF_SV = 4, LF_D = 5, LF_UU = 6, LF_VV = 7, LF_UV2 = 8, LF_GE = 9,
-  LF_RI1 = 10, LF_RI2 = 11, LF_RK1 = 12, LF_RK2 = 13, LF_QX = 14, LF_QY = 15,
+  LF_SV = 4, LF_D = 5, LF_UU = 6, LF_VV = 7,
+  LF_RI1 = 8, LF_RI2 = 9, LF_QX = 10, LF_UV2 = 11,     // xi metrics and contravariant velocity
+  LF_RK1 = 12, LF_RK2 = 13, LF_QY = 14, LF_GE = 15,    // eta
   LF_FCX = 16, LF_FSX = 17, LF_FCY = 18, LF_FSY = 19,  // forward chk / spec (xi, eta)
   LF_BCX = 20, LF_BSX = 21, LF_BCY = 22, LF_BSY = 23,  // backward chk / spec
   // preconditioned records only: chk*qq (xi, eta) and gm1 (bSq-1)/c**2 of
   // the forward (24..27) and the backward (28..31) sweep
   LF_PF = 24, LF_PB = 28
 };
-// element offset of field f of lane l within a chunk
+// element offset of field f of row r within a chunk
 template <class R, bool PRE = false>
-__host__ __device__ __forceinline__ int lu_idx(int f, int l) {
-  return l * LuLay<R, PRE>::LS + f;
+__host__ __device__ __forceinline__ int lu_idx(int f, int r) {
+  return r * LuLay<R, PRE>::LS + f;
 }
 
 __host__ __device__ __forceinline__ int lu_nrow(int kd) { return kd - 2; }
 __host__ __device__ __forceinline__ int lu_ncol(int jd) { return jd - 2; }
-__host__ __device__ __forceinline__ int lu_nband(int kd) { return (kd - 2 + 31) / 32; }
-__host__ __device__ __forceinline__ int lu_nstep(int jd) { return jd - 2 + 31; }
+// bands of rb rows and steps of a band
+__host__ __device__ __forceinline__ int lu_nband(int kd, int rb) { return (kd - 2 + rb - 1) / rb; }
+__host__ __device__ __forceinline__ int lu_nstep(int jd, int rb) { return jd - 2 + rb - 1; }
 // elements of one slice's record (element size esize bytes): chunks + 4
-// halo-contribution arrays, sized for the larger (preconditioned) layout so
-// that a slice can use either
+// halo-contribution arrays, enough for the plain and the preconditioned
+// layout so that a slice can use either (36 / 34 elements per cell in bands
+// of 32 rows bound both)
 __host__ __device__ __forceinline__ int64_t lu_rec_elems(int jd, int kd, int esize) {
-  const int ch = esize == 4 ? LuLay<float, true>::CH : LuLay<double, true>::CH;
-  return (int64_t)lu_nband(kd) * lu_nstep(jd) * ch + 8 * (int64_t)(lu_nrow(kd) + lu_ncol(jd)) + 64;
+  const int64_t ch = 32 * (esize == 4 ? 36 : 34);
+  return (int64_t)lu_nband(kd, 32) * lu_nstep(jd, 32) * ch + 8 * (int64_t)(lu_nrow(kd) + lu_ncol(jd)) + 64;
 }
 
-// fields f..f+3 of lane l of a chunk (f a multiple of 4) as 16-byte accesses
+// fields f..f+3 of row l of a chunk (f a multiple of 4) as 16-byte accesses
 template <class R>
 struct Lu4 { R x, y, z, w; };
-template <bool PRE = false>
-__device__ __forceinline__ Lu4<float> lu_ld4(const float* ch, int f, int l) {
-  const float4 v = *reinterpret_cast<const float4*>(ch + lu_idx<float, PRE>(f, l));
-  return {v.x, v.y, v.z, v.w};
-}
-template <bool PRE = false>
-__device__ __forceinline__ Lu4<double> lu_ld4(const double* ch, int f, int l) {
-  const double2 a = *reinterpret_cast<const double2*>(ch + lu_idx<double, PRE>(f, l));
-  const double2 b = *reinterpret_cast<const double2*>(ch + lu_idx<double, PRE>(f + 2, l));
-  return {a.x, a.y, b.x, b.y};
-}
 template <bool PRE = false>
 __device__ __forceinline__ void lu_st4(float* ch, int f, int l, float a, float b, float c, float d) {
   *reinterpret_cast<float4*>(ch + lu_idx<float, PRE>(f, l)) = make_float4(a, b, c, d);
@@ -96,22 +108,73 @@ __device__ __forceinline__ void lu_st4(double* ch, int f, int l, double a, doubl
   *reinterpret_cast<double2*>(ch + lu_idx<double, PRE>(f + 2, l)) = make_double2(c, d);
 }
 
-// four consecutive values at a 16-byte aligned shared address (the
-// cross-band ring slots and the staged halo contributions)
-__device__ __forceinline__ Lu4<float> lu_ldv(const float* a) {
-  const float4 v = *reinterpret_cast<const float4*>(a);
-  return {v.x, v.y, v.z, v.w};
+// Shared-memory accesses of the sweeps by 32-bit shared address (through
+// generic pointers the address arithmetic was a third of a step's
+// instructions): one, two or four consecutive values.
+__device__ __forceinline__ void lu_lds(uint32_t a, float& x) {
+  asm volatile("ld.shared.f32 %0, [%1];" : "=f"(x) : "r"(a) : "memory");
 }
-__device__ __forceinline__ Lu4<double> lu_ldv(const double* a) {
-  const double2 x = *reinterpret_cast<const double2*>(a), y = *reinterpret_cast<const double2*>(a + 2);
-  return {x.x, x.y, y.x, y.y};
+__device__ __forceinline__ void lu_lds(uint32_t a, double& x) {
+  asm volatile("ld.shared.f64 %0, [%1];" : "=d"(x) : "r"(a) : "memory");
 }
-__device__ __forceinline__ void lu_stv(float* a, const float* v) {
-  *reinterpret_cast<float4*>(a) = make_float4(v[0], v[1], v[2], v[3]);
+__device__ __forceinline__ void lu_lds2(uint32_t a, float& x, float& y) {
+  asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(x), "=f"(y) : "r"(a) : "memory");
 }
-__device__ __forceinline__ void lu_stv(double* a, const double* v) {
-  *reinterpret_cast<double2*>(a) = make_double2(v[0], v[1]);
-  *reinterpret_cast<double2*>(a + 2) = make_double2(v[2], v[3]);
+__device__ __forceinline__ void lu_lds2(uint32_t a, double& x, double& y) {
+  asm volatile("ld.shared.v2.f64 {%0, %1}, [%2];" : "=d"(x), "=d"(y) : "r"(a) : "memory");
+}
+__device__ __forceinline__ Lu4<float> lu_lds4(uint32_t a, float) {
+  Lu4<float> v;
+  asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(a) : "memory");
+  return v;
+}
+__device__ __forceinline__ Lu4<double> lu_lds4(uint32_t a, double) {
+  Lu4<double> v;
+  lu_lds2(a, v.x, v.y);
+  lu_lds2(a + 16, v.z, v.w);
+  return v;
+}
+__device__ __forceinline__ void lu_sts(uint32_t a, double x) {
+  asm volatile("st.shared.f64 [%0], %1;" ::"r"(a), "d"(x) : "memory");
+}
+__device__ __forceinline__ void lu_sts4(uint32_t a, const float* v) {
+  asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(a), "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3]) : "memory");
+}
+__device__ __forceinline__ void lu_sts4(uint32_t a, const double* v) {
+  asm volatile("st.shared.v2.f64 [%0], {%1, %2};" ::"r"(a), "d"(v[0]), "d"(v[1]) : "memory");
+  asm volatile("st.shared.v2.f64 [%0], {%1, %2};" ::"r"(a + 16), "d"(v[2]), "d"(v[3]) : "memory");
+}
+// The same stores under a predicate, so that no lane branches, and global
+// stores (to a 16-byte aligned address the four-value one).
+__device__ __forceinline__ void lu_sts_if(bool p, uint32_t a, double x) {
+  asm volatile("{\n .reg .pred q;\n setp.ne.s32 q, %2, 0;\n @q st.shared.f64 [%0], %1;\n}" ::"r"(a), "d"(x), "r"((int)p) : "memory");
+}
+__device__ __forceinline__ void lu_sts4_if(bool p, uint32_t a, const float* v) {
+  asm volatile("{\n .reg .pred q;\n setp.ne.s32 q, %5, 0;\n @q st.shared.v4.f32 [%0], {%1, %2, %3, %4};\n}" ::"r"(a), "f"(v[0]),
+               "f"(v[1]), "f"(v[2]), "f"(v[3]), "r"((int)p)
+               : "memory");
+}
+__device__ __forceinline__ void lu_sts4_if(bool p, uint32_t a, const double* v) {
+#pragma unroll
+  for (int n = 0; n < 4; ++n) lu_sts_if(p, a + 8 * n, v[n]);
+}
+__device__ __forceinline__ void lu_stg_if(bool p, float* a, float x) {
+  asm volatile("{\n .reg .pred q;\n setp.ne.s32 q, %2, 0;\n @q st.global.f32 [%0], %1;\n}" ::"l"(a), "f"(x), "r"((int)p) : "memory");
+}
+__device__ __forceinline__ void lu_stg_if(bool p, double* a, double x) {
+  asm volatile("{\n .reg .pred q;\n setp.ne.s32 q, %2, 0;\n @q st.global.f64 [%0], %1;\n}" ::"l"(a), "d"(x), "r"((int)p) : "memory");
+}
+__device__ __forceinline__ void lu_stg4_if(bool p, float* a, const float* v) {
+  asm volatile("{\n .reg .pred q;\n setp.ne.s32 q, %5, 0;\n @q st.global.v4.f32 [%0], {%1, %2, %3, %4};\n}" ::"l"(a), "f"(v[0]),
+               "f"(v[1]), "f"(v[2]), "f"(v[3]), "r"((int)p)
+               : "memory");
+}
+__device__ __forceinline__ void lu_stg4_if(bool p, double* a, const double* v) {
+#pragma unroll
+  for (int n = 0; n < 4; n += 2)
+    asm volatile("{\n .reg .pred q;\n setp.ne.s32 q, %3, 0;\n @q st.global.v2.f64 [%0], {%1, %2};\n}" ::"l"(a + n), "d"(v[n]),
+                 "d"(v[n + 1]), "r"((int)p)
+                 : "memory");
 }
 
 template <class R>
@@ -247,15 +310,14 @@ __device__ __forceinline__ void lu_contrib(const LuCell<R>& c, const R* s, R gm1
   }
 }
 
-// ---- kernel 1: records of the interior cells (one thread per (band, step, lane))
-// The record of lane l of chunk (band, t) into ch, the chunk as the warp
-// stages it in shared memory (k_lu_prep stores the staged chunk with
-// contiguous 16-byte accesses).
+// ---- kernel 1: records of the interior cells (one thread per (band, step, row))
+// The record of row l of chunk (band, t) into ch, the chunk as k_lu_prep
+// stages it in shared memory.
 template <class R, bool PRE = false>
 __device__ __forceinline__ void lu_prep_cell(const Slice<R>& S, const ot2d_params& p, int band, int t, int l, int scale,
                                              R* ch) {
   const int nrow = lu_nrow(S.kd), ncol = lu_ncol(S.jd);
-  const int r = 32 * band + l, c = t - l;
+  const int r = LuSplit<R, PRE>::RB * band + l, c = t - l;
   if (r >= nrow || c < 0 || c >= ncol) {
     const R z = (R)0;
 #pragma unroll
@@ -275,8 +337,8 @@ __device__ __forceinline__ void lu_prep_cell(const Slice<R>& S, const ot2d_param
   }
   lu_st4<PRE>(ch, LF_S, l, sv[0], sv[1], sv[2], sv[3]);
   lu_st4<PRE>(ch, LF_SV, l, ts * (R)0.5, cl.d, cl.uu, cl.vv);
-  lu_st4<PRE>(ch, LF_UV2, l, cl.uv2, cl.ge, cl.ri1, cl.ri2);
-  lu_st4<PRE>(ch, LF_RK1, l, cl.rk1, cl.rk2, cl.qx, cl.qy);
+  lu_st4<PRE>(ch, LF_RI1, l, cl.ri1, cl.ri2, cl.qx, cl.uv2);
+  lu_st4<PRE>(ch, LF_RK1, l, cl.rk1, cl.rk2, cl.qy, cl.ge);
   R a, b, a2, b2;
   if constexpr (PRE) {
     R q1, q2;
@@ -299,11 +361,12 @@ __device__ __forceinline__ void lu_prep_cell(const Slice<R>& S, const ot2d_param
 }
 
 // halo-contribution arrays after the chunks: A forward [nrow][4], A backward,
-// B forward [ncol][4], B backward
+// B forward [ncol][4], B backward (last column first: in sweep order)
 template <class R, bool PRE = false>
 __device__ __forceinline__ R* lu_halo(const Slice<R>& S, int which) {
   const int nrow = lu_nrow(S.kd), ncol = lu_ncol(S.jd);
-  R* base = S.lurec + (int64_t)lu_nband(S.kd) * lu_nstep(S.jd) * LuLay<R, PRE>::CH;
+  constexpr int RB = LuSplit<R, PRE>::RB;
+  R* base = S.lurec + (int64_t)lu_nband(S.kd, RB) * lu_nstep(S.jd, RB) * LuLay<R, PRE>::CH;
   switch (which) {
     case 0: return base;
     case 1: return base + 4 * nrow;
@@ -334,7 +397,7 @@ __device__ __forceinline__ void lu_edge_cell(const Slice<R>& S, const ot2d_param
       if (j == js - 1) { lu_contrib<R, true, true, PRE>(c, sv, gm1, eps2, a); dst = lu_halo<R, PRE>(S, 0) + 4 * (k - ks); }
       else if (j == je + 1) { lu_contrib<R, true, false, PRE>(c, sv, gm1, eps2, a); dst = lu_halo<R, PRE>(S, 1) + 4 * (k - ks); }
       else if (k == ks - 1) { lu_contrib<R, false, true, PRE>(c, sv, gm1, eps2, a); dst = lu_halo<R, PRE>(S, 2) + 4 * (j - js); }
-      else { lu_contrib<R, false, false, PRE>(c, sv, gm1, eps2, a); dst = lu_halo<R, PRE>(S, 3) + 4 * (j - js); }
+      else { lu_contrib<R, false, false, PRE>(c, sv, gm1, eps2, a); dst = lu_halo<R, PRE>(S, 3) + 4 * (je - j); }
 #pragma unroll
       for (int n = 0; n < 4; ++n) dst[n] = a[n];
     }
@@ -364,10 +427,8 @@ __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
 __device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
 }
-__device__ __forceinline__ void bulk_g2s(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
-  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_u32(dst)),
-               "l"(src), "r"(bytes), "r"(smem_u32(bar))
-               : "memory");
+__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
 __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
   uint32_t ok;
@@ -378,8 +439,6 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
       : "memory");
   return ok != 0;
 }
-__device__ __forceinline__ void fence_proxy_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
-
 // Polls a sweep wait makes before it gives up (the status word of the slice
 // records the timeout).  The solver can lower it (OT2D_OPT_POLL_LIMIT) to
 // make the waits run out on purpose; the drain of copies still in flight
@@ -393,264 +452,505 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity
   return false;
 }
 
-// Progress counters in shared memory: the producer publishes with a release
-// store, the consumer reads with an acquire load (CTA scope), so the data
-// written before the store is visible after the load.
-__device__ __forceinline__ int lu_ld_acquire(const int* cnt) {
-  int v;
-  asm volatile("ld.acquire.cta.shared::cta.s32 %0, [%1];" : "=r"(v) : "r"(smem_u32(cnt)) : "memory");
-  return v;
+// Cross-band ring: the last row of a band hands its outgoing (j,k-1)
+// contribution at its p-th column (in sweep order) to the next band through
+// slot p % LU_XB; the consumer's first row reads it at its own step p.
+constexpr int LU_XB = 64;         // a power of two; a band may run this many columns ahead of the next
+constexpr int LU_LG = 8;          // columns per barrier of a link between CTAs
+constexpr int LU_MAX_WARPS = 16;  // bands per CTA of a sweep
+constexpr int LU_MAX_CLUSTER = 8; // CTAs per slice
+
+// PG, the steps per group: a group's records arrive with one bulk copy, and
+// waits on the neighbouring bands are made and progress is published once per
+// group, so a band trails the one before it by RB + PG steps.  A group's
+// waits and bookkeeping cost about as much as two f32 steps: groups of 8 make
+// a step 215 cycles, groups of 4 294 (f32 sweeps of a 513x33 mesh, 147 and
+// 183 us), but hold twice the shared memory; in a batch whose sweeps share
+// their SMs with the turbulence solve the smaller groups are faster (64
+// 513x129 requests 1256 against 1402 us per iteration).  FP64 steps are an
+// order longer: groups of 2, which trail least.
+template <class R, bool WIDE>
+__host__ __device__ constexpr int lu_pg() { return sizeof(R) == 8 ? 2 : (WIDE ? 8 : 4); }
+// Exchange buffer of a warp, through which the lanes of a step pass values on
+// (a 16-byte store and load take the place of four shuffles).  A contribution
+// made at step t goes to slot (t+1) % lu_ks() of its lane; the slots of a lane
+// are 4 elements apart, as the columns of the cross-band ring are, so that a
+// cell takes its eta input at the same step stride from either.
+template <int PG>
+__host__ __device__ constexpr int lu_ks() { return PG < 4 ? 4 : PG; }
+template <class R, bool PRE, int PG>
+__host__ __device__ constexpr int lu_ex() {
+  return LuSplit<R, PRE>::LP == 2 ? 32 * 4 * (lu_ks<PG>() + 1) : 64 + 8 * 4 * (lu_ks<PG>() + 1);
 }
-__device__ __forceinline__ void lu_st_release(int* cnt, int v) {
-  asm volatile("st.release.cta.shared::cta.s32 [%0], %1;" ::"r"(smem_u32(cnt)), "r"(v) : "memory");
+
+// Shared memory of a sweep CTA: per warp D stages of a group's records with a
+// barrier each, its cross-band ring with a full and an empty barrier per
+// group of columns, and its exchange buffer; then one row of contributions
+// per column (at most maxcol): the halo's for the CTA with the first band in
+// sweep order, the previous CTA's last row for the others, with one barrier
+// per LU_LG columns.
+template <class R, bool PRE, int PG>
+__host__ __device__ __forceinline__ size_t lu_smem_bytes(int nwarp, int D, int maxcol) {
+  return (size_t)nwarp * (D * PG * LuLay<R, PRE>::CH + LU_XB * 4 + lu_ex<R, PRE, PG>()) * sizeof(R) +
+         (size_t)4 * maxcol * sizeof(R) + (size_t)nwarp * (D + 2 * (LU_XB / PG)) * sizeof(uint64_t) +
+         (size_t)((maxcol + LU_LG - 1) / LU_LG) * sizeof(uint64_t);
 }
-// Bounded wait until *cnt >= need; `seen` caches the last value read, so a
-// counter already known to be far enough ahead is not read again.
-__device__ __forceinline__ bool lu_wait_ge(const int* cnt, int need, int& seen, uint32_t lim) {
-  if (seen >= need) return true;
+
+// address of a local shared-memory object in CTA `rank` of the cluster
+__device__ __forceinline__ uint32_t lu_mapa(uint32_t local, int rank) {
+  uint32_t r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(local), "r"(rank));
+  return r;
+}
+// four values (one for FP64: lane v's own) into the next CTA's row, counted
+// on its barrier
+__device__ __forceinline__ void lu_send(uint32_t dst, uint32_t bar, const float* v) {
+  asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%1, %2, %3, %4}, [%5];" ::"r"(dst),
+               "r"(__float_as_uint(v[0])), "r"(__float_as_uint(v[1])), "r"(__float_as_uint(v[2])),
+               "r"(__float_as_uint(v[3])), "r"(bar)
+               : "memory");
+}
+__device__ __forceinline__ void lu_send1(uint32_t dst, uint32_t bar, double v) {
+  asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.b64 [%0], %1, [%2];" ::"r"(dst),
+               "l"(__double_as_longlong(v)), "r"(bar)
+               : "memory");
+}
+__device__ __forceinline__ void lu_send(uint32_t dst, uint32_t bar, const double* v) {
+#pragma unroll
+  for (int n = 0; n < 4; ++n) lu_send1(dst + 8 * n, bar, v[n]);
+}
+__device__ __forceinline__ bool lu_link_wait(uint64_t* bar, uint32_t lim) {
   for (uint32_t it = 0; it < lim; ++it) {
-    seen = lu_ld_acquire(cnt);
-    if (seen >= need) return true;
+    uint32_t ok;
+    asm volatile(
+        "{\n .reg .pred p;\n mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], 0;\n"
+        " selp.u32 %0, 1, 0, p;\n}\n"
+        : "=r"(ok)
+        : "r"(smem_u32(bar))
+        : "memory");
+    if (ok) return true;
   }
   return false;
 }
-
-// Cross-band ring: the boundary lane of band w hands its outgoing (j,k-1)
-// contribution of local step t to the next band in sweep order through
-// slot t % LU_XB; the consumer reads it at its step t - 31.
-constexpr int LU_XB = 128;   // a power of two
-
-// Shared memory of the sweep kernel: per warp a ring of two groups of G
-// chunks, its two barriers, its cross-band ring and its progress counter;
-// then the first-row halo contributions of the slice (4 per column, at most
-// maxcol columns).
-template <class R, bool PRE = false>
-__host__ __device__ __forceinline__ size_t lu_smem_bytes(int nwarp, int G, int maxcol) {
-  return (size_t)nwarp * 2 * G * LuLay<R, PRE>::CH * sizeof(R) + (size_t)nwarp * 2 * sizeof(uint64_t) +
-         (size_t)nwarp * LU_XB * 4 * sizeof(R) + (size_t)nwarp * sizeof(int) + 16 +
-         (size_t)4 * maxcol * sizeof(R);
+__device__ __forceinline__ void lu_cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release;\n barrier.cluster.wait.acquire;" ::: "memory");
 }
 
-// One sweep of one slice.  Warp w owns band w (rows 32w..32w+31, lane l ->
-// row 32w+l) and walks its nst local steps; at local step t lane l is on
-// column t-l (forward) or ncol-1-(t-(31-l)) (backward), so the lanes of a
-// warp are on 32 consecutive hyperplanes and the in-band dependency (the
-// neighbouring row) arrives by shuffle from the previous step.  The
-// dependency across bands -- lane 31 of band w-1 feeds lane 0 of band w
-// 31 steps later (backward: lane 0 of band w+1 feeds lane 31 of band w) --
-// goes through the cross-band ring guarded by per-warp progress counters,
-// so the warps run without block-wide barriers.  The records stream in
-// through cp.async.bulk, G chunks per copy, double-buffered.
-// PRE: the preilu2d records and contributions.
-template <class R, bool FWD, int G, bool PRE = false>
-__device__ void lu_sweep_slice(const Slice<R>& S, int nwarp, unsigned char* smem, uint32_t lim, int lag) {
-  const ot2d_params& p = *S.P;
-  const int nrow = lu_nrow(S.kd), ncol = lu_ncol(S.jd), nb = lu_nband(S.kd), nst = lu_nstep(S.jd);
-  const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-  const R gm1 = S.k_gm1;
-  R* rings = (R*)smem;
-  constexpr int CH = LuLay<R, PRE>::CH;
-  uint64_t* bars = (uint64_t*)(smem + (size_t)nwarp * 2 * G * CH * sizeof(R));
-  R* xrings = (R*)(bars + (size_t)nwarp * 2);
-  int* prog = (int*)(xrings + (size_t)nwarp * LU_XB * 4);
-  // halo contributions into the first (forward) / last (backward) row,
-  // read once per step by one lane: staged in shared memory
-  R* bhs = (R*)(((uintptr_t)(prog + nwarp) + 15) & ~(uintptr_t)15);
-  R* ring = rings + (size_t)w * 2 * G * CH;
-  uint64_t* bar = bars + (size_t)w * 2;
-  const bool wok = w < nb;
-  const R* rec_w = S.lurec + (int64_t)w * nst * CH;
-  R* recw = S.lurec + (int64_t)w * nst * CH;
-  const int ngrp = (nst + G - 1) / G;
-  // group g of the sweep covers local steps g*G .. g*G+G-1; its chunks are
-  // contiguous in memory starting at chunk c0(g) (ascending)
-  auto c0 = [&](int g) -> int { return FWD ? g * G : max(0, nst - (g + 1) * G); };
-  auto gsize = [&](int g) -> int { return min(G, nst - g * G); };
-  auto issue = [&](int g) {
-    const uint32_t bytes = (uint32_t)gsize(g) * CH * sizeof(R);
-    fence_proxy_async_smem();
-    mbar_expect_tx(&bar[g & 1], bytes);
-    bulk_g2s(ring + (size_t)(g & 1) * G * CH, rec_w + (int64_t)c0(g) * CH, bytes, &bar[g & 1]);
-  };
-  if (l == 0) {
-    if (wok) { mbar_init(&bar[0], 1); mbar_init(&bar[1], 1); }
-    prog[w] = 0;
+// The arithmetic of one wavefront step for the lanes of a warp.
+//
+// Two lanes per cell: lane 2r+d forms the whole correction of row r's cell
+// and the contribution of direction d (0 xi, 1 eta) in out[], which it leaves
+// in its slots of the exchange buffer for the cells that take it.
+template <class R, bool FWD, bool PRE, int LP, int KS>
+struct LuLanes;
+
+template <class R, bool FWD, bool PRE, int KS>
+struct LuLanes<R, FWD, PRE, 2, KS> {
+  static constexpr uint32_t B = sizeof(R), SB = 4 * B, LN = (KS + 1) * SB;   // bytes: value, slot, lane
+  // the lane's share of a cell's record
+  struct Rec { Lu4<R> s, p, m, pp; R chk, spec, other; };
+  R out[4], hx[4] = {0, 0, 0, 0};
+  uint32_t wr, ra, rb, oD, oO, oC;
+  int d;
+  __device__ __forceinline__ LuLanes(int l, uint32_t ex) {
+    d = l & 1;
+    wr = ex + l * LN;
+    ra = ex + (l & ~1) * LN;                                    // the row's xi lane
+    rb = ex + ((FWD ? (l & ~1) - 1 : (l | 1) + 2) & 31) * LN;   // the previous row's eta lane
+    oD = (d ? LF_RK1 : LF_RI1) * B;
+    oO = (d ? LF_UV2 : LF_GE) * B;
+    oC = ((FWD ? LF_FCX : LF_BCX) + 2 * d) * B;
   }
-  {
-    const R* Bg = lu_halo<R, PRE>(S, FWD ? 2 : 3);
-    for (int i = threadIdx.x; i < 4 * ncol; i += blockDim.x) bhs[i] = Bg[i];
+  __device__ __forceinline__ Rec load(uint32_t rec) const {
+    Rec r;
+    r.s = lu_lds4(rec + LF_S * B, R());
+    r.p = lu_lds4(rec + LF_SV * B, R());
+    r.m = lu_lds4(rec + oD, R());
+    lu_lds2(rec + oC, r.chk, r.spec);
+    lu_lds(rec + oO, r.other);
+    if constexpr (PRE) r.pp = lu_lds4(rec + (FWD ? LF_PF : LF_PB) * B, R());   // chk*qq xi, eta, preconditioner factor
+    return r;
   }
-  __syncthreads();
-  if (!wok) return;
-  if (l == 0) {
-    issue(0);
-    if (ngrp > 1) issue(1);
+  __device__ __forceinline__ uint32_t eta_base() const { return rb; }
+  __device__ __forceinline__ uint32_t eta_link(uint32_t slot) const { return slot; }
+  // the halo's xi contribution to the row's first column
+  __device__ __forceinline__ void halo_xi(const R* p) {
+#pragma unroll
+    for (int n = 0; n < 4; ++n) hx[n] = p[n];
   }
-  const R* Ah = lu_halo<R, PRE>(S, FWD ? 0 : 1);
-  const R* Bh = bhs;
-  // neighbouring bands in sweep order and the boundary lanes
-  const int wprev = FWD ? w - 1 : w + 1, wnext = FWD ? w + 1 : w - 1;
-  const bool has_prev = FWD ? w > 0 : w + 1 < nb, has_next = FWD ? w + 1 < nb : w > 0;
-  const int lout = FWD ? 31 : 0;
-  R* xout = xrings + (size_t)w * LU_XB * 4;
-  const R* xin = xrings + (size_t)(has_prev ? wprev : w) * LU_XB * 4;
-  const int r = 32 * w + l;
-  // this lane's row of s (backward sweep output), indexed by column
-  R* srow = S.s + (int64_t)(p.kbeg + r - 1) * S.jd + (p.jbeg - 1);
-  R aprev[4] = {0, 0, 0, 0}, bout[4] = {0, 0, 0, 0};
-  int seen_prev = 0, seen_next = 0;   // cached progress of the neighbouring bands
-  bool bad = false;
-  int gfail = -1;
-  // Band lag: start `lag` steps after the neighbouring band's first
-  // contribution is due, so that in the steady state the cross-band value
-  // is already there and the cached progress spares most polls (the
-  // operands of every cell are the same whatever the lag).
-  if (has_prev && lag > 0) {
-    if (l == 0 && !lu_wait_ge(&prog[wprev], min(32 + lag, nst), seen_prev, lim)) bad = true;
-    seen_prev = __shfl_sync(0xffffffffu, seen_prev, 0);
-  }
-  // This lane's record: residual, (tscale/2, d, u, v), (uv2, ge, xi
-  // metrics), (eta metrics, qx, qy), this sweep's (chk, spec) pairs.
-  struct Rec { Lu4<R> r0, r1, r2, r3, r4; };
-  auto ldrec = [&](const R* ch) -> Rec {
-    return {lu_ld4<PRE>(ch, LF_S, l), lu_ld4<PRE>(ch, LF_SV, l), lu_ld4<PRE>(ch, LF_UV2, l),
-            lu_ld4<PRE>(ch, LF_RK1, l), lu_ld4<PRE>(ch, FWD ? LF_FCX : LF_BCX, l)};
-  };
-  // The new correction of this lane's cell from its record and the summed
-  // neighbour contributions, its store (forward: into the record for the
-  // backward sweep; backward: into s), and its outgoing contributions:
-  // xi into aprev (the same lane's next step), eta into bout (the next lane).
-  auto cell = [&](const R* ch, const Rec& rc, int tl, int c, const R* bin) {
-    const Lu4<R>&r0 = rc.r0, &r1 = rc.r1, &r2 = rc.r2, &r3 = rc.r3, &r4 = rc.r4;
-    const R sv = r1.x, di = r1.y;
-    const R st[4] = {r0.x, r0.y, r0.z, r0.w};
+  // The cell of a step: eta the address of its incoming eta contribution, k
+  // and kn the exchange slots of this and of the next step; recg this step's
+  // global record, srow the row of s at the cell's column.  RAMP: some row may
+  // be on its first column (first) or outside its columns (not valid: its
+  // record is 0, so is its contribution, and nothing takes it).
+  template <bool RAMP>
+  __device__ __forceinline__ void cell(const Rec& r, uint32_t eta, int k, int kn, bool first, bool valid, R gm1, R* recg,
+                                       R* srow, int64_t qs) {
+    const Lu4<R> xb = lu_lds4(eta, R());
+    Lu4<R> xa = lu_lds4(ra + k * SB, R());
+    if (RAMP) {
+      xa.x = first ? hx[0] : xa.x; xa.y = first ? hx[1] : xa.y;
+      xa.z = first ? hx[2] : xa.z; xa.w = first ? hx[3] : xa.w;
+    }
+    const R uv2 = d ? r.other : r.m.w, ge = d ? r.m.w : r.other;
+    const R st[4] = {r.s.x, r.s.y, r.s.z, r.s.w};
+    const R in[4] = {xa.x + xb.x, xa.y + xb.y, xa.z + xb.z, xa.w + xb.w};
+    const R sv = r.p.x, di = r.p.y;
     R sn[4];
 #pragma unroll
-    for (int n = 0; n < 4; ++n)
-      sn[n] = FWD ? (st[n] + sv * (aprev[n] + bin[n])) * di : st[n] - sv * (aprev[n] + bin[n]) * di;
-    if (FWD) {
-      lu_st4<PRE>(recw + (int64_t)tl * CH, LF_S, l, sn[0], sn[1], sn[2], sn[3]);
-    } else {
-#pragma unroll
-      for (int n = 0; n < 4; ++n) srow[n * S.qs + c] = sn[n];
-    }
-    // xi: (chk, spec) = r4.x, r4.y with ri1, ri2, qx; eta: r4.z, r4.w
-    // with rk1, rk2, qy; u, v, uv2, ge shared
+    for (int n = 0; n < 4; ++n) sn[n] = FWD ? (st[n] + sv * in[n]) * di : st[n] - sv * in[n] * di;
     if constexpr (PRE) {
-      // (chk*qq xi, chk*qq eta, preconditioner factor)
-      const Lu4<R> r5 = lu_ld4<PRE>(ch, FWD ? LF_PF : LF_PB, l);
-      lu_apply_pre<R, FWD>(r4.x, r5.x, r4.y, r5.z, r2.z, r2.w, r3.z, r1.z, r1.w, r2.x, r2.y, gm1, sn, aprev);
-      lu_apply_pre<R, FWD>(r4.z, r5.y, r4.w, r5.z, r3.x, r3.y, r3.w, r1.z, r1.w, r2.x, r2.y, gm1, sn, bout);
+      lu_apply_pre<R, FWD>(r.chk, d ? r.pp.y : r.pp.x, r.spec, r.pp.z, r.m.x, r.m.y, r.m.z, r.p.z, r.p.w, uv2, ge, gm1,
+                           sn, out);
     } else {
-      lu_apply(r4.x, r4.y, r2.z, r2.w, r3.z, r1.z, r1.w, r2.x, r2.y, gm1, sn, aprev);
-      lu_apply(r4.z, r4.w, r3.x, r3.y, r3.w, r1.z, r1.w, r2.x, r2.y, gm1, sn, bout);
+      lu_apply(r.chk, r.spec, r.m.x, r.m.y, r.m.z, r.p.z, r.p.w, uv2, ge, gm1, sn, out);
     }
-  };
-  // Steady groups: a band of 32 rows, G steps all inside columns 1..ncol-1
-  // of every lane (local steps 32 .. ncol-1), so every lane is active, no
-  // lane is on the first column, and the waits on the neighbouring bands
-  // are made once per group -- for the last step's cross-band input and the
-  // last step's ring slot -- with the progress published once at the end.
-  // Its steps have no waits and no boundary cases (the boundary lane's
-  // input and output are predicated accesses); the cells see the same
-  // operands as in the per-step form below.
-  const bool full = 32 * (w + 1) <= nrow;
-  const int lin = FWD ? 0 : 31;
-  const bool pout = l == lout && has_next;
-  for (int g = 0; g < ngrp; ++g) {
-    const bool ok = mbar_wait_bounded(&bar[g & 1], (uint32_t)((g >> 1) & 1), lim);
-    if (__any_sync(0xffffffffu, !ok || bad)) { gfail = g; break; }
-    const int gs = gsize(g);
-    const R* gring = ring + (size_t)(g & 1) * G * CH;
-    const int t0 = g * G;
-    if (full && gs == G && t0 >= 32 && t0 + G <= ncol) {
-      if (has_prev && l == lin && !lu_wait_ge(&prog[wprev], t0 + G - 1 + 32, seen_prev, lim)) bad = true;
-      if (pout && !lu_wait_ge(&prog[wnext], t0 + G - 1 - LU_XB + 32, seen_next, lim)) bad = true;
-      if (__any_sync(0xffffffffu, bad)) { gfail = g; break; }
-#pragma unroll
-      for (int u = 0; u < G; ++u) {
-        const int tl = t0 + u;
-        const R* ch = gring + (FWD ? u : G - 1 - u) * CH;
-        const Rec rc = ldrec(ch);
-        R bin[4];
-#pragma unroll
-        for (int n = 0; n < 4; ++n)
-          bin[n] = FWD ? __shfl_up_sync(0xffffffffu, bout[n], 1) : __shfl_down_sync(0xffffffffu, bout[n], 1);
-        const int c = FWD ? tl - l : ncol - 1 - (tl - (31 - l));
-        // lane lin: from band wprev's step tl + 31, or the halo row
-        const R* xs = has_prev ? xin + ((tl + 31) & (LU_XB - 1)) * 4 : Bh + 4 * c;
-        if (l == lin) {
-          const Lu4<R> x = lu_ldv(xs);
-          bin[0] = x.x; bin[1] = x.y; bin[2] = x.z; bin[3] = x.w;
-        }
-        cell(ch, rc, tl, c, bin);
-        if (pout) lu_stv(xout + (tl & (LU_XB - 1)) * 4, bout);
-      }
-      if (l == lout) lu_st_release(&prog[w], t0 + G);
+    lu_sts4(wr + kn * SB, out);
+    if (FWD) {
+      lu_stg4_if(d == 0, recg + LF_S, sn);         // into the record, for the backward sweep
     } else {
-#pragma unroll 4
-      for (int u = 0; u < gs; ++u) {
-        const int tl = t0 + u;
-        // (loading the next step's record ahead of this step's arithmetic
-        // was measured slower: 0.81 against 0.71 ms at batch 64)
-        const R* ch = gring + (FWD ? u : gs - 1 - u) * CH;
-        const Rec rc = ldrec(ch);
-        R bin[4];
-#pragma unroll
-        for (int n = 0; n < 4; ++n)
-          bin[n] = FWD ? __shfl_up_sync(0xffffffffu, bout[n], 1) : __shfl_down_sync(0xffffffffu, bout[n], 1);
-        const int c = FWD ? tl - l : ncol - 1 - (tl - (31 - l));
-        const bool act = r < nrow && c >= 0 && c < ncol;
-        if (act) {
-          if (FWD ? c == 0 : c == ncol - 1) {
-#pragma unroll
-            for (int n = 0; n < 4; ++n) aprev[n] = Ah[4 * r + n];
-          }
-          // the (j,k-1) / (j,k+1) neighbour from outside the band
-          if (FWD ? l == 0 : (l == 31 || r == nrow - 1)) {
-            if (!has_prev || (!FWD && r == nrow - 1)) {
-#pragma unroll
-              for (int n = 0; n < 4; ++n) bin[n] = Bh[4 * c + n];
-            } else if (lu_wait_ge(&prog[wprev], tl + 32, seen_prev, lim)) {
-              // produced by band wprev at its step tl + 31
-              const R* x = xin + ((tl + 31) & (LU_XB - 1)) * 4;
-#pragma unroll
-              for (int n = 0; n < 4; ++n) bin[n] = x[n];
-            } else {
-              bad = true;
-            }
-          }
-          cell(ch, rc, tl, c, bin);
-        }
-        // hand the boundary contribution to the next band (its slot must have
-        // been read: the consumer is at least at step tl - LU_XB + 32), then
-        // publish this band's progress
-        if (l == lout) {
-          if (act && has_next) {
-            if (lu_wait_ge(&prog[wnext], tl - LU_XB + 32, seen_next, lim)) {
-              R* x = xout + (tl & (LU_XB - 1)) * 4;
-#pragma unroll
-              for (int n = 0; n < 4; ++n) x[n] = bout[n];
-            } else {
-              bad = true;
-            }
-          }
-          lu_st_release(&prog[w], tl + 1);
-        }
-      }
+      // two variables per lane (srow: the lane's first)
+      lu_stg_if(!RAMP || valid, srow, d ? sn[2] : sn[0]);
+      lu_stg_if(!RAMP || valid, srow + qs, d ? sn[3] : sn[1]);
     }
-    // group done: refill its buffer with group g + 2
-    __syncwarp();
-    if (l == 0 && g + 2 < ngrp) issue(g + 2);
   }
-  if (__any_sync(0xffffffffu, bad) && gfail < 0) gfail = ngrp;
-  if (gfail >= 0) {
-    if (l == lout) lu_st_release(&prog[w], 1 << 30);  // release a waiting neighbour
+  __device__ __forceinline__ int first_var() const { return 2 * d; }
+  __device__ __forceinline__ bool owns_eta() const { return d == 1; }
+  __device__ __forceinline__ void put_if(bool c, uint32_t p) const { lu_sts4_if(c, p, out); }
+  __device__ __forceinline__ void send(uint32_t dst, uint32_t bar) const { lu_send(dst, bar, out); }
+};
+
+// Four lanes per cell (FP64): lane 4r+v holds variable v.  Lanes 0..3 form
+// a4 and a2 (lu_apply) of xi, then of eta -- one instruction stream over
+// (A, B, C) = (ri1, ri2, qq) for a4 and (u, v, uv2) for a2 -- and each lane
+// its variable's contribution to both directions.  The corrections, the four
+// scalars and the eta contributions pass through parts of the exchange
+// buffer, a warp barrier between a part's write and its reads.
+template <bool FWD, int KS>
+struct LuLanes<double, FWD, false, 4, KS> {
+  static constexpr uint32_t B = 8, SB = 32, LN = (KS + 1) * SB;   // bytes: value, slot, row of slots
+  struct Rec { double sv, d, a, b, st, cc, chk, pe, px, q, fsx, fsy; };
+  double ox = 0, oe = 0, hx = 0;   // this variable's xi / eta contribution of the lane's last cell; the halo's xi
+  uint32_t wr, rd, wre, rb, oA, oC, oK, oX, oE, oQ, vb;
+  int v;
+  bool odd;
+  __device__ __forceinline__ LuLanes(int l, uint32_t exb) {
+    v = l & 3;
+    odd = v & 1;
+    vb = v * B;
+    wr = exb + l * B;
+    rd = exb + (l & ~3) * B;
+    wre = exb + 64 * B + (l >> 2) * LN + vb;
+    rb = exb + 64 * B + ((FWD ? (l >> 2) - 1 : (l >> 2) + 1) & 7) * LN + vb;
+    oA = (odd ? LF_UU : (v ? LF_RK1 : LF_RI1)) * B;
+    oC = (odd ? LF_UV2 : (v ? LF_QY : LF_QX)) * B;
+    oK = ((FWD ? LF_FCX : LF_BCX) + (v & 2)) * B;
+    oX = (LF_RI1 - 1 + v) * B;                     // ri1, ri2, qx for v = 1, 2, 3
+    oE = (LF_RK1 - 1 + v) * B;
+    oQ = (v == 1 ? LF_UU : (v == 2 ? LF_VV : LF_GE)) * B;
+  }
+  __device__ __forceinline__ Rec load(uint32_t rec) const {
+    Rec r;
+    lu_lds(rec + LF_S * B + vb, r.st);
+    lu_lds2(rec + LF_SV * B, r.sv, r.d);
+    lu_lds2(rec + oA, r.a, r.b);
+    lu_lds(rec + oC, r.cc);
+    lu_lds(rec + oK, r.chk);
+    lu_lds(rec + oE, r.pe);
+    lu_lds(rec + oX, r.px);
+    lu_lds(rec + oQ, r.q);
+    lu_lds(rec + (FWD ? LF_FSX : LF_BSX) * B, r.fsx);
+    lu_lds(rec + (FWD ? LF_FSY : LF_BSY) * B, r.fsy);
+    return r;
+  }
+  __device__ __forceinline__ uint32_t eta_base() const { return rb; }
+  __device__ __forceinline__ uint32_t eta_link(uint32_t slot) const { return slot + vb; }
+  __device__ __forceinline__ void halo_xi(const double* p) { hx = p[v]; }
+  template <bool RAMP>
+  __device__ __forceinline__ void cell(const Rec& r, uint32_t eta, int, int kn, bool first, bool valid, double gm1,
+                                       double* recg, double* srow, int64_t) {
+    double xb;
+    lu_lds(eta, xb);
+    const double xa = RAMP && first ? hx : ox;
+    const double sn = FWD ? (r.st + r.sv * (xa + xb)) * r.d : r.st - r.sv * (xa + xb) * r.d;
+    lu_sts(wr, sn);
+    __syncwarp();
+    if (FWD) lu_stg_if(true, recg + LF_S + v, sn);
+    else lu_stg_if(!RAMP || valid, srow, sn);
+    const Lu4<double> s = lu_lds4(rd, 0.0);
+    // a4 = chk*(ri1*s2 + ri2*s3 - qq*s1)
+    // a2 = chk*gm1*(uv2*s1 - (u*s2 + v*s3) + s4); chk is 0 or 1
+    const double x = r.a * s.y + r.b * s.z, y = r.cc * s.x;
+    const double t = (odd ? y : x) - (odd ? x : y);
+    const double w = (odd ? (__double2hiint(r.chk) ? gm1 : 0.0) : r.chk) * (odd ? t + s.w : t);
+    lu_sts(wr + 32 * B, w);
+    const double gx = r.fsx * sn, gy = r.fsy * sn;
+    __syncwarp();
+    const Lu4<double> a = lu_lds4(rd + 32 * B, 0.0);    // a4, a2 of xi; a4, a2 of eta
+    const double my = r.pe * a.w + r.q * a.z;
+    oe = (v ? my : a.z) + gy;
+    lu_sts(wre + kn * SB, oe);
+    const double mx = r.px * a.y + r.q * a.x;
+    ox = (v ? mx : a.x) + gx;
+  }
+  __device__ __forceinline__ int first_var() const { return v; }
+  __device__ __forceinline__ bool owns_eta() const { return true; }
+  __device__ __forceinline__ void put_if(bool c, uint32_t p) const { lu_sts_if(c, p + vb, oe); }
+  __device__ __forceinline__ void send(uint32_t dst, uint32_t bar) const { lu_send1(dst + vb, bar, oe); }
+};
+
+// bulk copy (TMA) into this CTA's shared memory, counted on bar; 16-byte
+// aligned ends and size
+__device__ __forceinline__ void lu_bulk(uint32_t dst, const void* src, uint32_t bytes, uint64_t* bar) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
+               "l"(src), "r"(bytes), "r"(smem_u32(bar))
+               : "memory");
+}
+
+// What a warp of a sweep works on (lu_sweep_slice), and where its first row's
+// input comes from (IN) and its last row's contributions go (OUT).
+enum { LU_HALO = 0, LU_NONE = 0, LU_RING = 1, LU_LINK = 2 };
+template <class R>
+struct LuBand {
+  int band, nrow, ncol, nst, row0;           // row0: first row of the band
+  uint32_t lim;
+  int lag, D;
+  R gm1;
+  const R* rec;                              // the band's records
+  R* rec_w;
+  R* s;                                      // s at (first interior row of the band, first interior column), variable 1
+  int64_t jd, qs;
+  const R* halo;                             // xi contributions of the halo to the first column, 4 per row
+  uint32_t stages, ex, xin, xout;            // shared addresses: record stages, exchange buffer, input row or ring, ring
+  uint64_t *bars, *xb_in, *xb_out, *lbars;   // barriers: stages; the input ring's, the own ring's; the link's
+  uint32_t ldst, lbar;                       // the next CTA's row and its barriers
+};
+
+// One band of one sweep.  Returns the group at which a bounded wait gave up,
+// or -1.
+template <class R, bool FWD, bool PRE, int PG, int IN, int OUT>
+__device__ __forceinline__ int lu_band(const LuBand<R>& B, int l) {
+  constexpr int CH = LuLay<R, PRE>::CH, LS = LuLay<R, PRE>::LS, LP = LuSplit<R, PRE>::LP, RB = LuSplit<R, PRE>::RB;
+  constexpr int NS = LU_XB / PG, KS = lu_ks<PG>();
+  constexpr uint32_t SB = 4 * sizeof(R), CHB = CH * sizeof(R);
+  static_assert(KS % PG == 0 && LU_LG % PG == 0 && LU_XB % PG == 0 && RB % PG == 0, "groups do not straddle");
+  const int ncol = B.ncol, nst = B.nst, D = B.D, ngrp = (nst + PG - 1) / PG;
+  const uint32_t lim = B.lim;
+  const int row = l / LP, r = B.row0 + row;
+  const int lout = FWD ? RB - 1 : 0;                         // the row the next band takes
+  // the row that takes from outside the band
+  const int lin = FWD ? 0 : min(RB - 1, B.nrow - 1 - B.row0);
+  const int prow = FWD ? row : RB - 1 - row;                 // steps this row trails the band's first
+  constexpr int xmask = IN == LU_RING ? LU_XB - 1 : 0x7fffffff;
+  LuLanes<R, FWD, PRE, LP, KS> L(l, B.ex);
+  const int cols = r < B.nrow ? ncol : 0;                    // columns of this row (none beyond the mesh)
+  if (cols) L.halo_xi(B.halo + 4 * r);
+  const bool is_lin = row == lin, out_lane = row == lout && L.owns_eta();
+  const int64_t qs = B.qs;
+  const R gm1 = B.gm1;
+  // this row's record of step 0 in global memory; its column of s at step 0,
+  // the lane's first variable (backward); both step on with the sweep
+  constexpr int SSTEP = FWD ? 1 : -1;
+  R* rg = B.rec_w + (int64_t)row * LS;
+  R* sr = B.s + (int64_t)L.first_var() * qs + (int64_t)row * B.jd + (FWD ? -prow : ncol - 1 + prow);
+  const uint32_t eta0 = L.eta_base(), lin0 = L.eta_link(B.xin);
+  // records of group g: chunks c0(g) .. c0(g)+size-1 of the band, ascending
+  auto issue = [&](int g, int st) {
+    const int n = min(PG, nst - g * PG), c0 = FWD ? g * PG : nst - g * PG - n;
+    // (the stage's earlier reads are ordered by the warp barrier before; a
+    // proxy fence here made each group wait for its global stores)
+    mbar_expect_tx(&B.bars[st], (uint32_t)n * CHB);
+    lu_bulk(B.stages + (uint32_t)st * PG * CHB, B.rec + (int64_t)c0 * CH, (uint32_t)n * CHB, &B.bars[st]);
+  };
+  if (l == 0)
+    for (int g = 0; g < min(D, ngrp); ++g) issue(g, g);
+  // Waits for group q of the previous band's, or the next band's, steps (each
+  // phase of a ring slot's barrier is one group).
+  const int qlast = ngrp - 1;
+  auto wait_full = [&](int q) { return mbar_wait_bounded(&B.xb_in[q % NS], (uint32_t)(q / NS) & 1, lim); };
+  auto wait_empty = [&](int q) { return mbar_wait_bounded(&B.xb_out[NS + q % NS], (uint32_t)(q / NS) & 1, lim); };
+  bool ok = true;
+  if (IN == LU_HALO) ok = __all_sync(0xffffffffu, mbar_wait_bounded(&B.lbars[0], 0, lim));
+  // Band lag: start `lag` steps after the neighbouring band's first
+  // contribution is due (the operands of every cell are the same whatever
+  // the lag; at most what the ring holds).
+  if (IN == LU_RING && B.lag > 0)
+    ok = __all_sync(0xffffffffu, wait_full(min(min(RB + B.lag, LU_XB) / PG - 1, qlast)));
+  // groups g0 .. g1-1 have every row active and none on its first column
+  const bool full = B.row0 + RB <= B.nrow;
+  const int g0 = full ? RB / PG : ngrp, g1 = full ? max(g0, ncol / PG) : ngrp;
+  int stage = 0;
+  uint32_t phase = 0;
+  int g = 0;
+  auto group = [&](auto ramp_) {
+    constexpr bool RAMP = decltype(ramp_)::value;
+    const int t0 = g * PG, ps = RAMP ? min(PG, nst - t0) : PG, p0 = t0 - prow;
+    ok = mbar_wait_bounded(&B.bars[stage], phase, lim) && ok;
+    // the first row's inputs of these steps (columns t0 .. t0+PG-1 in sweep
+    // order, produced RB-1 steps later by the previous band), and room in the
+    // ring for the last row's outputs
+    if (IN == LU_RING && (!RAMP || t0 < ncol)) ok = wait_full(min(g + RB / PG, qlast)) && ok;
+    if (IN == LU_LINK && (!RAMP || t0 < ncol)) ok = lu_link_wait(&B.lbars[t0 / LU_LG], lim) && ok;
+    if (OUT == LU_RING && g + 1 >= (RB + LU_XB) / PG) ok = wait_empty(g + 1 - (RB + LU_XB) / PG) && ok;
+    const uint32_t st0 = B.stages + (uint32_t)stage * PG * CHB + (uint32_t)row * LS * sizeof(R);
+    const uint32_t ch0 = FWD ? st0 : st0 + (uint32_t)(ps - 1) * CHB;
+    const int k0 = PG == KS ? 0 : t0 & (KS - 1);
+    const uint32_t eta = is_lin ? lin0 + (uint32_t)(t0 & xmask) * SB : eta0 + (uint32_t)k0 * SB;
+    auto rec = L.load(ch0);
+#pragma unroll
+    for (int u = 0; u < PG; ++u) {
+      if (RAMP && u >= ps) break;
+      const auto cur = rec;
+      if (u + 1 < PG && (!RAMP || u + 1 < ps)) rec = L.load(FWD ? ch0 + (u + 1) * CHB : ch0 - (u + 1) * CHB);
+      const bool valid = !RAMP || (unsigned)(p0 + u) < (unsigned)cols;
+      // (outside its columns the first row reads slot 0, in bounds)
+      const uint32_t ea = RAMP && is_lin ? lin0 + (uint32_t)(valid ? (p0 + u) & xmask : 0) * SB : eta + u * SB;
+      L.template cell<RAMP>(cur, ea, k0 + u, (k0 + u + 1) & (KS - 1), RAMP && p0 + u == 0, valid, gm1, rg + u * CH,
+                            sr + u * SSTEP, qs);
+      if (OUT == LU_RING) L.put_if(out_lane, B.xout + (uint32_t)((p0 + u) & (LU_XB - 1)) * SB);
+      if (OUT == LU_LINK) {
+        if (out_lane && valid) L.send(B.ldst + (uint32_t)(p0 + u) * SB, B.lbar + (uint32_t)((p0 + u) / LU_LG) * 8);
+      }
+      __syncwarp();
+    }
+    rg += PG * CH;
+    sr += PG * SSTEP;
     if (l == 0) {
-      // copies issued and not consumed: groups gfail .. gfail+1; wait
-      // (bounded) before the CTA's shared memory goes away, then flag
-      for (int g = gfail; g < gfail + 2 && g < ngrp; ++g) mbar_wait_bounded(&bar[g & 1], (uint32_t)((g >> 1) & 1));
-      if (S.ist) atomicOr(&S.ist[2], 4);
+      // these steps' ring slots are read and written by the whole warp, and
+      // its stage takes group g + D
+      if (OUT == LU_RING) mbar_arrive(&B.xb_out[g % NS]);
+      if (IN == LU_RING) mbar_arrive(&B.xb_in[NS + g % NS]);
+      if (g + D < ngrp) issue(g + D, stage);
+    }
+    if (++stage == D) { stage = 0; phase ^= 1; }
+    ++g;
+    ok = __all_sync(0xffffffffu, ok);
+  };
+  while (g < ngrp && ok) {
+    if (g == g0)
+#pragma unroll 1
+      while (g < g1 && ok) group(std::false_type());
+    if (g < ngrp && ok) group(std::true_type());
+  }
+  if (ok) return -1;
+  // copies issued and not consumed: wait (bounded) before the CTA's shared
+  // memory goes away
+  if (l == 0)
+    for (int h = max(0, g - 1); h < min(g + D, ngrp); ++h) mbar_wait_bounded(&B.bars[h % D], (uint32_t)(h / D) & 1);
+  __syncwarp();
+  return g;
+}
+
+// One sweep of one slice by the CTA `rank` of a cluster of cs.  The slice's
+// bands are dealt to the CTAs in contiguous runs, one warp per band; a warp
+// walks its nst local steps: at local step t row r of the band is on column
+// t-r (forward) or ncol-1-(t-(RB-1-r)) (backward), so the rows of a band are
+// on RB consecutive hyperplanes and the in-band dependency (the neighbouring
+// row) arrives through the warp's exchange buffer from the previous step.
+// The dependency across bands -- the last row of a band feeds the first row
+// of the next, RB-1 steps later -- goes through the producer's cross-band
+// ring guarded by mbarriers within a CTA (a counter published with a release
+// store cost a memory fence behind every group's global stores), and into the
+// next CTA's shared memory with st.async between CTAs (a whole row: nothing
+// is overwritten, so nothing flows back), so the warps run without block-wide
+// barriers.  Rows that have not reached their first column or are past their
+// last one run along on records of 0, so that no step branches; the groups
+// inside the columns of all rows of a full band also leave out their selects.
+// PRE: the preilu2d records and contributions.
+template <class R, bool FWD, bool PRE, int PG>
+__device__ void lu_sweep_slice(const Slice<R>& S, int nwarp, int cs, int rank, int maxcol, int D, unsigned char* smem,
+                               uint32_t lim, int lag) {
+  constexpr int CH = LuLay<R, PRE>::CH, RB = LuSplit<R, PRE>::RB, NS = LU_XB / PG;
+  const ot2d_params& p = *S.P;
+  const int nrow = lu_nrow(S.kd), ncol = lu_ncol(S.jd), nb = lu_nband(S.kd, RB), nst = lu_nstep(S.jd, RB);
+  const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
+  const int per = (nb + cs - 1) / cs, base = rank * per, mine = max(0, min(per, nb - base));
+  const int band = base + w;
+  R* stages = (R*)smem;
+  R* xrings = stages + (size_t)nwarp * D * PG * CH;
+  R* exs = xrings + (size_t)nwarp * LU_XB * 4;
+  R* rowbuf = exs + (size_t)nwarp * lu_ex<R, PRE, PG>();
+  uint64_t* bars = (uint64_t*)(rowbuf + (size_t)4 * maxcol);
+  uint64_t* xbars = bars + (size_t)nwarp * D;               // per warp: full[NS], empty[NS] of its ring
+  uint64_t* lbars = xbars + (size_t)nwarp * 2 * NS;
+  const bool wok = w < mine;
+  // the CTA of the first band in sweep order takes the halo's contributions
+  const bool first_cta = FWD ? rank == 0 : base + mine == nb;
+  const bool linked = cs > 1 && mine > 0 && !first_cta;     // takes its row from the previous CTA
+  for (int i = l; i < D; i += 32) mbar_init(&bars[(size_t)w * D + i], 1);
+  for (int i = l; i < 2 * NS; i += 32) mbar_init(&xbars[(size_t)w * 2 * NS + i], 1);
+  asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  for (int i = l; i < lu_ex<R, PRE, PG>(); i += 32) exs[(size_t)w * lu_ex<R, PRE, PG>() + i] = (R)0;
+  if (linked) {
+    for (int i = threadIdx.x; i < (ncol + LU_LG - 1) / LU_LG; i += blockDim.x) {
+      mbar_init(&lbars[i], 1);
+      asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+      mbar_expect_tx(&lbars[i], (uint32_t)min(LU_LG, ncol - i * LU_LG) * 4 * sizeof(R));
+    }
+  } else if (threadIdx.x == 0 && mine > 0) {
+    // the halo's row, one bulk copy (a loop of loads through registers took
+    // 10-20 us of a small mesh's sweep)
+    mbar_init(&lbars[0], 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    mbar_expect_tx(&lbars[0], (uint32_t)(4 * ncol * sizeof(R)));
+    lu_bulk(smem_u32(rowbuf), lu_halo<R, PRE>(S, FWD ? 2 : 3), (uint32_t)(4 * ncol * sizeof(R)), &lbars[0]);
+  }
+  __syncthreads();
+  if (cs > 1) lu_cluster_sync();
+  int gfail = -1;
+  if (wok) {
+    // neighbouring bands in sweep order
+    const bool has_next = FWD ? band + 1 < nb : band > 0;
+    const bool prev_here = FWD ? w > 0 : w + 1 < mine;
+    const bool next_here = has_next && (FWD ? w + 1 < mine : w > 0);
+    const bool from_link = linked && !prev_here, to_link = has_next && !next_here;
+    const int wprev = prev_here ? (FWD ? w - 1 : w + 1) : w;
+    LuBand<R> B;
+    B.band = band; B.nrow = nrow; B.ncol = ncol; B.nst = nst; B.row0 = RB * band;
+    B.lim = lim; B.lag = lag; B.D = D;
+    B.gm1 = S.k_gm1;
+    B.rec_w = S.lurec + (int64_t)band * nst * CH;
+    B.rec = B.rec_w;
+    B.s = S.s + (int64_t)(p.kbeg + RB * band - 1) * S.jd + (p.jbeg - 1);
+    B.jd = S.jd; B.qs = S.qs;
+    B.halo = lu_halo<R, PRE>(S, FWD ? 0 : 1);
+    B.stages = smem_u32(stages + (size_t)w * D * PG * CH);
+    B.ex = smem_u32(exs + (size_t)w * lu_ex<R, PRE, PG>());
+    B.xin = smem_u32(prev_here ? xrings + (size_t)wprev * LU_XB * 4 : rowbuf);
+    B.xout = smem_u32(xrings + (size_t)w * LU_XB * 4);
+    B.bars = bars + (size_t)w * D;
+    B.xb_in = xbars + (size_t)wprev * 2 * NS;
+    B.xb_out = xbars + (size_t)w * 2 * NS;
+    B.lbars = lbars;
+    const int nrank = FWD ? rank + 1 : rank - 1;
+    B.ldst = B.lbar = 0;
+    if (to_link) {
+      B.ldst = lu_mapa(smem_u32(rowbuf), nrank);
+      B.lbar = lu_mapa(smem_u32(lbars), nrank);
+    }
+    if (prev_here) {
+      if (next_here) gfail = lu_band<R, FWD, PRE, PG, LU_RING, LU_RING>(B, l);
+      else if (to_link) gfail = lu_band<R, FWD, PRE, PG, LU_RING, LU_LINK>(B, l);
+      else gfail = lu_band<R, FWD, PRE, PG, LU_RING, LU_NONE>(B, l);
+    } else if (from_link) {
+      if (next_here) gfail = lu_band<R, FWD, PRE, PG, LU_LINK, LU_RING>(B, l);
+      else if (to_link) gfail = lu_band<R, FWD, PRE, PG, LU_LINK, LU_LINK>(B, l);
+      else gfail = lu_band<R, FWD, PRE, PG, LU_LINK, LU_NONE>(B, l);
+    } else {
+      if (next_here) gfail = lu_band<R, FWD, PRE, PG, LU_HALO, LU_RING>(B, l);
+      else if (to_link) gfail = lu_band<R, FWD, PRE, PG, LU_HALO, LU_LINK>(B, l);
+      else gfail = lu_band<R, FWD, PRE, PG, LU_HALO, LU_NONE>(B, l);
+    }
+    if (gfail >= 0 && l == 0 && S.ist) atomicOr(&S.ist[2], 4);
+  }
+  // a give-up before the halo's row has landed: wait (bounded) for it
+  if (!linked && mine > 0 && threadIdx.x == 0) mbar_wait_bounded(&lbars[0], 0);
+  // no CTA leaves while another may still write into it; after a give-up
+  // the stores already under way get time to land too
+  if (cs > 1) {
+    lu_cluster_sync();
+    if (linked && __syncthreads_or(gfail >= 0)) {
+      for (int i = 0; i < 64; ++i) __nanosleep(1000);
     }
   }
 }

@@ -359,43 +359,42 @@ __global__ void k_rbc(const Slice<R>* __restrict__ sl) {
 
 // ilu2d (lhs.f:470-814), preceded by s *= tscale on all cells when `scale`
 // (step.f:141-148).  Records of the interior cells (prefix table lfirst):
-// a block of LU_PREP_BS threads builds LU_PREP_CH = 16 consecutive chunks of
-// the band layout.  Lane l of chunk (band, t) is cell (row 32 band + l,
-// column t - l), so the chunks' lanes walk the grid diagonally; thread i
-// computes lane i / 16 of chunk i % 16 instead, which makes sixteen
-// consecutive threads read sixteen consecutive cells (64 bytes of each
-// array) of one row (the lane-per-thread order would touch a different row,
-// and cache line, per thread).  The records go to the block's shared-memory
-// copy of its chunks (chunk stride padded by 16 bytes so the chunks of one
-// row land in different banks), then each warp stores one chunk with one
-// bulk copy.  PRE: the
-// preconditioned (preilu2d) records of the slices with k_mp2 >= 0; each
-// instantiation returns on the other kind's slices.
-constexpr int LU_PREP_CH = LU_PREP_BS / 32;   // chunks per block
+// a block of lu_prep_bs() threads builds NC = lu_prep_bs() / RB consecutive
+// chunks of the band layout.  Row l of chunk (band, t) is cell (row RB band +
+// l, column t - l), so the chunks' rows walk the grid diagonally; thread i
+// computes row i / NC of chunk i % NC, which makes NC consecutive threads
+// read NC (32) consecutive cells of one row.  The records go to
+// the block's shared-memory copy of its chunks (chunk stride padded by 16
+// bytes so the chunks of one row land in different banks), then each chunk
+// is stored with one bulk copy.  PRE: the preconditioned (preilu2d) records
+// of the slices with k_mp2 >= 0; each instantiation returns on the other
+// kind's slices.
+template <class R, bool PRE>
+__host__ __device__ constexpr int lu_prep_chunks() { return lu_prep_bs<R>() / LuSplit<R, PRE>::RB; }
 template <class R, bool PRE>
 __host__ __device__ constexpr int lu_prep_stride() { return LuLay<R, PRE>::CH + (int)(16 / sizeof(R)); }
 template <class R, bool PRE>
-__global__ void __launch_bounds__(LU_PREP_BS) k_lu_prep(const Slice<R>* __restrict__ sl, const int32_t* __restrict__ lfirst,
+__global__ void __launch_bounds__(lu_prep_bs<R>()) k_lu_prep(const Slice<R>* __restrict__ sl, const int32_t* __restrict__ lfirst,
                                                      int nslice, int scale, int only_lu) {
-  static_assert(LU_PREP_CH * 32 == LU_PREP_BS && (LU_PREP_CH & (LU_PREP_CH - 1)) == 0,
-                "thread -> (chunk, lane) map: a power-of-two number of 32-lane chunks");
   extern __shared__ __align__(16) unsigned char lp_smem[];
+  constexpr int RB = LuSplit<R, PRE>::RB, NC = lu_prep_chunks<R, PRE>();
+  static_assert(NC * RB == lu_prep_bs<R>(), "thread -> (chunk, row) map");
   const int si = find_slice(lfirst, nslice, blockIdx.x);
   const Slice<R>& S = sl[si];
   if ((S.k_mp2 >= (R)0) != PRE) return;                    // uniform over the block
   if (only_lu && S.P->ilhs != 1) return;                   // uniform over the block
-  const int nst = lu_nstep(S.jd), nb = lu_nband(S.kd);
-  const int c0 = (blockIdx.x - lfirst[si]) * LU_PREP_CH;   // first chunk of the block
+  const int nst = lu_nstep(S.jd, RB), nb = lu_nband(S.kd, RB);
+  const int c0 = (blockIdx.x - lfirst[si]) * NC;           // first chunk of the block
   constexpr int CH = LuLay<R, PRE>::CH, CHS = lu_prep_stride<R, PRE>();
   {
-    const int w = threadIdx.x & (LU_PREP_CH - 1), l = threadIdx.x / LU_PREP_CH;
+    const int w = threadIdx.x % NC, l = threadIdx.x / NC;
     const int c = c0 + w, band = c / nst, t = c - band * nst;
     if (band < nb) lu_prep_cell<R, PRE>(S, *S.P, band, t, l, scale, (R*)lp_smem + w * CHS);
   }
   __syncthreads();
-  const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
+  const int w = threadIdx.x;
   const int c = c0 + w, band = c / nst;
-  if (band >= nb || l != 0) return;
+  if (w >= NC || band >= nb) return;
   // one bulk copy (TMA) per staged chunk, shared -> global: chunk (band, t)
   // is chunk band*nst + t; both ends 16-byte aligned, 16-byte multiple size
   static_assert((CH * sizeof(R)) % 16 == 0 && (CHS * sizeof(R)) % 16 == 0, "bulk copy alignment");
@@ -435,12 +434,16 @@ __global__ void __launch_bounds__(128) k_lu_edges_ring(const Slice<R>* __restric
   lu_edge_cell<R, PRE>(S, *S.P, j, k, scale);
 }
 
-template <class R, bool FWD, int G, bool PRE>
-__global__ void k_lu_sweep(const Slice<R>* __restrict__ sl, int only_lu, uint32_t poll_limit, int lag) {
+// One sweep: a cluster of cs CTAs per slice (grid nslice * cs).
+template <class R, bool FWD, bool PRE, int PG>
+__global__ void __launch_bounds__(32 * LU_MAX_WARPS) k_lu_sweep(const Slice<R>* __restrict__ sl, int only_lu,
+                                                                uint32_t poll_limit, int lag, int cs, int maxcol,
+                                                                int stages) {
   extern __shared__ __align__(128) unsigned char lu_smem[];
-  if (only_lu && sl[blockIdx.x].P->ilhs != 1) return;
-  if ((sl[blockIdx.x].k_mp2 >= (R)0) != PRE) return;
-  lu_sweep_slice<R, FWD, G, PRE>(sl[blockIdx.x], blockDim.x >> 5, lu_smem, poll_limit, lag);
+  const Slice<R>& S = sl[blockIdx.x / cs];
+  if (only_lu && S.P->ilhs != 1) return;                   // uniform over the cluster
+  if ((S.k_mp2 >= (R)0) != PRE) return;                    // uniform over the cluster
+  lu_sweep_slice<R, FWD, PRE, PG>(S, blockDim.x >> 5, cs, blockIdx.x % cs, maxcol, stages, lu_smem, poll_limit, lag);
 }
 
 // vmu_sa's closing turbc (with the velocities k_sa_prep stored at the start

@@ -12,8 +12,10 @@ template <class R> struct Slice;
 struct NormPart;
 
 constexpr int CELL_BS = 256;
-// the LU-SGS record kernel: threads per block (LU_PREP_BS / 32 chunks each)
-constexpr int LU_PREP_BS = 512;
+// the LU-SGS record kernel: threads per block, one per cell record (FP64
+// records are twice as large: two blocks of 256 fit an SM's shared memory,
+// one of 512 would not leave room for a second)
+template <class R> constexpr int lu_prep_bs() { return sizeof(R) == 8 ? 256 : 512; }
 // threads of the one-CTA-per-slice boundary kernels (their loops run along
 // the boundary rows; more threads, fewer serial passes per row)
 constexpr int BC_BS = 512;
@@ -75,7 +77,6 @@ struct Batch {
   int lim_mask = 0;        // reconstruction families of the slices: 1 central, 2 MUSCL, 4 WENO, 8 quad
   int rt_shape = 0;        // residual tile shape of the tile table (rt_shape_dims)
   int cell_blocks = 0;     // blocks of the cell-parallel kernels
-  int max_lu_warps = 1;    // warps per CTA of the LU-SGS kernel
   int max_wall = 1;        // most wall cells of one slice (force kernel smem); also max jd
   int max_kd = 1;          // largest kd of the batch
   int max_nbc = 0;         // most &bcinp entries of one slice

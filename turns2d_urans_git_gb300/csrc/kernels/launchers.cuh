@@ -1,5 +1,6 @@
 // launchers.cuh -- launcher bodies, instantiated once per arithmetic type.
 #pragma once
+#include <algorithm>
 #include "kernels.cuh"
 
 namespace ot2d {
@@ -111,15 +112,15 @@ cudaError_t launch_rhslom(const Slice<R>* d_sl, const Batch& b, cudaStream_t st)
 template <class R, bool PRE>
 cudaError_t launch_lusgs_prep_t(const Slice<R>* d_sl, const Batch& b, int scale, cudaStream_t st, int only_lu,
                                 int parts) {
-  // one staged chunk per warp (f32 28 / 36 KB, f64 53 / 68 KB per block)
-  constexpr size_t prep_smem = (size_t)LU_PREP_CH * lu_prep_stride<R, PRE>() * sizeof(R);
+  // the block's staged chunks (f32 50 / 74 KB, f64 58 / 70 KB per block)
+  constexpr size_t prep_smem = (size_t)lu_prep_chunks<R, PRE>() * lu_prep_stride<R, PRE>() * sizeof(R);
   static DeviceOnce once;
   cudaError_t ae = once.run([&](int&) {
     return cudaFuncSetAttribute(k_lu_prep<R, PRE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)prep_smem);
   });
   if (ae != cudaSuccess) return ae;
   if (parts & 1)
-    k_lu_prep<R, PRE><<<b.lu_blocks, LU_PREP_BS, prep_smem, st>>>(d_sl, b.d_lfirst, b.nslice, scale, only_lu);
+    k_lu_prep<R, PRE><<<b.lu_blocks, lu_prep_bs<R>(), prep_smem, st>>>(d_sl, b.d_lfirst, b.nslice, scale, only_lu);
   if (!(parts & 2)) return cudaGetLastError();
   if constexpr (sizeof(R) == sizeof(double)) {
     // every cell: the FP64 path also round-trips q (lhs.f:524-531, :805-811)
@@ -138,26 +139,46 @@ cudaError_t launch_lusgs_prep(const Slice<R>* d_sl, const Batch& b, int scale, c
   if (e == cudaSuccess && b.precon) e = launch_lusgs_prep_t<R, true>(d_sl, b, scale, st, only_lu, parts);
   return e;
 }
+// CTAs per slice of the sweeps (a cluster), for nb bands.  One warp per SM
+// sub-partition (4 bands per CTA) makes a step fastest, but takes SMs from
+// the residual and the turbulence solve of a large batch.  Measured per
+// iteration (us), one CTA against ceil(nb / 4): FP32-mixed RANS-SA 769x193
+// alone 760, 454; 8 per launch 1127, 869; 32 per launch 2715, 2786; 513x129
+// 16 per launch 557, 477 (wide groups), 32 per launch 1276, 1328.  FP64
+// 513x129 alone 3769, 1877; 8 per launch 7577, 6801; 16 per launch 12638,
+// 13024.  The same line separates the wide groups of the f32 sweeps (lu_pg).
+// More CTAs than that only where the bands or their shared memory do not fit.
+constexpr int LU_SPREAD_SLICES = 16;
+template <class R, bool PRE, int PG>
+int lu_cluster(int nb, bool spread, int maxcol) {
+  const int want = spread ? std::min((nb + 3) / 4, LU_MAX_CLUSTER) : 1;
+  for (int cs = want; cs <= LU_MAX_CLUSTER; ++cs) {
+    const int nw = (nb + cs - 1) / cs;
+    if (nw <= LU_MAX_WARPS && lu_smem_bytes<R, PRE, PG>(nw, 2, maxcol) <= (size_t)SMEM_OPTIN_MAX) return cs;
+  }
+  return 0;
+}
 // ilu2d part 2: the forward and backward sweeps, launched at the device's
 // highest priority (they are the iteration's longest dependency chain and
 // run beside the turbulence branch)
-template <class R, bool PRE>
-cudaError_t launch_lusgs_sweeps_t(const Slice<R>* d_sl, const Batch& b, cudaStream_t st, int only_lu) {
-  const int nw = b.max_lu_warps;
-  // chunks per bulk copy: as many as ~200 KB of shared memory allows (1..8)
+template <class R, bool PRE, int PG>
+cudaError_t launch_lusgs_sweeps_t(const Slice<R>* d_sl, const Batch& b, cudaStream_t st, int only_lu, bool spread) {
   const int maxcol = b.max_wall;   // >= jd - 2 of every slice
-  int G = (b.lu_group == 1 || b.lu_group == 2 || b.lu_group == 4 || b.lu_group == 8) ? b.lu_group : 8;
-  while (G > 1 && lu_smem_bytes<R, PRE>(nw, G, maxcol) > 200 * 1024) G >>= 1;
-  const size_t smem = lu_smem_bytes<R, PRE>(nw, G, maxcol);
-  if (32 * nw > 1024 || smem > (size_t)SMEM_OPTIN_MAX) return cudaErrorInvalidConfiguration;
+  const int nb = lu_nband(b.max_kd, LuSplit<R, PRE>::RB);
+  const int cs = lu_cluster<R, PRE, PG>(nb, spread, maxcol);
+  if (cs < 1) return cudaErrorInvalidConfiguration;
+  const int nw = (nb + cs - 1) / cs;
+  // records in flight per band: two groups, or lu_group chunks where that is
+  // more (FP64: 16 by default), within ~200 KB of shared memory
+  const int G = (b.lu_group == 1 || b.lu_group == 2 || b.lu_group == 4 || b.lu_group == 8) ? b.lu_group : 8;
+  int D = std::max(2, (sizeof(R) == 8 ? 2 : 1) * G / PG);
+  while (D > 2 && lu_smem_bytes<R, PRE, PG>(nw, D, maxcol) > 200 * 1024) --D;
+  const size_t smem = lu_smem_bytes<R, PRE, PG>(nw, D, maxcol);
   static DeviceOnce once;
   int prio = 0;
   cudaError_t ae = once.run(
       [&](int& hi_prio) {
-        const void* ks[] = {(const void*)k_lu_sweep<R, true, 8, PRE>, (const void*)k_lu_sweep<R, false, 8, PRE>,
-                            (const void*)k_lu_sweep<R, true, 4, PRE>, (const void*)k_lu_sweep<R, false, 4, PRE>,
-                            (const void*)k_lu_sweep<R, true, 2, PRE>, (const void*)k_lu_sweep<R, false, 2, PRE>,
-                            (const void*)k_lu_sweep<R, true, 1, PRE>, (const void*)k_lu_sweep<R, false, 1, PRE>};
+        const void* ks[] = {(const void*)k_lu_sweep<R, true, PRE, PG>, (const void*)k_lu_sweep<R, false, PRE, PG>};
         for (const void* k : ks) {
           cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_OPTIN_MAX);
           if (e != cudaSuccess) return e;
@@ -168,35 +189,36 @@ cudaError_t launch_lusgs_sweeps_t(const Slice<R>* d_sl, const Batch& b, cudaStre
       },
       &prio);
   if (ae != cudaSuccess) return ae;
-  cudaLaunchAttribute at[1];
+  cudaLaunchAttribute at[2];
   at[0].id = cudaLaunchAttributePriority;
   at[0].val.priority = prio;
+  at[1].id = cudaLaunchAttributeClusterDimension;
+  at[1].val.clusterDim.x = cs;
+  at[1].val.clusterDim.y = 1;
+  at[1].val.clusterDim.z = 1;
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(b.nslice);
+  cfg.gridDim = dim3(b.nslice * cs);
   cfg.blockDim = dim3(32 * nw);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
   cfg.attrs = at;
-  cfg.numAttrs = 1;
-  auto run = [&](auto fwd, auto bwd) -> cudaError_t {
-    cudaError_t e = cudaLaunchKernelEx(&cfg, fwd, d_sl, only_lu, b.poll_limit, b.lu_lag);
-    if (e != cudaSuccess) return e;
-    return cudaLaunchKernelEx(&cfg, bwd, d_sl, only_lu, b.poll_limit, b.lu_lag);
-  };
-  cudaError_t e;
-  switch (G) {
-    case 8: e = run(k_lu_sweep<R, true, 8, PRE>, k_lu_sweep<R, false, 8, PRE>); break;
-    case 4: e = run(k_lu_sweep<R, true, 4, PRE>, k_lu_sweep<R, false, 4, PRE>); break;
-    case 2: e = run(k_lu_sweep<R, true, 2, PRE>, k_lu_sweep<R, false, 2, PRE>); break;
-    default: e = run(k_lu_sweep<R, true, 1, PRE>, k_lu_sweep<R, false, 1, PRE>); break;
-  }
+  cfg.numAttrs = 2;
+  cudaError_t e =
+      cudaLaunchKernelEx(&cfg, k_lu_sweep<R, true, PRE, PG>, d_sl, only_lu, b.poll_limit, b.lu_lag, cs, maxcol, D);
+  if (e != cudaSuccess) return e;
+  e = cudaLaunchKernelEx(&cfg, k_lu_sweep<R, false, PRE, PG>, d_sl, only_lu, b.poll_limit, b.lu_lag, cs, maxcol, D);
   if (e != cudaSuccess) return e;
   return cudaGetLastError();
 }
+template <class R, bool PRE>
+cudaError_t launch_lusgs_sweeps_p(const Slice<R>* d_sl, const Batch& b, cudaStream_t st, int only_lu) {
+  if (b.nslice <= LU_SPREAD_SLICES) return launch_lusgs_sweeps_t<R, PRE, lu_pg<R, true>()>(d_sl, b, st, only_lu, true);
+  return launch_lusgs_sweeps_t<R, PRE, lu_pg<R, false>()>(d_sl, b, st, only_lu, false);
+}
 template <class R>
 cudaError_t launch_lusgs_sweeps(const Slice<R>* d_sl, const Batch& b, cudaStream_t st, int only_lu) {
-  cudaError_t e = launch_lusgs_sweeps_t<R, false>(d_sl, b, st, only_lu);
-  if (e == cudaSuccess && b.precon) e = launch_lusgs_sweeps_t<R, true>(d_sl, b, st, only_lu);
+  cudaError_t e = launch_lusgs_sweeps_p<R, false>(d_sl, b, st, only_lu);
+  if (e == cudaSuccess && b.precon) e = launch_lusgs_sweeps_p<R, true>(d_sl, b, st, only_lu);
   return e;
 }
 template <class R>

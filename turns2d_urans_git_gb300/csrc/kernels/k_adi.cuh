@@ -15,14 +15,19 @@
 // so q leaves with the reference's bits.
 #pragma once
 #include "dev_common.cuh"
+#include "k_lines.cuh"
 #include "launch.h"
 
 namespace ot2d {
 
-// scratch arrays of one slice (stride S.wstride); dm/em: per variable
-// i = 1..4 the modified super-diagonals of pentadag's forward sweep
-enum ADIw { A_P = 0, A_QX, A_QY, A_CX, A_CY, A_UV, A_VN, A_GE, A_U, A_V, A_E, A_D2P, A_AT, A_BT, A_CT, A_DT, A_ET,
-            A_DM, A_EM = A_DM + 4, A_N = A_EM + 4 };
+// scratch arrays of one slice (stride S.wstride).  Rows of the line systems
+// (adi_row_cell): A_RB / A_RD one array per system; pentadiagonal (ilhs 2)
+// A_RA, A_RE, A_RC shared by the systems; tridiagonal (ilhs 3) A_RA = 0 =
+// A_RE and the diagonals of the three systems in A_RA, A_RE, A_RC.  A_EM: per
+// system the second super-diagonal of pentadag's forward sweep (the first
+// replaces A_RD); A_DN, the dissipation's diagonal, is used before it.
+enum ADIw { A_P = 0, A_QX, A_QY, A_CX, A_CY, A_UV, A_VN, A_GE, A_U, A_V, A_E, A_D2P, A_RA, A_RE, A_RC,
+            A_RB, A_RD = A_RB + 3, A_EM = A_RD + 3, A_N = A_EM + 3, A_DN = A_EM };
 static_assert(A_N <= ADI_NSCRATCH, "ADI scratch layout");
 
 __device__ __forceinline__ bool adi_slice(const ot2d_params& p) { return p.ilhs == 2 || p.ilhs == 3; }
@@ -107,21 +112,6 @@ __device__ void adi_txi_cell(const Slice<R>& S, const ot2d_params& p, int j, int
   S.s[3 * qs + o] = (R)0.5 * (a3 + a4 / cjkl);
 }
 
-// pressure switch of line direction dir (:919-935, :977-993): interior of
-// the line, 0 at its two ends
-template <class R>
-__device__ __forceinline__ void adi_d2p_cell(const Slice<R>& S, int dir, int m, int n, int ms, int me) {
-  const int jd = S.jd; const int64_t ws = S.wstride;
-  const R* P = S.w + A_P * ws;
-  R v = (R)0;
-  if (m > ms && m < me) {
-    const R pp = P[adi_at(jd, dir, m + 1, n)], pc = P[adi_at(jd, dir, m, n)], pm = P[adi_at(jd, dir, m - 1, n)];
-    v = fabs(pp - (R)2. * pc + pm);
-    v = v / fabs(pp + (R)2. * pc + pm);
-  }
-  S.w[A_D2P * ws + adi_at(jd, dir, m, n)] = v;
-}
-
 // spectral-radius diagonal of lhsinv (:1587-1596): d[0] = diag(m,1) =
 // diag(m,2), d[1] = diag(m,3), d[2] = diag(m,4), d[3] = diag(m,nq)
 template <class R>
@@ -138,12 +128,41 @@ __device__ __forceinline__ void adi_diag(const Slice<R>& S, const ot2d_params& p
   d[3] = (R)0.5 * ((bSq + (R)1.) * fabs(qv) + X) / S.q[(int64_t)(p.nq - 1) * S.qs + o];
 }
 
+// pressure switch of line direction dir (:919-935, :977-993): interior of
+// the line, 0 at its two ends; and diag(m,nq) of lhsinv
+template <class R>
+__device__ __forceinline__ void adi_d2p_cell(const Slice<R>& S, const ot2d_params& p, int dir, int m, int n, int ms,
+                                             int me) {
+  const int jd = S.jd; const int64_t ws = S.wstride;
+  const R* P = S.w + A_P * ws;
+  R v = (R)0;
+  if (m > ms && m < me) {
+    const R pp = P[adi_at(jd, dir, m + 1, n)], pc = P[adi_at(jd, dir, m, n)], pm = P[adi_at(jd, dir, m - 1, n)];
+    v = fabs(pp - (R)2. * pc + pm);
+    v = v / fabs(pp + (R)2. * pc + pm);
+  }
+  const int64_t o = adi_at(jd, dir, m, n);
+  S.w[A_D2P * ws + o] = v;
+  R d[4];
+  adi_diag(S, p, dir, o, d);
+  S.w[A_DN * ws + o] = d[3];
+}
+
+template <class R>
+struct AdiRow { R a, b, c, d, e; };
+
+// a product rounded on its own (the compiler must not fuse it with the
+// addition that follows)
+__device__ __forceinline__ float adi_mul(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ double adi_mul(double a, double b) { return __dmul_rn(a, b); }
+
 // Dissipation coefficients atmp..etmp of lhsinv (:1655-1732) at line
 // position m, times J (:1734-1740); the entries the reference leaves
 // unassigned (both line ends, and the ones its end-point formulas skip) are
 // 0.  Requires lines of at least 8 points.
 template <class R>
-__device__ void adi_coef_cell(const Slice<R>& S, const ot2d_params& p, int dir, int m, int n, int ms, int me) {
+__device__ __forceinline__ AdiRow<R> adi_coef(const Slice<R>& S, const ot2d_params& p, int dir, int m, int n, int ms,
+                                              int me) {
   const int jd = S.jd; const int64_t ws = S.wstride, qs = S.qs;
   const R dis2 = (R)10.0, dis4 = (R)0.1;
   R g[5], dn[5];   // positions m-2 .. m+2
@@ -152,9 +171,7 @@ __device__ void adi_coef_cell(const Slice<R>& S, const ot2d_params& p, int dir, 
     if (mm < ms || mm > me) { g[t] = (R)0; dn[t] = (R)0; continue; }
     const int64_t oo = adi_at(jd, dir, mm, n);
     g[t] = S.w[A_D2P * ws + oo];
-    R d[4];
-    adi_diag(S, p, dir, oo, d);
-    dn[t] = d[3];
+    dn[t] = S.w[A_DN * ws + oo];
   }
   auto G = [&](int dm) { return g[dm + 2]; };
   auto D = [&](int dm) { return dn[dm + 2]; };
@@ -204,26 +221,19 @@ __device__ void adi_coef_cell(const Slice<R>& S, const ot2d_params& p, int dir, 
   }
   const int64_t o = adi_at(jd, dir, m, n);
   const R J = S.q[(int64_t)(p.nq - 1) * qs + o];
-  S.w[A_AT * ws + o] = at * J;
-  S.w[A_BT * ws + o] = bt * J;
-  S.w[A_CT * ws + o] = ct * J;
-  S.w[A_DT * ws + o] = dt * J;
-  S.w[A_ET * ws + o] = et * J;
+  return {adi_mul(at, J), adi_mul(bt, J), adi_mul(ct, J), adi_mul(dt, J), adi_mul(et, J)};
 }
 
-// The five scaled bands a1..e1 of lhsinv (:1742-1785) for variable i at
-// line position m
+// The five scaled bands a1..e1 of lhsinv (:1742-1785) for system sys (0:
+// variables 1 and 2, 1: variable 3, 2: variable 4) at line position m; cf:
+// adi_coef of the position, dg: adi_diag
 template <class R>
-struct AdiRow { R a, b, c, d, e; };
-template <class R>
-__device__ __forceinline__ AdiRow<R> adi_row(const Slice<R>& S, const ot2d_params& p, int dir, int i, int m, int n,
-                                            int ms, int me) {
+__device__ __forceinline__ AdiRow<R> adi_row(const Slice<R>& S, const ot2d_params& p, int dir, int sys, int m, int n,
+                                            int ms, int me, const AdiRow<R>& cf, const R* dg) {
   const int jd = S.jd; const int64_t ws = S.wstride, qs = S.qs;
   const int64_t o = adi_at(jd, dir, m, n);
   const R* ts = S.tscale;
-  R dg[4];
-  adi_diag(S, p, dir, o, dg);
-  const R di = (i <= 2) ? dg[0] : (i == 3 ? dg[1] : dg[2]);
+  const R di = dg[sys];
   R v1 = (R)0, v2 = (R)0, v3 = (R)0;
   if (m > ms && m < me) {
     const R* xn = dir == 0 ? S.xx : S.yx;
@@ -261,8 +271,7 @@ __device__ __forceinline__ AdiRow<R> adi_row(const Slice<R>& S, const ot2d_param
     r.c = r.c * T(m) + (R)1.0;
     return r;
   }
-  r.a = S.w[A_AT * ws + o]; r.b = S.w[A_BT * ws + o]; r.c = S.w[A_CT * ws + o];
-  r.d = S.w[A_DT * ws + o]; r.e = S.w[A_ET * ws + o];
+  r = cf;
   r.b = r.b - di * (R)0.5;
   r.d = r.d + di * (R)0.5;
   r.b = r.b - (R)0.5 * v1;
@@ -276,85 +285,222 @@ __device__ __forceinline__ AdiRow<R> adi_row(const Slice<R>& S, const ot2d_param
   return r;
 }
 
-// One pentadiagonal system (variable i, line n): the reduced system over
-// m = ms+1..me-1 with the end corrections of :1787-1797, solved with
-// pentadag's recurrences (:1819-1873) in a sliding window; the modified
-// super-diagonals go to scratch for the backward sweep, the solution into s.
+// The rows of the three systems at line position m, for the recurrences of
+// adi_forward: a step takes a(m-2), b(m-1), c(m), d(m+1) and e(m+2) of the
+// reference's rows, so each is stored where it is used, with 0 where a step
+// takes none (its end rows ms and me are no part of the system).  The two end
+// positions correct the right-hand sides next to them (:1787-1797).
 template <class R>
-__device__ void adi_solve_line(const Slice<R>& S, const ot2d_params& p, int dir, int i, int n, int ms, int me) {
-  const int jd = S.jd; const int64_t ws = S.wstride, qs = S.qs;
-  R* sv = S.s + (int64_t)(i - 1) * qs;
-  R* Dm = S.w + (A_DM + i - 1) * ws;
-  R* Em = S.w + (A_EM + i - 1) * ws;
-  const int N = me - ms - 1;
-  auto O = [&](int ii) { return adi_at(jd, dir, ms + ii, n); };   // system index -> cell
-  // end rows of the full line
-  const AdiRow<R> r0 = adi_row(S, p, dir, i, ms, n, ms, me), rN1 = adi_row(S, p, dir, i, me, n, ms, me);
-  const R f1ms = sv[adi_at(jd, dir, ms, n)], f1me = sv[adi_at(jd, dir, me, n)];
-  // original bands of system row ii (1..N), with d(1)=e(1)=e(2)=0,
-  // b(N)=a(N)=a(N-1)=0, and f with its end corrections
-  auto row = [&](int ii) {
-    AdiRow<R> r = adi_row(S, p, dir, i, ms + ii, n, ms, me);
-    if (ii == 1) { r.d = (R)0; r.e = (R)0; }
-    if (ii == 2) r.e = (R)0;
-    if (ii == N) { r.b = (R)0; r.a = (R)0; }
-    if (ii == N - 1) r.a = (R)0;
-    return r;
-  };
-  auto fval = [&](int ii) {
-    R f = sv[O(ii)];
-    if (ii == 1) f = f - r0.b * f1ms / r0.c;
-    if (ii == N) f = f - rN1.d * f1me / rN1.c;
-    return f;
-  };
-  // i = 1
-  AdiRow<R> R1 = row(1), R2 = row(2), R3 = row(3);
-  R d0 = (R)1.0 / R1.c;
-  R Dn = R2.d * d0;                 // D(2)
-  R En1 = R3.e * d0;                // E(3)
-  R F1 = fval(1) * d0;
-  sv[O(1)] = F1;
-  Dm[O(2)] = Dn; Em[O(3)] = En1;
-  // i = 2
-  R d1 = R1.b;
-  d0 = (R)1.0 / (R2.c - d1 * Dn);
-  R F2 = (fval(2) - d1 * F1) * d0;
-  sv[O(2)] = F2;
-  const AdiRow<R> R4 = row(4);
-  R Dp = (R3.d - d1 * En1) * d0;    // D(3)
-  R Ep = R4.e * d0;                 // E(4)
-  Dm[O(3)] = Dp; Em[O(4)] = Ep;
-  // window: Dprev = D(i-1), Dcur = D(i), Ecur = E(i), Enext = E(i+1)
-  R Dprev = Dn, Dcur = Dp, Ecur = En1, Enext = Ep;
-  R Fm2 = F1, Fm1 = F2;
-  AdiRow<R> Rm2 = R1, Rm1 = R2, Rc = R3, Rn1 = R4;   // rows i-2, i-1, i, i+1
-  for (int ii = 3; ii <= N; ++ii) {
-    const AdiRow<R> Rn2 = (ii + 2 <= N) ? row(ii + 2) : AdiRow<R>{(R)0, (R)0, (R)0, (R)0, (R)0};
-    d1 = Rm2.a;
-    const R d2 = (Rm1.b - Rm2.a * Dprev);
-    d0 = (R)1. / (Rc.c - d2 * Dcur - d1 * Ecur);
-    const R Fi = (fval(ii) - d2 * Fm1 - d1 * Fm2) * d0;
-    sv[O(ii)] = Fi;
-    R Dnew = (R)0, Enew = (R)0;
-    if (ii <= N - 1) {
-      Dnew = (Rn1.d - d2 * Enext) * d0;
-      Dm[O(ii + 1)] = Dnew;
-      if (ii <= N - 2) { Enew = (Rn2.e) * d0; Em[O(ii + 2)] = Enew; }
+__device__ void adi_row_cell(const Slice<R>& S, const ot2d_params& p, int dir, int m, int n, int ms, int me) {
+  const int64_t ws = S.wstride, qs = S.qs;
+  const bool tri = p.ilhs == 3;
+  auto put = [&](int arr, int mm, R v) { S.w[arr * ws + adi_at(S.jd, dir, mm, n)] = v; };
+  AdiRow<R> cf{(R)0, (R)0, (R)0, (R)0, (R)0};
+  if (!tri) cf = adi_coef(S, p, dir, m, n, ms, me);
+  R dg[4];
+  adi_diag(S, p, dir, adi_at(S.jd, dir, m, n), dg);
+  for (int sys = 0; sys < 3; ++sys) {
+    const AdiRow<R> r = adi_row(S, p, dir, sys, m, n, ms, me, cf, dg);
+    if (m == ms || m == me) {
+      const int mi = m == ms ? ms + 1 : me - 1;
+      const R x = m == ms ? r.b : r.d;
+      for (int v = sys ? sys + 1 : 0; v < (sys ? sys + 2 : 2); ++v) {
+        R* sv = S.s + (int64_t)v * qs;
+        const int64_t oi = adi_at(S.jd, dir, mi, n);
+        sv[oi] = sv[oi] - x * sv[adi_at(S.jd, dir, m, n)] / r.c;
+      }
+      if (m == ms) put(A_RB + sys, ms + 1, (R)0);
+      else put(A_RD + sys, me - 1, (R)0);
+      if (!tri && sys == 0) {
+        if (m == ms) { put(A_RA, ms + 1, (R)0); put(A_RA, ms + 2, (R)0); }
+        else { put(A_RE, me - 1, (R)0); put(A_RE, me - 2, (R)0); }
+      }
+      continue;
     }
-    Dprev = Dcur; Dcur = Dnew; Ecur = Enext; Enext = Enew;
-    Fm2 = Fm1; Fm1 = Fi;
-    Rm2 = Rm1; Rm1 = Rc; Rc = Rn1; Rn1 = Rn2;
+    if (m < me - 1) put(A_RB + sys, m + 1, r.b);
+    if (m > ms + 1) put(A_RD + sys, m - 1, r.d);
+    if (tri) {
+      put(sys == 0 ? A_RA : (sys == 1 ? A_RE : A_RC), m, r.c);
+    } else if (sys == 0) {
+      put(A_RC, m, r.c);
+      if (m < me - 2) put(A_RA, m + 2, r.a);
+      if (m > ms + 2) put(A_RE, m - 2, r.e);
+    }
   }
-  // backward sweep
-  R Fa = sv[O(N)];                  // F(i+1)
-  R Fb = sv[O(N - 1)] - Dm[O(N)] * Fa;
-  sv[O(N - 1)] = Fb;
-  R Fc = Fa;                        // F(i+2)
-  Fa = Fb;
-  for (int ii = N - 2; ii >= 1; --ii) {
-    const R Fi = sv[O(ii)] - Dm[O(ii + 1)] * Fa - Em[O(ii + 2)] * Fc;
-    sv[O(ii)] = Fi;
-    Fc = Fa; Fa = Fi;
+}
+
+// pentadag's forward recurrences (:1819-1873) for NF right-hand sides: one
+// row in, the modified super-diagonals (d, e) and right-hand sides (f) out
+template <class R, int NF>
+struct AdiForward {
+  R Dp = (R)0, Dc = (R)0, Ec = (R)0, En = (R)0, f1[NF], f2[NF];
+  __device__ __forceinline__ AdiForward() {
+#pragma unroll
+    for (int v = 0; v < NF; ++v) f1[v] = f2[v] = (R)0;
+  }
+  __device__ __forceinline__ void step(R a, R b, R c, R& d, R& e, R* f) {
+    const R d2 = (b - a * Dp);
+    const R d0 = (R)1. / (c - d2 * Dc - a * Ec);
+#pragma unroll
+    for (int v = 0; v < NF; ++v) {
+      f[v] = (f[v] - d2 * f1[v] - a * f2[v]) * d0;
+      f2[v] = f1[v]; f1[v] = f[v];
+    }
+    d = (d - d2 * En) * d0;
+    e = e * d0;
+    Dp = Dc; Dc = d; Ec = En; En = e;
+  }
+};
+// ... and its back substitution
+template <class R, int NF>
+struct AdiBackward {
+  R f1[NF], f2[NF];
+  __device__ __forceinline__ AdiBackward() {
+#pragma unroll
+    for (int v = 0; v < NF; ++v) f1[v] = f2[v] = (R)0;
+  }
+  __device__ __forceinline__ void step(R d, R e, R* f) {
+#pragma unroll
+    for (int v = 0; v < NF; ++v) {
+      f[v] = f[v] - d * f1[v] - e * f2[v];
+      f2[v] = f1[v]; f1[v] = f[v];
+    }
+  }
+};
+
+// System sys of 32 lines along j (rows k0 .. k0+31 of the mesh) by a CTA of
+// JL_THREADS threads through staged tiles.  Arrays: a, b, c, d, e, f (f of
+// variable 2 too); the forward pass stores d, e and f.  TRI: a = e = 0.
+template <class R, bool TRI, int NF>
+__device__ void adi_solve_j(const Slice<R>& S, const ot2d_params& p, int sys, int k0, R* sm) {
+  const int64_t ws = S.wstride;
+  R* w = S.w;
+  const int var = sys ? sys + 1 : 0;
+  R* const f = S.s + (int64_t)var * S.qs;
+  constexpr int NA = TRI ? 3 + NF : 5 + NF, ND = TRI ? 2 : 3;   // d is array ND, then e, then f
+  R* src[NA];
+  R* dst[NA];
+  if (TRI) {
+    src[0] = w + (A_RB + sys) * ws;
+    src[1] = w + (sys == 0 ? A_RA : (sys == 1 ? A_RE : A_RC)) * ws;
+  } else {
+    src[0] = w + A_RA * ws; src[1] = w + (A_RB + sys) * ws; src[2] = w + A_RC * ws;
+    src[ND + 1] = w + A_RE * ws;
+  }
+  src[ND] = w + (A_RD + sys) * ws;
+#pragma unroll
+  for (int v = 0; v < NF; ++v) src[NA - NF + v] = f + (int64_t)v * S.qs;
+#pragma unroll
+  for (int a = 0; a < NA; ++a) dst[a] = src[a];
+  if (!TRI) dst[ND + 1] = w + (A_EM + sys) * ws;
+  constexpr unsigned OUT = ((1u << NA) - 1) & ~((1u << ND) - 1), RHS = ((1u << NF) - 1) << (NA - NF);
+  AdiForward<R, NF> F;
+  AdiBackward<R, NF> B;
+  jl_solve<R, NA, OUT, OUT, RHS>(
+      src, dst, S.jd, p.jbeg, p.jend, k0, min(32, S.kd - k0 + 1), sm,
+      [&](R* t, int) {
+        R f_[NF], e = TRI ? (R)0 : t[(ND + (TRI ? 0 : 1)) * JL_TILE];
+#pragma unroll
+        for (int v = 0; v < NF; ++v) f_[v] = t[(NA - NF + v) * JL_TILE];
+        R d = t[ND * JL_TILE];
+        F.step(TRI ? (R)0 : t[0], t[(ND - 2) * JL_TILE], t[(ND - 1) * JL_TILE], d, e, f_);
+        t[ND * JL_TILE] = d;
+        if (!TRI) t[(ND + 1) * JL_TILE] = e;
+#pragma unroll
+        for (int v = 0; v < NF; ++v) t[(NA - NF + v) * JL_TILE] = f_[v];
+      },
+      [&](R* t, int) {
+        R f_[NF];
+#pragma unroll
+        for (int v = 0; v < NF; ++v) f_[v] = t[(NA - NF + v) * JL_TILE];
+        B.step(t[ND * JL_TILE], TRI ? (R)0 : t[(ND + (TRI ? 0 : 1)) * JL_TILE], f_);
+#pragma unroll
+        for (int v = 0; v < NF; ++v) t[(NA - NF + v) * JL_TILE] = f_[v];
+      });
+}
+
+// System sys of the line along k at column j, one thread: rows a chunk ahead
+template <class R, bool TRI, int NF>
+__device__ void adi_solve_k(const Slice<R>& S, const ot2d_params& p, int sys, int j) {
+  constexpr int U = sizeof(R) == 4 ? 8 : 4;
+  const int64_t ws = S.wstride;
+  const int ks = p.kbeg, ke = p.kend, jd = S.jd;
+  const int var = sys ? sys + 1 : 0;
+  R* f = S.s + (int64_t)var * S.qs;
+  const R* ga = S.w + A_RA * ws;
+  const R* gb = S.w + (A_RB + sys) * ws;
+  const R* gc = S.w + (TRI ? (sys == 0 ? A_RA : (sys == 1 ? A_RE : A_RC)) : A_RC) * ws;
+  const R* ge = S.w + A_RE * ws;
+  R* gd = S.w + (A_RD + sys) * ws;
+  R* gem = S.w + (A_EM + sys) * ws;
+  {
+    AdiForward<R, NF> F;
+    AdiRow<R> nr[U];
+    R nf[U][NF];
+    auto load = [&](int k0) {
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+        if (k0 + u <= ke) {
+          const int64_t o = at(jd, j, k0 + u);
+          nr[u] = {TRI ? (R)0 : ga[o], gb[o], gc[o], gd[o], TRI ? (R)0 : ge[o]};
+#pragma unroll
+          for (int v = 0; v < NF; ++v) nf[u][v] = f[(int64_t)v * S.qs + o];
+        }
+    };
+    load(ks);
+    for (int k0 = ks; k0 <= ke; k0 += U) {
+      AdiRow<R> rr[U];
+      R rf[U][NF];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        rr[u] = nr[u];
+#pragma unroll
+        for (int v = 0; v < NF; ++v) rf[u][v] = nf[u][v];
+      }
+      if (k0 + U <= ke) load(k0 + U);
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+        if (k0 + u <= ke) {
+          const int64_t o = at(jd, j, k0 + u);
+          R d = rr[u].d, e = rr[u].e;
+          F.step(rr[u].a, rr[u].b, rr[u].c, d, e, rf[u]);
+          gd[o] = d;
+          if (!TRI) gem[o] = e;
+#pragma unroll
+          for (int v = 0; v < NF; ++v) f[(int64_t)v * S.qs + o] = rf[u][v];
+        }
+    }
+  }
+  AdiBackward<R, NF> B;
+  R nd[U], ne[U], nf[U][NF];
+  auto load = [&](int k0) {   // positions k0, k0-1, ...
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (k0 - u >= ks) {
+        const int64_t o = at(jd, j, k0 - u);
+        nd[u] = gd[o];
+        ne[u] = TRI ? (R)0 : gem[o];
+#pragma unroll
+        for (int v = 0; v < NF; ++v) nf[u][v] = f[(int64_t)v * S.qs + o];
+      }
+  };
+  load(ke);
+  for (int k0 = ke; k0 >= ks; k0 -= U) {
+    R rd[U], re[U], rf[U][NF];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      rd[u] = nd[u]; re[u] = ne[u];
+#pragma unroll
+      for (int v = 0; v < NF; ++v) rf[u][v] = nf[u][v];
+    }
+    if (k0 - U >= ks) load(k0 - U);
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (k0 - u >= ks) {
+        B.step(rd[u], re[u], rf[u]);
+#pragma unroll
+        for (int v = 0; v < NF; ++v) f[(int64_t)v * S.qs + at(jd, j, k0 - u)] = rf[u][v];
+      }
   }
 }
 

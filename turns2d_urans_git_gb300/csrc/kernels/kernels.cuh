@@ -679,7 +679,8 @@ __global__ void __launch_bounds__(CELL_BS) k_adi_txi(const Slice<R>* __restrict_
   if (!inside || (only && !adi_slice(*S.P))) return;
   adi_txi_cell(S, *S.P, j, k, scale);
 }
-// line direction dir over all cells: d2p (what = 0) or the coefficients (1)
+// line direction dir over all cells: the pressure switch and dissipation
+// diagonal (what = 0), then the rows of the line systems (1)
 template <class R>
 __global__ void __launch_bounds__(CELL_BS) k_adi_line_cells(const Slice<R>* __restrict__ sl,
                                                             const int32_t* __restrict__ first, int nslice, int dir,
@@ -690,21 +691,43 @@ __global__ void __launch_bounds__(CELL_BS) k_adi_line_cells(const Slice<R>* __re
   if (only && !adi_slice(p)) return;
   const int m = dir == 0 ? j : k, n = dir == 0 ? k : j;
   const int ms = dir == 0 ? p.jbeg - 1 : p.kbeg - 1, me = dir == 0 ? p.jend + 1 : p.kend + 1;
-  if (what == 0) adi_d2p_cell(S, dir, m, n, ms, me);
-  else adi_coef_cell(S, p, dir, m, n, ms, me);
+  if (what == 0) adi_d2p_cell(S, p, dir, m, n, ms, me);
+  else adi_row_cell(S, p, dir, m, n, ms, me);
 }
-// one thread per (line, variable); blockIdx.y = slice
+// the three systems (blockIdx.z) of 32 lines along j (blockIdx.x) of a slice
+// (blockIdx.y)
 template <class R>
-__global__ void k_adi_solve(const Slice<R>* __restrict__ sl, int dir, int only) {
+__global__ void __launch_bounds__(JL_THREADS) k_adi_solve_j(const Slice<R>* __restrict__ sl, int only) {
+  extern __shared__ __align__(16) unsigned char jl_raw[];
+  R* sm = (R*)jl_raw;
   const Slice<R>& S = sl[blockIdx.y];
   const ot2d_params& p = *S.P;
   if (only && !adi_slice(p)) return;
-  const int nlines = dir == 0 ? S.kd : S.jd;   // n = ks-1..ke+1 / js-1..je+1
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= 4 * nlines) return;
-  const int n = 1 + t % nlines, i = 1 + t / nlines;
-  const int ms = dir == 0 ? p.jbeg - 1 : p.kbeg - 1, me = dir == 0 ? p.jend + 1 : p.kend + 1;
-  adi_solve_line(S, p, dir, i, n, ms, me);
+  const int k0 = 1 + 32 * blockIdx.x, sys = blockIdx.z;       // lines of every row, ks-1..ke+1
+  if (k0 > S.kd) return;
+  if (p.ilhs == 3) {
+    if (sys == 0) adi_solve_j<R, true, 2>(S, p, sys, k0, sm);
+    else adi_solve_j<R, true, 1>(S, p, sys, k0, sm);
+  } else {
+    if (sys == 0) adi_solve_j<R, false, 2>(S, p, sys, k0, sm);
+    else adi_solve_j<R, false, 1>(S, p, sys, k0, sm);
+  }
+}
+// one thread per (line along k, system): blockIdx.y = slice, blockIdx.z = system
+template <class R>
+__global__ void __launch_bounds__(32) k_adi_solve_k(const Slice<R>* __restrict__ sl, int only) {
+  const Slice<R>& S = sl[blockIdx.y];
+  const ot2d_params& p = *S.P;
+  if (only && !adi_slice(p)) return;
+  const int j = 1 + blockIdx.x * 32 + threadIdx.x, sys = blockIdx.z;   // js-1..je+1
+  if (j > S.jd) return;
+  if (p.ilhs == 3) {
+    if (sys == 0) adi_solve_k<R, true, 2>(S, p, sys, j);
+    else adi_solve_k<R, true, 1>(S, p, sys, j);
+  } else {
+    if (sys == 0) adi_solve_k<R, false, 2>(S, p, sys, j);
+    else adi_solve_k<R, false, 1>(S, p, sys, j);
+  }
 }
 template <class R>
 __global__ void __launch_bounds__(CELL_BS) k_adi_ninv(const Slice<R>* __restrict__ sl, const int32_t* __restrict__ first,

@@ -276,13 +276,21 @@ cudaError_t launch_sst(const Slice<R>* d_sl, const Batch& b, cudaStream_t st) {
 }
 template <class R>
 cudaError_t launch_adi(const Slice<R>* d_sl, const Batch& b, int scale, cudaStream_t st, int only_adi) {
+  constexpr size_t jl_smem = (size_t)jl_smem_elems(7) * sizeof(R);
+  static DeviceOnce once;
+  cudaError_t ae = once.run([&](int&) {
+    return cudaFuncSetAttribute(k_adi_solve_j<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)jl_smem);
+  });
+  if (ae != cudaSuccess) return ae;
   k_adi_txi<R><<<b.cell_blocks, CELL_BS, 0, st>>>(d_sl, b.d_first, b.nslice, scale, only_adi);
   for (int dir = 0; dir < 2; ++dir) {
     if (dir == 1) k_adi_ninv<R><<<b.cell_blocks, CELL_BS, 0, st>>>(d_sl, b.d_first, b.nslice, only_adi);
     k_adi_line_cells<R><<<b.cell_blocks, CELL_BS, 0, st>>>(d_sl, b.d_first, b.nslice, dir, 0, only_adi);
     k_adi_line_cells<R><<<b.cell_blocks, CELL_BS, 0, st>>>(d_sl, b.d_first, b.nslice, dir, 1, only_adi);
-    const int nl = 4 * (dir == 0 ? b.max_kd : b.max_wall);
-    k_adi_solve<R><<<dim3((nl + 63) / 64, b.nslice), 64, 0, st>>>(d_sl, dir, only_adi);
+    if (dir == 0)
+      k_adi_solve_j<R><<<dim3((b.max_kd + 31) / 32, b.nslice, 3), JL_THREADS, jl_smem, st>>>(d_sl, only_adi);
+    else
+      k_adi_solve_k<R><<<dim3((b.max_wall + 31) / 32, b.nslice, 3), 32, 0, st>>>(d_sl, only_adi);
   }
   k_adi_teta<R><<<b.cell_blocks, CELL_BS, 0, st>>>(d_sl, b.d_first, b.nslice, only_adi);
   return cudaGetLastError();

@@ -147,4 +147,87 @@ __device__ __forceinline__ void jl_solve(R* const (&src)[NA], R* const (&dst)[NA
   if (mover) store(BST, 0, (ntile - 1) % JL_NBUF);
 }
 
+// lsolvej (samodel2d.f:1306-1344, komegasst.f:1435-1475) of the tridiagonal
+// systems a, b, c, s along the j-lines k0 .. k0+nrow-1: x * b replaces s, c is
+// overwritten.  SAOUT: ((x + 0) - 0) * b, as vmu_sa forms it with s2 = 0
+// (samodel2d.f:150-153).
+template <class R, bool SAOUT>
+__device__ void tri_solve_j(R* a, R* b, R* c, R* s, int jd, int js, int je, int k0, int nrow, R* sm) {
+  R* const arr[4] = {a, b, c, s};
+  R cp = (R)0, sp = (R)0, xn = (R)0;
+  jl_solve<R, 4, 12u, 14u, 8u>(
+      arr, arr, jd, js, je, k0, nrow, sm,
+      [&](R* t, int j) {
+        const R av = j == js ? (R)0 : t[0];
+        const R bb = (R)1. / (t[JL_TILE] - av * cp);
+        sp = (t[3 * JL_TILE] - av * sp) * bb;
+        cp = t[2 * JL_TILE] * bb;
+        t[3 * JL_TILE] = sp;
+        t[2 * JL_TILE] = cp;
+      },
+      [&](R* t, int j) {
+        const R sv = t[3 * JL_TILE];
+        xn = j == je ? sv : sv - t[2 * JL_TILE] * xn;
+        if constexpr (SAOUT) t[3 * JL_TILE] = ((xn + (R)0.) - (R)0.) * t[JL_TILE];
+        else t[3 * JL_TILE] = xn * t[JL_TILE];
+      });
+}
+
+// lsolvek (samodel2d.f:1347-1385, komegasst.f:1478-1518) of the systems a, b,
+// c, s along the line at column j, one thread per line: x replaces s.  The
+// line is walked in chunks whose loads are issued one chunk ahead.  Lanes are
+// neighbouring columns, so the loads coalesce; a warp per SM leaves nothing
+// to hide them, which is why the chunks are long and what follows the solve
+// (updates of the state) is a kernel over the cells.
+template <class R>
+__device__ void tri_solve_k(const R* a, const R* b, R* c, R* s, int jd, int ks, int ke, int j) {
+  constexpr int U = sizeof(R) == 4 ? 16 : 8;
+  R sp = (R)0, cp = (R)0;
+  {
+    R na[U], nb[U], nc[U], ns[U];
+    auto load = [&](int k0) {
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+        if (k0 + u <= ke) { const int64_t o = at(jd, j, k0 + u); na[u] = a[o]; nb[u] = b[o]; nc[u] = c[o]; ns[u] = s[o]; }
+    };
+    load(ks);
+    for (int k0 = ks; k0 <= ke; k0 += U) {
+      R ra[U], rb[U], rc[U], rs[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) { ra[u] = na[u]; rb[u] = nb[u]; rc[u] = nc[u]; rs[u] = ns[u]; }
+      if (k0 == ks) ra[0] = (R)0;
+      if (k0 + U <= ke) load(k0 + U);
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+        if (k0 + u <= ke) {
+          const int64_t o = at(jd, j, k0 + u);
+          const R bb = (R)1. / (rb[u] - ra[u] * cp);
+          sp = (rs[u] - ra[u] * sp) * bb;
+          cp = rc[u] * bb;
+          s[o] = sp;
+          c[o] = cp;
+        }
+    }
+  }
+  R nc[U], ns[U], x = sp;
+  auto load = [&](int k0) {   // rows k0, k0-1, ...
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (k0 - u >= ks) { const int64_t o = at(jd, j, k0 - u); nc[u] = c[o]; ns[u] = s[o]; }
+  };
+  load(ke);
+  for (int k0 = ke; k0 >= ks; k0 -= U) {
+    R rc[U], rs[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) { rc[u] = nc[u]; rs[u] = ns[u]; }
+    if (k0 - U >= ks) load(k0 - U);
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (k0 - u >= ks) {
+        if (k0 - u < ke) x = rs[u] - rc[u] * x;
+        s[at(jd, j, k0 - u)] = x;
+      }
+  }
+}
+
 }  // namespace ot2d

@@ -5,6 +5,7 @@
 // the reference's order, so each band entry carries the same bits.
 #pragma once
 #include "dev_common.cuh"
+#include "k_lines.cuh"
 
 namespace ot2d {
 
@@ -225,301 +226,54 @@ __device__ void sa_rhs_cell(const Slice<R>& S, const ot2d_params& p, int j, int 
   S.w[W_BJ * ws + o] = (R)1. + (bj + bk) * tscal;
 }
 
-// lsolvej (samodel2d.f:1306-1344) on one k-line, then s1 = x,
-// sjmat = (s1 - s2)*bjmat with s2 = 0 (samodel2d.f:150-153)
+// The update after the line solves: s2 = x, q5 = max(q5 + x*max(iblank,0),
+// 1e-20) (samodel2d.f:184-188) in FP64 and c_turm of the cell
+// (samodel2d.f:193; the second turbc only changes halo cells, so mu_t here
+// equals the reference's).  Interior cells.
 template <class R>
-__device__ void sa_lsolvej_line(const Slice<R>& S, const ot2d_params& p, int k) {
-  const int jd = S.jd; const int64_t ws = S.wstride;
-  R* a = S.w + W_AJ * ws; R* c = S.w + W_CJ * ws; R* s = S.w + W_SJ * ws; const R* b = S.w + W_BJ * ws;
-  const int js = p.jbeg, je = p.jend;
-  int64_t o = at(jd, js, k);
-  R bb = (R)1. / b[o];
-  R sp = s[o] * bb, cp = c[o] * bb;
-  s[o] = sp; c[o] = cp;
-  for (int j = js + 1; j <= je; ++j) {
-    o = at(jd, j, k);
-    bb = (R)1. / (b[o] - a[o] * cp);
-    sp = (s[o] - a[o] * sp) * bb;
-    cp = c[o] * bb;
-    s[o] = sp; c[o] = cp;
-  }
-  R snext = sp;
-  s[o] = ((snext + (R)0.) - (R)0.) * b[o];
-  for (int j = je - 1; j >= js; --j) {
-    o = at(jd, j, k);
-    R x = s[o] - c[o] * snext;
-    snext = x;
-    s[o] = ((x + (R)0.) - (R)0.) * b[o];
-  }
-}
-
-// lsolvej for 32 consecutive k-lines by a CTA of two warps.  The lines run
-// along j, the fast index of the arrays, so 32 x 32 tiles are staged
-// through shared memory (one row of a tile per copy, then one line per
-// lane).  Warp 0 eliminates: lane l walks line kline0+l through the tile
-// with the arithmetic of sa_lsolvej_line, in its order, and reads and
-// writes only shared memory.  Warp 1 moves the data through three buffers:
-// while warp 0 works on tile t it stores the results of tile t-1 and
-// fetches tile t+2 (cp.async) into that buffer, so the recurrence neither
-// waits on global memory nor spends its issue slots on copies.  The two
-// warps meet at one named barrier per tile.
-// smem: LJ_SMEM elements of R.
-constexpr int LJ_TILE = 32 * 33;
-constexpr int LJ_NBUF = 3;
-constexpr int LJ_SMEM = LJ_NBUF * 4 * LJ_TILE;
-constexpr int LJ_THREADS = 64;
-
-template <class R>
-__device__ __forceinline__ void lj_cp_async(R* dst, const R* src) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], %2;\n" ::"r"((uint32_t)__cvta_generic_to_shared(dst)),
-               "l"(src), "n"((int)sizeof(R)));
-}
-__device__ __forceinline__ void lj_commit() { asm volatile("cp.async.commit_group;\n" ::); }
-template <int N>
-__device__ __forceinline__ void lj_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
-// the two warps of the CTA meet (named barrier 1, 64 threads)
-__device__ __forceinline__ void lj_meet() { asm volatile("bar.sync 1, 64;" ::: "memory"); }
-
-// The bands are the scratch slots sa, sb, sc, ss.  SAOUT: the result is
-// ((x + 0) - 0) * b as vmu_sa forms it (samodel2d.f:150-153); otherwise
-// x * b as komegasst does (komegasst.f:134-139).
-template <class R, bool SAOUT = true>
-__device__ void sa_lsolvej_group(const Slice<R>& S, const ot2d_params& p, int kline0, R* sm, int sa = W_AJ,
-                                 int sb = W_BJ, int sc = W_CJ, int ss = W_SJ) {
-  const int lane = threadIdx.x & 31;
-  const bool mover = (threadIdx.x >> 5) == 1;
-  const int jd = S.jd; const int64_t ws = S.wstride;
-  const R* ga = S.w + sa * ws; R* gc = S.w + sc * ws; R* gs = S.w + ss * ws; const R* gb = S.w + sb * ws;
-  const int js = p.jbeg, je = p.jend, ks = p.kbeg, ke = p.kend;
-  const int ntile = (je - js + 1 + 31) / 32;
-  const bool mine = ks + kline0 + lane <= ke;
-  // buffer b of array m: sm + (b*4 + m)*LJ_TILE; element (row r, column c) at r*33 + c
-  auto buf = [&](int b, int m) { return sm + (b * 4 + m) * LJ_TILE; };
-  // mover: issue the copies of tile t (columns j0..j0+31) of {a,} b, c, s
-  // into buffer b as one cp.async group.  Each lane copies column lane of
-  // every row, the same elements it stores below.
-  auto fetch = [&](int t, int b, bool fwd) {
-    const int j = js + 32 * t + lane;
-    for (int r = 0; r < 32; ++r) {
-      const int kr = ks + kline0 + r;
-      if (kr <= ke && j <= je) {
-        const int64_t o = at(jd, j, kr);
-        if (fwd) lj_cp_async(buf(b, 0) + r * 33 + lane, ga + o);
-        lj_cp_async(buf(b, 1) + r * 33 + lane, gb + o);
-        lj_cp_async(buf(b, 2) + r * 33 + lane, gc + o);
-        lj_cp_async(buf(b, 3) + r * 33 + lane, gs + o);
-      }
-    }
-    lj_commit();
-  };
-  // mover: store tile t's results from buffer b (forward: c and s; backward: s)
-  auto store = [&](int t, int b, bool fwd) {
-    const int j = js + 32 * t + lane;
-    const R *Cm = buf(b, 2), *Sm = buf(b, 3);
-    for (int r = 0; r < 32; ++r) {
-      const int kr = ks + kline0 + r;
-      if (kr <= ke && j <= je) {
-        const int64_t o = at(jd, j, kr);
-        if (fwd) gc[o] = Cm[r * 33 + lane];
-        gs[o] = Sm[r * 33 + lane];
-      }
-    }
-  };
-  // ---- forward elimination.  Round t: warp 0 eliminates tile t (buffer
-  // t%3); warp 1 stores tile t-1 and then fetches tile t+2 into the buffer
-  // tile t-1 used (the stores read it before the copies overwrite it), and
-  // waits for tile t+1.
-  R cp = (R)0, sp = (R)0;
-  if (mover) {
-    fetch(0, 0, true);
-    if (ntile > 1) { fetch(1, 1, true); lj_wait<1>(); }
-    else lj_wait<0>();
-  }
-  lj_meet();
-  for (int t = 0; t < ntile; ++t) {
-    const int b = t % LJ_NBUF;
-    if (!mover) {
-      if (mine) {
-        const R *A = buf(b, 0), *B = buf(b, 1);
-        R *Cm = buf(b, 2), *Sm = buf(b, 3);
-        const int j0 = js + 32 * t;
-        for (int jj = 0; jj < 32 && j0 + jj <= je; ++jj) {
-          const int i = lane * 33 + jj;
-          R bb;
-          if (j0 + jj == js) { bb = (R)1. / B[i]; sp = Sm[i] * bb; cp = Cm[i] * bb; }
-          else { bb = (R)1. / (B[i] - A[i] * cp); sp = (Sm[i] - A[i] * sp) * bb; cp = Cm[i] * bb; }
-          Sm[i] = sp; Cm[i] = cp;
-        }
-      }
-    } else {
-      const int bf = (t + 2) % LJ_NBUF;   // = (t - 1) % 3
-      if (t >= 1) store(t - 1, bf, true);
-      __syncwarp();
-      if (t + 2 < ntile) { fetch(t + 2, bf, true); lj_wait<1>(); }
-      else lj_wait<0>();
-    }
-    lj_meet();
-  }
-  // ---- back substitution; output x * bjmat (samodel2d.f:150-153).  Round
-  // n (tile t = ntile-1-n, buffer n%3): warp 1 stores tile t+1 and fetches
-  // tile t-2.
-  if (mover) {
-    store(ntile - 1, (ntile - 1) % LJ_NBUF, true);
-    // the stores are read back below by the same lanes (same element ->
-    // lane mapping); order them before the asynchronous copies
-    __threadfence_block();
-    fetch(ntile - 1, 0, false);
-    if (ntile > 1) { fetch(ntile - 2, 1, false); lj_wait<1>(); }
-    else lj_wait<0>();
-  }
-  lj_meet();
-  R snext = sp;
-  for (int t = ntile - 1, n = 0; t >= 0; --t, ++n) {
-    const int b = n % LJ_NBUF;
-    if (!mover) {
-      if (mine) {
-        const R *B = buf(b, 1), *Cm = buf(b, 2);
-        R* Sm = buf(b, 3);
-        const int j0 = js + 32 * t;
-        const int jjmax = (je - j0 < 31) ? je - j0 : 31;
-        for (int jj = jjmax; jj >= 0; --jj) {
-          const int i = lane * 33 + jj;
-          R x = (j0 + jj == je) ? Sm[i] : Sm[i] - Cm[i] * snext;
-          snext = x;
-          if constexpr (SAOUT) Sm[i] = ((x + (R)0.) - (R)0.) * B[i];
-          else Sm[i] = x * B[i];
-        }
-      }
-    } else {
-      const int bf = (n + 2) % LJ_NBUF;   // = (n - 1) % 3
-      if (n >= 1) store(t + 1, bf, false);
-      __syncwarp();
-      if (t - 2 >= 0) { fetch(t - 2, bf, false); lj_wait<1>(); }
-      else lj_wait<0>();
-    }
-    lj_meet();
-  }
-  if (mover) store(0, (ntile - 1) % LJ_NBUF, false);
-}
-
-// lsolvek (samodel2d.f:1347-1385) on one j-line, then s2 = x and the
-// update q5 = max(q5 + x*max(iblank,0), 1e-20) (samodel2d.f:184-188) in FP64
-// and c_turm of the cell (samodel2d.f:193; the second turbc only changes
-// halo cells, so mu_t here equals the reference's).  The line is walked in
-// chunks of LK_U cells whose loads are issued one chunk ahead, before the
-// stores of the current chunk, so the recurrence does not wait on memory.
-template <class R>
-__device__ void sa_lsolvek_line(const Slice<R>& S, const ot2d_params& p, int j) {
-  constexpr int LK_U = sizeof(R) == 4 ? 8 : 4;
-  const int jd = S.jd; const int64_t ws = S.wstride, qs = S.qs;
-  R* a = S.w + W_AK * ws; R* c = S.w + W_CK * ws; R* s = S.w + W_SJ * ws; const R* b = S.w + W_BJ * ws;
-  const R* vmul = S.w + W_VMUL * ws;
-  const int ks = p.kbeg, ke = p.kend, n5 = p.nmv + 1;
+__device__ __forceinline__ void sa_update_cell(const Slice<R>& S, const ot2d_params& p, int j, int k) {
+  const int64_t oo = at(S.jd, j, k), qs = S.qs, ws = S.wstride;
+  const int n5 = p.nmv + 1;
   const R cv1 = (R)SAc::cv1;
-  int64_t o = at(jd, j, ks);
-  R bb = (R)1. / b[o];
-  R sp = s[o] * bb, cp = c[o] * bb;
-  s[o] = sp; c[o] = cp;
-  // forward elimination
-  {
-    R na[LK_U], nb[LK_U], nc[LK_U], ns[LK_U];
-    auto load = [&](int k0) {
-#pragma unroll
-      for (int u = 0; u < LK_U; ++u)
-        if (k0 + u <= ke) { const int64_t ou = at(jd, j, k0 + u); na[u] = a[ou]; nb[u] = b[ou]; nc[u] = c[ou]; ns[u] = s[ou]; }
-    };
-    load(ks + 1);
-    for (int k0 = ks + 1; k0 <= ke; k0 += LK_U) {
-      R ra[LK_U], rb[LK_U], rc[LK_U], rs[LK_U];
-#pragma unroll
-      for (int u = 0; u < LK_U; ++u) { ra[u] = na[u]; rb[u] = nb[u]; rc[u] = nc[u]; rs[u] = ns[u]; }
-      if (k0 + LK_U <= ke) load(k0 + LK_U);
-#pragma unroll
-      for (int u = 0; u < LK_U; ++u) {
-        if (k0 + u <= ke) {
-          o = at(jd, j, k0 + u);
-          bb = (R)1. / (rb[u] - ra[u] * cp);
-          sp = (rs[u] - ra[u] * sp) * bb;
-          cp = rc[u] * bb;
-          s[o] = sp; c[o] = cp;
-        }
-      }
-    }
-  }
-  // back substitution + update + mu_t
   double* q5 = S.q64 + (int64_t)(n5 - 1) * qs;
-  R nc[LK_U], ns[LK_U], nq1[LK_U], nJ[LK_U], nvm[LK_U];
-  double nq5[LK_U];
-  int nib[LK_U];
-  auto load = [&](int k0) {  // cells k0, k0-1, ..., k0-LK_U+1
-#pragma unroll
-    for (int u = 0; u < LK_U; ++u)
-      if (k0 - u >= ks) {
-        const int64_t ou = at(jd, j, k0 - u);
-        nc[u] = c[ou]; ns[u] = s[ou]; nq1[u] = S.q[ou]; nJ[u] = S.q[(int64_t)(p.nq - 1) * qs + ou];
-        nvm[u] = vmul[ou]; nq5[u] = q5[ou]; nib[u] = S.iblank[ou];
-      }
-  };
-  auto upd = [&](int64_t oo, R x, double q5o, int ibi, R q1, R J, R vm) {
-    R x2 = (R)0. + x;            // s2 = s2 + sjmat, s2 = 0 on entry
-    R relx = (R)1.0 * x2;        // relfac * sjmat
-    s[oo] = relx;
-    double v;
-    R qv;
-    if constexpr (sizeof(R) == sizeof(double)) {
-      double ib = (double)(ibi > 0 ? ibi : 0);
-      v = q5o + (double)relx * ib;
-      v = (1.0e-20 > v) ? 1.0e-20 : v;
-      qv = (R)v;
-    } else {
-      // The same values with one FP64 operation (GB300's FP64 pipe is
-      // narrow): relx * max(iblank, 0) is exact for iblank 0 (a signed zero,
-      // or NaN for a non-finite relx) and 1, so it is formed in f32 and
-      // widened on the integer pipe; the clamp compares IEEE bit patterns;
-      // the narrowing is the f32 path's round-to-nearest with flush to zero.
-      double dx;
-      if (ibi == 1) dx = f2d_bits_ftz(relx);
-      else if (ibi <= 0) dx = f2d_bits_ftz(relx * 0.0f);
-      else dx = (double)relx * (double)ibi;
-      v = q5o + dx;
-      const uint64_t vb = (uint64_t)__double_as_longlong(v), mag = vb & 0x7fffffffffffffffull;
-      // 1e-20 > v: v negative (not NaN), or positive below 1e-20
-      const bool below = (vb >> 63) ? mag <= 0x7ff0000000000000ull
-                                    : vb < (uint64_t)__double_as_longlong(1.0e-20);
-      if (below) v = 1.0e-20;
-      qv = d2f_bits_rn_ftz(v);
-    }
-    q5[oo] = v;
-    if constexpr (sizeof(R) != sizeof(double)) S.q[(int64_t)(n5 - 1) * qs + oo] = qv;
-    // c_turm (samodel2d.f:372-399) with q5 as just stored
-    const R rhoJ = q1 * J;
-    const R vnul = vm / rhoJ;
-    const R chi = qv / vnul;
-    const R fv1 = cube(chi) / (cube(chi) + cube(cv1));
-    S.turmu[oo] = rhoJ * qv * fv1;
-  };
-  R snext = sp;
-  load(ke);
-  for (int k0 = ke; k0 >= ks; k0 -= LK_U) {
-    R rc[LK_U], rs[LK_U], rq1[LK_U], rJ[LK_U], rvm[LK_U];
-    double rq5[LK_U];
-    int rib[LK_U];
-#pragma unroll
-    for (int u = 0; u < LK_U; ++u) {
-      rc[u] = nc[u]; rs[u] = ns[u]; rq1[u] = nq1[u]; rJ[u] = nJ[u]; rvm[u] = nvm[u]; rq5[u] = nq5[u]; rib[u] = nib[u];
-    }
-    if (k0 - LK_U >= ks) load(k0 - LK_U);
-#pragma unroll
-    for (int u = 0; u < LK_U; ++u) {
-      const int k = k0 - u;
-      if (k >= ks) {
-        o = at(jd, j, k);
-        const R x = (k == ke) ? snext : rs[u] - rc[u] * snext;
-        snext = x;
-        upd(o, x, rq5[u], rib[u], rq1[u], rJ[u], rvm[u]);
-      }
-    }
+  const R x = S.w[W_SJ * ws + oo], q1 = S.q[oo], J = S.q[(int64_t)(p.nq - 1) * qs + oo], vm = S.w[W_VMUL * ws + oo];
+  const double q5o = q5[oo];
+  const int ibi = S.iblank[oo];
+  R x2 = (R)0. + x;            // s2 = s2 + sjmat, s2 = 0 on entry
+  R relx = (R)1.0 * x2;        // relfac * sjmat
+  double v;
+  R qv;
+  if constexpr (sizeof(R) == sizeof(double)) {
+    double ib = (double)(ibi > 0 ? ibi : 0);
+    v = q5o + (double)relx * ib;
+    v = (1.0e-20 > v) ? 1.0e-20 : v;
+    qv = (R)v;
+  } else {
+    // The same values with one FP64 operation (GB300's FP64 pipe is
+    // narrow): relx * max(iblank, 0) is exact for iblank 0 (a signed zero,
+    // or NaN for a non-finite relx) and 1, so it is formed in f32 and
+    // widened on the integer pipe; the clamp compares IEEE bit patterns;
+    // the narrowing is the f32 path's round-to-nearest with flush to zero.
+    double dx;
+    if (ibi == 1) dx = f2d_bits_ftz(relx);
+    else if (ibi <= 0) dx = f2d_bits_ftz(relx * 0.0f);
+    else dx = (double)relx * (double)ibi;
+    v = q5o + dx;
+    const uint64_t vb = (uint64_t)__double_as_longlong(v), mag = vb & 0x7fffffffffffffffull;
+    // 1e-20 > v: v negative (not NaN), or positive below 1e-20
+    const bool below = (vb >> 63) ? mag <= 0x7ff0000000000000ull
+                                  : vb < (uint64_t)__double_as_longlong(1.0e-20);
+    if (below) v = 1.0e-20;
+    qv = d2f_bits_rn_ftz(v);
   }
+  q5[oo] = v;
+  if constexpr (sizeof(R) != sizeof(double)) S.q[(int64_t)(n5 - 1) * qs + oo] = qv;
+  // c_turm (samodel2d.f:372-399) with q5 as just stored
+  const R rhoJ = q1 * J;
+  const R vnul = vm / rhoJ;
+  const R chi = qv / vnul;
+  const R fv1 = cube(chi) / (cube(chi) + cube(cv1));
+  S.turmu[oo] = rhoJ * qv * fv1;
 }
 
 // c_turm, samodel2d.f:372-399 (all cells)

@@ -406,57 +406,30 @@ __device__ void sst_rhs_cell(const Slice<R>& S, const ot2d_params& p, int j, int
   }
 }
 
-// lsolvek2 (komegasst.f:1478-1518) of both equations on one j-line, then
-// the update of :135-152 (s = sjmat, q += s*max(iblank,0), clipped at
-// 1e-20*rho, in FP64) and findturm of the updated cell (:185; the second
-// komegabc changes only halo cells).
+// The update after the line solves (komegasst.f:135-152: s = sjmat, q +=
+// s*max(iblank,0), clipped at 1e-20*rho, in FP64) and findturm of the updated
+// cell (:185; the second komegabc changes only halo cells).  Interior cells.
 template <class R>
-__device__ void sst_lsolvek_line(const Slice<R>& S, const ot2d_params& p, int j) {
-  const int jd = S.jd; const int64_t ws = S.wstride, qs = S.qs;
-  const int ks = p.kbeg, ke = p.kend, nmv = p.nmv;
-  for (int n = 0; n < 2; ++n) {
-    const R* a = S.w + kband(KB_AK, n) * ws; R* c = S.w + kband(KB_CK, n) * ws;
-    const R* b = S.w + kband(KB_BJ, n) * ws; R* sv = S.w + kband(KB_SJ, n) * ws;
-    int64_t o = at(jd, j, ks);
-    R bb = (R)1. / b[o];
-    R sp = sv[o] * bb, cp = c[o] * bb;
-    sv[o] = sp; c[o] = cp;
-    for (int k = ks + 1; k <= ke; ++k) {
-      o = at(jd, j, k);
-      bb = (R)1. / (b[o] - a[o] * cp);
-      sp = (sv[o] - a[o] * sp) * bb;
-      cp = c[o] * bb;
-      sv[o] = sp; c[o] = cp;
-    }
-    R snext = sp;
-    for (int k = ke - 1; k >= ks; --k) {
-      o = at(jd, j, k);
-      const R x = sv[o] - c[o] * snext;
-      sv[o] = x;
-      snext = x;
-    }
-  }
-  const R* s0 = S.w + kband(KB_SJ, 0) * ws; const R* s1 = S.w + kband(KB_SJ, 1) * ws;
+__device__ __forceinline__ void sst_update_cell(const Slice<R>& S, const ot2d_params& p, int j, int k) {
+  const int64_t ws = S.wstride, qs = S.qs, o = at(S.jd, j, k);
+  const int nmv = p.nmv;
   double* q5 = S.q64 + (int64_t)nmv * qs; double* q6 = S.q64 + (int64_t)(nmv + 1) * qs;
   const double tkelim = 1e-20, tomegalim = 1e-20, relfac = 1.;
-  for (int k = ks; k <= ke; ++k) {
-    const int64_t o = at(jd, j, k);
-    const R r5 = (R)relfac * s0[o], r6 = (R)relfac * s1[o];
-    S.s[(int64_t)nmv * qs + o] = r5;
-    S.s[(int64_t)(nmv + 1) * qs + o] = r6;
-    const int ibi = S.iblank[o];
-    const double ib = (double)(ibi > 0 ? ibi : 0);
-    const double rho = (double)S.w[K_RHO * ws + o];
-    double v5 = q5[o] + (double)r5 * ib, v6 = q6[o] + (double)r6 * ib;
-    v5 = fmax2(v5, tkelim * rho);
-    v6 = fmax2(v6, tomegalim * rho);
-    q5[o] = v5; q6[o] = v6;
-    if constexpr (sizeof(R) != sizeof(double)) {
-      S.q[(int64_t)nmv * qs + o] = (R)v5;
-      S.q[(int64_t)(nmv + 1) * qs + o] = (R)v6;
-    }
-    S.turmu[o] = sst_turm(p, (R)rho, (R)v5, (R)v6, S.w[K_STRAIN * ws + o], S.w[K_F2 * ws + o]);
+  const R r5 = (R)relfac * S.w[kband(KB_SJ, 0) * ws + o], r6 = (R)relfac * S.w[kband(KB_SJ, 1) * ws + o];
+  S.s[(int64_t)nmv * qs + o] = r5;
+  S.s[(int64_t)(nmv + 1) * qs + o] = r6;
+  const int ibi = S.iblank[o];
+  const double ib = (double)(ibi > 0 ? ibi : 0);
+  const double rho = (double)S.w[K_RHO * ws + o];
+  double v5 = q5[o] + (double)r5 * ib, v6 = q6[o] + (double)r6 * ib;
+  v5 = fmax2(v5, tkelim * rho);
+  v6 = fmax2(v6, tomegalim * rho);
+  q5[o] = v5; q6[o] = v6;
+  if constexpr (sizeof(R) != sizeof(double)) {
+    S.q[(int64_t)nmv * qs + o] = (R)v5;
+    S.q[(int64_t)(nmv + 1) * qs + o] = (R)v6;
   }
+  S.turmu[o] = sst_turm(p, (R)rho, (R)v5, (R)v6, S.w[K_STRAIN * ws + o], S.w[K_F2 * ws + o]);
 }
 
 }  // namespace ot2d

@@ -553,33 +553,54 @@ __host__ __device__ constexpr size_t sa_rhs_smem() {
   return sizeof(R) * (size_t)SA_NST * (TJ + 2) * (TK + 2);
 }
 
-// line solves: slice i owns lines [lfirst[i], lfirst[i+1]) (one thread each)
+// lsolvej by CTAs of 32 k-lines; slice i owns groups [gfirst[i], gfirst[i+1])
 template <class R>
-__global__ void k_sa_lsolve(const Slice<R>* __restrict__ sl, const int32_t* __restrict__ lfirst, int nslice, int dir) {
-  const int gid = blockIdx.x * blockDim.x + threadIdx.x;
-  if (gid >= lfirst[nslice]) return;
-  int lo = 0, hi = nslice - 1;
-  while (lo < hi) { int mid = (lo + hi + 1) >> 1; if (lfirst[mid] <= gid) lo = mid; else hi = mid - 1; }
-  const Slice<R>& S = sl[lo];
-  const ot2d_params& p = *S.P;
-  if (p.lamin || p.iturb != 1) return;
-  const int line = gid - lfirst[lo];
-  if (dir == 0) { int k = p.kbeg + line; if (k <= p.kend) sa_lsolvej_line(S, p, k); }
-  else { int j = p.jbeg + line; if (j <= p.jend) sa_lsolvek_line(S, p, j); }
-}
-
-// lsolvej by CTAs of 32 k-lines (two warps: elimination and data
-// movement); slice i owns groups [gfirst[i], gfirst[i+1])
-template <class R>
-__global__ void __launch_bounds__(LJ_THREADS) k_sa_lsolvej(const Slice<R>* __restrict__ sl, const int32_t* __restrict__ gfirst,
-                                                   int nslice) {
-  extern __shared__ __align__(16) unsigned char lj_raw[];
-  R* sm = (R*)lj_raw;   // LJ_SMEM elements
+__global__ void __launch_bounds__(JL_THREADS) k_sa_lsolvej(const Slice<R>* __restrict__ sl,
+                                                           const int32_t* __restrict__ gfirst, int nslice) {
+  extern __shared__ __align__(16) unsigned char jl_raw[];
   const int si = find_slice(gfirst, nslice, blockIdx.x);
   const Slice<R>& S = sl[si];
   const ot2d_params& p = *S.P;
   if (p.lamin || p.iturb != 1) return;
-  sa_lsolvej_group(S, p, 32 * (blockIdx.x - gfirst[si]), sm);
+  const int k0 = p.kbeg + 32 * (blockIdx.x - gfirst[si]);
+  const int64_t ws = S.wstride;
+  tri_solve_j<R, true>(S.w + W_AJ * ws, S.w + W_BJ * ws, S.w + W_CJ * ws, S.w + W_SJ * ws, S.jd, p.jbeg, p.jend, k0,
+                       min(32, p.kend - k0 + 1), (R*)jl_raw);
+}
+// slice and line of a thread of the k-line solves (one thread per j-line;
+// slice i owns lines [lfirst[i], lfirst[i+1]))
+__device__ __forceinline__ bool k_line_of(const int32_t* lfirst, int nslice, int& si, int& line) {
+  const int gid = blockIdx.x * blockDim.x + threadIdx.x;
+  if (gid >= lfirst[nslice]) return false;
+  int lo = 0, hi = nslice - 1;
+  while (lo < hi) { int mid = (lo + hi + 1) >> 1; if (lfirst[mid] <= gid) lo = mid; else hi = mid - 1; }
+  si = lo; line = gid - lfirst[lo];
+  return true;
+}
+template <class R>
+__global__ void __launch_bounds__(32) k_sa_lsolvek(const Slice<R>* __restrict__ sl, const int32_t* __restrict__ lfirst,
+                                                   int nslice) {
+  int si, line;
+  if (!k_line_of(lfirst, nslice, si, line)) return;
+  const Slice<R>& S = sl[si];
+  const ot2d_params& p = *S.P;
+  if (p.lamin || p.iturb != 1 || p.jbeg + line > p.jend) return;
+  const int64_t ws = S.wstride;
+  tri_solve_k(S.w + W_AK * ws, S.w + W_BJ * ws, S.w + W_CK * ws, S.w + W_SJ * ws, S.jd, p.kbeg, p.kend, p.jbeg + line);
+}
+// the nu_tilde update and mu_t of the interior cells
+template <class R>
+__global__ void __launch_bounds__(CELL_BS / CELL_PT) k_sa_update(const Slice<R>* __restrict__ sl,
+                                                                 const int32_t* __restrict__ first, int nslice) {
+  OT2D_CELL_MAP_PT();
+  const ot2d_params& p = *S.P;
+  if (p.lamin || p.iturb != 1) return;
+#pragma unroll
+  for (int u = 0; u < CELL_PT; ++u) {
+    const int cid = cid0 + u * (CELL_BS / CELL_PT);
+    const int j = cid % S.jd + 1, k = cid / S.jd + 1;
+    if (cid < ncell && j >= p.jbeg && j <= p.jend && k >= p.kbeg && k <= p.kend) sa_update_cell(S, p, j, k);
+  }
 }
 
 // ---- k-omega SST (komegasst.f:2-187) ---------------------------------------
@@ -642,33 +663,43 @@ __global__ void __launch_bounds__(CELL_BS) k_sst_rhs(const Slice<R>* __restrict_
   sst_rhs_cell(S, p, j, k);
 }
 
-// lsolvej2 of equation blockIdx.y by warps of 32 k-lines; output x * bjmat
+// lsolvej2 by CTAs of 32 k-lines, blockIdx.y = equation
 template <class R>
-__global__ void __launch_bounds__(LJ_THREADS) k_sst_lsolvej(const Slice<R>* __restrict__ sl, const int32_t* __restrict__ gfirst,
-                                                    int nslice) {
-  extern __shared__ __align__(16) unsigned char lj_raw[];
-  R* sm = (R*)lj_raw;   // LJ_SMEM elements
+__global__ void __launch_bounds__(JL_THREADS) k_sst_lsolvej(const Slice<R>* __restrict__ sl,
+                                                            const int32_t* __restrict__ gfirst, int nslice) {
+  extern __shared__ __align__(16) unsigned char jl_raw[];
   const int si = find_slice(gfirst, nslice, blockIdx.x);
   const Slice<R>& S = sl[si];
   const ot2d_params& p = *S.P;
   if (!sst_slice(p)) return;
-  const int n = blockIdx.y;
-  sa_lsolvej_group<R, false>(S, p, 32 * (blockIdx.x - gfirst[si]), sm, kband(KB_AJ, n), kband(KB_BJ, n),
-                             kband(KB_CJ, n), kband(KB_SJ, n));
+  const int n = blockIdx.y, k0 = p.kbeg + 32 * (blockIdx.x - gfirst[si]);
+  const int64_t ws = S.wstride;
+  tri_solve_j<R, false>(S.w + kband(KB_AJ, n) * ws, S.w + kband(KB_BJ, n) * ws, S.w + kband(KB_CJ, n) * ws,
+                        S.w + kband(KB_SJ, n) * ws, S.jd, p.jbeg, p.jend, k0, min(32, p.kend - k0 + 1), (R*)jl_raw);
 }
-
-// lsolvek2 + update + findturm, one thread per j-line
+// lsolvek2, one thread per j-line, blockIdx.y = equation
 template <class R>
-__global__ void k_sst_lsolvek(const Slice<R>* __restrict__ sl, const int32_t* __restrict__ lfirst, int nslice) {
-  const int gid = blockIdx.x * blockDim.x + threadIdx.x;
-  if (gid >= lfirst[nslice]) return;
-  int lo = 0, hi = nslice - 1;
-  while (lo < hi) { int mid = (lo + hi + 1) >> 1; if (lfirst[mid] <= gid) lo = mid; else hi = mid - 1; }
-  const Slice<R>& S = sl[lo];
+__global__ void __launch_bounds__(32) k_sst_lsolvek(const Slice<R>* __restrict__ sl, const int32_t* __restrict__ lfirst,
+                                                    int nslice) {
+  int si, line;
+  if (!k_line_of(lfirst, nslice, si, line)) return;
+  const Slice<R>& S = sl[si];
   const ot2d_params& p = *S.P;
-  if (!sst_slice(p)) return;
-  const int j = p.jbeg + gid - lfirst[lo];
-  if (j <= p.jend) sst_lsolvek_line(S, p, j);
+  if (!sst_slice(p) || p.jbeg + line > p.jend) return;
+  const int n = blockIdx.y;
+  const int64_t ws = S.wstride;
+  tri_solve_k(S.w + kband(KB_AK, n) * ws, S.w + kband(KB_BJ, n) * ws, S.w + kband(KB_CK, n) * ws,
+              S.w + kband(KB_SJ, n) * ws, S.jd, p.kbeg, p.kend, p.jbeg + line);
+}
+// the update of k and omega and mu_t of the interior cells
+template <class R>
+__global__ void __launch_bounds__(CELL_BS) k_sst_update(const Slice<R>* __restrict__ sl,
+                                                        const int32_t* __restrict__ first, int nslice) {
+  OT2D_CELL_MAP();
+  if (!inside) return;
+  const ot2d_params& p = *S.P;
+  if (!sst_slice(p) || j < p.jbeg || j > p.jend || k < p.kbeg || k > p.kend) return;
+  sst_update_cell(S, p, j, k);
 }
 
 // ---- ADI operator arc2d (lhs.f:817-1057), ilhs = 2 ------------------------

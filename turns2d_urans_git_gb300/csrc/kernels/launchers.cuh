@@ -238,14 +238,15 @@ cudaError_t launch_sa(const Slice<R>* d_sl, const Batch& b, cudaStream_t st, int
     case 3: k_sa_rhs<R, 32, 16><<<b.tile_blocks, 512, sa_rhs_smem<R, 32, 16>(), st>>>(d_sl, b.d_tfirst, b.nslice); break;
     default: k_sa_rhs<R, 16, 16><<<b.tile_blocks, 256, sa_rhs_smem<R, 16, 16>(), st>>>(d_sl, b.d_tfirst, b.nslice);
   }
-  constexpr size_t lj_smem = sizeof(R) * LJ_SMEM;
+  constexpr size_t jl_smem = sizeof(R) * jl_smem_elems(4);
   static DeviceOnce once;
   cudaError_t ae = once.run([&](int&) {
-    return cudaFuncSetAttribute(k_sa_lsolvej<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lj_smem);
+    return cudaFuncSetAttribute(k_sa_lsolvej<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)jl_smem);
   });
   if (ae != cudaSuccess) return ae;
-  k_sa_lsolvej<R><<<b.jgroups, LJ_THREADS, lj_smem, st>>>(d_sl, b.d_gfirst, b.nslice);
-  k_sa_lsolve<R><<<(b.klines + 63) / 64, 64, 0, st>>>(d_sl, b.d_kfirst, b.nslice, 1);
+  k_sa_lsolvej<R><<<b.jgroups, JL_THREADS, jl_smem, st>>>(d_sl, b.d_gfirst, b.nslice);
+  k_sa_lsolvek<R><<<(b.klines + 31) / 32, 32, 0, st>>>(d_sl, b.d_kfirst, b.nslice);
+  k_sa_update<R><<<b.cell_blocks, CELL_BS / CELL_PT, 0, st>>>(d_sl, b.d_first, b.nslice);
   if (final_bc) k_turbc<R><<<b.nslice, BC_BS, 0, st>>>(d_sl);
   return cudaGetLastError();
 }
@@ -263,14 +264,15 @@ cudaError_t launch_sst(const Slice<R>* d_sl, const Batch& b, cudaStream_t st) {
   k_sst_fields<R><<<b.cell_blocks, CELL_BS, 0, st>>>(d_sl, b.d_first, b.nslice);
   k_sst_turm<R><<<b.cell_blocks, CELL_BS, 0, st>>>(d_sl, b.d_first, b.nslice);
   k_sst_rhs<R><<<b.cell_blocks, CELL_BS, 0, st>>>(d_sl, b.d_first, b.nslice);
-  constexpr size_t lj_smem = sizeof(R) * LJ_SMEM;
+  constexpr size_t jl_smem = sizeof(R) * jl_smem_elems(4);
   static DeviceOnce once;
   cudaError_t ae = once.run([&](int&) {
-    return cudaFuncSetAttribute(k_sst_lsolvej<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lj_smem);
+    return cudaFuncSetAttribute(k_sst_lsolvej<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)jl_smem);
   });
   if (ae != cudaSuccess) return ae;
-  k_sst_lsolvej<R><<<dim3(b.jgroups, 2), LJ_THREADS, lj_smem, st>>>(d_sl, b.d_gfirst, b.nslice);
-  k_sst_lsolvek<R><<<(b.klines + 63) / 64, 64, 0, st>>>(d_sl, b.d_kfirst, b.nslice);
+  k_sst_lsolvej<R><<<dim3(b.jgroups, 2), JL_THREADS, jl_smem, st>>>(d_sl, b.d_gfirst, b.nslice);
+  k_sst_lsolvek<R><<<dim3((b.klines + 31) / 32, 2), 32, 0, st>>>(d_sl, b.d_kfirst, b.nslice);
+  k_sst_update<R><<<b.cell_blocks, CELL_BS, 0, st>>>(d_sl, b.d_first, b.nslice);
   k_sst_bc<R><<<b.nslice, 256, 0, st>>>(d_sl, 1);
   return cudaGetLastError();
 }

@@ -8,6 +8,7 @@
 #include <cstdint>
 #include <cuda_runtime.h>
 #include "ot2d_params.h"
+#include "soft64.h"
 
 namespace ot2d {
 
@@ -160,7 +161,13 @@ template <class R> __device__ __forceinline__ R fmin2(R a, R b) { return (b < a)
 template <class R> __device__ __forceinline__ R sq(R x) { return x * x; }
 template <class R> __device__ __forceinline__ R cube(R x) { return (x * x) * x; }
 template <class R> __device__ __forceinline__ R pow6(R x) { R t = (x * x) * x; return t * t; }
-__device__ __forceinline__ double rsqrt_(double x) { return sqrt(x); }
+// a / by(b) and root(x): FP64 on the integer pipe (soft64.h), f32 as written
+struct Den64 { double v; };
+__device__ __forceinline__ Den64 by(double b) { return {b}; }
+__device__ __forceinline__ float by(float b) { return b; }
+__device__ __forceinline__ double operator/(double a, Den64 b) { return soft64::div(a, b.v); }
+__device__ __forceinline__ double root(double x) { return soft64::sqrt_rn(x); }
+__device__ __forceinline__ float root(float x) { return sqrt(x); }
 
 // exact widening to double
 __device__ __forceinline__ double to_d(float x) { return (double)x; }

@@ -39,7 +39,7 @@ __device__ __forceinline__ int64_t adi_at(int jd, int dir, int m, int n) { retur
 template <class R>
 __device__ __forceinline__ R adi_bsq(const Slice<R>& S, int64_t o) {
   const R btv = S.bt ? S.bt[o] : (R)1.;
-  return S.k_mp2 / (btv - S.k_mp2 * (btv - (R)1));
+  return S.k_mp2 / by(btv - S.k_mp2 * (btv - (R)1));
 }
 
 // s *= tscale when `scale` (step.f:141-148), primitive variables (:853-860) and the
@@ -50,7 +50,7 @@ __device__ void adi_txi_cell(const Slice<R>& S, const ot2d_params& p, int j, int
   const int64_t o = at(S.jd, j, k), qs = S.qs, ws = S.wstride;
   const R gm1 = S.k_gm1, ggm1 = S.k_ggm1;
   const R q1 = S.q[o], J = S.q[(p.nq - 1) * qs + o];
-  const R dj = (R)1.0 / q1;
+  const R dj = (R)1.0 / by(q1);
   const R uu = S.q[qs + o] * dj, vv = S.q[2 * qs + o] * dj, e = S.q[3 * qs + o] * dj;
   const R rho = q1 * J;
   R s1 = S.s[o], s2 = S.s[qs + o], s3 = S.s[2 * qs + o], s4 = S.s[3 * qs + o];
@@ -59,8 +59,8 @@ __device__ void adi_txi_cell(const Slice<R>& S, const ot2d_params& p, int j, int
     s1 = s1 * ts; s2 = s2 * ts; s3 = s3 * ts; s4 = s4 * ts;
   }
   const R uv2 = (R)0.5 * (uu * uu + vv * vv);
-  const R cjkl = sqrt(ggm1 * (e - uv2));
-  const R c2i = (R)1.0 / (cjkl * cjkl);
+  const R cjkl = root(ggm1 * (e - uv2));
+  const R c2i = (R)1.0 / by(cjkl * cjkl);
   S.w[A_P * ws + o] = (e - uv2) * gm1 * rho;
   R rj1 = S.xx[o], rj2 = S.xy[o];
   const R ugc = S.ug ? S.ug[o] : (R)0, vgc = S.vg ? S.vg[o] : (R)0;
@@ -69,8 +69,8 @@ __device__ void adi_txi_cell(const Slice<R>& S, const ot2d_params& p, int j, int
   const bool pre = S.k_mp2 >= (R)0;
   const R qq1 = pre ? rj1 * (uu - ugc) + rj2 * (vv - vgc) : rj1 * uu + rj2 * vv;
   S.w[A_QX * ws + o] = pre ? qq1 : qq1 - (rj1 * ugc + rj2 * vgc);
-  const R rr1 = sqrt(sq(rj1) + sq(rj2));
-  rj1 = rj1 / rr1; rj2 = rj2 / rr1;
+  const R rr1 = root(sq(rj1) + sq(rj2));
+  rj1 = rj1 / by(rr1); rj2 = rj2 / by(rr1);
   const R rk1 = S.yx[o], rk2 = S.yy[o];
   if (pre) {
     S.w[A_QY * ws + o] = rk1 * (uu - ugc) + rk2 * (vv - vgc);
@@ -78,11 +78,11 @@ __device__ void adi_txi_cell(const Slice<R>& S, const ot2d_params& p, int j, int
     const R qq2 = rk1 * uu + rk2 * vv;
     S.w[A_QY * ws + o] = qq2 - (rk1 * ugc + rk2 * vgc);
   }
-  const R rr2 = sqrt(sq(rk1) + sq(rk2));
+  const R rr2 = root(sq(rk1) + sq(rk2));
   S.w[A_UV * ws + o] = uv2;
   S.w[A_CX * ws + o] = cjkl * rr1;
   S.w[A_CY * ws + o] = cjkl * rr2;
-  S.w[A_VN * ws + o] = (S.k_rmue + S.turmu[o]) / (S.k_rey * rho);
+  S.w[A_VN * ws + o] = (S.k_rmue + S.turmu[o]) / by(S.k_rey * rho);
   S.w[A_GE * ws + o] = S.k_gamma * e - gm1 * uv2;
   S.w[A_U * ws + o] = uu; S.w[A_V * ws + o] = vv; S.w[A_E * ws + o] = e;
   R a1 = s2 * uu + s3 * vv - s4;
@@ -97,19 +97,19 @@ __device__ void adi_txi_cell(const Slice<R>& S, const ot2d_params& p, int j, int
     // arc2d_precon :1141-1164: the preconditioned acoustic eigenvectors
     const R bSq = adi_bsq(S, o), omb = (R)1. - bSq;
     const R cx = cjkl * rr1;
-    const R X = sqrt((omb * qq1) * (omb * qq1) + (R)4. * bSq * cx * cx) / rr1;
-    const R Y = (R)0.5 * (omb * qq1 / rr1 + X);
-    const R Z = (R)0.5 * (omb * qq1 / rr1 - X);
+    const R X = root((omb * qq1) * (omb * qq1) + (R)4. * bSq * cx * cx) / by(rr1);
+    const R Y = (R)0.5 * (omb * qq1 / by(rr1) + X);
+    const R Z = (R)0.5 * (omb * qq1 / by(rr1) - X);
     const R qqmxt = qq1 + ugc * rj1 * rr1 + vgc * rj2 * rr1;
-    R a4 = qqmxt * s1 / rr1 - rj1 * s2 - rj2 * s3;
+    R a4 = qqmxt * s1 / by(rr1) - rj1 * s2 - rj2 * s3;
     a4 = a4 * bSq;
-    S.s[2 * qs + o] = -(Z * a3 + a4) / X;
-    S.s[3 * qs + o] = (Y * a3 + a4) / X;
+    S.s[2 * qs + o] = -(Z * a3 + a4) / by(X);
+    S.s[3 * qs + o] = (Y * a3 + a4) / by(X);
     return;
   }
-  const R a4 = qq1 * s1 / rr1 - rj1 * s2 - rj2 * s3;
-  S.s[2 * qs + o] = (R)0.5 * (a3 - a4 / cjkl);
-  S.s[3 * qs + o] = (R)0.5 * (a3 + a4 / cjkl);
+  const R a4 = qq1 * s1 / by(rr1) - rj1 * s2 - rj2 * s3;
+  S.s[2 * qs + o] = (R)0.5 * (a3 - a4 / by(cjkl));
+  S.s[3 * qs + o] = (R)0.5 * (a3 + a4 / by(cjkl));
 }
 
 // spectral-radius diagonal of lhsinv (:1587-1596): d[0] = diag(m,1) =
@@ -119,13 +119,13 @@ __device__ __forceinline__ void adi_diag(const Slice<R>& S, const ot2d_params& p
   const int64_t ws = S.wstride;
   const R Mp = (R)p.Mp;
   const R btv = S.bt ? S.bt[o] : (R)1.;
-  const R bSq = (Mp * Mp) / (btv - (Mp * Mp) * (btv - (R)1));
+  const R bSq = (Mp * Mp) / by(btv - (Mp * Mp) * (btv - (R)1));
   const R qv = S.w[(dir == 0 ? A_QX : A_QY) * ws + o], cv = S.w[(dir == 0 ? A_CX : A_CY) * ws + o];
-  const R X = sqrt(((R)1. - bSq) * qv * (((R)1. - bSq) * qv) + (R)4. * bSq * cv * cv);
+  const R X = root(((R)1. - bSq) * qv * (((R)1. - bSq) * qv) + (R)4. * bSq * cv * cv);
   d[0] = qv;
   d[1] = (R)0.5 * ((bSq + (R)1.) * qv + X);
   d[2] = (R)0.5 * ((bSq + (R)1.) * qv - X);
-  d[3] = (R)0.5 * ((bSq + (R)1.) * fabs(qv) + X) / S.q[(int64_t)(p.nq - 1) * S.qs + o];
+  d[3] = (R)0.5 * ((bSq + (R)1.) * fabs(qv) + X) / by(S.q[(int64_t)(p.nq - 1) * S.qs + o]);
 }
 
 // pressure switch of line direction dir (:919-935, :977-993): interior of
@@ -139,7 +139,7 @@ __device__ __forceinline__ void adi_d2p_cell(const Slice<R>& S, const ot2d_param
   if (m > ms && m < me) {
     const R pp = P[adi_at(jd, dir, m + 1, n)], pc = P[adi_at(jd, dir, m, n)], pm = P[adi_at(jd, dir, m - 1, n)];
     v = fabs(pp - (R)2. * pc + pm);
-    v = v / fabs(pp + (R)2. * pc + pm);
+    v = v / by(fabs(pp + (R)2. * pc + pm));
   }
   const int64_t o = adi_at(jd, dir, m, n);
   S.w[A_D2P * ws + o] = v;
@@ -241,11 +241,11 @@ __device__ __forceinline__ AdiRow<R> adi_row(const Slice<R>& S, const ot2d_param
     const R* Jq = S.q + (int64_t)(p.nq - 1) * qs;
     const int64_t op = adi_at(jd, dir, m + 1, n), om = adi_at(jd, dir, m - 1, n);
     const R vnu = S.w[A_VN * ws + o];
-    v1 = (xn[o] * xn[o] + yn[o] * yn[o]) / Jq[o];
-    v1 = v1 + (xn[op] * xn[op] + yn[op] * yn[op]) / Jq[op];
+    v1 = (xn[o] * xn[o] + yn[o] * yn[o]) / by(Jq[o]);
+    v1 = v1 + (xn[op] * xn[op] + yn[op] * yn[op]) / by(Jq[op]);
     v1 = v1 * Jq[o] * vnu;
-    v3 = (xn[o] * xn[o] + yn[o] * yn[o]) / Jq[o];
-    v3 = v3 + (xn[om] * xn[om] + yn[om] * yn[om]) / Jq[om];
+    v3 = (xn[o] * xn[o] + yn[o] * yn[o]) / by(Jq[o]);
+    v3 = v3 + (xn[om] * xn[om] + yn[om] * yn[om]) / by(Jq[om]);
     v3 = v3 * Jq[o] * vnu;
     v2 = (R)0.5 * (v1 + v3);
   }
@@ -255,10 +255,10 @@ __device__ __forceinline__ AdiRow<R> adi_row(const Slice<R>& S, const ot2d_param
     // lhsinv_up (lhs.f:1387-1501): upwind split eigenvalues, tridiagonal
     const R* xn = dir == 0 ? S.xx : S.yx;
     const R* yn = dir == 0 ? S.xy : S.yy;
-    const R eps = (R)0.05 * sqrt(sq(xn[o]) + sq(yn[o]));
+    const R eps = (R)0.05 * root(sq(xn[o]) + sq(yn[o]));
     const R fac = (R)1.05;
-    const R dpl = (R)0.5 * (di + fac * sqrt(sq(di) + sq(eps)));
-    const R dmi = (R)0.5 * (di - fac * sqrt(sq(di) + sq(eps)));
+    const R dpl = (R)0.5 * (di + fac * root(sq(di) + sq(eps)));
+    const R dmi = (R)0.5 * (di - fac * root(sq(di) + sq(eps)));
     r.a = (R)0.; r.b = (R)0.; r.c = (R)0.; r.d = (R)0.; r.e = (R)0.;
     r.b = r.b - dpl;
     r.d = r.d + dmi;
@@ -307,7 +307,7 @@ __device__ void adi_row_cell(const Slice<R>& S, const ot2d_params& p, int dir, i
       for (int v = sys ? sys + 1 : 0; v < (sys ? sys + 2 : 2); ++v) {
         R* sv = S.s + (int64_t)v * qs;
         const int64_t oi = adi_at(S.jd, dir, mi, n);
-        sv[oi] = sv[oi] - x * sv[adi_at(S.jd, dir, m, n)] / r.c;
+        sv[oi] = sv[oi] - x * sv[adi_at(S.jd, dir, m, n)] / by(r.c);
       }
       if (m == ms) put(A_RB + sys, ms + 1, (R)0);
       else put(A_RD + sys, me - 1, (R)0);
@@ -340,7 +340,7 @@ struct AdiForward {
   }
   __device__ __forceinline__ void step(R a, R b, R c, R& d, R& e, R* f) {
     const R d2 = (b - a * Dp);
-    const R d0 = (R)1. / (c - d2 * Dc - a * Ec);
+    const R d0 = (R)1. / by(c - d2 * Dc - a * Ec);
 #pragma unroll
     for (int v = 0; v < NF; ++v) {
       f[v] = (f[v] - d2 * f1[v] - a * f2[v]) * d0;
@@ -508,30 +508,30 @@ __device__ void adi_solve_k(const Slice<R>& S, const ot2d_params& p, int sys, in
 template <class R>
 __device__ void adi_ninv_cell(const Slice<R>& S, const ot2d_params& p, int j, int k) {
   const int64_t o = at(S.jd, j, k), qs = S.qs, ws = S.wstride;
-  const R cjkl = sqrt(S.k_ggm1 * (S.w[A_E * ws + o] - S.w[A_UV * ws + o]));
-  const R rj1 = S.xx[o], rj2 = S.xy[o], rr1 = sqrt(rj1 * rj1 + rj2 * rj2);
-  const R rk1 = S.yx[o], rk2 = S.yy[o], rr2 = sqrt(rk1 * rk1 + rk2 * rk2);
-  const R a1 = (rj1 * rk1 + rj2 * rk2) / rr1 / rr2;
-  const R a2 = (rj1 * rk2 - rj2 * rk1) / rr1 / rr2;
+  const R cjkl = root(S.k_ggm1 * (S.w[A_E * ws + o] - S.w[A_UV * ws + o]));
+  const R rj1 = S.xx[o], rj2 = S.xy[o], rr1 = root(rj1 * rj1 + rj2 * rj2);
+  const R rk1 = S.yx[o], rk2 = S.yy[o], rr2 = root(rk1 * rk1 + rk2 * rk2);
+  const R a1 = (rj1 * rk1 + rj2 * rk2) / by(rr1) / by(rr2);
+  const R a2 = (rj1 * rk2 - rj2 * rk1) / by(rr1) / by(rr2);
   const R s2 = S.s[qs + o], s3 = S.s[2 * qs + o], s4 = S.s[3 * qs + o];
   if (S.k_mp2 >= (R)0) {
     // arc2d_precon :1207-1231
     const R bSq = adi_bsq(S, o), omb = (R)1.0 - bSq;
     const R qx = S.w[A_QX * ws + o], qy = S.w[A_QY * ws + o], cx = S.w[A_CX * ws + o], cy = S.w[A_CY * ws + o];
-    const R X = sqrt((omb * qx) * (omb * qx) + (R)4. * bSq * cx * cx) / rr1;
-    const R Y = (R)0.5 * (omb * qx / rr1 + X);
-    const R Z = (R)0.5 * (omb * qx / rr1 - X);
-    const R X1 = sqrt((omb * qy) * (omb * qy) + (R)4. * bSq * cy * cy) / rr2;
-    const R Y1 = (R)0.5 * (omb * qy / rr2 + X1);
-    const R Z1 = (R)0.5 * (omb * qy / rr2 - X1);
-    S.s[qs + o] = a1 * s2 + (Y * s3 + Z * s4) * a2 / bSq;
-    S.s[2 * qs + o] = -(a2 * bSq * s2 - (Y * a1 - Z1) * s3 - (Z * a1 - Z1) * s4) / X1;
-    S.s[3 * qs + o] = (a2 * bSq * s2 - (Y * a1 - Y1) * s3 - (Z * a1 - Y1) * s4) / X1;
+    const R X = root((omb * qx) * (omb * qx) + (R)4. * bSq * cx * cx) / by(rr1);
+    const R Y = (R)0.5 * (omb * qx / by(rr1) + X);
+    const R Z = (R)0.5 * (omb * qx / by(rr1) - X);
+    const R X1 = root((omb * qy) * (omb * qy) + (R)4. * bSq * cy * cy) / by(rr2);
+    const R Y1 = (R)0.5 * (omb * qy / by(rr2) + X1);
+    const R Z1 = (R)0.5 * (omb * qy / by(rr2) - X1);
+    S.s[qs + o] = a1 * s2 + (Y * s3 + Z * s4) * a2 / by(bSq);
+    S.s[2 * qs + o] = -(a2 * bSq * s2 - (Y * a1 - Z1) * s3 - (Z * a1 - Z1) * s4) / by(X1);
+    S.s[3 * qs + o] = (a2 * bSq * s2 - (Y * a1 - Y1) * s3 - (Z * a1 - Y1) * s4) / by(X1);
     return;
   }
   const R a4 = a1 * s2 + (cjkl * s3 - cjkl * s4) * a2;
-  const R a5 = (R)-0.5 * (a2 * s2 / cjkl - (a1 + (R)1) * s3 + (a1 - (R)1) * s4);
-  const R a6 = (R)0.5 * (a2 * s2 / cjkl - (a1 - (R)1) * s3 + (a1 + (R)1) * s4);
+  const R a5 = (R)-0.5 * (a2 * s2 / by(cjkl) - (a1 + (R)1) * s3 + (a1 - (R)1) * s4);
+  const R a6 = (R)0.5 * (a2 * s2 / by(cjkl) - (a1 - (R)1) * s3 + (a1 + (R)1) * s4);
   S.s[qs + o] = a4; S.s[2 * qs + o] = a5; S.s[3 * qs + o] = a6;
 }
 
@@ -541,53 +541,53 @@ template <class R>
 __device__ void adi_teta_cell(const Slice<R>& S, const ot2d_params& p, int j, int k) {
   const int64_t o = at(S.jd, j, k), qs = S.qs, ws = S.wstride;
   const R uu = S.w[A_U * ws + o], vv = S.w[A_V * ws + o], uv = S.w[A_UV * ws + o], ge = S.w[A_GE * ws + o];
-  const R cjkl = sqrt(S.k_ggm1 * (S.w[A_E * ws + o] - uv));
+  const R cjkl = root(S.k_ggm1 * (S.w[A_E * ws + o] - uv));
   R rk1 = S.yx[o], rk2 = S.yy[o];
   const R ugc = S.ug ? S.ug[o] : (R)0, vgc = S.vg ? S.vg[o] : (R)0;
   const bool pre = S.k_mp2 >= (R)0;
   const R qq2 = pre ? S.w[A_QY * ws + o] : S.w[A_QY * ws + o] + (rk1 * ugc + rk2 * vgc);
-  const R rr2 = sqrt(rk1 * rk1 + rk2 * rk2);
-  rk1 = rk1 / rr2; rk2 = rk2 / rr2;
+  const R rr2 = root(rk1 * rk1 + rk2 * rk2);
+  rk1 = rk1 / by(rr2); rk2 = rk2 / by(rr2);
   const R s1 = S.s[o], s2 = S.s[qs + o], s3 = S.s[2 * qs + o], s4 = S.s[3 * qs + o];
   const R a1 = s1 + s3 + s4;
   R a2, a3, a4;
   if (pre) {
     // arc2d_precon :1264-1298
     const R bSq = adi_bsq(S, o), omb = (R)1. - bSq, cy = S.w[A_CY * ws + o];
-    const R X = sqrt((omb * qq2) * (omb * qq2) + (R)4. * bSq * cy * cy) / rr2;
-    const R Y = (R)0.5 * (omb * qq2 / rr2 + X);
-    const R Z = (R)0.5 * (omb * qq2 / rr2 - X);
+    const R X = root((omb * qq2) * (omb * qq2) + (R)4. * bSq * cy * cy) / by(rr2);
+    const R Y = (R)0.5 * (omb * qq2 / by(rr2) + X);
+    const R Z = (R)0.5 * (omb * qq2 / by(rr2) - X);
     const R qqmxt = qq2 + ugc * rk1 * rr2 + vgc * rk2 * rr2;
-    a2 = uu * s1 + rk2 * s2 + (uu + rk1 * Y / bSq) * s3;
-    a2 = a2 + (uu + rk1 * Z / bSq) * s4;
-    a3 = vv * s1 - rk1 * s2 + (vv + rk2 * Y / bSq) * s3;
-    a3 = a3 + (vv + rk2 * Z / bSq) * s4;
+    a2 = uu * s1 + rk2 * s2 + (uu + rk1 * Y / by(bSq)) * s3;
+    a2 = a2 + (uu + rk1 * Z / by(bSq)) * s4;
+    a3 = vv * s1 - rk1 * s2 + (vv + rk2 * Y / by(bSq)) * s3;
+    a3 = a3 + (vv + rk2 * Z / by(bSq)) * s4;
     a4 = uv * s1 + (rk2 * uu - rk1 * vv) * s2;
-    a4 = a4 + (ge + Y * qqmxt / rr2 / bSq) * s3;
-    a4 = a4 + (ge + Z * qqmxt / rr2 / bSq) * s4;
+    a4 = a4 + (ge + Y * qqmxt / by(rr2) / by(bSq)) * s3;
+    a4 = a4 + (ge + Z * qqmxt / by(rr2) / by(bSq)) * s4;
   } else {
     a2 = uu * s1 + rk2 * s2 + (uu + rk1 * cjkl) * s3;
     a2 = a2 + (uu - rk1 * cjkl) * s4;
     a3 = vv * s1 - rk1 * s2 + (vv + rk2 * cjkl) * s3;
     a3 = a3 + (vv - rk2 * cjkl) * s4;
     a4 = uv * s1 + (rk2 * uu - rk1 * vv) * s2;
-    a4 = a4 + (ge + cjkl * qq2 / rr2) * s3;
-    a4 = a4 + (ge - cjkl * qq2 / rr2) * s4;
+    a4 = a4 + (ge + cjkl * qq2 / by(rr2)) * s3;
+    a4 = a4 + (ge - cjkl * qq2 / by(rr2)) * s4;
   }
   R o2 = a2, o3 = a3;
   if (p.iunst == 2) {
     const R tsr = S.tscale[o] * (R)p.rotf;
     const R d = (R)1.0 + sq(S.tscale[o] * (R)p.rotf);
-    o2 = (a2 + tsr * a3) / d;
-    o3 = (a3 - tsr * a2) / d;
+    o2 = (a2 + tsr * a3) / by(d);
+    o3 = (a3 - tsr * a2) / by(d);
   }
   S.s[o] = a1; S.s[qs + o] = o2; S.s[2 * qs + o] = o3; S.s[3 * qs + o] = a4;
   if constexpr (sizeof(R) == sizeof(double)) {
     double* q = S.q64;
     const double q1 = q[o], J = q[(int64_t)(p.nq - 1) * qs + o];
-    const double dj = 1.0 / q1;
+    const double dj = 1.0 / by(q1);
     const double u = q[qs + o] * dj, v = q[2 * qs + o] * dj, e = q[3 * qs + o] * dj;
-    const double q1n = (q1 * J) / J;
+    const double q1n = (q1 * J) / by(J);
     q[o] = q1n;
     q[qs + o] = u * q1n;
     q[2 * qs + o] = v * q1n;

@@ -45,19 +45,19 @@ static __device__ __forceinline__ void extrap_prim(const BcK<T>& K, QVT<T> q, in
   const int nq = K.nq; const T gm1 = K.gm1;
   T rho1 = q(j1, k1, 1) * q(j1, k1, nq);
   T rho2 = q(j2, k2, 1) * q(j2, k2, nq);
-  T u1 = q(j1, k1, 2) / q(j1, k1, 1);
-  T u2 = q(j2, k2, 2) / q(j2, k2, 1);
-  T v1 = q(j1, k1, 3) / q(j1, k1, 1);
-  T v2 = q(j2, k2, 3) / q(j2, k2, 1);
-  T p1 = gm1 * (q(j1, k1, 4) - (T)0.5 * (sq(q(j1, k1, 2)) + sq(q(j1, k1, 3))) / q(j1, k1, 1)) * q(j1, k1, nq);
-  T pp2 = gm1 * (q(j2, k2, 4) - (T)0.5 * (sq(q(j2, k2, 2)) + sq(q(j2, k2, 3))) / q(j2, k2, 1)) * q(j2, k2, nq);
-  T r = (((T)1. + foso) * rho1 - foso * rho2) / q(j, k, nq);
+  T u1 = q(j1, k1, 2) / by(q(j1, k1, 1));
+  T u2 = q(j2, k2, 2) / by(q(j2, k2, 1));
+  T v1 = q(j1, k1, 3) / by(q(j1, k1, 1));
+  T v2 = q(j2, k2, 3) / by(q(j2, k2, 1));
+  T p1 = gm1 * (q(j1, k1, 4) - (T)0.5 * (sq(q(j1, k1, 2)) + sq(q(j1, k1, 3))) / by(q(j1, k1, 1))) * q(j1, k1, nq);
+  T pp2 = gm1 * (q(j2, k2, 4) - (T)0.5 * (sq(q(j2, k2, 2)) + sq(q(j2, k2, 3))) / by(q(j2, k2, 1))) * q(j2, k2, nq);
+  T r = (((T)1. + foso) * rho1 - foso * rho2) / by(q(j, k, nq));
   q(j, k, 1) = r;
   T a = (((T)1. + foso) * u1 - foso * u2) * r;
   T b = (((T)1. + foso) * v1 - foso * v2) * r;
   q(j, k, 2) = a; q(j, k, 3) = b;
   T press = ((T)1. + foso) * p1 - foso * pp2;
-  q(j, k, 4) = press / (gm1 * q(j, k, nq)) + (T)0.5 * (sq(a) + sq(b)) / r;
+  q(j, k, 4) = press / by(gm1 * q(j, k, nq)) + (T)0.5 * (sq(a) + sq(b)) / by(r);
 }
 
 // bcwall (bc.f:1669-1801) with bctany + uv (bc.f:1328-1415, :2224-2264),
@@ -76,10 +76,10 @@ static __device__ void bcwall_col(const BcK<T>& K, QVT<T> q, const T* xx, const 
   T u, v;
   {
     T ft = (T)1.0;
-    T u1 = (q(j, k1, 2) * M(xx, j, k) + q(j, k1, 3) * M(xy, j, k)) / q(j, k1, 1);
-    T v1 = (q(j, k1, 2) * M(yx, j, k) + q(j, k1, 3) * M(yy, j, k)) / q(j, k1, 1);
+    T u1 = (q(j, k1, 2) * M(xx, j, k) + q(j, k1, 3) * M(xy, j, k)) / by(q(j, k1, 1));
+    T v1 = (q(j, k1, 2) * M(yx, j, k) + q(j, k1, 3) * M(yy, j, k)) / by(q(j, k1, 1));
     if (invsc) {
-      T u2 = (q(j, k2, 2) * M(xx, j, k) + q(j, k2, 3) * M(xy, j, k)) / q(j, k2, 1);
+      T u2 = (q(j, k2, 2) * M(xx, j, k) + q(j, k2, 3) * M(xy, j, k)) / by(q(j, k2, 1));
       u = ((T)1. + ft) * u1 - ft * u2;
     } else {
       u = G(ug, j, k) * M(xx, j, k) + G(vg, j, k) * M(xy, j, k) + G(ug, j, k1) * M(xx, j, k1) +
@@ -89,32 +89,32 @@ static __device__ void bcwall_col(const BcK<T>& K, QVT<T> q, const T* xx, const 
         G(vg, j, k1) * M(yy, j, k1) - v1;
   }
   T t11 = (M(yy, j, k)), t12 = -(M(xy, j, k)), t21 = -(M(yx, j, k)), t22 = (M(xx, j, k));
-  T vol = (T)1. / (t22 * t11 - t12 * t21);
+  T vol = (T)1. / by(t22 * t11 - t12 * t21);
   T uwall = (t11 * u + t12 * v) * vol;
   T vwall = (t21 * u + t22 * v) * vol;
   {
     T rho1 = q(j, k1, 1) * q(j, k1, nq);
     T rho2 = q(j, k2, 1) * q(j, k2, nq);
-    T p1 = gm1 * (q(j, k1, 4) - (T)0.5 * (sq(q(j, k1, 2)) + sq(q(j, k1, 3))) / q(j, k1, 1)) * q(j, k1, nq);
-    T pp2 = gm1 * (q(j, k2, 4) - (T)0.5 * (sq(q(j, k2, 2)) + sq(q(j, k2, 3))) / q(j, k2, 1)) * q(j, k2, nq);
-    T r = (((T)1. + foso) * rho1 - foso * rho2) / q(j, k, nq);
+    T p1 = gm1 * (q(j, k1, 4) - (T)0.5 * (sq(q(j, k1, 2)) + sq(q(j, k1, 3))) / by(q(j, k1, 1))) * q(j, k1, nq);
+    T pp2 = gm1 * (q(j, k2, 4) - (T)0.5 * (sq(q(j, k2, 2)) + sq(q(j, k2, 3))) / by(q(j, k2, 1))) * q(j, k2, nq);
+    T r = (((T)1. + foso) * rho1 - foso * rho2) / by(q(j, k, nq));
     q(j, k, 1) = r;
     T a = uwall * r, b = vwall * r;
     q(j, k, 2) = a; q(j, k, 3) = b;
     T press = ((T)1. + foso) * p1 - foso * pp2;
-    q(j, k, 4) = press / (gm1 * q(j, k, nq)) + (T)0.5 * (sq(a) + sq(b)) / r;
+    q(j, k, 4) = press / by(gm1 * q(j, k, nq)) + (T)0.5 * (sq(a) + sq(b)) / by(r);
   }
   for (int kc = 1; kc <= ke - ks; ++kc) {
     int kk = (idir == 2) ? ke - kc : ks + kc;
     int kk1 = kk + iadd, kk2 = kk1 + iadd;
     extrap_prim(K, q, j, kk, j, kk1, j, kk2, (T)1.0);
   }
-  T t = (T)istep0 / (T)30.;
+  T t = (T)istep0 / by((T)30.);
   if (t > (T)1. || K.iread > 0) t = (T)1.;
   T scal = ((T)10. - (T)15. * t + (T)6. * t * t) * cube(t);
   T rscal = (T)1. - scal;
   for (int kk = ks; kk <= ke; ++kk) {
-    T ajacinv = (T)1. / q(j, kk, nq);
+    T ajacinv = (T)1. / by(q(j, kk, nq));
     q(j, kk, 1) = q(j, kk, 1) * scal + rscal * K.rinf * ajacinv;
     q(j, kk, 2) = q(j, kk, 2) * scal + rscal * K.rinf * K.uinf * ajacinv;
     q(j, kk, 3) = q(j, kk, 3) * scal + rscal * K.rinf * K.vinf * ajacinv;
@@ -128,7 +128,7 @@ static __device__ void trkl_cell(const BcK<T>& K, QVT<T> q, int j, int k, int j1
                           T ugc, T vgc, T btc, int iadd) {
   const int nq = K.nq; const T gm1 = K.gm1, ggm1 = K.ggm1, gamma = K.gamma, Mp = K.mp;
   const T foso = (T)1.0;
-  T snorm = -(T)1. * iadd / sqrt(sq(mx) + sq(my));
+  T snorm = -(T)1. * iadd / by(root(sq(mx) + sq(my)));
   T xxn = mx * snorm, xyn = my * snorm;
   T qext[4], qbar[4], delq[4], delw[4];
   for (int n = 1; n <= 4; ++n) qext[n - 1] = ((T)1. + foso) * q(j1, k1, n) * q(j1, k1, nq) - foso * q(j2, k2, n) * q(j2, k2, nq);
@@ -140,16 +140,16 @@ static __device__ void trkl_cell(const BcK<T>& K, QVT<T> q, int j, int k, int j1
   delq[1] = (T)0.5 * (K.rinf * K.uinf - qext[1]);
   delq[2] = (T)0.5 * (K.rinf * K.vinf - qext[2]);
   delq[3] = (T)0.5 * (K.einf - qext[3]);
-  T rho = qbar[0], rrho = (T)1. / rho;
+  T rho = qbar[0], rrho = (T)1. / by(rho);
   T uu = qbar[1] * rrho, vv = qbar[2] * rrho, e = qbar[3] * rrho;
   T uv2 = (T)0.5 * (uu * uu + vv * vv);
-  T cjkl = sqrt(ggm1 * (e - uv2));
-  T c2i = (T)1. / (cjkl * cjkl);
+  T cjkl = root(ggm1 * (e - uv2));
+  T c2i = (T)1. / by(cjkl * cjkl);
   T ge = gamma * e - gm1 * uv2;
   T qq = (uu - ugc) * xxn + (vv - vgc) * xyn;
-  T bSq = sq(Mp) / (btc - sq(Mp) * (btc - 1));
-  T Z = sqrt(((T)1. - bSq) * qq * ((T)1. - bSq) * qq + (T)4. * bSq * cjkl * cjkl);
-  T Zi = (T)1. / Z;
+  T bSq = sq(Mp) / by(btc - sq(Mp) * (btc - 1));
+  T Z = root(((T)1. - bSq) * qq * ((T)1. - bSq) * qq + (T)4. * bSq * cjkl * cjkl);
+  T Zi = (T)1. / by(Z);
   T R = (T)0.5 * (((T)1. - bSq) * qq + Z);
   T S = (T)0.5 * (((T)1. - bSq) * qq - Z);
   T sqs = fsign((T)1., qq), sR = fsign((T)1., R + bSq * qq), sR2 = fsign((T)1., R + qq * bSq);
@@ -170,15 +170,15 @@ static __device__ void trkl_cell(const BcK<T>& K, QVT<T> q, int j, int k, int j1
   delw[3] = delw[3] - (xyn * bSq + R * vv * gm1 * c2i) * Zi * sS2 * delq[2];
   delw[3] = delw[3] + R * gm1 * c2i * Zi * sS2 * delq[3];
   delq[0] = delw[0] + delw[2] + delw[3];
-  delq[1] = uu * delw[0] + xyn * delw[1] + (uu + xxn * R / bSq) * delw[2];
-  delq[1] = delq[1] + (uu + xxn * S / bSq) * delw[3];
-  delq[2] = vv * delw[0] - xxn * delw[1] + (vv + xyn * R / bSq) * delw[2];
-  delq[2] = delq[2] + (vv + xyn * S / bSq) * delw[3];
+  delq[1] = uu * delw[0] + xyn * delw[1] + (uu + xxn * R / by(bSq)) * delw[2];
+  delq[1] = delq[1] + (uu + xxn * S / by(bSq)) * delw[3];
+  delq[2] = vv * delw[0] - xxn * delw[1] + (vv + xyn * R / by(bSq)) * delw[2];
+  delq[2] = delq[2] + (vv + xyn * S / by(bSq)) * delw[3];
   delq[3] = uv2 * delw[0] + (uu * xyn - vv * xxn) * delw[1];
-  delq[3] = delq[3] + (ge + R * qq / bSq) * delw[2];
-  delq[3] = delq[3] + (ge + S * qq / bSq) * delw[3];
+  delq[3] = delq[3] + (ge + R * qq / by(bSq)) * delw[2];
+  delq[3] = delq[3] + (ge + S * qq / by(bSq)) * delw[3];
   T J = q(j, k, nq);
-  for (int n = 1; n <= 4; ++n) q(j, k, n) = (qbar[n - 1] - delq[n - 1]) / J;
+  for (int n = 1; n <= 4; ++n) q(j, k, n) = (qbar[n - 1] - delq[n - 1]) / by(J);
 }
 
 // bc.f:2-86 for BC entry ib of one slice (the &bcinp table's order is kept
@@ -214,8 +214,8 @@ __device__ void bc_entry(const Slice<R>& S, int istep0, int ib, int tid, int nth
             int k, k1;
             if (idir == 2) { k = ke - kc + 1; k1 = ke + kc; } else { k = ks + kc - 1; k1 = ks - kc; }
             int jj = jd - j + 1;
-            T scale1 = q(jj, k1, p.nq) / q(j, k, p.nq);
-            T scale2 = q(j, k1, p.nq) / q(jj, k, p.nq);
+            T scale1 = q(jj, k1, p.nq) / by(q(j, k, p.nq));
+            T scale2 = q(j, k1, p.nq) / by(q(jj, k, p.nq));
             for (int n = 1; n <= 4; ++n) q(j, k, n) = q(jj, k1, n) * scale1;
             for (int n = 1; n <= 4; ++n) q(jj, k, n) = q(j, k1, n) * scale2;
           }
@@ -244,10 +244,10 @@ __device__ void bc_entry(const Slice<R>& S, int istep0, int ib, int tid, int nth
     } else if (t == 46) {
       for (int idx = tid; idx < (je - js + 1) * (ke - ks + 1); idx += nthr) {
         int j = js + idx % (je - js + 1), k = ks + idx / (je - js + 1);
-        T rj = (T)1. / q(j, k, p.nq);
+        T rj = (T)1. / by(q(j, k, p.nq));
         T r = K.rinf * rj, a = K.rinf * K.uinf * rj, b = K.rinf * K.vinf * rj;
         q(j, k, 1) = r; q(j, k, 2) = a; q(j, k, 3) = b;
-        q(j, k, 4) = K.pinf / K.gm1 * rj + (T)0.5 * (sq(a) + sq(b)) / r;
+        q(j, k, 4) = K.pinf / by(K.gm1) * rj + (T)0.5 * (sq(a) + sq(b)) / by(r);
       }
     } else if (t == 10 || t == 11) {
       const int nq = p.nq;
@@ -256,12 +256,12 @@ __device__ void bc_entry(const Slice<R>& S, int istep0, int ib, int tid, int nth
           for (int jc = 1; jc <= je - js + 1; ++jc) {
             if (t == 10) {
               int j = (idir == 1) ? je - jc + 1 : js + jc - 1, j1 = j + iadd;
-              T s1 = q(j1, k, nq) / q(j, k, nq);
-              for (int n = 1; n <= 4; ++n) q(j, k, n) = ((T)1. + (T)0.0) * q(j1, k, n) * s1 - (T)0.0 * q(j1 + iadd, k, n) * (q(j1 + iadd, k, nq) / q(j, k, nq));
+              T s1 = q(j1, k, nq) / by(q(j, k, nq));
+              for (int n = 1; n <= 4; ++n) q(j, k, n) = ((T)1. + (T)0.0) * q(j1, k, n) * s1 - (T)0.0 * q(j1 + iadd, k, n) * (q(j1 + iadd, k, nq) / by(q(j, k, nq)));
             } else {
               int j, j1;
               if (idir == 1) { j = je - jc + 1; j1 = je + jc; } else { j = js + jc - 1; j1 = js - jc; }
-              T sc = q(j1, k, nq) / q(j, k, nq);
+              T sc = q(j1, k, nq) / by(q(j, k, nq));
               q(j, k, 1) = q(j1, k, 1) * sc; q(j, k, 2) = -q(j1, k, 2) * sc;
               q(j, k, 3) = q(j1, k, 3) * sc; q(j, k, 4) = q(j1, k, 4) * sc;
             }
@@ -271,12 +271,12 @@ __device__ void bc_entry(const Slice<R>& S, int istep0, int ib, int tid, int nth
           for (int kc = 1; kc <= ke - ks + 1; ++kc) {
             if (t == 10) {
               int k = (idir == 2) ? ke - kc + 1 : ks + kc - 1, k1 = k + iadd;
-              T s1 = q(j, k1, nq) / q(j, k, nq);
-              for (int n = 1; n <= 4; ++n) q(j, k, n) = ((T)1. + (T)0.0) * q(j, k1, n) * s1 - (T)0.0 * q(j, k1 + iadd, n) * (q(j, k1 + iadd, nq) / q(j, k, nq));
+              T s1 = q(j, k1, nq) / by(q(j, k, nq));
+              for (int n = 1; n <= 4; ++n) q(j, k, n) = ((T)1. + (T)0.0) * q(j, k1, n) * s1 - (T)0.0 * q(j, k1 + iadd, n) * (q(j, k1 + iadd, nq) / by(q(j, k, nq)));
             } else {
               int k, k1;
               if (idir == 2) { k = ke - kc + 1; k1 = ke + kc; } else { k = ks + kc - 1; k1 = ks - kc; }
-              T sc = q(j, k1, nq) / q(j, k, nq);
+              T sc = q(j, k1, nq) / by(q(j, k, nq));
               q(j, k, 1) = q(j, k1, 1) * sc; q(j, k, 2) = q(j, k1, 2) * sc;
               q(j, k, 3) = -q(j, k1, 3) * sc; q(j, k, 4) = q(j, k1, 4) * sc;
             }
@@ -289,7 +289,7 @@ __device__ void bc_entry(const Slice<R>& S, int istep0, int ib, int tid, int nth
         for (int j = js + tid; j <= je; j += nthr) {
           int jc = (idir == 1) ? jd - 2 * jj + (j - js + 1) : 1 + 2 * jj - (je - j + 1);
           for (int k = ks; k <= ke; ++k) {
-            T sc = q(jc, k, nq) / q(j, k, nq);
+            T sc = q(jc, k, nq) / by(q(j, k, nq));
             for (int n = 1; n <= 4; ++n) q(j, k, n) = q(jc, k, n) * sc;
           }
         }
@@ -298,7 +298,7 @@ __device__ void bc_entry(const Slice<R>& S, int istep0, int ib, int tid, int nth
         for (int j = js + tid; j <= je; j += nthr)
           for (int k = ks; k <= ke; ++k) {
             int kc = (idir == 2) ? p.kd - 2 * kk + (k - ks + 1) : 1 + 2 * kk - (ke - k + 1);
-            T sc = q(j, kc, nq) / q(j, k, nq);
+            T sc = q(j, kc, nq) / by(q(j, k, nq));
             for (int n = 1; n <= 4; ++n) q(j, k, n) = q(j, kc, n) * sc;
           }
       }
@@ -372,8 +372,8 @@ __device__ void rbc_slice(const Slice<R>& S) {
           int k, k1;
           if (idir == 2) { k = ke - kc + 1; k1 = ke + kc; } else { k = ks + kc - 1; k1 = ks - kc; }
           int jj = jd - j + 1;
-          R scale1 = (R)(q(jj, k1, nq) / q(j, k, nq));
-          R scale2 = (R)(q(j, k1, nq) / q(jj, k, nq));
+          R scale1 = (R)(q(jj, k1, nq) / by(q(j, k, nq)));
+          R scale2 = (R)(q(j, k1, nq) / by(q(jj, k, nq)));
           for (int n = 1; n <= 4; ++n) s(j, k, n) = s(jj, k1, n) * scale1;
           for (int n = 1; n <= 4; ++n) s(jj, k, n) = s(j, k1, n) * scale2;
         }
@@ -384,7 +384,7 @@ __device__ void rbc_slice(const Slice<R>& S) {
             int j, j1;
             if (t == 10) { j = (idir == 1) ? je - jc + 1 : js + jc - 1; j1 = j + iadd; }
             else if (idir == 1) { j = je - jc + 1; j1 = je + jc; } else { j = js + jc - 1; j1 = js - jc; }
-            R sc = (R)(q(j1, k, nq) / q(j, k, nq));
+            R sc = (R)(q(j1, k, nq) / by(q(j, k, nq)));
             for (int n = 1; n <= 4; ++n) s(j, k, n) = (t == 11 && n == 2) ? -s(j1, k, n) * sc : (t == 10 ? (R)(1. + 0.0) * s(j1, k, n) * sc - (R)0 : s(j1, k, n) * sc);
           }
       } else if (iadir == 2) {
@@ -393,7 +393,7 @@ __device__ void rbc_slice(const Slice<R>& S) {
             int k, k1;
             if (t == 10) { k = (idir == 2) ? ke - kc + 1 : ks + kc - 1; k1 = k + iadd; }
             else if (idir == 2) { k = ke - kc + 1; k1 = ke + kc; } else { k = ks + kc - 1; k1 = ks - kc; }
-            R sc = (R)(q(j, k1, nq) / q(j, k, nq));
+            R sc = (R)(q(j, k1, nq) / by(q(j, k, nq)));
             for (int n = 1; n <= 4; ++n) s(j, k, n) = (t == 11 && n == 3) ? -s(j, k1, n) * sc : (t == 10 ? (R)(1. + 0.0) * s(j, k1, n) * sc - (R)0 : s(j, k1, n) * sc);
           }
       }
@@ -403,7 +403,7 @@ __device__ void rbc_slice(const Slice<R>& S) {
         for (int j = js + threadIdx.x; j <= je; j += blockDim.x) {
           int jc = (idir == 1) ? jd - 2 * jj + (j - js + 1) : 1 + 2 * jj - (je - j + 1);
           for (int k = ks; k <= ke; ++k) {
-            R sc = (R)(q(jc, k, nq) / q(j, k, nq));
+            R sc = (R)(q(jc, k, nq) / by(q(j, k, nq)));
             for (int n = 1; n <= 4; ++n) s(j, k, n) = s(jc, k, n) * sc;
           }
         }
@@ -412,7 +412,7 @@ __device__ void rbc_slice(const Slice<R>& S) {
         for (int j = js + threadIdx.x; j <= je; j += blockDim.x)
           for (int k = ks; k <= ke; ++k) {
             int kc = (idir == 2) ? p.kd - 2 * kk + (k - ks + 1) : 1 + 2 * kk - (ke - k + 1);
-            R sc = (R)(q(j, kc, nq) / q(j, k, nq));
+            R sc = (R)(q(j, kc, nq) / by(q(j, k, nq)));
             for (int n = 1; n <= 4; ++n) s(j, k, n) = s(j, kc, n) * sc;
           }
       }
@@ -435,7 +435,7 @@ __device__ void turbc_slice(const Slice<R>& S, const R* u, const R* v) {
   auto U = [&](const R* a, int n, int j, int k) {
     const int64_t o = at(jd, j, k);
     if (a) return (double)a[o];
-    return (double)(S.q[n * S.qs + o] / S.q[o]);
+    return (double)(S.q[n * S.qs + o] / by(S.q[o]));
   };
   auto G = [&](const double* a, int j, int k) { return a ? a[at(jd, j, k)] : 0.0; };
   for (int ib = 0; ib < p.nbc; ++ib) {

@@ -159,7 +159,7 @@ __device__ void tri_solve_j(R* a, R* b, R* c, R* s, int jd, int js, int je, int 
       arr, arr, jd, js, je, k0, nrow, sm,
       [&](R* t, int j) {
         const R av = j == js ? (R)0 : t[0];
-        const R bb = (R)1. / (t[JL_TILE] - av * cp);
+        const R bb = (R)1. / by(t[JL_TILE] - av * cp);
         sp = (t[3 * JL_TILE] - av * sp) * bb;
         cp = t[2 * JL_TILE] * bb;
         t[3 * JL_TILE] = sp;
@@ -201,7 +201,7 @@ __device__ void tri_solve_k(const R* a, const R* b, R* c, R* s, int jd, int ks, 
       for (int u = 0; u < U; ++u)
         if (k0 + u <= ke) {
           const int64_t o = at(jd, j, k0 + u);
-          const R bb = (R)1. / (rb[u] - ra[u] * cp);
+          const R bb = (R)1. / by(rb[u] - ra[u] * cp);
           sp = (rs[u] - ra[u] * sp) * bb;
           cp = rc[u] * bb;
           s[o] = sp;

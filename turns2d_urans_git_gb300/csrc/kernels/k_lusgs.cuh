@@ -191,38 +191,38 @@ __device__ __forceinline__ LuCell<R> lu_cell(const Slice<R>& S, const ot2d_param
   const int64_t o = at(S.jd, j, k), qs = S.qs;
   LuCell<R> c;
   R q1 = S.q[o];
-  R dj = (R)1.0 / q1;
+  R dj = (R)1.0 / by(q1);
   c.uu = S.q[qs + o] * dj;
   c.vv = S.q[2 * qs + o] * dj;
   R e = S.q[3 * qs + o] * dj;
   R rho = q1 * S.q[(p.nq - 1) * qs + o];
   c.uv2 = (R)0.5 * (c.uu * c.uu + c.vv * c.vv);
-  R cjkl = sqrt(S.k_ggm1 * (e - c.uv2));
+  R cjkl = root(S.k_ggm1 * (e - c.uv2));
   c.ri1 = S.xx[o]; c.ri2 = S.xy[o]; c.rk1 = S.yx[o]; c.rk2 = S.yy[o];
   c.ugc = S.ug ? S.ug[o] : (R)0; c.vgc = S.vg ? S.vg[o] : (R)0;
   R qq1 = c.ri1 * c.uu + c.ri2 * c.vv;
   R qqx = fabs(-c.ri1 * c.ugc - c.ri2 * c.vgc + qq1);
-  R rr1 = sqrt(sq(c.ri1) + sq(c.ri2));
+  R rr1 = root(sq(c.ri1) + sq(c.ri2));
   R qq2 = c.rk1 * c.uu + c.rk2 * c.vv;
   R qqy = fabs(-c.rk1 * c.ugc - c.rk2 * c.vgc + qq2);
-  R rr2 = sqrt(sq(c.rk1) + sq(c.rk2));
-  R vnu = (R)2.0 * rr2 * rr2 * (S.k_rmue + S.turmu[o]) / (S.k_rey * rho);
+  R rr2 = root(sq(c.rk1) + sq(c.rk2));
+  R vnu = (R)2.0 * rr2 * rr2 * (S.k_rmue + S.turmu[o]) / by(S.k_rey * rho);
   R svt = S.tscale[o];
   c.qx = qq1; c.cx = cjkl * rr1; c.qy = qq2; c.cy = cjkl * rr2; c.vn = vnu;
   c.ge = S.k_gamma * e - S.k_gm1 * c.uv2;
   if constexpr (PRE) {
     const R btv = S.bt[o], mp2 = S.k_mp2;
-    const R bSq = mp2 / (btv - mp2 * (btv - (R)1));
+    const R bSq = mp2 / by(btv - mp2 * (btv - (R)1));
     const R omb = (R)1. - bSq, opb = bSq + (R)1., fb = (R)4. * bSq;
-    const R X = sqrt((omb * qqx) * (omb * qqx) + (fb * c.cx) * c.cx);
+    const R X = root((omb * qqx) * (omb * qqx) + (fb * c.cx) * c.cx);
     R term = (R)0.5 * (opb * qqx + X);
-    const R Y = sqrt((omb * qqy) * (omb * qqy) + (fb * c.cy) * c.cy);
+    const R Y = root((omb * qqy) * (omb * qqy) + (fb * c.cy) * c.cy);
     term = term + (R)0.5 * (opb * qqy + Y);
-    c.d = (R)1.0 / ((R)1.0 + svt * (term * epsv + vnu));
+    c.d = (R)1.0 / by((R)1.0 + svt * (term * epsv + vnu));
     c.bsq = bSq;
-    c.term = S.k_gm1 * (bSq - (R)1.) / (cjkl * cjkl);
+    c.term = S.k_gm1 * (bSq - (R)1.) / by(cjkl * cjkl);
   } else {
-    c.d = (R)1.0 / ((R)1.0 + svt * ((qqx + qqy + cjkl * (rr1 + rr2)) * epsv + vnu));
+    c.d = (R)1.0 / by((R)1.0 + svt * ((qqx + qqy + cjkl * (rr1 + rr2)) * epsv + vnu));
     c.bsq = (R)0; c.term = (R)0;
   }
   return c;
@@ -265,7 +265,7 @@ __device__ __forceinline__ void lu_chkspec_pre(const LuCell<R>& c, R eps2, R& ch
   R ri1 = XI ? c.ri1 : c.rk1, ri2 = XI ? c.ri2 : c.rk2, qq = XI ? c.qx : c.qy, cc = XI ? c.cx : c.cy;
   R qqn = -ri1 * c.ugc - ri2 * c.vgc + qq;
   const R bSq = c.bsq, omb = (R)1. - bSq, opb = bSq + (R)1.;
-  R X = sqrt((omb * qqn) * (omb * qqn) + (((R)4. * bSq) * cc) * cc);
+  R X = root((omb * qqn) * (omb * qqn) + (((R)4. * bSq) * cc) * cc);
   if (FWD) chk = (R)0.5 + fsign((R)0.5, opb * qqn + X);
   else chk = (R)0.5 - fsign((R)0.5, opb * qqn - X);
   R sp1 = (R)0.5 * (opb * fabs(qqn) + X);
@@ -408,9 +408,9 @@ __device__ __forceinline__ void lu_edge_cell(const Slice<R>& S, const ot2d_param
   if constexpr (sizeof(R) == sizeof(double)) {
     const int64_t qs = S.qs;
     double q1 = S.q[o], J = S.q[(p.nq - 1) * qs + o];
-    double dj = 1.0 / q1;
+    double dj = 1.0 / by(q1);
     double u = S.q[qs + o] * dj, v = S.q[2 * qs + o] * dj, e = S.q[3 * qs + o] * dj;
-    double q1n = (q1 * J) / J;
+    double q1n = (q1 * J) / by(J);
     S.q[o] = q1n;
     S.q[qs + o] = u * q1n;
     S.q[2 * qs + o] = v * q1n;

@@ -64,13 +64,13 @@ __device__ void mv_pitch_cell(const Slice<R>& S, int cid) {
     const double ynew = -((x - p.xac) * sn) + (y - p.yac) * cn + p.yac;
     double ug, vg;
     if (p.ntac == 1) {
-      ug = (xnew - x) / p.dt;
-      vg = (ynew - y) / p.dt;
+      ug = (xnew - x) / by(p.dt);
+      vg = (ynew - y) / by(p.dt);
     } else {
       const double xo = (x - p.xac) * cnold + (y - p.yac) * snold + p.xac;
       const double yo = -((x - p.xac) * snold) + (y - p.yac) * cnold + p.yac;
-      ug = (1.5 * xnew - 2. * x + 0.5 * xo) / p.dt;
-      vg = (1.5 * ynew - 2. * y + 0.5 * yo) / p.dt;
+      ug = (1.5 * xnew - 2. * x + 0.5 * xo) / by(p.dt);
+      vg = (1.5 * ynew - 2. * y + 0.5 * yo) / by(p.dt);
     }
     S.xc[cid] = xnew;
     S.yc[cid] = ynew;
@@ -113,7 +113,7 @@ __device__ void mv_geom_cell(const Slice<R>& S, int j, int k) {
     const int a = j - nh + 1, b = k - nh + 1;
     const double dx1 = XV(a, b) - XV(a - 1, b - 1), dy1 = YV(a, b) - YV(a - 1, b - 1);
     const double dx2 = XV(a - 1, b) - XV(a, b - 1), dy2 = YV(a - 1, b) - YV(a, b - 1);
-    const double qj = 1. / (0.5 * (dx1 * dy2 - dx2 * dy1));
+    const double qj = 1. / by(0.5 * (dx1 * dy2 - dx2 * dy1));
     const double xx = qj * (0.5 * (YV(a, b) - YV(a, b - 1) + YV(a - 1, b) - YV(a - 1, b - 1)));
     const double xy = qj * (-(0.5 * (XV(a, b) - XV(a, b - 1) + XV(a - 1, b) - XV(a - 1, b - 1))));
     const double yx = qj * (-(0.5 * (YV(a, b) - YV(a - 1, b) + YV(a, b - 1) - YV(a - 1, b - 1))));
@@ -146,12 +146,12 @@ __device__ void mv_geom_cell(const Slice<R>& S, int j, int k) {
     {
       const double dx1 = XV(a, b) - XO(a, b - 1), dy1 = YV(a, b) - YO(a, b - 1);
       const double dx2 = XO(a, b) - XV(a, b - 1), dy2 = YO(a, b) - YV(a, b - 1);
-      tj = -(0.5 * (dx1 * dy2 - dx2 * dy1) / p.dt);
+      tj = -(0.5 * (dx1 * dy2 - dx2 * dy1) / by(p.dt));
     }
     if (second) {
       const double dx1 = XO(a, b) - XE(a, b - 1), dy1 = YO(a, b) - YE(a, b - 1);
       const double dx2 = XE(a, b) - XO(a, b - 1), dy2 = YE(a, b) - YO(a, b - 1);
-      const double temp = -(0.5 * (dx1 * dy2 - dx2 * dy1) / p.dt);
+      const double temp = -(0.5 * (dx1 * dy2 - dx2 * dy1) / by(p.dt));
       tj = 1.5 * tj - 0.5 * temp;
     }
     const_cast<R*>(S.fxa)[o] = (R)fx; const_cast<R*>(S.fya)[o] = (R)fy; const_cast<R*>(S.ftj)[o] = (R)tj;
@@ -164,12 +164,12 @@ __device__ void mv_geom_cell(const Slice<R>& S, int j, int k) {
     {
       const double dx1 = XV(a, b) - XO(a - 1, b), dy1 = YV(a, b) - YO(a - 1, b);
       const double dx2 = XO(a, b) - XV(a - 1, b), dy2 = YO(a, b) - YV(a - 1, b);
-      tj = 0.5 * (dx1 * dy2 - dx2 * dy1) / p.dt;
+      tj = 0.5 * (dx1 * dy2 - dx2 * dy1) / by(p.dt);
     }
     if (second) {
       const double dx1 = XO(a, b) - XE(a - 1, b), dy1 = YO(a, b) - YE(a - 1, b);
       const double dx2 = XE(a, b) - XO(a - 1, b), dy2 = YE(a, b) - YO(a - 1, b);
-      const double temp = 0.5 * (dx1 * dy2 - dx2 * dy1) / p.dt;
+      const double temp = 0.5 * (dx1 * dy2 - dx2 * dy1) / by(p.dt);
       tj = 1.5 * tj - 0.5 * temp;
     }
     const_cast<R*>(S.gxa)[o] = (R)gx; const_cast<R*>(S.gya)[o] = (R)gy; const_cast<R*>(S.gtj)[o] = (R)tj;
@@ -184,12 +184,12 @@ __device__ void mv_geom_cell(const Slice<R>& S, int j, int k) {
         const int a = j - nh;
         const double fx = 0.5 * (XV(a, 1) + XV(a + 1, 1)), fy = 0.5 * (YV(a, 1) + YV(a + 1, 1));
         const double dx = S.xc[o] - fx, dy = S.yc[o] - fy;
-        d = sqrt(dx * dx + dy * dy);
+        d = root(dx * dx + dy * dy);
       }
     } else {
       const int a = p.jtail1 - nh;
       const double dx = S.xc[o] - XV(a, 1), dy = S.yc[o] - YV(a, 1);
-      d = sqrt(dx * dx + dy * dy);
+      d = root(dx * dx + dy * dy);
     }
     const_cast<R*>(S.sn)[o] = (R)d;
   }

@@ -46,9 +46,9 @@ __device__ __forceinline__ R quad_sonic(R at, R ati1, R sl) {
 // curvature (curv = true) at interior line position i, is2 < i < ie2.
 template <class R>
 __device__ __forceinline__ R quad_rhs(const LineRd<R>& L, int v, int i, bool curv) {
-  if (!curv) return (L.f(i + 2, v) + (R)28. * L.f(i + 1, v) - (R)28. * L.f(i - 1, v) - L.f(i - 2, v)) / (R)36.;
+  if (!curv) return (L.f(i + 2, v) + (R)28. * L.f(i + 1, v) - (R)28. * L.f(i - 1, v) - L.f(i - 2, v)) / by((R)36.);
   return ((R)3. * L.f(i + 2, v) + (R)48. * L.f(i + 1, v) - (R)102. * L.f(i, v) + (R)48. * L.f(i - 1, v) +
-          (R)3. * L.f(i - 2, v)) / (R)44.;
+          (R)3. * L.f(i - 2, v)) / by((R)44.);
 }
 
 // tridag over positions is2..ie2 of one line: sub- and super-diagonal c1,
@@ -65,7 +65,7 @@ __device__ __forceinline__ void quad_tridag(const LineRd<R>& L, R* D, R* W, int 
     const R a = j == ie2 ? c1e : c1i;
     const R f = j == ie2 ? rhs_e : rhs(j);
     const R d = (R)1. - a * w;
-    const R rd = (R)1.0 / d;
+    const R rd = (R)1.0 / by(d);
     w = a * rd;
     g = (f - a * g) * rd;
     W[L.off(j)] = w; D[L.off(j)] = g;
@@ -173,8 +173,8 @@ __device__ void quad_line(const Slice<R>& S, const LineRd<R>& L, int dir, int v,
         ci = ammd(cl, d2);
       }
     }
-    QL[o] = f0 + (R)0.5 * si + ci / (R)12.;
-    QR[o] = f0 - (R)0.5 * si + ci / (R)12.;
+    QL[o] = f0 + (R)0.5 * si + ci / by((R)12.);
+    QR[o] = f0 - (R)0.5 * si + ci / by((R)12.);
   }
   // the end cells from their sonic-A slopes, and quad's consistency of the
   // third cell from each end with them

@@ -132,27 +132,27 @@ __device__ __forceinline__ void rt_store_cell(const Slice<R>& S, const SM& sm, i
                                               bool visc) {
   const R q1 = a.q1, q2 = a.q2, q3 = a.q3, q4 = a.q4, J = a.J;
   const R gm1 = S.k_gm1;
-  const R rhoi = (R)1.0 / q1;
+  const R rhoi = (R)1.0 / by(q1);
   sm.at(RS_RHO, r) = q1 * J;
   const R u = q2 * rhoi, v = q3 * rhoi;
   sm.at(RS_U, r) = u;
   sm.at(RS_V, r) = v;
-  const R ppp = gm1 * (q4 - (R)0.5 * (sq(q2) + sq(q3)) / q1);
+  const R ppp = gm1 * (q4 - (R)0.5 * (sq(q2) + sq(q3)) / by(q1));
   sm.at(RS_P, r) = ppp * J;
   if (visc) {
     const R c2b = S.k_c2b, c2bp = S.k_c2bp, prtr = S.k_prtr;
     const R e = q4 * rhoi - (R).5 * (sq(u) + sq(v));
     const R tt = S.k_ggm1 * e;
-    const R vmue = c2bp * tt * sqrt(tt) / (c2b + tt);
+    const R vmue = c2bp * tt * root(tt) / by(c2b + tt);
     const R turm = a.turm;
     sm.at(RS_E, r) = e;
     sm.at(RS_VNU, r) = vmue + turm;
     sm.at(RS_GKAP, r) = vmue + prtr * turm;
-    sm.at(RS_RJ, r) = (R)1. / J;
-    const R ud = q2 / q1, vd = q3 / q1;
+    sm.at(RS_RJ, r) = (R)1. / by(J);
+    const R ud = q2 / by(q1), vd = q3 / by(q1);
     sm.at(RS_UD, r) = ud;
     sm.at(RS_VD, r) = vd;
-    sm.at(RS_ED, r) = q4 / q1 - (R).5 * (sq(ud) + sq(vd));
+    sm.at(RS_ED, r) = q4 / by(q1) - (R).5 * (sq(ud) + sq(vd));
     sm.at(RS_XX, r) = a.xx; sm.at(RS_XY, r) = a.xy; sm.at(RS_YX, r) = a.yx; sm.at(RS_YY, r) = a.yy;
   }
   const int ia = a.ib < 0 ? -a.ib : a.ib;
@@ -191,9 +191,9 @@ __device__ __forceinline__ void rt_visc_eta(const SM& sm, int r, R gkpr, R dre, 
     uu[m] = sm.at(RS_U, rr); vv[m] = sm.at(RS_V, rr); ee[m] = sm.at(RS_E, rr);
     const R yx = sm.at(RS_YX, rr), yy = sm.at(RS_YY, rr);
     const R b4 = (sq(yx) + sq(yy)) * rj;
-    bv[m][0] = (b4 + sq(yx) / (R)3. * rj) * vnu * dre;
-    bv[m][1] = (b4 + sq(yy) / (R)3. * rj) * vnu * dre;
-    bv[m][3] = (yx * yy / (R)3. * rj) * vnu * dre;
+    bv[m][0] = (b4 + sq(yx) / by((R)3.) * rj) * vnu * dre;
+    bv[m][1] = (b4 + sq(yy) / by((R)3.) * rj) * vnu * dre;
+    bv[m][3] = (yx * yy / by((R)3.) * rj) * vnu * dre;
     bv[m][2] = b4 * gkpr * gkap * dre;
   }
   const int rm = r - 1, rp = r + 1;
@@ -253,9 +253,9 @@ __device__ __forceinline__ void rt_visc_xi(const SM& sm, int r, R gkpr, R dre, R
     uu[m] = sm.at(RS_U, rr); vv[m] = sm.at(RS_V, rr); ee[m] = sm.at(RS_E, rr);
     const R xx = sm.at(RS_XX, rr), xy = sm.at(RS_XY, rr);
     const R a4 = (sq(xx) + sq(xy)) * rj;
-    av[m][0] = (a4 + sq(xx) / (R)3. * rj) * vnu * dre;
-    av[m][1] = (a4 + sq(xy) / (R)3. * rj) * vnu * dre;
-    av[m][3] = (xx * xy / (R)3. * rj) * vnu * dre;
+    av[m][0] = (a4 + sq(xx) / by((R)3.) * rj) * vnu * dre;
+    av[m][1] = (a4 + sq(xy) / by((R)3.) * rj) * vnu * dre;
+    av[m][3] = (xx * xy / by((R)3.) * rj) * vnu * dre;
     av[m][2] = a4 * gkpr * gkap * dre;
   }
   const int rm = r - SM::RW, rp = r + SM::RW;
@@ -310,16 +310,16 @@ template <class R>
 __device__ __forceinline__ void rhslom_cell(const Slice<R>& S, const ot2d_params& p, int64_t o, R* s) {
   const int64_t qs = S.qs;
   const R q1 = S.q[o], gm1 = S.k_gm1, gamma = S.k_gamma, mp2 = S.k_mp2;
-  const R u = S.q[qs + o] / q1;
-  const R v = S.q[2 * qs + o] / q1;
+  const R u = S.q[qs + o] / by(q1);
+  const R v = S.q[2 * qs + o] / by(q1);
   const R phiSq = (R)0.5 * (u * u + v * v);
-  const R ge = S.q[3 * qs + o] / q1 * gamma - phiSq * gm1;
-  const R aSq = (S.q[3 * qs + o] / q1 - phiSq) * gm1 * gamma;
+  const R ge = S.q[3 * qs + o] / by(q1) * gamma - phiSq * gm1;
+  const R aSq = (S.q[3 * qs + o] / by(q1) - phiSq) * gm1 * gamma;
   const R t1 = s[0], t2 = s[1], t3 = s[2], t4 = s[3];
   const R a = phiSq * t1 - u * t2 - v * t3 + t4;
   const R btv = S.bt[o];
-  const R bSq = mp2 / (btv - mp2 * (btv - (R)1));
-  const R f = gm1 * (bSq - (R)1.) / aSq;
+  const R bSq = mp2 / by(btv - mp2 * (btv - (R)1));
+  const R f = gm1 * (bSq - (R)1.) / by(aSq);
   s[0] = a * f + t1;
   s[1] = (u * a) * f + t2;
   s[2] = (v * a) * f + t3;
@@ -554,7 +554,7 @@ __device__ void resid_tile(const Slice<R>& S, const RtSmem<R, TJ, TK>& sm, int t
         for (int n = 0; n < 8; ++n) {
           if (n >= nv) continue;
           const int64_t on = (int64_t)n * S.qs + o;
-          const double ssv = 0.0 - (S.q64[on] - S.qnewt[on]) / (double)ts;
+          const double ssv = 0.0 - (S.q64[on] - S.qnewt[on]) / by((double)ts);
           s[n] = s[n] + (R)ssv;
         }
       }

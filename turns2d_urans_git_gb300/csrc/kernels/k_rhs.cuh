@@ -20,36 +20,36 @@ __device__ __forceinline__ void time_step_vals(const Slice<R>& S, const ot2d_par
   R jac_factor = p.invisc ? (R)0.01 : (R)0.002;
   if (p.iconstant_cfl == 0) {
     if (p.idual == 0) {
-      S.tscale[o] = oat * h * ib * ((R)1.0 + jac_factor * ((R)1. - timeac) * sqrt(J)) / ((R)1.0 + ((R)1. - timeac) * sqrt(J));
+      S.tscale[o] = oat * h * ib * ((R)1.0 + jac_factor * ((R)1. - timeac) * root(J)) / by((R)1.0 + ((R)1. - timeac) * root(J));
       S.bt[o] = (R)1.;
     } else {
-      R t = ib * ((R)1.0 + jac_factor * sqrt(J)) / ((R)1.0 + sqrt(J));
-      if (p.iprecon) t = (R)100. * ib * ((R)1.0 + (R)0.005 * sqrt(J)) / ((R)1.0 + sqrt(J));   // time.f:62-66
+      R t = ib * ((R)1.0 + jac_factor * root(J)) / by((R)1.0 + root(J));
+      if (p.iprecon) t = (R)100. * ib * ((R)1.0 + (R)0.005 * root(J)) / by((R)1.0 + root(J));   // time.f:62-66
       t = t * S.k_dualtime;
-      S.bt[o] = (R)1. / ((R)1. + t / h / oat);
-      S.tscale[o] = t / ((R)1. + t / h / oat);
+      S.bt[o] = (R)1. / by((R)1. + t / by(h) / by(oat));
+      S.tscale[o] = t / by((R)1. + t / by(h) / by(oat));
     }
     return;
   }
-  R u = q2 / q1, v = q3 / q1, e = q4 / q1;
+  R u = q2 / by(q1), v = q3 / by(q1), e = q4 / by(q1);
   R ugc = S.ug ? S.ug[o] : (R)0, vgc = S.vg ? S.vg[o] : (R)0;
   R xx = S.xx[o], xy = S.xy[o], yx = S.yx[o], yy = S.yy[o];
   R uu = (u - ugc) * xx + (v - vgc) * xy;
   R vv = (u - ugc) * yx + (v - vgc) * yy;
   R dxdx = sq(xx) + sq(xy), dydy = sq(yx) + sq(yy);
   R asq = S.k_ggm1 * (e - (R)0.5 * (sq(u) + sq(v)));
-  R lam_j = fabs(uu) + sqrt(asq * dxdx);
-  R lam_k = fabs(vv) + sqrt(asq * dydy);
+  R lam_j = fabs(uu) + root(asq * dxdx);
+  R lam_k = fabs(vv) + root(asq * dydy);
   if (p.idual == 0) {
-    R t = h / (lam_j + lam_k);
+    R t = h / by(lam_j + lam_k);
     S.tscale[o] = t * ib;
     S.bt[o] = (R)1.;
   } else {
-    R hnew = S.k_dualtime / (lam_j + lam_k);
+    R hnew = S.k_dualtime / by(lam_j + lam_k);
     R t = hnew * ib;
-    t = t / ((R)1. + t / h / oat);
+    t = t / by((R)1. + t / by(h) / by(oat));
     S.tscale[o] = t;
-    S.bt[o] = (R)1. / ((R)1. + t / h / oat);
+    S.bt[o] = (R)1. / by((R)1. + t / by(h) / by(oat));
   }
 }
 template <class R>
@@ -80,18 +80,18 @@ struct LineRd {
     int64_t o = off(i);
     R q1 = q[o];
     if (n == 1) return q1 * q[(nq - 1) * qs + o];
-    if (n == 2) { R rhoi = (R)1.0 / q1; return q[qs + o] * rhoi; }
-    if (n == 3) { R rhoi = (R)1.0 / q1; return q[2 * qs + o] * rhoi; }
+    if (n == 2) { R rhoi = (R)1.0 / by(q1); return q[qs + o] * rhoi; }
+    if (n == 3) { R rhoi = (R)1.0 / by(q1); return q[2 * qs + o] * rhoi; }
     R q2 = q[qs + o], q3 = q[2 * qs + o];
-    R ppp = gm1 * (q[3 * qs + o] - (R)0.5 * (sq(q2) + sq(q3)) / q1);
+    R ppp = gm1 * (q[3 * qs + o] - (R)0.5 * (sq(q2) + sq(q3)) / by(q1));
     return ppp * q[(nq - 1) * qs + o];
   }
   __device__ __forceinline__ void f4(int i, R* out) const {
     int64_t o = off(i);
     R q1 = q[o], q2 = q[qs + o], q3 = q[2 * qs + o], q4 = q[3 * qs + o], J = q[(nq - 1) * qs + o];
-    R rhoi = (R)1.0 / q1;
+    R rhoi = (R)1.0 / by(q1);
     out[0] = q1 * J; out[1] = q2 * rhoi; out[2] = q3 * rhoi;
-    R ppp = gm1 * (q4 - (R)0.5 * (sq(q2) + sq(q3)) / q1);
+    R ppp = gm1 * (q4 - (R)0.5 * (sq(q2) + sq(q3)) / by(q1));
     out[3] = ppp * J;
   }
   __device__ __forceinline__ int iba(int i) const { int v = ib[off(i)]; return v < 0 ? -v : v; }
@@ -111,9 +111,9 @@ template <class R> __device__ __forceinline__ R weno5(R a, R b, R c, R d, R e) {
   R dis1 = b1 * dj * dj + (R)0.25 * ej * ej + epsw;
   R dis2 = b1 * djp1 * djp1 + (R)0.25 * ejp1 * ejp1 + epsw;
   R q30 = (R)2. * a - (R)7. * b + (R)11. * c, q31 = -b + (R)5. * c + (R)2. * d, q32 = (R)2. * c + (R)5. * d - e;
-  R d01 = dis0 / dis1, d02 = dis0 / dis2;
+  R d01 = dis0 / by(dis1), d02 = dis0 / by(dis2);
   R a1ba0 = (R)6. * d01, a2ba0 = (R)3. * d02;
-  R w0 = (R)1. / ((R)1. + a1ba0 + a2ba0);
+  R w0 = (R)1. / by((R)1. + a1ba0 + a2ba0);
   R w1 = a1ba0 * w0;
   R w2 = (R)1. - w0 - w1;
   return b2 * (w0 * q30 + w1 * q31 + w2 * q32);
@@ -137,7 +137,7 @@ struct Recon {
     R f2i = wp - w0, f2i1 = w0 - wm;
     R a1 = (R)3.0 * (f2i * f2i1 + epsl);
     R a2 = (R)2.0 * sq(f2i - f2i1) + a1;
-    R f3i = a1 / a2;
+    R f3i = a1 / by(a2);
     R f3qt = qt * f3i * (R)ib0 * (R)ibp * (R)ibm;
     ql = w0 + f3qt * (thm * f2i1 + thp * f2i);
     qr = w0 - f3qt * (thp * f2i1 + thm * f2i);
@@ -192,35 +192,35 @@ template <class R>
 __device__ __forceinline__ void roe(R gm1, const R* L, const R* Rr, R ri1, R ri2, R ri3, R* f) {
   const R eps = (R)1.e-6;
   R rlft = L[0], ulft = L[1], vlft = L[2], plft = L[3];
-  R rlfti = (R)1.0 / rlft;
+  R rlfti = (R)1.0 / by(rlft);
   R rulft = rlft * ulft, rvlft = rlft * vlft;
   R uvl = (R)0.5 * (ulft * ulft + vlft * vlft);
-  R elft = plft / gm1 + rlft * uvl;
+  R elft = plft / by(gm1) + rlft * uvl;
   R hlft = (elft + plft) * rlfti;
-  R clft = sqrt(gm1 * (hlft - uvl));
+  R clft = root(gm1 * (hlft - uvl));
   R rrht = Rr[0], urht = Rr[1], vrht = Rr[2], prht = Rr[3];
-  R rrhti = (R)1.0 / rrht;
+  R rrhti = (R)1.0 / by(rrht);
   R rurht = rrht * urht, rvrht = rrht * vrht;
   R uvr = (R)0.5 * (urht * urht + vrht * vrht);
-  R erht = prht / gm1 + rrht * uvr;
+  R erht = prht / by(gm1) + rrht * uvr;
   R hrht = (erht + prht) * rrhti;
-  R crht = sqrt(gm1 * (hrht - uvr));
-  R rat = sqrt(rrht * rlfti);
-  R rati = (R)1.0 / (rat + (R)1.);
+  R crht = root(gm1 * (hrht - uvr));
+  R rat = root(rrht * rlfti);
+  R rati = (R)1.0 / by(rat + (R)1.);
   R rav = rat * rlft;
   R uav = (rat * urht + ulft) * rati;
   R vav = (rat * vrht + vlft) * rati;
   R hav = (rat * hrht + hlft) * rati;
   R uv = (R)0.5 * (uav * uav + vav * vav);
-  R cav = sqrt(gm1 * (hav - uv));
+  R cav = root(gm1 * (hav - uv));
   R aq1 = rrht - rlft, aq2 = urht - ulft, aq3 = vrht - vlft, aq4 = prht - plft;
   R rr2 = ri1 * ri1 + ri2 * ri2;
-  R rr = sqrt(rr2);
-  R r0 = (R)1.0 / rr;
+  R rr = root(rr2);
+  R r0 = (R)1.0 / by(rr);
   R r1 = ri1 * r0, r2 = ri2 * r0, r3 = ri3 * r0;
   R uu = r1 * uav + r2 * vav + r3;
   R c2 = cav * cav;
-  R c2i = (R)1.0 / c2;
+  R c2i = (R)1.0 / by(c2);
   R auu = fabs(uu), aupc = fabs(uu + cav), aumc = fabs(uu - cav);
   R uulft = r1 * ulft + r2 * vlft + r3;
   R uurht = r1 * urht + r2 * vrht + r3;
@@ -228,13 +228,13 @@ __device__ __forceinline__ void roe(R gm1, const R* L, const R* Rr, R ri1, R ri2
   R umclft = uulft - clft, umcrht = uurht - crht;
   R dauu = (R)4. * (uurht - uulft) + eps;
   R dauus = fmax2(dauu, (R)0.0);
-  if (auu <= (R)0.5 * dauus) auu = auu * auu / dauu + (R)0.25 * dauu;
+  if (auu <= (R)0.5 * dauus) auu = auu * auu / by(dauu) + (R)0.25 * dauu;
   R daupc = (R)4. * (upcrht - upclft) + eps;
   R daupcs = fmax2(daupc, (R)0.0);
-  if (aupc <= (R)0.5 * daupcs) aupc = aupc * aupc / daupc + (R)0.25 * daupc;
+  if (aupc <= (R)0.5 * daupcs) aupc = aupc * aupc / by(daupc) + (R)0.25 * daupc;
   R daumc = (R)4. * (umcrht - umclft) + eps;
   R daumcs = fmax2(daumc, (R)0.0);
-  if (aumc <= (R)0.5 * daumcs) aumc = aumc * aumc / daumc + (R)0.25 * daumc;
+  if (aumc <= (R)0.5 * daumcs) aumc = aumc * aumc / by(daumc) + (R)0.25 * daumc;
   R rcav = rav * cav;
   R aquu = uurht - uulft;
   R c2ih = (R)0.5 * c2i;
@@ -249,7 +249,7 @@ __device__ __forceinline__ void roe(R gm1, const R* L, const R* Rr, R ri1, R ri2
   aq1 = b4;
   aq2 = uav * b4 + r1 * b5 + b6;
   aq3 = vav * b4 + r2 * b5 + b7;
-  aq4 = hav * b4 + (uu - r3) * b5 + uav * b6 + vav * b7 - c2 * b1 / gm1;
+  aq4 = hav * b4 + (uu - r3) * b5 + uav * b6 + vav * b7 - c2 * b1 / by(gm1);
   R aj = (R)0.5 * rr;
   R plar = plft + prht;
   R eplft = elft + plft, eprht = erht + prht;
@@ -269,66 +269,66 @@ template <class R>
 __device__ __forceinline__ void roe_turkel(R gm1, R bSq, const R* L, const R* Rr, R ri1, R ri2, R ri3, R* f) {
   const R eps = (R)1.e-6;
   R rlft = L[0], ulft = L[1], vlft = L[2], plft = L[3];
-  R rlfti = (R)1.0 / rlft;
+  R rlfti = (R)1.0 / by(rlft);
   R rulft = rlft * ulft, rvlft = rlft * vlft;
   R uvl = (R)0.5 * (ulft * ulft + vlft * vlft);
-  R elft = plft / gm1 + rlft * uvl;
+  R elft = plft / by(gm1) + rlft * uvl;
   R hlft = (elft + plft) * rlfti;
-  R clft = sqrt(gm1 * (hlft - uvl));
+  R clft = root(gm1 * (hlft - uvl));
   R rrht = Rr[0], urht = Rr[1], vrht = Rr[2], prht = Rr[3];
-  R rrhti = (R)1.0 / rrht;
+  R rrhti = (R)1.0 / by(rrht);
   R rurht = rrht * urht, rvrht = rrht * vrht;
   R uvr = (R)0.5 * (urht * urht + vrht * vrht);
-  R erht = prht / gm1 + rrht * uvr;
+  R erht = prht / by(gm1) + rrht * uvr;
   R hrht = (erht + prht) * rrhti;
-  R crht = sqrt(gm1 * (hrht - uvr));
-  R rat = sqrt(rrht * rlfti);
-  R rati = (R)1.0 / (rat + (R)1.);
+  R crht = root(gm1 * (hrht - uvr));
+  R rat = root(rrht * rlfti);
+  R rati = (R)1.0 / by(rat + (R)1.);
   R rav = rat * rlft;
   R uav = (rat * urht + ulft) * rati;
   R vav = (rat * vrht + vlft) * rati;
   R hav = (rat * hrht + hlft) * rati;
   R uv = (R)0.5 * (uav * uav + vav * vav);
-  R cav = sqrt(gm1 * (hav - uv));
+  R cav = root(gm1 * (hav - uv));
   R aq1 = rrht - rlft, aq2 = urht - ulft, aq3 = vrht - vlft, aq4 = prht - plft;
   R rr2 = ri1 * ri1 + ri2 * ri2;
-  R rr = sqrt(rr2);
-  R r0 = (R)1.0 / rr;
+  R rr = root(rr2);
+  R r0 = (R)1.0 / by(rr);
   R r1 = ri1 * r0, r2 = ri2 * r0, r3 = ri3 * r0;
   R uumxt = r1 * uav + r2 * vav;
   R uu = uumxt + r3;
   R c2 = cav * cav;
-  R c2i = (R)1.0 / c2;
+  R c2i = (R)1.0 / by(c2);
   const R omb = (R)1. - bSq, opb = (R)1. + bSq, fb = (R)4. * bSq;
-  R X = sqrt(((omb * uu) * omb) * uu + fb * c2);
+  R X = root(((omb * uu) * omb) * uu + fb * c2);
   R auu = fabs(uu);
   R aupc = (R)0.5 * fabs(opb * uu + X);
   R aumc = (R)0.5 * fabs(opb * uu - X);
   R uulft = r1 * ulft + r2 * vlft + r3;
   R uurht = r1 * urht + r2 * vrht + r3;
-  X = sqrt((omb * uulft) * (omb * uulft) + (fb * clft) * clft);
+  X = root((omb * uulft) * (omb * uulft) + (fb * clft) * clft);
   R upclft = (R)0.5 * (opb * uulft + X);
   R umclft = (R)0.5 * (opb * uulft - X);
-  X = sqrt((omb * uurht) * (omb * uurht) + (fb * crht) * crht);
+  X = root((omb * uurht) * (omb * uurht) + (fb * crht) * crht);
   R upcrht = (R)0.5 * (opb * uurht + X);
   R umcrht = (R)0.5 * (opb * uurht - X);
   R dauu = (R)4. * (uurht - uulft) + eps;
   R dauus = fmax2(dauu, (R)0.0);
-  if (auu <= (R)0.5 * dauus) auu = auu * auu / dauu + (R)0.25 * dauu;
+  if (auu <= (R)0.5 * dauus) auu = auu * auu / by(dauu) + (R)0.25 * dauu;
   R daupc = (R)4. * (upcrht - upclft) + eps;
   R daupcs = fmax2(daupc, (R)0.0);
-  if (aupc <= (R)0.5 * daupcs) aupc = aupc * aupc / daupc + (R)0.25 * daupc;
+  if (aupc <= (R)0.5 * daupcs) aupc = aupc * aupc / by(daupc) + (R)0.25 * daupc;
   R daumc = (R)4. * (umcrht - umclft) + eps;
   R daumcs = fmax2(daumc, (R)0.0);
-  if (aumc <= (R)0.5 * daumcs) aumc = aumc * aumc / daumc + (R)0.25 * daumc;
+  if (aumc <= (R)0.5 * daumcs) aumc = aumc * aumc / by(daumc) + (R)0.25 * daumc;
   R aquu = uurht - uulft;
   R ruuav = auu * rav;
-  X = sqrt((omb * uu) * (omb * uu) + fb * c2);
+  X = root((omb * uu) * (omb * uu) + fb * c2);
   R Rw = (R)0.5 * (omb * uu + X);
   R Sw = (R)0.5 * (omb * uu - X);
   R b1 = auu * (aq1 - c2i * aq4);
-  R b2 = aupc * (aq4 / Rw + rav * aquu) / X;
-  R b3 = aumc * (-(aq4 / Sw) - rav * aquu) / X;
+  R b2 = aupc * (aq4 / by(Rw) + rav * aquu) / by(X);
+  R b3 = aumc * (-(aq4 / by(Sw)) - rav * aquu) / by(X);
   R b4 = b1 + b2 + b3;
   R b5 = (Rw * b2 + Sw * b3);
   R b6 = ruuav * (aq2 - r1 * aquu);
@@ -336,7 +336,7 @@ __device__ __forceinline__ void roe_turkel(R gm1, R bSq, const R* L, const R* Rr
   aq1 = b4;
   aq2 = uav * b4 + r1 * b5 + b6;
   aq3 = vav * b4 + r2 * b5 + b7;
-  aq4 = hav * b4 + uumxt * b5 + uav * b6 + vav * b7 - c2 * b1 / gm1;
+  aq4 = hav * b4 + uumxt * b5 + uav * b6 + vav * b7 - c2 * b1 / by(gm1);
   R aj = (R)0.5 * rr;
   R plar = plft + prht;
   R eplft = elft + plft, eprht = erht + prht;
@@ -441,9 +441,9 @@ template <class R>
 __device__ __forceinline__ Recon<R> make_recon(const ot2d_params& p, int dir) {
   Recon<R> rc;
   int irhs = p.irhsy < 0 ? -p.irhsy : p.irhsy;
-  rc.th = (R)((double)(irhs - 2) / (double)irhs);
+  rc.th = (R)((double)(irhs - 2) / by((double)irhs));
   rc.qt = (irhs == 1) ? (R)0.0 : (R)0.25;
-  double ep = (dir == 0) ? 10. / (double)p.jmax : 10. / (double)p.kmax;
+  double ep = (dir == 0) ? 10. / by((double)p.jmax) : 10. / by((double)p.kmax);
   rc.epsl = (R)((ep * ep) * ep);
   rc.ilim = p.ilim;
   rc.bsq = p.iprecon ? (R)(p.Mp * p.Mp) : (R)-1;
@@ -489,14 +489,14 @@ __device__ __forceinline__ ViscCell<R> visc_cell(const Slice<R>& S, const ot2d_p
   const int64_t o = at(S.jd, j, k), qs = S.qs;
   const R c2b = S.k_c2b, c2bp = S.k_c2bp, prtr = S.k_prtr;
   ViscCell<R> c;
-  R ra = (R)1. / S.q[o];
+  R ra = (R)1. / by(S.q[o]);
   c.u = S.q[qs + o] * ra; c.v = S.q[2 * qs + o] * ra;
   c.e = S.q[3 * qs + o] * ra - (R).5 * (sq(c.u) + sq(c.v));
   R tt = S.k_ggm1 * c.e;
-  R vmue = c2bp * tt * sqrt(tt) / (c2b + tt);
+  R vmue = c2bp * tt * root(tt) / by(c2b + tt);
   R turm = S.turmu[o];
   c.vnu = vmue + turm; c.gkap = vmue + prtr * turm;
-  c.rj = (R)1. / S.q[(p.nq - 1) * qs + o];
+  c.rj = (R)1. / by(S.q[(p.nq - 1) * qs + o]);
   return c;
 }
 
@@ -516,12 +516,12 @@ __device__ void visc_eta_face(const Slice<R>& S, int j, int k, R* V) {
     uu[m] = c.u; vv[m] = c.v; ee[m] = c.e;
     R yx = M(S.yx, j, kk), yy = M(S.yy, j, kk);
     R b4 = (sq(yx) + sq(yy)) * c.rj;
-    bv[m][0] = (b4 + sq(yx) / (R)3. * c.rj) * c.vnu * dre;
-    bv[m][1] = (b4 + sq(yy) / (R)3. * c.rj) * c.vnu * dre;
-    bv[m][3] = (yx * yy / (R)3. * c.rj) * c.vnu * dre;
+    bv[m][0] = (b4 + sq(yx) / by((R)3.) * c.rj) * c.vnu * dre;
+    bv[m][1] = (b4 + sq(yy) / by((R)3.) * c.rj) * c.vnu * dre;
+    bv[m][3] = (yx * yy / by((R)3.) * c.rj) * c.vnu * dre;
     bv[m][2] = b4 * gkpr * c.gkap * dre;
     if (m == 0) {
-      R rjm = (R)1. / S.q[(p.nq - 1) * qs + at(jd, j - 1, kk)], rjp = (R)1. / S.q[(p.nq - 1) * qs + at(jd, j + 1, kk)];
+      R rjm = (R)1. / by(S.q[(p.nq - 1) * qs + at(jd, j - 1, kk)]), rjp = (R)1. / by(S.q[(p.nq - 1) * qs + at(jd, j + 1, kk)]);
       R xxm = M(S.xx, j - 1, kk), xym = M(S.xy, j - 1, kk), yxm = M(S.yx, j - 1, kk), yym = M(S.yy, j - 1, kk);
       R xxp = M(S.xx, j + 1, kk), xyp = M(S.xy, j + 1, kk), yxp = M(S.yx, j + 1, kk), yyp = M(S.yy, j + 1, kk);
       d1 = ((R)(4. / 3.) * xxm * yxm + xym * yym) * rjm;
@@ -543,12 +543,12 @@ __device__ void visc_eta_face(const Slice<R>& S, int j, int k, R* V) {
   }
   R b1 = bv[1][0] + bv[0][0], b2 = bv[1][1] + bv[0][1], b5 = bv[1][3] + bv[0][3];
   const int64_t op = at(jd, j + 1, k), om = at(jd, j - 1, k);
-  R ujp1 = S.q[qs + op] / S.q[op], ujm1 = S.q[qs + om] / S.q[om];
+  R ujp1 = S.q[qs + op] / by(S.q[op]), ujm1 = S.q[qs + om] / by(S.q[om]);
   R duj = (R)0.5 * (ujp1 - ujm1);
-  R vjp1 = S.q[2 * qs + op] / S.q[op], vjm1 = S.q[2 * qs + om] / S.q[om];
+  R vjp1 = S.q[2 * qs + op] / by(S.q[op]), vjm1 = S.q[2 * qs + om] / by(S.q[om]);
   R dvj = (R)0.5 * (vjp1 - vjm1);
-  R ejp1 = S.q[3 * qs + op] / S.q[op] - (R).5 * (sq(ujp1) + sq(vjp1));
-  R ejm1 = S.q[3 * qs + om] / S.q[om] - (R).5 * (sq(ujm1) + sq(vjm1));
+  R ejp1 = S.q[3 * qs + op] / by(S.q[op]) - (R).5 * (sq(ujp1) + sq(vjp1));
+  R ejm1 = S.q[3 * qs + om] / by(S.q[om]) - (R).5 * (sq(ujm1) + sq(vjm1));
   R dej = (R)0.5 * (ejp1 - ejm1);
   R t4 = uu[1] * bv[1][0] + uu[0] * bv[0][0];
   R t5 = vv[1] * bv[1][1] + vv[0] * bv[0][1];
@@ -586,12 +586,12 @@ __device__ void visc_xi_face(const Slice<R>& S, int j, int k, R* V) {
     uu[m] = c.u; vv[m] = c.v; ee[m] = c.e;
     R xx = M(S.xx, jj, k), xy = M(S.xy, jj, k);
     R a4 = (sq(xx) + sq(xy)) * c.rj;
-    av[m][0] = (a4 + sq(xx) / (R)3. * c.rj) * c.vnu * dre;
-    av[m][1] = (a4 + sq(xy) / (R)3. * c.rj) * c.vnu * dre;
-    av[m][3] = (xx * xy / (R)3. * c.rj) * c.vnu * dre;
+    av[m][0] = (a4 + sq(xx) / by((R)3.) * c.rj) * c.vnu * dre;
+    av[m][1] = (a4 + sq(xy) / by((R)3.) * c.rj) * c.vnu * dre;
+    av[m][3] = (xx * xy / by((R)3.) * c.rj) * c.vnu * dre;
     av[m][2] = a4 * gkpr * c.gkap * dre;
     if (m == 0) {
-      R rkm = (R)1. / S.q[(p.nq - 1) * qs + at(jd, jj, k - 1)], rkp = (R)1. / S.q[(p.nq - 1) * qs + at(jd, jj, k + 1)];
+      R rkm = (R)1. / by(S.q[(p.nq - 1) * qs + at(jd, jj, k - 1)]), rkp = (R)1. / by(S.q[(p.nq - 1) * qs + at(jd, jj, k + 1)]);
       R xxm = M(S.xx, jj, k - 1), xym = M(S.xy, jj, k - 1), yxm = M(S.yx, jj, k - 1), yym = M(S.yy, jj, k - 1);
       R xxp = M(S.xx, jj, k + 1), xyp = M(S.xy, jj, k + 1), yxp = M(S.yx, jj, k + 1), yyp = M(S.yy, jj, k + 1);
       d1 = ((R)(4. / 3.) * xxm * yxm + xym * yym) * rkm;
@@ -613,12 +613,12 @@ __device__ void visc_xi_face(const Slice<R>& S, int j, int k, R* V) {
   }
   R a1 = av[1][0] + av[0][0], a2 = av[1][1] + av[0][1], a5 = av[1][3] + av[0][3];
   const int64_t op = at(jd, j, k + 1), om = at(jd, j, k - 1);
-  R ukp1 = S.q[qs + op] / S.q[op], ukm1 = S.q[qs + om] / S.q[om];
+  R ukp1 = S.q[qs + op] / by(S.q[op]), ukm1 = S.q[qs + om] / by(S.q[om]);
   R duk = (R)0.5 * (ukp1 - ukm1);
-  R vkp1 = S.q[2 * qs + op] / S.q[op], vkm1 = S.q[2 * qs + om] / S.q[om];
+  R vkp1 = S.q[2 * qs + op] / by(S.q[op]), vkm1 = S.q[2 * qs + om] / by(S.q[om]);
   R dvk = (R)0.5 * (vkp1 - vkm1);
-  R ekp1 = S.q[3 * qs + op] / S.q[op] - (R).5 * (sq(ukp1) + sq(vkp1));
-  R ekm1 = S.q[3 * qs + om] / S.q[om] - (R).5 * (sq(ukm1) + sq(vkm1));
+  R ekp1 = S.q[3 * qs + op] / by(S.q[op]) - (R).5 * (sq(ukp1) + sq(vkp1));
+  R ekm1 = S.q[3 * qs + om] / by(S.q[om]) - (R).5 * (sq(ukm1) + sq(vkm1));
   R dek = (R)0.5 * (ekp1 - ekm1);
   R t4 = uu[1] * av[1][0] + uu[0] * av[0][0];
   R t5 = vv[1] * av[1][1] + vv[0] * av[0][1];

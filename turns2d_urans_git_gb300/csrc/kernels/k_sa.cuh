@@ -38,13 +38,13 @@ __device__ __forceinline__ void sa_prep_cell(const Slice<R>& S, const ot2d_param
   const int64_t o = at(S.jd, j, k), qs = S.qs, ws = S.wstride;
   const R c2b = S.k_c2b, c2bp = S.k_c2bp;
   R q1 = S.q[o], q2 = S.q[qs + o], q3 = S.q[2 * qs + o], q4 = S.q[3 * qs + o];
-  R ra = (R)1. / q1;
+  R ra = (R)1. / by(q1);
   R uvel = q2 * ra, vvel = q3 * ra;
   R ei = q4 * ra - (R)0.5 * (sq(uvel) + sq(vvel));
   R tt = S.k_ggm1 * ei;
-  S.w[W_VMUL * ws + o] = c2bp * tt * sqrt(tt) / (c2b + tt);
-  S.w[W_U * ws + o] = q2 / q1;
-  S.w[W_V * ws + o] = q3 / q1;
+  S.w[W_VMUL * ws + o] = c2bp * tt * root(tt) / by(c2b + tt);
+  S.w[W_U * ws + o] = q2 / by(q1);
+  S.w[W_V * ws + o] = q3 / by(q1);
 }
 
 template <class R>
@@ -111,8 +111,8 @@ __device__ void sa_rhs_cell(const Slice<R>& S, const ot2d_params& p, int j, int 
   if (k <= ke - 1) ck = ck + ((c0.vm < (R)-1.0e-12) ? (R)1.0 : (R)0.0) * (ckp.vp + ckp.vm);
   R bk = (R)0. + c0.vp - c0.vm;
   // ---- diffus
-  const R chpc = (R)((1. + SAc::cb2) / SAc::sigma) / rey;
-  const R c2c = (R)(SAc::cb2 / SAc::sigma) / rey;
+  const R chpc = (R)((1. + SAc::cb2) / SAc::sigma) / by(rey);
+  const R c2c = (R)(SAc::cb2 / SAc::sigma) / by(rey);
   auto nul = [&](int jj, int kk) { return a.nul(jj, kk); };
   {
     // half points j-1/2 (index j-1) and j+1/2 (index j)
@@ -160,41 +160,41 @@ __device__ void sa_rhs_cell(const Slice<R>& S, const ot2d_params& p, int j, int 
       d = S.sn[o];
     }
     R vnul = a.nul(j, k);
-    R chi = q5 / vnul;
+    R chi = q5 / by(vnul);
     chi = fmax2(chi, (R)1.e-12);
-    R fv1 = (cube(chi)) / (cube(chi) + cube(cv1));
-    R fv2 = (R)1. - chi / ((R)1. + chi * fv1);
+    R fv1 = (cube(chi)) / by(cube(chi) + cube(cv1));
+    R fv2 = (R)1. - chi / by((R)1. + chi * fv1);
     R fv3 = (R)1.0;
     // ft2 = fturf * ct3 * exp(-ct4 chi^2) with fturf = 0: +0 exactly (the
     // exponential is finite and positive), so it is not evaluated
     R ft2 = (R)0.0;
     (void)fturf; (void)ct3;
-    R dchi = (R)1. / vnul;
-    R dfv1 = ((R)3. * cube(cv1)) * (sq(chi)) * dchi * sq((R)1. / (cube(chi) + cube(cv1)));
-    R dfv2 = (fv2 - (R)1.) / chi / vnul + ((R)1. - fv2) * ((R)1 - fv2) * (dfv1 + fv1 / chi / vnul);
+    R dchi = (R)1. / by(vnul);
+    R dfv1 = ((R)3. * cube(cv1)) * (sq(chi)) * dchi * sq((R)1. / by(cube(chi) + cube(cv1)));
+    R dfv2 = (fv2 - (R)1.) / by(chi) / by(vnul) + ((R)1. - fv2) * ((R)1 - fv2) * (dfv1 + fv1 / by(chi) / by(vnul));
     R dfv3 = (R)0.0;
     R dft2 = ((R)-2. * ct4) * chi * dchi * ft2;
     R d2 = fmax2(sq(d), d2min);
-    R stilda = vort * fv3 + vnul / (d2 * akt * akt * rey) * chi * fv2;
+    R stilda = vort * fv3 + vnul / by(d2 * akt * akt * rey) * chi * fv2;
     stilda = fmax2(stilda, stilim);
-    R r = q5 / (d2 * akt * akt * rey) / stilda;
+    R r = q5 / by(d2 * akt * akt * rey) / by(stilda);
     r = fmin2(r, rmax);
     R g = r + cw2 * (pow6(r) - r);
     // ((1 + cw3^6) / (g^6 + cw3^6))^(1/6), which fw and its derivative
     // both take (samodel2d.f:767-778): one power for the two
-    const R fw6 = sa_pow_pos(((R)1. + pow6(cw3)) / (pow6(g) + pow6(cw3)), (R)(1. / 6.));
+    const R fw6 = sa_pow_pos(((R)1. + pow6(cw3)) / by(pow6(g) + pow6(cw3)), (R)(1. / 6.));
     R fw = g * fw6;
-    R dstild = vort * dfv3 + vnul * (dchi * fv2 + chi * dfv2) / (d2 * akt * akt * rey);
-    R dr = vnul * (dchi - chi * dstild / stilda) / stilda / (d2 * akt * akt * rey);
+    R dstild = vort * dfv3 + vnul * (dchi * fv2 + chi * dfv2) / by(d2 * akt * akt * rey);
+    R dr = vnul * (dchi - chi * dstild / by(stilda)) / by(stilda) / by(d2 * akt * akt * rey);
     R dg = dr * ((R)1. + cw2 * ((R)6. * sa_pow5(r) - (R)1.));
     R dfw = fw6;
-    dfw = dfw * dg * ((R)1. - pow6(g) / (pow6(g) + pow6(cw3)));
+    dfw = dfw * dg * ((R)1. - pow6(g) / by(pow6(g) + pow6(cw3)));
     R pro = cb1 * stilda * ((R)1. - ft2);
-    R des = (cw1 * fw - cb1 / (akt * akt) * ft2) / d2 / rey;
+    R des = (cw1 * fw - cb1 / (akt * akt) * ft2) / by(d2) / by(rey);
     R prod = cb1 * stilda * ((R)1. - ft2) * q5;
-    R dest = (cw1 * fw - cb1 / (akt * akt) * ft2) * q5 * q5 / d2 / rey;
-    R dpro = pro * dstild / stilda - cb1 * stilda * dft2;
-    R ddes = (cw1 * dfw - cb1 / (akt * akt) * dft2) / d2 / rey * vnul * chi;
+    R dest = (cw1 * fw - cb1 / (akt * akt) * ft2) * q5 * q5 / by(d2) / by(rey);
+    R dpro = pro * dstild / by(stilda) - cb1 * stilda * dft2;
+    R ddes = (cw1 * dfw - cb1 / (akt * akt) * dft2) / by(d2) / by(rey) * vnul * chi;
     ddes = ddes + des;
     ddes = ddes * q5;
     dpro = dpro * q5;
@@ -207,16 +207,16 @@ __device__ void sa_rhs_cell(const Slice<R>& S, const ot2d_params& p, int j, int 
   R tscal = S.tscale[o];
   int ibi = S.iblank[o];
   if (p.cfltur > 1 && p.idual_turb == 1) {
-    R dtp = S.k_cfltur / (bj + bk);
+    R dtp = S.k_cfltur / by(bj + bk);
     tscal = dtp * (R)ibi;
-    tscal = tscal / ((R)1. + tscal / S.k_h);
+    tscal = tscal / by((R)1. + tscal / by(S.k_h));
   }
   if (p.timeac == 1) {
     R ib = (R)(ibi > 0 ? ibi : 0);
     R J = Q(j, k, nq);
-    tscal = ib * ((R)1.0 + (R)0.002 * sqrt(J)) / ((R)1. + sqrt(J));
+    tscal = ib * ((R)1.0 + (R)0.002 * root(J)) / by((R)1. + root(J));
     tscal = tscal * (R)1.0;
-    tscal = tscal / ((R)1. + tscal / S.k_h);
+    tscal = tscal / by((R)1. + tscal / by(S.k_h));
   }
   S.w[W_SJ * ws + o] = sj * tscal;
   S.w[W_AJ * ws + o] = aj * tscal;
@@ -270,9 +270,9 @@ __device__ __forceinline__ void sa_update_cell(const Slice<R>& S, const ot2d_par
   if constexpr (sizeof(R) != sizeof(double)) S.q[(int64_t)(n5 - 1) * qs + oo] = qv;
   // c_turm (samodel2d.f:372-399) with q5 as just stored
   const R rhoJ = q1 * J;
-  const R vnul = vm / rhoJ;
-  const R chi = qv / vnul;
-  const R fv1 = cube(chi) / (cube(chi) + cube(cv1));
+  const R vnul = vm / by(rhoJ);
+  const R chi = qv / by(vnul);
+  const R fv1 = cube(chi) / by(cube(chi) + cube(cv1));
   S.turmu[oo] = rhoJ * qv * fv1;
 }
 
@@ -282,10 +282,10 @@ __device__ __forceinline__ void sa_turm_cell(const Slice<R>& S, const ot2d_param
   const int64_t o = at(S.jd, j, k), qs = S.qs, ws = S.wstride;
   const R cv1 = (R)SAc::cv1;
   R rhoJ = S.q[o] * S.q[(p.nq - 1) * qs + o];
-  R vnul = S.w[W_VMUL * ws + o] / rhoJ;
+  R vnul = S.w[W_VMUL * ws + o] / by(rhoJ);
   R q5 = S.q[(int64_t)p.nmv * qs + o];
-  R chi = q5 / vnul;
-  R fv1 = cube(chi) / (cube(chi) + cube(cv1));
+  R chi = q5 / by(vnul);
+  R fv1 = cube(chi) / by(cube(chi) + cube(cv1));
   S.turmu[o] = rhoJ * q5 * fv1;
 }
 

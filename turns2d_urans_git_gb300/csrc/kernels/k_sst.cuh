@@ -43,14 +43,14 @@ __device__ __forceinline__ void sst_prep_cell(const Slice<R>& S, const ot2d_para
   const int64_t o = at(S.jd, j, k), qs = S.qs, ws = S.wstride;
   const R c2b = S.k_c2b, c2bp = S.k_c2bp;
   const R q1 = S.q[o], q2 = S.q[qs + o], q3 = S.q[2 * qs + o], q4 = S.q[3 * qs + o], J = S.q[(p.nq - 1) * qs + o];
-  const R ra = (R)1. / q1;
+  const R ra = (R)1. / by(q1);
   const R uvel = q2 * ra, vvel = q3 * ra;
   const R ei = q4 * ra - (R)0.5 * (sq(uvel) + sq(vvel));
   const R tt = S.k_ggm1 * ei;
-  S.w[K_VMUL * ws + o] = c2bp * tt * sqrt(tt) / (c2b + tt);
+  S.w[K_VMUL * ws + o] = c2bp * tt * root(tt) / by(c2b + tt);
   S.w[K_RHO * ws + o] = q1 * J;
-  S.w[K_U * ws + o] = q2 / q1;
-  S.w[K_V * ws + o] = q3 / q1;
+  S.w[K_U * ws + o] = q2 / by(q1);
+  S.w[K_V * ws + o] = q3 / by(q1);
   if (j < p.jbeg || j > p.jend || k < p.kbeg || k > p.kend) {
     S.w[K_STRAIN * ws + o] = (R)0;
     S.w[K_F1 * ws + o] = (R)0;
@@ -69,7 +69,7 @@ __device__ void sst_fields_cell(const Slice<R>& S, const ot2d_params& p, int j, 
   auto Q = [&](int jj, int kk, int n) { return S.q[(int64_t)(n - 1) * qs + at(jd, jj, kk)]; };
   const int64_t o = at(jd, j, k);
   const R xx = S.xx[o], xy = S.xy[o], yx = S.yx[o], yy = S.yy[o];
-  const R rei = (R)1. / S.k_rey;
+  const R rei = (R)1. / by(S.k_rey);
   // kwvortic / turbstress share the velocity gradients
   const R usi = (R)0.5 * (W(K_U, j + 1, k) - W(K_U, j - 1, k)), vsi = (R)0.5 * (W(K_V, j + 1, k) - W(K_V, j - 1, k));
   const R ueta = (R)0.5 * (W(K_U, j, k + 1) - W(K_U, j, k - 1)), veta = (R)0.5 * (W(K_V, j, k + 1) - W(K_V, j, k - 1));
@@ -77,7 +77,7 @@ __device__ void sst_fields_cell(const Slice<R>& S, const ot2d_params& p, int j, 
   const R vx = xx * vsi + yx * veta, vy = xy * vsi + yy * veta;
   {
     const R sxx = ux, sxy = (R)0.5 * (uy + vx), syy = vy;
-    S.w[K_STRAIN * ws + o] = sqrt((R)2. * (sxx * sxx + (R)2. * sxy * sxy + syy * syy));
+    S.w[K_STRAIN * ws + o] = root((R)2. * (sxx * sxx + (R)2. * sxy * sxy + syy * syy));
   }
   S.w[K_UX * ws + o] = ux; S.w[K_UY * ws + o] = uy; S.w[K_VX * ws + o] = vx; S.w[K_VY * ws + o] = vy;
   const R sfdiv = (R)(2. / 3) * (ux + vy);
@@ -87,21 +87,21 @@ __device__ void sst_fields_cell(const Slice<R>& S, const ot2d_params& p, int j, 
   S.w[K_TXY * ws + o] = tm * rei * (uy + vx);
   // crossdiff
   const R rho = W(K_RHO, j, k);
-  const R ksi = (R)0.5 * (Q(j + 1, k, nmv + 1) / W(K_RHO, j + 1, k) - Q(j - 1, k, nmv + 1) / W(K_RHO, j - 1, k));
-  const R keta = (R)0.5 * (Q(j, k + 1, nmv + 1) / W(K_RHO, j, k + 1) - Q(j, k - 1, nmv + 1) / W(K_RHO, j, k - 1));
-  const R omegasi = (R)0.5 * (Q(j + 1, k, nmv + 2) / W(K_RHO, j + 1, k) - Q(j - 1, k, nmv + 2) / W(K_RHO, j - 1, k));
-  const R omegaeta = (R)0.5 * (Q(j, k + 1, nmv + 2) / W(K_RHO, j, k + 1) - Q(j, k - 1, nmv + 2) / W(K_RHO, j, k - 1));
+  const R ksi = (R)0.5 * (Q(j + 1, k, nmv + 1) / by(W(K_RHO, j + 1, k)) - Q(j - 1, k, nmv + 1) / by(W(K_RHO, j - 1, k)));
+  const R keta = (R)0.5 * (Q(j, k + 1, nmv + 1) / by(W(K_RHO, j, k + 1)) - Q(j, k - 1, nmv + 1) / by(W(K_RHO, j, k - 1)));
+  const R omegasi = (R)0.5 * (Q(j + 1, k, nmv + 2) / by(W(K_RHO, j + 1, k)) - Q(j - 1, k, nmv + 2) / by(W(K_RHO, j - 1, k)));
+  const R omegaeta = (R)0.5 * (Q(j, k + 1, nmv + 2) / by(W(K_RHO, j, k + 1)) - Q(j, k - 1, nmv + 2) / by(W(K_RHO, j, k - 1)));
   const R kx = ksi * xx + keta * yx, ky = ksi * xy + keta * yy;
   const R omegax = omegasi * xx + omegaeta * yx, omegay = omegasi * xy + omegaeta * yy;
   R cdkw = kx * omegax + ky * omegay;
-  cdkw = cdkw * (R)2 * (R)SSTc::sigmaw2 * rho * rho / q6;
+  cdkw = cdkw * (R)2 * (R)SSTc::sigmaw2 * rho * rho / by(q6);
   S.w[K_CDKW * ws + o] = cdkw;
   // blend
   const R sn = S.sn[o];
-  const R a1 = rei * sqrt(q5 * rho) / ((R)0.09 * q6 * sn);
-  const R a2 = (R)500 * rei * rei * W(K_VMUL, j, k) / (q6 * sq(sn));
+  const R a1 = rei * root(q5 * rho) / by((R)0.09 * q6 * sn);
+  const R a2 = (R)500 * rei * rei * W(K_VMUL, j, k) / by(q6 * sq(sn));
   const R cd = fmax2(cdkw, (R)1e-10);
-  const R a3 = (R)4 * q5 * (R)SSTc::sigmaw2 / (cd * sq(sn));
+  const R a3 = (R)4 * q5 * (R)SSTc::sigmaw2 / by(cd * sq(sn));
   const R arg1 = fmin2(fmax2(a1, a2), a3);
   const R arg2 = fmax2((R)2 * a1, a2);
   S.w[K_F1 * ws + o] = tanh(sq(sq(arg1)));
@@ -111,8 +111,8 @@ __device__ void sst_fields_cell(const Slice<R>& S, const ot2d_params& p, int j, 
 // findturm, komegasst.f:190-215, at one cell (rho, strain, F2 of this step)
 template <class R>
 __device__ __forceinline__ R sst_turm(const ot2d_params& p, R rho, R q5, R q6, R strain, R F2) {
-  const R a1 = (R)0.31, rei = (R)1. / (R)p.rey;
-  R t = a1 * rho * q5 / fmax2(a1 * q6, F2 * rho * strain * rei);
+  const R a1 = (R)0.31, rei = (R)1. / by((R)p.rey);
+  R t = a1 * rho * q5 / by(fmax2(a1 * q6, F2 * rho * strain * rei));
   return fmax2(t, (R)1e-20);
 }
 template <class R>
@@ -157,7 +157,7 @@ __device__ void sst_bc_slice(const Slice<R>& S, const double* wd2) {
           }
       }
     } else if (t == 5) {
-      const double rei = 1. / p.rey;
+      const double rei = 1. / by(p.rey);
       const int istep0 = S.ist ? S.ist[0] : p.istep0;
       double tt = ((double)istep0 - 1.) / 30.;
       if (tt > 1. || p.iread > 0) tt = 1.;
@@ -168,9 +168,9 @@ __device__ void sst_bc_slice(const Slice<R>& S, const double* wd2) {
         for (int k = ks + threadIdx.x; k <= ke; k += blockDim.x) {
           const double dely2 = wd2[at(jd, j, k)];
           const double vmulwall = 0.5 * (W(K_VMUL, j1, k) + W(K_VMUL, j, k));
-          const double omegawall = 60. * vmulwall * rei * rei / (SSTc::beta1 * dely2);
+          const double omegawall = 60. * vmulwall * rei * rei / by(SSTc::beta1 * dely2);
           const double qwall5 = -q(j1, k, n5);
-          const double qwall6 = 2 * omegawall - 6. * W(K_VMUL, j1, k) * rei * rei / (SSTc::beta1 * dely2);
+          const double qwall6 = 2 * omegawall - 6. * W(K_VMUL, j1, k) * rei * rei / by(SSTc::beta1 * dely2);
           q(j, k, n5) = scal * qwall5 + (1. - scal) * q(j, k, n5);
           q(j, k, n6) = scal * qwall6 + (1. - scal) * q(j, k, n6);
         }
@@ -179,9 +179,9 @@ __device__ void sst_bc_slice(const Slice<R>& S, const double* wd2) {
           const int k = (idir == 2) ? ke : ks, k1 = k + iadd;
           const double dely2 = wd2[at(jd, j, k)];
           const double vmulwall = 0.5 * (W(K_VMUL, j, k1) + W(K_VMUL, j, k1));
-          const double omegawall = 60. * vmulwall * rei * rei / (SSTc::beta1 * dely2);
+          const double omegawall = 60. * vmulwall * rei * rei / by(SSTc::beta1 * dely2);
           const double qwall5 = -q(j, k1, n5);
-          const double qwall6 = 2 * omegawall - 6. * W(K_VMUL, j, k1) * rei * rei / (SSTc::beta1 * dely2);
+          const double qwall6 = 2 * omegawall - 6. * W(K_VMUL, j, k1) * rei * rei / by(SSTc::beta1 * dely2);
           q(j, k, n5) = scal * qwall5 + (1. - scal) * q(j, k, n5);
           q(j, k, n6) = scal * qwall6 + (1. - scal) * q(j, k, n6);
           for (int kc = 1; kc <= ke - ks; ++kc) {
@@ -286,7 +286,7 @@ __device__ void sst_rhs_cell(const Slice<R>& S, const ot2d_params& p, int j, int
   auto Q = [&](int jj, int kk, int n) { return S.q[(int64_t)(n - 1) * qs + at(jd, jj, kk)]; };
   auto X = [&](const R* a, int jj, int kk) { return a[at(jd, jj, kk)]; };
   const int64_t o = at(jd, j, k);
-  const R rey = S.k_rey, rei = (R)1. / S.k_rey;
+  const R rey = S.k_rey, rei = (R)1. / by(S.k_rey);
   // ---- convection: upwind split of this cell (:508-511, :546-549)
   const R ugc = S.ug ? S.ug[o] : (R)0, vgc = S.vg ? S.vg[o] : (R)0;
   const R u0 = W(K_U, j, k), v0 = W(K_V, j, k);
@@ -313,20 +313,20 @@ __device__ void sst_rhs_cell(const Slice<R>& S, const ot2d_params& p, int j, int
   {
     R prod = W(K_TXX, j, k) * W(K_UX, j, k) + W(K_TXY, j, k) * (W(K_UY, j, k) + W(K_VX, j, k)) +
              W(K_TYY, j, k) * W(K_VY, j, k);
-    const R kdes = (R)SSTc::betastar * rey * q6 * q5 / rho;
+    const R kdes = (R)SSTc::betastar * rey * q6 * q5 / by(rho);
     const R ksust = (R)SSTc::betastar * rey * (R)p.tkeinf * (R)p.tomegainf * rho;
     const R prodlim = (R)10. * kdes;
     prod = fmin2(prod, prodlim);
     const R kprod = prod;
     const R beta = F1 * (R)SSTc::beta1 + ((R)1 - F1) * (R)SSTc::beta2;
-    const R omegades = beta * rey * q6 * q6 / rho;
+    const R omegades = beta * rey * q6 * q6 / by(rho);
     const R omegasust = beta * rey * sq((R)p.tomegainf) * rho;
     const R omegacrossdiff = ((R)1 - F1) * W(K_CDKW, j, k) * rei;
     sj[0] = sj[0] + kprod - kdes + ksust;
     const R gammap = F1 * (R)SSTc::gamma1 + ((R)1 - F1) * (R)SSTc::gamma2;
-    sj[1] = sj[1] + gammap * rho / S.turmu[o] * prod - omegades + omegacrossdiff + omegasust;
-    bj[0] = bj[0] + kdes / q5;
-    bj[1] = bj[1] + ((R)2 * omegades + fabs(omegacrossdiff)) / q6;
+    sj[1] = sj[1] + gammap * rho / by(S.turmu[o]) * prod - omegades + omegacrossdiff + omegasust;
+    bj[0] = bj[0] + kdes / by(q5);
+    bj[1] = bj[1] + ((R)2 * omegades + fabs(omegacrossdiff)) / by(q6);
   }
   // ---- diffusion, j direction: faces j-1/2 (chp(j-1)) and j+1/2 (chp(j))
   {
@@ -344,14 +344,14 @@ __device__ void sst_rhs_cell(const Slice<R>& S, const ot2d_params& p, int j, int
       const R sg1 = (R)(n == 0 ? SSTc::sigmak1 : SSTc::sigmaw1), sg2 = (R)(n == 0 ? SSTc::sigmak2 : SSTc::sigmaw2);
       const R chpp = rei * (vnulp + (F1 * sg1 + ((R)1. - F1) * sg2) * vnup);
       const R chpm = rei * (vnulm + (F1m * sg1 + ((R)1. - F1m) * sg2) * vnum);
-      const R dnp = Q(j + 1, k, nn) / rp - Q(j, k, nn) / rho;
-      const R dnm = Q(j, k, nn) / rho - Q(j - 1, k, nn) / rm;
+      const R dnp = Q(j + 1, k, nn) / by(rp) - Q(j, k, nn) / by(rho);
+      const R dnm = Q(j, k, nn) / by(rho) - Q(j - 1, k, nn) / by(rm);
       const R dcp = dxp * (chpp), dcm = dxm * (chpm);
       const R ax = fmax2(dcm, (R)0.0), cx = fmax2(dcp, (R)0.0);
       sj[n] = sj[n] - ax * dnm + cx * dnp;
-      aj[n] = aj[n] - ax / rm;
-      cj[n] = cj[n] - cx / rp;
-      bj[n] = bj[n] + (ax + cx) / rho;
+      aj[n] = aj[n] - ax / by(rm);
+      cj[n] = cj[n] - cx / by(rp);
+      bj[n] = bj[n] + (ax + cx) / by(rho);
     }
   }
   // ---- diffusion, k direction
@@ -370,14 +370,14 @@ __device__ void sst_rhs_cell(const Slice<R>& S, const ot2d_params& p, int j, int
       const R sg1 = (R)(n == 0 ? SSTc::sigmak1 : SSTc::sigmaw1), sg2 = (R)(n == 0 ? SSTc::sigmak2 : SSTc::sigmaw2);
       const R chpp = rei * (vnulp + (F1 * sg1 + ((R)1. - F1) * sg2) * vnup);
       const R chpm = rei * (vnulm + (F1m * sg1 + ((R)1. - F1m) * sg2) * vnum);
-      const R dnp = Q(j, k + 1, nn) / rp - Q(j, k, nn) / rho;
-      const R dnm = Q(j, k, nn) / rho - Q(j, k - 1, nn) / rm;
+      const R dnp = Q(j, k + 1, nn) / by(rp) - Q(j, k, nn) / by(rho);
+      const R dnm = Q(j, k, nn) / by(rho) - Q(j, k - 1, nn) / by(rm);
       const R dcp = dyp * (chpp), dcm = dym * (chpm);
       const R ay = fmax2(dcm, (R)0.0), cy = fmax2(dcp, (R)0.0);
       sj[n] = sj[n] - ay * dnm + cy * dnp;
-      ak[n] = ak[n] - ay / rm;
-      ck[n] = ck[n] - cy / rp;
-      bj[n] = bj[n] + (ay + cy) / rho;
+      ak[n] = ak[n] - ay / by(rm);
+      ck[n] = ck[n] - cy / by(rp);
+      bj[n] = bj[n] + (ay + cy) / by(rho);
     }
   }
   // ---- time scaling (:100-131)
@@ -392,9 +392,9 @@ __device__ void sst_rhs_cell(const Slice<R>& S, const ot2d_params& p, int j, int
     const int ibi = S.iblank[o];
     const R ib = (R)(ibi > 0 ? ibi : 0);
     const R Jc = S.q[(int64_t)(nq - 1) * qs + o];
-    tscal = ib * ((R)1.0 + (R)0.002 * sqrt(Jc)) / ((R)1. + sqrt(Jc));
+    tscal = ib * ((R)1.0 + (R)0.002 * root(Jc)) / by((R)1. + root(Jc));
     tscal = tscal * dtpseudo_turb;
-    tscal = tscal / ((R)1. + tscal / S.k_h / oat);
+    tscal = tscal / by((R)1. + tscal / by(S.k_h) / by(oat));
   }
   for (int n = 0; n < 2; ++n) {
     S.w[kband(KB_AJ, n) * ws + o] = aj[n] * tscal;

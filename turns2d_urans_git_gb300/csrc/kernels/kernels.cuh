@@ -80,7 +80,7 @@ __device__ __forceinline__ void iter_begin_slice(const Slice<R>& S) {
   double oat = 1.0;
   if (p.ntac >= 2 && istep > 1) oat = 2. / 3.;
   if (p.ntac == 3 && istep > 2) oat = 6. / 11.;
-  if (S.red) S.red[8] = 1. / (oat * p.h);
+  if (S.red) S.red[8] = 1. / by(oat * p.h);
 }
 template <class R>
 __global__ void k_iter_begin(const Slice<R>* __restrict__ sl, int nslice) {
@@ -323,7 +323,7 @@ __global__ void k_norm_final(const Slice<R>* __restrict__ sl, const int32_t* __r
   acc = warp_norm_reduce(acc);
   if (lane != 0) return;
   double volum = (double)(S.jd * S.kd);
-  double rsum = sqrt(acc.rsum / volum), resrho = sqrt(acc.resrho / volum);
+  double rsum = root(acc.rsum / by(volum)), resrho = root(acc.resrho / by(volum));
   S.red[0] = rsum; S.red[1] = resrho; S.red[2] = acc.resmax; S.red[3] = (double)acc.key;
   if (S.ist) {
     const int it = S.ist[1];
@@ -539,7 +539,7 @@ __global__ void __launch_bounds__(TJ * TK, (sizeof(R) == 4 ? 1024 : 512) / (TJ *
     if (r >= NR || j < 1 || j > jd || k < 1 || k > kd) continue;
 #pragma unroll
     for (int a = 0; a < SA_UG; ++a)
-      sm[a * NR + r] = a == SA_NUL ? val[i][SA_NUL] / val[i][SA_NST] / val[i][SA_NST + 1] : val[i][a];
+      sm[a * NR + r] = a == SA_NUL ? val[i][SA_NUL] / by(val[i][SA_NST]) / by(val[i][SA_NST + 1]) : val[i][a];
     if (gs) { sm[SA_UG * NR + r] = val[i][SA_UG]; sm[SA_VG * NR + r] = val[i][SA_VG]; }
   }
   __syncthreads();
@@ -873,7 +873,7 @@ __global__ void __launch_bounds__(CELL_BS) k_monitor(const Slice<R>* __restrict_
     const int64_t o = at(S.jd, j, k);
     double rho = S.q64[o];
     double qq = sq(S.q64[S.qs + o]) + sq(S.q64[2 * S.qs + o]);
-    double asq = p.ggm1 * (S.q64[3 * S.qs + o] - .5 * qq / rho) / rho;
+    double asq = p.ggm1 * (S.q64[3 * S.qs + o] - .5 * qq / by(rho)) / by(rho);
     bad = (asq <= 0.002) || (asq + 1 == asq) || (asq != asq);
   }
   bad = __syncthreads_or(bad);
@@ -899,15 +899,15 @@ __global__ void k_forces(const Slice<R>* __restrict__ sl, const double* const* _
   const double fmm = (p.fsmach != 0) ? p.fsmach : ((p.fmtip != 0) ? p.fmtip : 1.0);
   const double gm1 = p.gm1, gamma = p.gamma;
   for (int j = j1 + threadIdx.x; j <= j2; j += blockDim.x) {
-    double rr = 1. / Q(j, k, 1), rho = Q(j, k, 1) * Q(j, k, nq);
+    double rr = 1. / by(Q(j, k, 1)), rho = Q(j, k, 1) * Q(j, k, nq);
     double u = Q(j, k, 2) * rr, v = Q(j, k, 3) * rr, e = Q(j, k, 4) * Q(j, k, nq);
-    double vsq = u * u + v * v, pp = gm1 * (e - rho * vsq / 2.), pp1 = pp / p.pinf;
-    double cp = 2. * (pp1 - 1.) / (gamma * sq(fmm));
+    double vsq = u * u + v * v, pp = gm1 * (e - rho * vsq / 2.), pp1 = pp / by(p.pinf);
+    double cp = 2. * (pp1 - 1.) / by(gamma * sq(fmm));
     double z = cp;
-    rr = 1. / Q(j, k - 1, 1); rho = Q(j, k - 1, 1) * Q(j, k - 1, nq);
+    rr = 1. / by(Q(j, k - 1, 1)); rho = Q(j, k - 1, 1) * Q(j, k - 1, nq);
     u = Q(j, k - 1, 2) * rr; v = Q(j, k - 1, 3) * rr; e = Q(j, k - 1, 4) * Q(j, k - 1, nq);
-    vsq = u * u + v * v; pp = gm1 * (e - rho * vsq / 2.); pp1 = pp / p.pinf;
-    cp = 2. * (pp1 - 1.) / (gamma * sq(fmm));
+    vsq = u * u + v * v; pp = gm1 * (e - rho * vsq / 2.); pp1 = pp / by(p.pinf);
+    cp = 2. * (pp1 - 1.) / by(gamma * sq(fmm));
     zz[j - j1] = 0.5 * (z + cp);
   }
   __syncthreads();
@@ -920,8 +920,8 @@ __global__ void k_forces(const Slice<R>* __restrict__ sl, const double* const* _
       cc = cc + z * (YV(jv + 1, kv) - YV(jv, kv));
       cmle = cmle + z * (0.5 * (XV(jv + 1, kv) + XV(jv, kv)) * (XV(jv + 1, kv) - XV(jv, kv)) +
                          0.5 * (YV(jv + 1, kv) + YV(jv, kv)) * (YV(jv + 1, kv) - YV(jv, kv)));
-      double u = Q(j, k, 2) / Q(j, k, 1), v = Q(j, k, 3) / Q(j, k, 1);
-      double um = Q(j, k - 1, 2) / Q(j, k - 1, 1), vm = Q(j, k - 1, 3) / Q(j, k - 1, 1);
+      double u = Q(j, k, 2) / by(Q(j, k, 1)), v = Q(j, k, 3) / by(Q(j, k, 1));
+      double um = Q(j, k - 1, 2) / by(Q(j, k - 1, 1)), vm = Q(j, k - 1, 3) / by(Q(j, k - 1, 1));
       cpinv = cpinv + 0.5 * (u + um) * z * (YV(jv + 1, kv) - YV(jv, kv)) - 0.5 * (v + vm) * z * (XV(jv + 1, kv) - XV(jv, kv));
     }
     double half = (double)p.half;
@@ -930,31 +930,31 @@ __global__ void k_forces(const Slice<R>* __restrict__ sl, const double* const* _
   __syncthreads();
   double cnv = 0., ccv = 0., cmlev = 0., cpv = 0.;
   if (!p.invisc) {
-    const double amu = p.rinf * 1. / p.rey, uinf2 = sq(fmm);
+    const double amu = p.rinf * 1. / by(p.rey), uinf2 = sq(fmm);
     const double *xx = S.xx64, *xy = S.xy64, *yx = S.yx64, *yy = S.yy64;
     for (int j = j1 + threadIdx.x; j <= j2; j += blockDim.x) {
       double uxi, vxi;
       if (j == j1) {
-        uxi = Q(j + 1, k, 2) / Q(j + 1, k, 1) - Q(j, k, 2) / Q(j, k, 1);
-        vxi = Q(j + 1, k, 3) / Q(j + 1, k, 1) - Q(j, k, 3) / Q(j, k, 1);
+        uxi = Q(j + 1, k, 2) / by(Q(j + 1, k, 1)) - Q(j, k, 2) / by(Q(j, k, 1));
+        vxi = Q(j + 1, k, 3) / by(Q(j + 1, k, 1)) - Q(j, k, 3) / by(Q(j, k, 1));
       } else if (j == j2) {
-        uxi = Q(j, k, 2) / Q(j, k, 1) - Q(j - 1, k, 2) / Q(j - 1, k, 1);
-        vxi = Q(j, k, 3) / Q(j, k, 1) - Q(j - 1, k, 3) / Q(j - 1, k, 1);
+        uxi = Q(j, k, 2) / by(Q(j, k, 1)) - Q(j - 1, k, 2) / by(Q(j - 1, k, 1));
+        vxi = Q(j, k, 3) / by(Q(j, k, 1)) - Q(j - 1, k, 3) / by(Q(j - 1, k, 1));
       } else {
-        uxi = .5 * (Q(j + 1, k, 2) / Q(j + 1, k, 1) - Q(j - 1, k, 2) / Q(j - 1, k, 1));
-        vxi = .5 * (Q(j + 1, k, 3) / Q(j + 1, k, 1) - Q(j - 1, k, 3) / Q(j - 1, k, 1));
+        uxi = .5 * (Q(j + 1, k, 2) / by(Q(j + 1, k, 1)) - Q(j - 1, k, 2) / by(Q(j - 1, k, 1)));
+        vxi = .5 * (Q(j + 1, k, 3) / by(Q(j + 1, k, 1)) - Q(j - 1, k, 3) / by(Q(j - 1, k, 1)));
       }
-      double ueta = -1.5 * Q(j, k, 2) / Q(j, k, 1) + 2. * Q(j, k2, 2) / Q(j, k2, 1) - .5 * Q(j, k3, 2) / Q(j, k3, 1);
-      double veta = -1.5 * Q(j, k, 3) / Q(j, k, 1) + 2. * Q(j, k2, 3) / Q(j, k2, 1) - .5 * Q(j, k3, 3) / Q(j, k3, 1);
+      double ueta = -1.5 * Q(j, k, 2) / by(Q(j, k, 1)) + 2. * Q(j, k2, 2) / by(Q(j, k2, 1)) - .5 * Q(j, k3, 2) / by(Q(j, k3, 1));
+      double veta = -1.5 * Q(j, k, 3) / by(Q(j, k, 1)) + 2. * Q(j, k2, 3) / by(Q(j, k2, 1)) - .5 * Q(j, k3, 3) / by(Q(j, k3, 1));
       const int64_t o = at(jd, j, k);
       double xix = xx[o], xiy = xy[o], etax = yx[o], etay = yy[o];
       double sfdiv = 2. / 3 * (uxi * xix + ueta * etax + vxi * xiy + veta * etay);
       double a = amu * (2. * (uxi * xix + ueta * etax) - sfdiv);
       double b = amu * (2. * (vxi * xiy + veta * etay) - sfdiv);
       double tauw = amu * ((uxi * xiy + ueta * etay) + (vxi * xix + veta * etax));
-      sxx[j - j1] = a / (.5 * p.rinf * uinf2);
-      syy[j - j1] = b / (.5 * p.rinf * uinf2);
-      zz[j - j1] = tauw / (.5 * p.rinf * uinf2);
+      sxx[j - j1] = a / by(.5 * p.rinf * uinf2);
+      syy[j - j1] = b / by(.5 * p.rinf * uinf2);
+      zz[j - j1] = tauw / by(.5 * p.rinf * uinf2);
     }
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -967,8 +967,8 @@ __global__ void k_forces(const Slice<R>* __restrict__ sl, const double* const* _
                              0.5 * (YV(jv + 1, kv) + YV(jv, kv)) * (XV(jv + 1, kv) - XV(jv, kv))) -
                 0.5 * (XV(jv + 1, kv) + XV(jv, kv)) * (XV(jv + 1, kv) - XV(jv, kv)) * sy -
                 0.5 * (YV(jv + 1, kv) + YV(jv, kv)) * (YV(jv + 1, kv) - YV(jv, kv)) * sx;
-        double u = Q(j, k, 2) / Q(j, k, 1), v = Q(j, k, 3) / Q(j, k, 1);
-        double um = Q(j, k - 1, 2) / Q(j, k - 1, 1), vm = Q(j, k - 1, 3) / Q(j, k - 1, 1);
+        double u = Q(j, k, 2) / by(Q(j, k, 1)), v = Q(j, k, 3) / by(Q(j, k, 1));
+        double um = Q(j, k - 1, 2) / by(Q(j, k - 1, 1)), vm = Q(j, k - 1, 3) / by(Q(j, k - 1, 1));
         cpv = cpv + 0.5 * (u + um) * z * (XV(jv + 1, kv) - XV(jv, kv)) - 0.5 * (u + um) * sx * (YV(jv + 1, kv) - YV(jv, kv)) -
               0.5 * (v + vm) * z * (YV(jv + 1, kv) - YV(jv, kv)) + 0.5 * (v + vm) * sy * (XV(jv + 1, kv) - XV(jv, kv));
       }
@@ -980,7 +980,7 @@ __global__ void k_forces(const Slice<R>* __restrict__ sl, const double* const* _
     out[4 * blockIdx.x + 0] = cc + ccv;
     out[4 * blockIdx.x + 1] = cn + cnv;
     out[4 * blockIdx.x + 2] = cmle + cmlev;
-    out[4 * blockIdx.x + 3] = (cpinv + cpv) / fmm;
+    out[4 * blockIdx.x + 3] = (cpinv + cpv) / by(fmm);
   }
 }
 

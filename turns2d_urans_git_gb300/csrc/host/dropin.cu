@@ -31,7 +31,7 @@ constexpr size_t DW_SLOTS = SST_NSCRATCH + 1;
 
 struct Ctx {
   ot2d_params P{};
-  bool has = false;
+  bool has = false, fresh = true;   // fresh: P not yet on the device
   int err = 0;
   cudaStream_t st = nullptr;
   ot2d_params* dP = nullptr;
@@ -40,10 +40,18 @@ struct Ctx {
   int nslice = 1;
   DevBatch<double> batch;
   std::vector<Staged> staged;
-  std::vector<void*> pool;                         // staging buffers of this call
+  char* arena = nullptr; size_t acap = 0;          // staging space kept between calls (at most ARENA_MAX)
+  size_t aused = 0, awant = 0;                     // of this call: handed out, asked for
+  std::vector<void*> pool;                         // buffers of this call that the arena had no room for
+  cudaEvent_t geo = nullptr;
+  bool geo_waits = false;                          // this call's stream waits for the caller's geometry
   std::vector<double> norms;
-  ~Ctx() {}
+  ~Ctx() { if (arena) cudaFree(arena); }
 };
+// A call whose arguments need more staging than this allocates it and gives
+// it back (a cudaMalloc / cudaFree pair is a few microseconds per array,
+// which shows in calls of well under a millisecond only).
+constexpr size_t ARENA_MAX = (size_t)256 << 20;
 thread_local Ctx g_ctx;
 
 int fail(int e) { if (e) g_ctx.err = e; return e; }
@@ -56,6 +64,21 @@ int ensure_stream() {
     if (cudaMalloc(&g_ctx.dist, sizeof(int32_t) * IST_N * 64) != cudaSuccess) return OT2D_ERR_NOMEM;
   }
   return OT2D_OK;
+}
+
+// Device space for this call
+void* stage(size_t bytes, int& err) {
+  const size_t b = (bytes + 255) / 256 * 256;
+  g_ctx.awant += b;
+  if (g_ctx.aused + b <= g_ctx.acap) {
+    void* d = g_ctx.arena + g_ctx.aused;
+    g_ctx.aused += b;
+    return d;
+  }
+  void* d = nullptr;
+  if (cudaMalloc(&d, bytes) != cudaSuccess) { cudaGetLastError(); err = OT2D_ERR_NOMEM; return nullptr; }
+  g_ctx.pool.push_back(d);
+  return d;
 }
 
 // Resolve one argument.  `in`: the routine reads it; `out`: it writes it.
@@ -75,9 +98,8 @@ void* resolve(void* p, size_t bytes, bool in, bool out, int& err) {
       if ((uintptr_t)p + bytes <= base + it->second.bytes) return (char*)it->second.dev + ((uintptr_t)p - base);
     }
   }
-  void* d = nullptr;
-  if (cudaMalloc(&d, bytes) != cudaSuccess) { err = OT2D_ERR_NOMEM; return nullptr; }
-  g_ctx.pool.push_back(d);
+  void* d = stage(bytes, err);
+  if (!d) return nullptr;
   if (in) {
     if (cudaMemcpyAsync(d, p, bytes, cudaMemcpyHostToDevice, g_ctx.st) != cudaSuccess) err = OT2D_ERR_CUDA;
   } else if (cudaMemsetAsync(d, 0, bytes, g_ctx.st) != cudaSuccess) {
@@ -94,9 +116,17 @@ int finish(int err) {
       if (cudaMemcpyAsync(s.host, s.dev, s.bytes, cudaMemcpyDeviceToHost, g_ctx.st) != cudaSuccess) err = OT2D_ERR_CUDA;
   }
   if (cudaStreamSynchronize(g_ctx.st) != cudaSuccess && !err) err = OT2D_ERR_CUDA;
+  const bool grow = !g_ctx.pool.empty() && g_ctx.awant > g_ctx.acap && g_ctx.awant <= ARENA_MAX;
   for (void* d : g_ctx.pool) cudaFree(d);
   g_ctx.pool.clear();
   g_ctx.staged.clear();
+  if (grow) {
+    if (g_ctx.arena) cudaFree(g_ctx.arena);
+    g_ctx.acap = g_ctx.awant;
+    if (cudaMalloc(&g_ctx.arena, g_ctx.acap) != cudaSuccess) { cudaGetLastError(); g_ctx.arena = nullptr; g_ctx.acap = 0; }
+  }
+  g_ctx.aused = g_ctx.awant = 0;
+  g_ctx.geo_waits = false;
   return fail(err);
 }
 
@@ -122,9 +152,33 @@ void host_store(double* p, const double* v, size_t n) {
   }
 }
 
+// A geometry array (centres, vertices, vertex speeds) on the device.  Device
+// memory is used in place, after the work that the default stream has been
+// given; host memory is copied as it stands, registered or not.
+const double* geo_view(const double* p, size_t n, int& err) {
+  if (!p || err) return nullptr;
+  cudaPointerAttributes a;
+  if (cudaPointerGetAttributes(&a, p) == cudaSuccess && (a.type == cudaMemoryTypeDevice || a.type == cudaMemoryTypeManaged)) {
+    if (!g_ctx.geo_waits) {
+      if (!g_ctx.geo && cudaEventCreateWithFlags(&g_ctx.geo, cudaEventDisableTiming) != cudaSuccess) err = OT2D_ERR_CUDA;
+      if (!err && (cudaEventRecord(g_ctx.geo, cudaStreamLegacy) != cudaSuccess ||
+                   cudaStreamWaitEvent(g_ctx.st, g_ctx.geo) != cudaSuccess))
+        err = OT2D_ERR_CUDA;
+      g_ctx.geo_waits = !err;
+    }
+    return p;
+  }
+  cudaGetLastError();
+  double* d = (double*)stage(n * sizeof(double), err);
+  if (d && cudaMemcpyAsync(d, p, n * sizeof(double), cudaMemcpyHostToDevice, g_ctx.st) != cudaSuccess) err = OT2D_ERR_CUDA;
+  return d;
+}
+
 // Scratch arrays for nslice slices; upload params.
 int prepare(int nslice, int& err) {
   if ((err = ensure_stream())) return err;
+  g_ctx.aused = g_ctx.awant = 0;   // a call that was refused may have staged some
+  g_ctx.geo_waits = false;
   if (!g_ctx.has) return err = OT2D_ERR_NOPARAMS;
   const size_t n2 = (size_t)g_ctx.P.jd * g_ctx.P.kd, ws = (n2 + 63) / 64 * 64;
   const size_t rec = (size_t)lu_rec_elems(g_ctx.P.jd, g_ctx.P.kd, 8);
@@ -136,8 +190,9 @@ int prepare(int nslice, int& err) {
     if (cudaMalloc(&g_ctx.dwork, need * sizeof(double)) != cudaSuccess) { g_ctx.dwork = nullptr; g_ctx.wcap = 0; return err = OT2D_ERR_NOMEM; }
     g_ctx.wcap = need;
   }
-  if (cudaMemcpyAsync(g_ctx.dP, &g_ctx.P, sizeof(ot2d_params), cudaMemcpyHostToDevice, g_ctx.st) != cudaSuccess)
+  if (g_ctx.fresh && cudaMemcpyAsync(g_ctx.dP, &g_ctx.P, sizeof(ot2d_params), cudaMemcpyHostToDevice, g_ctx.st) != cudaSuccess)
     return err = OT2D_ERR_CUDA;
+  g_ctx.fresh = false;
   return err;
 }
 
@@ -179,7 +234,7 @@ Slice<double> base_slice(int nsp, int nspec, int64_t qs) {
 
 int run_batch(const std::vector<Slice<double>>& sl, int& err) {
   if (err) return err;
-  if ((err = g_ctx.batch.build(sl, g_ctx.st))) return err;
+  if ((err = g_ctx.batch.build(sl, g_ctx.st, false))) return err;
   return err;
 }
 
@@ -189,34 +244,46 @@ bool dims_ok(const int32_t* jd, const int32_t* kd) {
 
 // face normals (and time-spectral face speeds) from the vertex grid
 // (xold..yole: the previous vertex levels of a time-accurate moving grid,
-// or null)
+// or null), formed on the device
 int faces_upload(double* dst4, double* dst2, const double* xv, const double* yv, const double* ugv, const double* vgv,
                  size_t ws, int& err, const double* xold = nullptr, const double* yold = nullptr,
                  const double* xole = nullptr, const double* yole = nullptr) {
   const ot2d_params& p = g_ctx.P;
-  const size_t nv = (size_t)p.jmax * p.kmax, n2 = (size_t)p.jd * p.kd;
-  std::vector<double> hx = host_copy(xv, nv), hy = host_copy(yv, nv), hu, hvv;
-  std::vector<double> f(4 * n2), t(2 * n2, 0.0);
+  const size_t nv = (size_t)p.jmax * p.kmax;
   const bool swept = p.iunst > 0 && xold && yold && xole && yole;
   const bool ts = !swept && p.timespectral && ugv && vgv;
-  if (ts) { hu = host_copy(ugv, nv); hvv = host_copy(vgv, nv); }
-  face_normals(p, hx.data(), hy.data(), ts ? hu.data() : nullptr, ts ? hvv.data() : nullptr, f.data(), f.data() + n2,
-               f.data() + 2 * n2, f.data() + 3 * n2, ts ? t.data() : nullptr, ts ? t.data() + n2 : nullptr);
+  GeomArgs g{};
+  g.xv = geo_view(xv, nv, err); g.yv = geo_view(yv, nv, err);
+  if (ts) { g.ugv = geo_view(ugv, nv, err); g.vgv = geo_view(vgv, nv, err); }
   if (swept) {
-    std::vector<double> a = host_copy(xold, nv), b = host_copy(yold, nv), c = host_copy(xole, nv), d = host_copy(yole, nv);
-    face_speeds_swept(p, hx.data(), hy.data(), a.data(), b.data(), c.data(), d.data(), t.data(), t.data() + n2);
+    g.xold = geo_view(xold, nv, err); g.yold = geo_view(yold, nv, err);
+    g.xole = geo_view(xole, nv, err); g.yole = geo_view(yole, nv, err);
   }
-  for (int a = 0; a < 4; ++a)
-    if (cudaMemcpyAsync(dst4 + a * ws, f.data() + a * n2, n2 * 8, cudaMemcpyHostToDevice, g_ctx.st) != cudaSuccess)
-      err = OT2D_ERR_CUDA;
-  if ((ts || swept) && dst2)
-    for (int a = 0; a < 2; ++a)
-      if (cudaMemcpyAsync(dst2 + a * ws, t.data() + a * n2, n2 * 8, cudaMemcpyHostToDevice, g_ctx.st) != cudaSuccess)
-        err = OT2D_ERR_CUDA;
-  cudaStreamSynchronize(g_ctx.st);  // host vectors go out of scope
+  g.faces = dst4;
+  g.speeds = ts || swept ? dst2 : nullptr;
+  g.ws = (int64_t)ws;
+  if (!err && launch_geometry(g_ctx.dP, p.jd * p.kd, g, g_ctx.st) != cudaSuccess) err = OT2D_ERR_CUDA;
   return err;
 }
 
+// SA wall distance into dsn, formed on the device.  (A wall range outside the
+// mesh is left to the host's loop.)
+void wall_upload(double* dsn, const double* x, const double* y, const double* xv, const double* yv, int& err) {
+  const ot2d_params& p = g_ctx.P;
+  const size_t n2 = (size_t)p.jd * p.kd, nv = (size_t)p.jmax * p.kmax;
+  if (p.jtail1 >= 2 && p.jtail1 <= p.jd && p.jtail2 <= p.jmax) {
+    GeomArgs g{};
+    g.x = geo_view(x, n2, err); g.y = geo_view(y, n2, err);
+    g.xv = geo_view(xv, nv, err); g.yv = geo_view(yv, nv, err);
+    g.sn = dsn;
+    if (!err && launch_geometry(g_ctx.dP, (int)n2, g, g_ctx.st) != cudaSuccess) err = OT2D_ERR_CUDA;
+    return;
+  }
+  std::vector<double> hx = host_copy(x, n2), hy = host_copy(y, n2), hxv = host_copy(xv, nv), hyv = host_copy(yv, nv);
+  std::vector<double> sn(n2);
+  wall_distance(p, hx.data(), hy.data(), hxv.data(), hyv.data(), sn.data());
+  if (!err && cudaMemcpy(dsn, sn.data(), n2 * 8, cudaMemcpyHostToDevice) != cudaSuccess) err = OT2D_ERR_CUDA;
+}
 
 // Device view of an argument without staging: the pointer itself for device
 // memory, the registered mirror for registered host memory, else nullptr.
@@ -502,7 +569,7 @@ int ot2d_set_params(const ot2d_params* p) {
   if (!rt_lim_known(p->ilim)) return fail(OT2D_ERR_ARG);   // reconstructions of rhsup (eulerrhs.f:84-97)
   if (rt_lim_class(p->ilim) == 2 && (p->jd < 7 || p->kd < 7)) return fail(OT2D_ERR_ARG);   // quad's end stencils
   g_ctx.P = *p;
-  g_ctx.has = true;
+  g_ctx.has = g_ctx.fresh = true;
   return OT2D_OK;
 }
 
@@ -719,16 +786,11 @@ int ot2d_vmu_sa(double* q, double* s, double* turmu, double* x, double* y, doubl
   const ot2d_params& p = g_ctx.P;
   if (!dims_ok(jd, kd) || p.iturb != 1 || p.lamin || !q || !s || !turmu || !x || !y || !xv || !yv || !tscale || !iblank)
     return fail(OT2D_ERR_ARG);
-  const size_t n2 = (size_t)p.jd * p.kd, nv = (size_t)p.jmax * p.kmax;
+  const size_t n2 = (size_t)p.jd * p.kd;
   Slice<double> S = base_slice(1, 1, (int64_t)n2);
   const size_t ws = (size_t)S.wstride;
   double* dsn = g_ctx.dwork + ws * DW_SLOTS;
-  {
-    std::vector<double> hx = host_copy(x, n2), hy = host_copy(y, n2), hxv = host_copy(xv, nv), hyv = host_copy(yv, nv);
-    std::vector<double> sn(n2);
-    wall_distance(p, hx.data(), hy.data(), hxv.data(), hyv.data(), sn.data());
-    if (cudaMemcpy(dsn, sn.data(), n2 * 8, cudaMemcpyHostToDevice) != cudaSuccess) err = OT2D_ERR_CUDA;
-  }
+  wall_upload(dsn, x, y, xv, yv, err);
   S.q = S.q64 = (double*)resolve(q, n2 * p.nq * 8, true, true, err);
   S.s = (double*)resolve(s, n2 * p.nv * 8, true, false, err);
   S.turmu = (double*)resolve(turmu, n2 * 8, true, true, err);
@@ -857,23 +919,25 @@ int ot2d_step(double* q, double* qtn, double* qtnm1, double* qnewt, double* s, d
   double* dDs = p.timespectral ? (double*)resolve(Ds, ns * ns * 8, true, false, err) : nullptr;
   // per-instance face normals and wall distance from the host grid
   const size_t ws = (n2 + 63) / 64 * 64;
-  double* extra = nullptr;
-  if (!err && cudaMalloc(&extra, sizeof(double) * ws * 8 * ns) != cudaSuccess) err = OT2D_ERR_NOMEM;
-  if (extra) g_ctx.pool.push_back(extra);
+  double* extra = err ? nullptr : (double*)stage(sizeof(double) * ws * 8 * ns, err);
   std::vector<Slice<double>> sl;
-  std::vector<double> hx = host_copy(x, qs), hy = host_copy(y, qs), hxv = host_copy(xv, nv * ns), hyv = host_copy(yv, nv * ns);
+  std::vector<double> hx, hy, hxv, hyv;
+  if (sst_params(p)) { hx = host_copy(x, qs); hy = host_copy(y, qs); hxv = host_copy(xv, nv * ns); hyv = host_copy(yv, nv * ns); }
   for (int nsp = 1; nsp <= nspec && !err; ++nsp) {
     double* e = extra + (size_t)(nsp - 1) * ws * 8;
     faces_upload(e, e + 4 * ws, xv + (nsp - 1) * nv, yv + (nsp - 1) * nv, ugv ? ugv + (nsp - 1) * nv : nullptr,
                  vgv ? vgv + (nsp - 1) * nv : nullptr, ws, err, swept ? xold : nullptr, swept ? yold : nullptr,
                  swept ? xole : nullptr, swept ? yole : nullptr);
-    std::vector<double> sn(n2);
-    wall_distance(p, hx.data() + (nsp - 1) * n2, hy.data() + (nsp - 1) * n2, hxv.data() + (nsp - 1) * nv,
-                  hyv.data() + (nsp - 1) * nv, sn.data());
-    if (sst_params(p))
+    if (sst_params(p)) {
+      std::vector<double> sn(n2);
+      wall_distance(p, hx.data() + (nsp - 1) * n2, hy.data() + (nsp - 1) * n2, hxv.data() + (nsp - 1) * nv,
+                    hyv.data() + (nsp - 1) * nv, sn.data());
       sst_geometry(p, hx.data() + (nsp - 1) * n2, hy.data() + (nsp - 1) * n2, hxv.data() + (nsp - 1) * nv,
                    hyv.data() + (nsp - 1) * nv, sn.data(), e + 7 * ws, err);
-    if (cudaMemcpy(e + 6 * ws, sn.data(), n2 * 8, cudaMemcpyHostToDevice) != cudaSuccess) err = OT2D_ERR_CUDA;
+      if (cudaMemcpy(e + 6 * ws, sn.data(), n2 * 8, cudaMemcpyHostToDevice) != cudaSuccess) err = OT2D_ERR_CUDA;
+    } else {
+      wall_upload(e + 6 * ws, x + (nsp - 1) * n2, y + (nsp - 1) * n2, xv + (nsp - 1) * nv, yv + (nsp - 1) * nv, err);
+    }
     Slice<double> S = base_slice(nsp, nspec, (int64_t)qs);
     const size_t o = (size_t)(nsp - 1) * n2;
     S.q = S.q64 = dq + o; S.s = ds + o; S.iblank = dib + o;
@@ -1114,7 +1178,7 @@ int ot2d_restr2(double* q, int32_t* jd, int32_t* kd, int32_t* logq) {
   std::vector<double> h(4 * n2);
   int err = rec_read(f, hdr, sizeof(hdr));   // fstip, alf, reypr, totime
   if (!err) err = rec_read(f, h.data(), h.size() * 8);
-  if (!err) { g_ctx.P.totime = hdr[3]; err = put(q, h.data(), h.size() * 8); }
+  if (!err) { g_ctx.P.totime = hdr[3]; g_ctx.fresh = true; err = put(q, h.data(), h.size() * 8); }
   return fail(err);
 }
 

@@ -419,7 +419,7 @@ template Slice<double> make_slice<double>(const DevSolve&, int, double*, int32_t
 template Slice<float> make_slice<float>(const DevSolve&, int, double*, int32_t*);
 
 template <class R>
-int DevBatch<R>::build(const std::vector<Slice<R>>& sl, cudaStream_t st) {
+int DevBatch<R>::build(const std::vector<Slice<R>>& sl, cudaStream_t st, bool sync) {
   const int n = (int)sl.size();
   // six prefix tables of n+1 entries: cell blocks, k-lines, j-lines, LU
   // record blocks, 32-line groups, residual tiles
@@ -454,21 +454,28 @@ int DevBatch<R>::build(const std::vector<Slice<R>>& sl, cudaStream_t st) {
   idx[5 * (n + 1) - 1] = grp; idx[6 * (n + 1) - 1] = tiles;
   if ((size_t)n > cap_sl) {
     if (d_sl) cudaFree(d_sl);
-    if (d_idx) cudaFree(d_idx);
     cap_sl = std::max((size_t)n, (size_t)2 * cap_sl);
-    if (cudaMalloc(&d_sl, cap_sl * sizeof(Slice<R>)) != cudaSuccess) return OT2D_ERR_NOMEM;
-    if (cudaMalloc(&d_idx, 6 * (cap_sl + 1) * sizeof(int32_t)) != cudaSuccess) return OT2D_ERR_NOMEM;
+    // the slices and, behind them, the tables: one copy uploads both
+    if (cudaMalloc(&d_sl, cap_sl * sizeof(Slice<R>) + 6 * (cap_sl + 1) * sizeof(int32_t)) != cudaSuccess) return OT2D_ERR_NOMEM;
   }
+  d_idx = (int32_t*)(d_sl + n);
   const size_t nparts = (size_t)std::max(cells, tiles);
   if (nparts > cap_part) {
     if (d_part) cudaFree(d_part);
     cap_part = std::max(nparts, (size_t)2 * cap_part);
     if (cudaMalloc(&d_part, cap_part * sizeof(NormPart)) != cudaSuccess) return OT2D_ERR_NOMEM;
   }
-  if (cudaMemcpyAsync(d_sl, sl.data(), n * sizeof(Slice<R>), cudaMemcpyHostToDevice, st) != cudaSuccess) return OT2D_ERR_CUDA;
-  if (cudaMemcpyAsync(d_idx, idx.data(), idx.size() * sizeof(int32_t), cudaMemcpyHostToDevice, st) != cudaSuccess)
-    return OT2D_ERR_CUDA;
-  if (cudaStreamSynchronize(st) != cudaSuccess) return OT2D_ERR_CUDA;
+  const size_t nsl = n * sizeof(Slice<R>), nup = nsl + idx.size() * sizeof(int32_t);
+  if (nup > cap_up) {
+    if (h_up) cudaFreeHost(h_up);
+    cap_up = 0;
+    if (cudaMallocHost(&h_up, nup) != cudaSuccess) { h_up = nullptr; return OT2D_ERR_NOMEM; }
+    cap_up = nup;
+  }
+  std::memcpy(h_up, sl.data(), nsl);
+  std::memcpy(h_up + nsl, idx.data(), nup - nsl);
+  if (cudaMemcpyAsync(d_sl, h_up, nup, cudaMemcpyHostToDevice, st) != cudaSuccess) return OT2D_ERR_CUDA;
+  if (sync && cudaStreamSynchronize(st) != cudaSuccess) return OT2D_ERR_CUDA;
   b.nslice = n;
   b.moving = moving;
   b.precon = precon;
@@ -492,8 +499,9 @@ int DevBatch<R>::build(const std::vector<Slice<R>>& sl, cudaStream_t st) {
 template <class R>
 void DevBatch<R>::release() {
   if (d_sl) cudaFree(d_sl);
-  if (d_idx) cudaFree(d_idx);
   if (d_part) cudaFree(d_part);
+  if (h_up) cudaFreeHost(h_up);
+  h_up = nullptr; cap_up = 0;
   d_sl = nullptr; d_idx = nullptr; d_part = nullptr; cap_sl = cap_part = 0;
 }
 

@@ -85,7 +85,11 @@ struct DevBatch {
   NormPart* d_part = nullptr;
   size_t cap_sl = 0, cap_part = 0;
   int rt_shape = 0;   // residual tile shape the next build lays out (rt_shape_dims)
-  int build(const std::vector<Slice<R>>& sl, cudaStream_t st);  // returns OT2D status
+  char* h_up = nullptr;       // pinned copy of what a build uploads
+  size_t cap_up = 0;
+  // returns OT2D status.  sync = false: the uploads are still on st when it
+  // returns; the caller synchronises st before its next build
+  int build(const std::vector<Slice<R>>& sl, cudaStream_t st, bool sync = true);
   void release();
 };
 

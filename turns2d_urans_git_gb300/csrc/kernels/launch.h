@@ -126,6 +126,15 @@ template <class R> cudaError_t launch_time_step(const Slice<R>* d_sl, const Batc
 template <class R> cudaError_t launch_pitch(const Slice<R>* d_sl, const Batch& b, cudaStream_t st);
 // stqol over n elements of each of nv variables (stride qs): q of the
 // current step, the stored levels and the Newton target (time.f:110-175)
+// Geometry of one mesh (nhalo 1) from its vertices: the four face-normal
+// arrays (faces, ws apart) with, when speeds is not null, the two face-speed
+// arrays, and / or the SA wall distance sn of the centres (x, y).
+struct GeomArgs {
+  const double *x, *y, *xv, *yv, *ugv, *vgv, *xold, *yold, *xole, *yole;
+  double *faces, *speeds, *sn;
+  int64_t ws;
+};
+cudaError_t launch_geometry(const ot2d_params* d_p, int cells, const GeomArgs& g, cudaStream_t st);
 cudaError_t launch_stqol(const double* q, double* qtn, double* qtnm1, double* qnewt, int64_t qs, int nv, int ntac,
                          int istep, cudaStream_t st);
 // begin = 1 (mixed path): each slice's boundary CTA first applies the

@@ -425,7 +425,7 @@ int DevBatch<R>::build(const std::vector<Slice<R>>& sl, cudaStream_t st, bool sy
   // record blocks, 32-line groups, residual tiles
   std::vector<int32_t> idx(6 * (n + 1));
   int cells = 0, jl = 0, kl = 0, lub = 0, grp = 0, tiles = 0, maxwall = 1, maxkd = 1, moving = 0, precon = 0;
-  int maxnbc = 0, limmask = 0;
+  int maxnbc = 0, limmask = 0, bands = 0;
   int tj = 16, tk = 16;
   rt_shape_dims(rt_shape, tj, tk);
   for (int i = 0; i < n; ++i) {
@@ -442,6 +442,7 @@ int DevBatch<R>::build(const std::vector<Slice<R>>& sl, cudaStream_t st, bool sy
     // record blocks: enough for the plain and the preconditioned band layout
     auto rec_blocks = [&](int rb) { return (lu_nband(kd, rb) * lu_nstep(jd, rb) * rb + lu_prep_bs<R>() - 1) / lu_prep_bs<R>(); };
     lub += std::max(rec_blocks(LuSplit<R, false>::RB), rec_blocks(LuSplit<R, true>::RB));
+    bands += lu_nband(kd, LuSplit<R, false>::RB);
     grp += (kd - 2 + 31) / 32;
     tiles += ((jd - 2 + tj - 1) / tj) * ((kd - 2 + tk - 1) / tk);
     maxwall = std::max(maxwall, jd);
@@ -487,6 +488,7 @@ int DevBatch<R>::build(const std::vector<Slice<R>>& sl, cudaStream_t st, bool sy
   b.rt_shape = rt_shape;
   b.jlines = jl; b.klines = kl;
   b.lu_blocks = lub;
+  b.bands = bands;
   b.jgroups = grp;
   b.d_gfirst = d_idx + 4 * (n + 1);
   b.d_tfirst = d_idx + 5 * (n + 1);

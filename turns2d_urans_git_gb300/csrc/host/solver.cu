@@ -128,7 +128,8 @@ struct ot2d_solver {
   // Host-buffer path: the batch in HP parts of about equal cells, a graph
   // and a stream each, so that some parts' copies run while others iterate
   // (built once that path is used)
-  static constexpr int HP = 4;
+  static constexpr int HP = 8, HP_MIN = 4;
+  int np = HP_MIN;                        // parts of this batch
   bool want_parts = false;
   bool parts = false;
   DevBatch<double> p64[HP];
@@ -137,6 +138,8 @@ struct ot2d_solver {
   cudaGraphExec_t pexec[HP] = {};
   cudaStream_t pst[HP] = {};
   cudaEvent_t ev_pdone[HP] = {};
+  cudaStream_t st_h2d = nullptr;          // the parts' uploads, one part after another
+  cudaEvent_t ev_pup[HP] = {}, ev_pdown[HP] = {};   // a part's uploads / downloads finished
   int next_id = 0;
   double t0 = 0;
   int check_every = 25;
@@ -227,7 +230,7 @@ cudaError_t launch_graph_iteration(ot2d_solver* s) {
     // four independent parts, each on its own stream after what the solver
     // stream holds (uploads, a rebuild's time step)
     cudaError_t e = cudaEventRecord(s->ev_step, s->st);
-    for (int q = 0; q < ot2d_solver::HP && e == cudaSuccess; ++q) {
+    for (int q = 0; q < s->np && e == cudaSuccess; ++q) {
       e = cudaStreamWaitEvent(s->pst[q], s->ev_step, 0);
       if (e == cudaSuccess) e = cudaGraphLaunch(s->pexec[q], s->pst[q]);
     }
@@ -247,7 +250,7 @@ cudaError_t launch_graph_iteration(ot2d_solver* s) {
 cudaError_t join_halves(ot2d_solver* s) {
   if (s->split4) {
     cudaError_t e = cudaSuccess;
-    for (int q = 0; q < ot2d_solver::HP && e == cudaSuccess; ++q) {
+    for (int q = 0; q < s->np && e == cudaSuccess; ++q) {
       e = cudaEventRecord(s->ev_pdone[q], s->pst[q]);
       if (e == cudaSuccess) e = cudaStreamWaitEvent(s->st, s->ev_pdone[q], 0);
     }
@@ -271,6 +274,7 @@ template <> DevBatch<float>* parts_of<float>(ot2d_solver* s) { return s->p32; }
 template <class R>
 int build_parts(ot2d_solver* s, const DevBatch<R>& B, int visc) {
   constexpr int HP = ot2d_solver::HP;
+  const int np = s->np;
   std::vector<int> ids = s->live;
   auto cells_of = [&](int id) { const ot2d_params& p = s->recs[id].d.P; return (size_t)p.jd * p.kd * p.nspec; };
   std::stable_sort(ids.begin(), ids.end(), [&](int a, int b) { return cells_of(a) > cells_of(b); });
@@ -278,20 +282,21 @@ int build_parts(ot2d_solver* s, const DevBatch<R>& B, int visc) {
   size_t load[HP] = {};
   for (int id : ids) {
     int q = 0;
-    for (int i = 1; i < HP; ++i)
+    for (int i = 1; i < np; ++i)
       if (load[i] < load[q]) q = i;
     load[q] += cells_of(id);
     slices_of<R>(s, s->recs[id], slp[q]);
     s->recs[id].part = q;
   }
   DevBatch<R>* P = parts_of<R>(s);
-  for (int q = 0; q < HP; ++q) {
+  for (int q = 0; q < np; ++q) {
     if (!s->pst[q] && cudaStreamCreateWithFlags(&s->pst[q], cudaStreamNonBlocking) != cudaSuccess) return OT2D_ERR_CUDA;
-    if (!s->ev_pdone[q] && cudaEventCreateWithFlags(&s->ev_pdone[q], cudaEventDisableTiming) != cudaSuccess)
-      return OT2D_ERR_CUDA;
+    for (cudaEvent_t* e : {&s->ev_pdone[q], &s->ev_pup[q], &s->ev_pdown[q]})
+      if (!*e && cudaEventCreateWithFlags(e, cudaEventDisableTiming) != cudaSuccess) return OT2D_ERR_CUDA;
     P[q].rt_shape = B.rt_shape;
     int e = P[q].build(slp[q], s->st);
     if (e) return e;
+    P[q].b.shared_bands = B.b.bands;
     P[q].b.poll_limit = B.b.poll_limit;
     P[q].b.ts_in_update = B.b.ts_in_update;
     P[q].b.lu_lag = B.b.lu_lag;
@@ -367,7 +372,7 @@ int rebuild_t(ot2d_solver* s, DevBatch<R>& B) {
   const int visc = s->any_viscous ? 1 : 0;
   const bool can_split = sl.size() >= (size_t)PIPE_MIN_SLICES && s->live.size() >= 2;
   const bool split = ch.pipeline == 1 && can_split;
-  const bool can_parts = sl.size() >= (size_t)PIPE_MIN_SLICES && s->live.size() >= (size_t)ot2d_solver::HP;
+  const bool can_parts = sl.size() >= (size_t)PIPE_MIN_SLICES && s->live.size() >= (size_t)ot2d_solver::HP_MIN;
   const bool split4 = ch.pipeline == 2 && can_parts;
   if (split4 && !s->ev_step && cudaEventCreateWithFlags(&s->ev_step, cudaEventDisableTiming) != cudaSuccess)
     return OT2D_ERR_CUDA;
@@ -375,7 +380,12 @@ int rebuild_t(ot2d_solver* s, DevBatch<R>& B) {
   // the parts: for the device-resident iteration (OT2D_OPT_PIPELINE 2) or
   // once the host-buffer path has been used
   const bool want_parts = (s->want_parts || ch.pipeline == 2) && sl.size() >= (size_t)PIPE_MIN_SLICES &&
-                          s->live.size() >= (size_t)ot2d_solver::HP;
+                          s->live.size() >= (size_t)ot2d_solver::HP_MIN;
+  // Eight parts for the host-buffer path, four for the device-resident one.
+  // Two host iterations in 4, 6, 8 parts (us): 64 instances of 513x129 4155,
+  // 3825, 3847; 16 of them 1632, 1585, 1554; 64 of 257x65 1523, 1416, 1395;
+  // 64 of 129x33 761, 748, 724.
+  s->np = ch.pipeline != 2 && s->live.size() >= (size_t)ot2d_solver::HP ? ot2d_solver::HP : ot2d_solver::HP_MIN;
   if (!split) {
     if (cudaStreamBeginCapture(s->st, cudaStreamCaptureModeThreadLocal) != cudaSuccess) return OT2D_ERR_CUDA;
     cudaError_t le = launch_iteration<R>(B.d_sl, B.b, visc, s->turb_bits, s->lhs_bits, s->st);
@@ -408,6 +418,7 @@ int rebuild_t(ot2d_solver* s, DevBatch<R>& B) {
   for (int h = 0; h < 2; ++h) {
     H[h].rt_shape = ch.rt_shape;
     if ((e = H[h].build(slh[h], s->st))) return e;
+    H[h].b.shared_bands = B.b.bands;
     H[h].b.poll_limit = s->poll_limit;
     H[h].b.ts_in_update = B.b.ts_in_update;
     H[h].b.lu_lag = ch.lu_lag;
@@ -827,7 +838,7 @@ void ot2d_solver_destroy(ot2d_solver* s) {
   if (s->ev_join) cudaEventDestroy(s->ev_join);
   for (int q = 0; q < ot2d_solver::HP; ++q) {
     s->p64[q].release(); s->p32[q].release();
-    if (s->ev_pdone[q]) cudaEventDestroy(s->ev_pdone[q]);
+    for (cudaEvent_t e : {s->ev_pdone[q], s->ev_pup[q], s->ev_pdown[q]}) if (e) cudaEventDestroy(e);
     if (s->pst[q]) { cudaStreamSynchronize(s->pst[q]); cudaStreamDestroy(s->pst[q]); }
   }
   if (s->st2) cudaStreamDestroy(s->st2);
@@ -835,6 +846,7 @@ void ot2d_solver_destroy(ot2d_solver* s) {
   for (cudaEvent_t e : s->ev_d2h) cudaEventDestroy(e);
   if (s->ev_step) cudaEventDestroy(s->ev_step);
   if (s->st_d2h) cudaStreamDestroy(s->st_d2h);
+  if (s->st_h2d) cudaStreamDestroy(s->st_h2d);
   s->b64.release(); s->b32.release(); s->f64.release(); s->f32.release();
   if (s->h_out) cudaFreeHost(s->h_out);
   for (cudaEvent_t e : s->ev_out) if (e) cudaEventDestroy(e);
@@ -1048,7 +1060,7 @@ int ot2d_solver_graph_kernels(ot2d_solver* s) {
   if (s->live.empty()) return 0;
   if (s->split4) {
     int k = 0;
-    for (int q = 0; q < ot2d_solver::HP; ++q) {
+    for (int q = 0; q < s->np; ++q) {
       const int a = kernel_nodes(s->pgraph[q]);
       if (a < 0) return a;
       k += a;
@@ -1072,28 +1084,39 @@ cudaError_t host_time_step(ot2d_solver* s, int part, cudaStream_t st) {
 }
 
 // Host-buffer iterations over a batch in parts: per iteration, part q
-// uploads its listed instances on its stream (each upload after that
-// instance's previous download), makes its compute copy and time step, runs
-// its graph and downloads its instances on the download stream.  Some
-// parts' copies thus run while others iterate; every instance computes what
-// it computes in the single graph.
+// uploads its listed instances after its previous downloads, makes its
+// compute copy and time step, runs its graph and downloads its instances.
+// Uploads and downloads have a stream each, so the parts follow one another
+// on the link and some parts' copies run while others iterate.  (With each
+// part's uploads on its own stream the parts shared the link, all started
+// to iterate when all uploads were in, and their downloads came together
+// again: two iterations of 64 instances of 513x129 in four parts 4450 us,
+// 4160 now.)  Every instance computes what it computes in the single graph.
 int iterate_host_parts(ot2d_solver* s, int32_t n, std::vector<Rec*>& rs, double* const* q_host, int32_t iters,
                        int32_t& done) {
-  constexpr int HP = ot2d_solver::HP;
   done = 0;
   int err = OT2D_OK;
   bool parts = true;
+  // uploads come after everything launched before
+  if (!s->st_h2d && cudaStreamCreateWithFlags(&s->st_h2d, cudaStreamNonBlocking) != cudaSuccess) return OT2D_ERR_CUDA;
+  if (cudaEventRecord(s->ev_step, s->st) != cudaSuccess || cudaStreamWaitEvent(s->st_h2d, s->ev_step, 0) != cudaSuccess)
+    return OT2D_ERR_CUDA;
+  for (int q = 0; q < s->np; ++q)
+    if (cudaEventRecord(s->ev_pdown[q], s->pst[q]) != cudaSuccess) return OT2D_ERR_CUDA;
   for (int it = 0; it < iters && !err && parts; ++it) {
     done = it + 1;
-    for (int q = 0; q < HP && !err; ++q) {
+    for (int q = 0; q < s->np && !err; ++q) {
       cudaStream_t sq = s->pst[q];
+      if (cudaStreamWaitEvent(s->st_h2d, s->ev_pdown[q], 0) != cudaSuccess) err = OT2D_ERR_CUDA;
       for (int i = 0; i < n && !err; ++i) {
         if (rs[i]->part != q) continue;
         const size_t bytes = rs[i]->d.n2 * rs[i]->d.nspec * rs[i]->d.P.nq * sizeof(double);
-        if ((it > 0 && cudaStreamWaitEvent(sq, s->ev_d2h[i], 0) != cudaSuccess) ||
-            cudaMemcpyAsync(rs[i]->d.q64, q_host[i], bytes, cudaMemcpyHostToDevice, sq) != cudaSuccess)
+        if (cudaMemcpyAsync(rs[i]->d.q64, q_host[i], bytes, cudaMemcpyHostToDevice, s->st_h2d) != cudaSuccess)
           err = OT2D_ERR_CUDA;
       }
+      if (!err && (cudaEventRecord(s->ev_pup[q], s->st_h2d) != cudaSuccess ||
+                   cudaStreamWaitEvent(sq, s->ev_pup[q], 0) != cudaSuccess))
+        err = OT2D_ERR_CUDA;
       if (!err && s->precision == OT2D_FP32_MIXED &&
           launch_shadow<float>(s->p32[q].d_sl, s->p32[q].b, sq) != cudaSuccess)
         err = OT2D_ERR_CUDA;
@@ -1106,10 +1129,10 @@ int iterate_host_parts(ot2d_solver* s, int32_t n, std::vector<Rec*>& rs, double*
       for (int i = 0; i < n && !err; ++i) {
         if (rs[i]->part != q) continue;
         const size_t bytes = rs[i]->d.n2 * rs[i]->d.nspec * rs[i]->d.P.nq * sizeof(double);
-        if (cudaMemcpyAsync(q_host[i], rs[i]->d.q64, bytes, cudaMemcpyDeviceToHost, s->st_d2h) != cudaSuccess ||
-            cudaEventRecord(s->ev_d2h[i], s->st_d2h) != cudaSuccess)
+        if (cudaMemcpyAsync(q_host[i], rs[i]->d.q64, bytes, cudaMemcpyDeviceToHost, s->st_d2h) != cudaSuccess)
           err = OT2D_ERR_CUDA;
       }
+      if (!err && cudaEventRecord(s->ev_pdown[q], s->st_d2h) != cudaSuccess) err = OT2D_ERR_CUDA;
     }
     bool capped = false;
     for (int id : s->live) {
@@ -1118,7 +1141,7 @@ int iterate_host_parts(ot2d_solver* s, int32_t n, std::vector<Rec*>& rs, double*
     }
     if (!err && (++s->since_check >= s->check_every || capped)) {
       // the status read sees every part done and no upload in flight
-      for (int q = 0; q < HP && !err; ++q)
+      for (int q = 0; q < s->np && !err; ++q)
         if (cudaStreamWaitEvent(s->st, s->ev_pdone[q], 0) != cudaSuccess) err = OT2D_ERR_CUDA;
       if (!err && cudaStreamSynchronize(s->st_d2h) != cudaSuccess) err = OT2D_ERR_CUDA;
       if (!err) err = check(s);
@@ -1130,8 +1153,9 @@ int iterate_host_parts(ot2d_solver* s, int32_t n, std::vector<Rec*>& rs, double*
       }
     }
   }
+  if (cudaStreamSynchronize(s->st_h2d) != cudaSuccess && !err) err = OT2D_ERR_CUDA;
   if (cudaStreamSynchronize(s->st_d2h) != cudaSuccess && !err) err = OT2D_ERR_CUDA;
-  for (int q = 0; q < HP; ++q)
+  for (int q = 0; q < s->np; ++q)
     if (cudaStreamSynchronize(s->pst[q]) != cudaSuccess && !err) err = OT2D_ERR_CUDA;
   if (cudaStreamSynchronize(s->st) != cudaSuccess && !err) err = OT2D_ERR_CUDA;
   return err;
@@ -1159,7 +1183,7 @@ int ot2d_solver_iterate_host(ot2d_solver* s, int32_t n, const int32_t* ids, doub
   }
   // A batch large enough for parts overlaps some parts' copies with the
   // others' iterations.
-  if (!s->parts && !s->want_parts && s->live.size() >= (size_t)ot2d_solver::HP) {
+  if (!s->parts && !s->want_parts && s->live.size() >= (size_t)ot2d_solver::HP_MIN) {
     s->want_parts = true;
     s->dirty = true;
     int e = rebuild(s);

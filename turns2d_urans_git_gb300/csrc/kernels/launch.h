@@ -73,6 +73,8 @@ struct Batch {
   // the solver's batches of steady requests with a first-order time step
   // factor: the local time step of the next iteration is computed by the
   // state update (k_update<R, true>), not by a kernel of its own
+  int bands = 0;           // LU-SGS bands of the batch
+  int shared_bands = 0;    // and, where others run beside it, of all of them together
   int ts_in_update = 0;
   int lim_mask = 0;        // reconstruction families of the slices: 1 central, 2 MUSCL, 4 WENO, 8 quad
   int rt_shape = 0;        // residual tile shape of the tile table (rt_shape_dims)

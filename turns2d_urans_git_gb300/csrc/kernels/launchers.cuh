@@ -147,8 +147,12 @@ cudaError_t launch_lusgs_prep(const Slice<R>* d_sl, const Batch& b, int scale, c
 // 16 per launch 557, 477 (wide groups), 32 per launch 1276, 1328.  FP64
 // 513x129 alone 3769, 1877; 8 per launch 7577, 6801; 16 per launch 12638,
 // 13024.  The same line separates the wide groups of the f32 sweeps (lu_pg).
+// Batches that run beside each other (halves, parts) share the SMs: in four
+// parts, 64 slices of 513x129 (512 bands) 1228, 1269, of 385x97 (384) 747,
+// 787, of 257x65 (256) 394, 383; 32 of 385x97 (192) 492, 483; FP64 257x65,
+// 64 slices (512) 4697, 4759, 32 (256) 2680, 2641.
 // More CTAs than that only where the bands or their shared memory do not fit.
-constexpr int LU_SPREAD_SLICES = 16;
+constexpr int LU_SPREAD_SLICES = 16, LU_SPREAD_BANDS = 256;
 template <class R, bool PRE, int PG>
 int lu_cluster(int nb, bool spread, int maxcol) {
   const int want = spread ? std::min((nb + 3) / 4, LU_MAX_CLUSTER) : 1;
@@ -212,7 +216,7 @@ cudaError_t launch_lusgs_sweeps_t(const Slice<R>* d_sl, const Batch& b, cudaStre
 }
 template <class R, bool PRE>
 cudaError_t launch_lusgs_sweeps_p(const Slice<R>* d_sl, const Batch& b, cudaStream_t st, int only_lu) {
-  if (b.nslice <= LU_SPREAD_SLICES) return launch_lusgs_sweeps_t<R, PRE, lu_pg<R, true>()>(d_sl, b, st, only_lu, true);
+  if (b.nslice <= LU_SPREAD_SLICES && b.shared_bands <= LU_SPREAD_BANDS) return launch_lusgs_sweeps_t<R, PRE, lu_pg<R, true>()>(d_sl, b, st, only_lu, true);
   return launch_lusgs_sweeps_t<R, PRE, lu_pg<R, false>()>(d_sl, b, st, only_lu, false);
 }
 template <class R>

@@ -276,11 +276,12 @@ typedef struct ot2d_result {
 #define OT2D_OPT_LU_GROUP      8  /* LU-SGS records streamed per bulk copy: 1, 2, 4 or 8
                                      (default 0: the largest the shared memory allows) */
 #define OT2D_OPT_RT_SHAPE      9  /* residual tile: 0 16x16 (default), 1 32x8, 2 8x32, 3 32x16 cells */
-#define OT2D_OPT_PIPELINE     10  /* 1 (default): a batch of 16 or more time instances runs
+#define OT2D_OPT_PIPELINE     10  /* 1: a batch of 16 or more time instances runs
                                      as two halves on two streams, each half's residual
                                      beside the other half's LU-SGS sweeps; 2: as four
                                      independent parts on four streams (and at least four
-                                     requests); 0: one graph */
+                                     requests); 0: one graph; not set: as 2 where there
+                                     are four requests, else as 1 */
 #define OT2D_OPT_POLL_LIMIT    5  /* polls a LU-SGS sweep wait makes before it gives up
                                      (default 4194304).  An instance whose wait gave up
                                      keeps its state and retires with OT2D_ERR_TIMEOUT;

@@ -114,7 +114,7 @@ struct ot2d_solver {
   // once the other half's residual of the same (or the previous) iteration
   // is done, so one half's residual fills the SMs the other half's LU-SGS
   // sweeps leave idle.
-  int pipeline = 1;
+  int pipeline = 3;   // OT2D_OPT_PIPELINE; 3: not set
   bool split = false;        // the device-resident iteration runs as the halves
   bool halves = false;       // the halves' graphs exist
   bool split4 = false;       // the device-resident iteration runs as the four parts (OT2D_OPT_PIPELINE 2)
@@ -220,7 +220,7 @@ void drop_graph(ot2d_solver* s) {
   s->parts = false;
 }
 
-// batches of at least this many slices run as two pipelined halves
+// batches of at least this many slices run in parts or as two pipelined halves
 constexpr int PIPE_MIN_SLICES = 16;
 
 // one iteration of every live instance: the single graph, or the two halves
@@ -370,22 +370,26 @@ int rebuild_t(ot2d_solver* s, DevBatch<R>& B) {
   Branch* br = nullptr;   // the turbulence branch's stream, created outside the capture
   if (branch_of_device(br) != cudaSuccess) return OT2D_ERR_CUDA;
   const int visc = s->any_viscous ? 1 : 0;
-  const bool can_split = sl.size() >= (size_t)PIPE_MIN_SLICES && s->live.size() >= 2;
-  const bool split = ch.pipeline == 1 && can_split;
-  const bool can_parts = sl.size() >= (size_t)PIPE_MIN_SLICES && s->live.size() >= (size_t)ot2d_solver::HP_MIN;
-  const bool split4 = ch.pipeline == 2 && can_parts;
+  const bool big = sl.size() >= (size_t)PIPE_MIN_SLICES;
+  const bool can_parts = big && s->live.size() >= (size_t)ot2d_solver::HP_MIN;
+  // Unless the option says which: four independent parts where there are four
+  // requests, else two halves.
+  // Per iteration (us) in halves, in parts: five time instances of four
+  // requests 257x65 250, 234; 16 pitching slices 257x65 261, 247; 24 slices
+  // of five sizes 684, 668; 64 slices 513x129 1257, 1227, 129x33 188, 151.
+  const bool split4 = ch.pipeline >= 2 && can_parts;
+  const bool split = (ch.pipeline & 1) && big && s->live.size() >= 2 && !split4;
   if (split4 && !s->ev_step && cudaEventCreateWithFlags(&s->ev_step, cudaEventDisableTiming) != cudaSuccess)
     return OT2D_ERR_CUDA;
   for (int id : s->live) { s->recs[id].half = -1; s->recs[id].part = -1; }
-  // the parts: for the device-resident iteration (OT2D_OPT_PIPELINE 2) or
-  // once the host-buffer path has been used
-  const bool want_parts = (s->want_parts || ch.pipeline == 2) && sl.size() >= (size_t)PIPE_MIN_SLICES &&
-                          s->live.size() >= (size_t)ot2d_solver::HP_MIN;
-  // Eight parts for the host-buffer path, four for the device-resident one.
+  // the parts: for the device-resident iteration or once the host-buffer
+  // path has been used
+  const bool want_parts = (s->want_parts || split4) && can_parts;
+  // Eight parts once the host-buffer path has been used, four before.
   // Two host iterations in 4, 6, 8 parts (us): 64 instances of 513x129 4155,
   // 3825, 3847; 16 of them 1632, 1585, 1554; 64 of 257x65 1523, 1416, 1395;
   // 64 of 129x33 761, 748, 724.
-  s->np = ch.pipeline != 2 && s->live.size() >= (size_t)ot2d_solver::HP ? ot2d_solver::HP : ot2d_solver::HP_MIN;
+  s->np = s->want_parts && ch.pipeline != 2 && s->live.size() >= (size_t)ot2d_solver::HP ? ot2d_solver::HP : ot2d_solver::HP_MIN;
   if (!split) {
     if (cudaStreamBeginCapture(s->st, cudaStreamCaptureModeThreadLocal) != cudaSuccess) return OT2D_ERR_CUDA;
     cudaError_t le = launch_iteration<R>(B.d_sl, B.b, visc, s->turb_bits, s->lhs_bits, s->st);
@@ -1164,6 +1168,9 @@ int iterate_host_parts(ot2d_solver* s, int32_t n, std::vector<Rec*>& rs, double*
 int ot2d_solver_iterate_host(ot2d_solver* s, int32_t n, const int32_t* ids, double* const* q_host, int32_t iters) {
   if (!s || n < 0 || (n && (!ids || !q_host)) || iters < 0) return OT2D_ERR_ARG;
   cudaSetDevice(s->device);
+  // A batch large enough for parts overlaps some parts' copies with the
+  // others' iterations.
+  if (!s->want_parts && s->live.size() >= (size_t)ot2d_solver::HP_MIN) s->want_parts = s->dirty = true;
   if (s->dirty) { int e = rebuild(s); if (e) return e; }
   std::vector<Rec*> rs;
   for (int i = 0; i < n; ++i) {
@@ -1180,14 +1187,6 @@ int ot2d_solver_iterate_host(ot2d_solver* s, int32_t n, const int32_t* ids, doub
     cudaEvent_t e;
     if (cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess) return OT2D_ERR_CUDA;
     s->ev_d2h.push_back(e);
-  }
-  // A batch large enough for parts overlaps some parts' copies with the
-  // others' iterations.
-  if (!s->parts && !s->want_parts && s->live.size() >= (size_t)ot2d_solver::HP_MIN) {
-    s->want_parts = true;
-    s->dirty = true;
-    int e = rebuild(s);
-    if (e) return e;
   }
   int err = OT2D_OK;
   int32_t done = 0;

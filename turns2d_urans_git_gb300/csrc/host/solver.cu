@@ -148,7 +148,7 @@ struct ot2d_solver {
   int force_decades = 1;                 // norm drop below the peak the force rule needs
   uint32_t poll_limit = 1u << 22;        // polls of a sweep wait (OT2D_OPT_POLL_LIMIT)
   int lu_lag = 0, lu_group = 0;          // LU-SGS schedule (OT2D_OPT_LU_LAG, OT2D_OPT_LU_GROUP)
-  int rt_shape = 0;                      // residual tile shape (OT2D_OPT_RT_SHAPE)
+  int rt_shape = -1;                     // residual tile shape (OT2D_OPT_RT_SHAPE; -1: not set)
   std::vector<ot2d_tuning> tuning;       // per size class (ot2d_solver_set_tuning)
   ot2d_tuning applied{};                 // the choice of the current batch
   int keep_q = 0;
@@ -337,7 +337,14 @@ int rebuild_t(ot2d_solver* s, DevBatch<R>& B) {
   s->dirty = false;
   if (sl.empty()) return OT2D_OK;
   // launch choices: the tuning entry of the batch's largest mesh, else the options
-  ot2d_tuning ch{0, 0, s->rt_shape, s->lu_group, s->lu_lag, s->pipeline};
+  // (residual tiles when the option is not set: 32x8 cells in f32, 16x16 in
+  // FP64.  The kernel is bound by issue in f32, where longer rows load in
+  // fewer instructions, and by the FP64 pipe else, where the squarer tile has
+  // fewer faces.  16x16, 32x8 per iteration, us: 64 slices 513x129 1228, 1196,
+  // its residual 440, 425; 24 slices of five sizes 672, 665; smaller batches
+  // within 1; FP64 385x97 in eights 2114, 2138.)
+  const int tile = s->rt_shape >= 0 ? s->rt_shape : (s->precision == OT2D_FP32_MIXED ? 1 : 0);
+  ot2d_tuning ch{0, 0, tile, s->lu_group, s->lu_lag, s->pipeline};
   {
     size_t best = 0;
     int kd = 0, jd = 0;

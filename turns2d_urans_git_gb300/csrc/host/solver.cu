@@ -396,7 +396,7 @@ int rebuild_t(ot2d_solver* s, DevBatch<R>& B) {
   // Two host iterations in 4, 6, 8 parts (us): 64 instances of 513x129 4155,
   // 3825, 3847; 16 of them 1632, 1585, 1554; 64 of 257x65 1523, 1416, 1395;
   // 64 of 129x33 761, 748, 724.
-  s->np = s->want_parts && ch.pipeline != 2 && s->live.size() >= (size_t)ot2d_solver::HP ? ot2d_solver::HP : ot2d_solver::HP_MIN;
+  s->np = s->want_parts && s->live.size() >= (size_t)ot2d_solver::HP ? ot2d_solver::HP : ot2d_solver::HP_MIN;
   if (!split) {
     if (cudaStreamBeginCapture(s->st, cudaStreamCaptureModeThreadLocal) != cudaSuccess) return OT2D_ERR_CUDA;
     cudaError_t le = launch_iteration<R>(B.d_sl, B.b, visc, s->turb_bits, s->lhs_bits, s->st);

@@ -271,10 +271,10 @@ typedef struct ot2d_result {
 #define OT2D_OPT_BUDGET_MB     6  /* device memory the live instances may hold, MiB
                                      (default 0: 90 % of the memory free when the solver
                                      was created) */
-#define OT2D_OPT_LU_LAG        7  /* LU-SGS schedule: steps each 32-row band trails the
-                                     band it depends on beyond the minimum (default 0) */
-#define OT2D_OPT_LU_GROUP      8  /* LU-SGS records streamed per bulk copy: 1, 2, 4 or 8
-                                     (default 0: the largest the shared memory allows) */
+#define OT2D_OPT_LU_LAG        7  /* LU-SGS schedule: steps each band trails the band it
+                                     depends on beyond the minimum (default 0) */
+#define OT2D_OPT_LU_GROUP      8  /* LU-SGS record chunks in flight per band: 1, 2, 4 or 8
+                                     (default 0: 8, as the shared memory allows) */
 #define OT2D_OPT_RT_SHAPE      9  /* residual tile: 0 16x16 (default in FP64), 1 32x8 (default in
                                      FP32-mixed), 2 8x32, 3 32x16 cells */
 #define OT2D_OPT_PIPELINE     10  /* 1: a batch of 16 or more time instances runs

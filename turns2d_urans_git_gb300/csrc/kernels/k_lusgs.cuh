@@ -41,7 +41,7 @@ namespace ot2d {
 // variable (1930 cycles; the exchange between the lanes is the rest).  The
 // preconditioned FP64 operator, whose preconditioner couples the four
 // variables once more, stays at two.  Both sweeps and their records, 257x65
-// FP64: 1710 -> 765 us; 385x97: 2658 -> 1220; FP32-mixed 769x193: 485 -> 301.
+// FP64: 1710 -> 755 us; 385x97: 2658 -> 1150; FP32-mixed 769x193: 485 -> 301.
 template <class R, bool PRE = false>
 struct LuSplit {
   static constexpr int LP = (sizeof(R) == 8 && !PRE) ? 4 : 2;   // lanes per cell

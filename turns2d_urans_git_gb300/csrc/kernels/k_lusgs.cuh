@@ -618,6 +618,10 @@ struct LuLanes<R, FWD, PRE, 2, KS> {
   __device__ __forceinline__ bool owns_eta() const { return d == 1; }
   __device__ __forceinline__ void put_if(bool c, uint32_t p) const { lu_sts4_if(c, p, out); }
   __device__ __forceinline__ void send(uint32_t dst, uint32_t bar) const { lu_send(dst, bar, out); }
+  __device__ __forceinline__ void send_zero(uint32_t dst, uint32_t bar) const {
+    const R z[4] = {0, 0, 0, 0};
+    lu_send(dst, bar, z);
+  }
 };
 
 // Four lanes per cell (FP64): lane 4r+v holds variable v.  Lanes 0..3 form
@@ -697,6 +701,7 @@ struct LuLanes<double, FWD, false, 4, KS> {
   __device__ __forceinline__ bool owns_eta() const { return true; }
   __device__ __forceinline__ void put_if(bool c, uint32_t p) const { lu_sts_if(c, p + vb, oe); }
   __device__ __forceinline__ void send(uint32_t dst, uint32_t bar) const { lu_send1(dst + vb, bar, oe); }
+  __device__ __forceinline__ void send_zero(uint32_t dst, uint32_t bar) const { lu_send1(dst + vb, bar, 0.0); }
 };
 
 // bulk copy (TMA) into this CTA's shared memory, counted on bar; 16-byte
@@ -727,7 +732,8 @@ struct LuBand {
 };
 
 // One band of one sweep.  Returns the group at which a bounded wait gave up,
-// or -1.
+// or -1.  A group whose waits did not all end is left alone: its records may
+// not have landed, so nothing of it is read, stored, handed on or refilled.
 template <class R, bool FWD, bool PRE, int PG, int IN, int OUT>
 __device__ __forceinline__ int lu_band(const LuBand<R>& B, int l) {
   constexpr int CH = LuLay<R, PRE>::CH, LS = LuLay<R, PRE>::LS, LP = LuSplit<R, PRE>::LP, RB = LuSplit<R, PRE>::RB;
@@ -785,13 +791,15 @@ __device__ __forceinline__ int lu_band(const LuBand<R>& B, int l) {
   auto group = [&](auto ramp_) {
     constexpr bool RAMP = decltype(ramp_)::value;
     const int t0 = g * PG, ps = RAMP ? min(PG, nst - t0) : PG, p0 = t0 - prow;
-    ok = mbar_wait_bounded(&B.bars[stage], phase, lim) && ok;
+    ok = mbar_wait_bounded(&B.bars[stage], phase, lim);
     // the first row's inputs of these steps (columns t0 .. t0+PG-1 in sweep
     // order, produced RB-1 steps later by the previous band), and room in the
     // ring for the last row's outputs
     if (IN == LU_RING && (!RAMP || t0 < ncol)) ok = wait_full(min(g + RB / PG, qlast)) && ok;
     if (IN == LU_LINK && (!RAMP || t0 < ncol)) ok = lu_link_wait(&B.lbars[t0 / LU_LG], lim) && ok;
     if (OUT == LU_RING && g + 1 >= (RB + LU_XB) / PG) ok = wait_empty(g + 1 - (RB + LU_XB) / PG) && ok;
+    ok = __all_sync(0xffffffffu, ok);
+    if (!ok) return;
     const uint32_t st0 = B.stages + (uint32_t)stage * PG * CHB + (uint32_t)row * LS * sizeof(R);
     const uint32_t ch0 = FWD ? st0 : st0 + (uint32_t)(ps - 1) * CHB;
     const int k0 = PG == KS ? 0 : t0 & (KS - 1);
@@ -824,7 +832,6 @@ __device__ __forceinline__ int lu_band(const LuBand<R>& B, int l) {
     }
     if (++stage == D) { stage = 0; phase ^= 1; }
     ++g;
-    ok = __all_sync(0xffffffffu, ok);
   };
   while (g < ngrp && ok) {
     if (g == g0)
@@ -833,10 +840,16 @@ __device__ __forceinline__ int lu_band(const LuBand<R>& B, int l) {
     if (g < ngrp && ok) group(std::true_type());
   }
   if (ok) return -1;
-  // copies issued and not consumed: wait (bounded) before the CTA's shared
-  // memory goes away
+  // The rest of the row that the next CTA takes, as zeros (its results are
+  // discarded with the slice's): with it every barrier of the link completes,
+  // so that CTA can wait for the last store before its shared memory goes.
+  if (OUT == LU_LINK && out_lane)
+    for (int q = max(0, g * PG - (RB - 1)); q < ncol; ++q)
+      L.send_zero(B.ldst + (uint32_t)q * SB, B.lbar + (uint32_t)(q / LU_LG) * 8);
+  // copies issued and not consumed, each in its own phase: wait (bounded)
+  // before the CTA's shared memory goes away
   if (l == 0)
-    for (int h = max(0, g - 1); h < min(g + D, ngrp); ++h) mbar_wait_bounded(&B.bars[h % D], (uint32_t)(h / D) & 1);
+    for (int h = g; h < min(g + D, ngrp); ++h) mbar_wait_bounded(&B.bars[h % D], (uint32_t)(h / D) & 1);
   __syncwarp();
   return g;
 }
@@ -945,13 +958,13 @@ __device__ void lu_sweep_slice(const Slice<R>& S, int nwarp, int cs, int rank, i
   }
   // a give-up before the halo's row has landed: wait (bounded) for it
   if (!linked && mine > 0 && threadIdx.x == 0) mbar_wait_bounded(&lbars[0], 0);
-  // no CTA leaves while another may still write into it; after a give-up
-  // the stores already under way get time to land too
+  // no CTA leaves while another may still write into it: past the cluster
+  // barrier the previous CTA has issued its whole row, and what a band that
+  // gave up has not waited for is waited for (bounded) here
   if (cs > 1) {
     lu_cluster_sync();
-    if (linked && __syncthreads_or(gfail >= 0)) {
-      for (int i = 0; i < 64; ++i) __nanosleep(1000);
-    }
+    if (linked && __syncthreads_or(gfail >= 0))
+      for (int i = threadIdx.x; i < (ncol + LU_LG - 1) / LU_LG; i += blockDim.x) lu_link_wait(&lbars[i], LU_POLL_DEFAULT);
   }
 }
 

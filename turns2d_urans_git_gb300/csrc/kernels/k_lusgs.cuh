@@ -452,6 +452,17 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity
   return false;
 }
 
+// The same by a whole warp.  The vote makes the loop and its result uniform:
+// the band leaves at the first wait that runs out, and a step costs what it
+// costs without a check (one vote over the lanes' results ahead of a group's
+// first read cost 85 cycles a group: both sweeps of a 1025x33 mesh 252 us with
+// a vote at the end of the group, 263 ahead of it, 249 so).
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, uint32_t lim) {
+  for (uint32_t it = 0; it < lim; ++it)
+    if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+  return false;
+}
+
 // Cross-band ring: the last row of a band hands its outgoing (j,k-1)
 // contribution at its p-th column (in sweep order) to the next band through
 // slot p % LU_XB; the consumer's first row reads it at its own step p.
@@ -519,6 +530,7 @@ __device__ __forceinline__ void lu_send(uint32_t dst, uint32_t bar, const double
 #pragma unroll
   for (int n = 0; n < 4; ++n) lu_send1(dst + 8 * n, bar, v[n]);
 }
+// a whole warp's wait (as mbar_wait_warp) for a barrier of the link
 __device__ __forceinline__ bool lu_link_wait(uint64_t* bar, uint32_t lim) {
   for (uint32_t it = 0; it < lim; ++it) {
     uint32_t ok;
@@ -528,7 +540,7 @@ __device__ __forceinline__ bool lu_link_wait(uint64_t* bar, uint32_t lim) {
         : "=r"(ok)
         : "r"(smem_u32(bar))
         : "memory");
-    if (ok) return true;
+    if (__all_sync(0xffffffffu, (int)ok)) return true;
   }
   return false;
 }
@@ -773,15 +785,15 @@ __device__ __forceinline__ int lu_band(const LuBand<R>& B, int l) {
   // Waits for group q of the previous band's, or the next band's, steps (each
   // phase of a ring slot's barrier is one group).
   const int qlast = ngrp - 1;
-  auto wait_full = [&](int q) { return mbar_wait_bounded(&B.xb_in[q % NS], (uint32_t)(q / NS) & 1, lim); };
-  auto wait_empty = [&](int q) { return mbar_wait_bounded(&B.xb_out[NS + q % NS], (uint32_t)(q / NS) & 1, lim); };
+  auto wait_full = [&](int q) { return mbar_wait_warp(&B.xb_in[q % NS], (uint32_t)(q / NS) & 1, lim); };
+  auto wait_empty = [&](int q) { return mbar_wait_warp(&B.xb_out[NS + q % NS], (uint32_t)(q / NS) & 1, lim); };
   bool ok = true;
-  if (IN == LU_HALO) ok = __all_sync(0xffffffffu, mbar_wait_bounded(&B.lbars[0], 0, lim));
+  if (IN == LU_HALO) ok = mbar_wait_warp(&B.lbars[0], 0, lim);
   // Band lag: start `lag` steps after the neighbouring band's first
   // contribution is due (the operands of every cell are the same whatever
   // the lag; at most what the ring holds).
   if (IN == LU_RING && B.lag > 0)
-    ok = __all_sync(0xffffffffu, wait_full(min(min(RB + B.lag, LU_XB) / PG - 1, qlast)));
+    ok = wait_full(min(min(RB + B.lag, LU_XB) / PG - 1, qlast));
   // groups g0 .. g1-1 have every row active and none on its first column
   const bool full = B.row0 + RB <= B.nrow;
   const int g0 = full ? RB / PG : ngrp, g1 = full ? max(g0, ncol / PG) : ngrp;
@@ -791,15 +803,13 @@ __device__ __forceinline__ int lu_band(const LuBand<R>& B, int l) {
   auto group = [&](auto ramp_) {
     constexpr bool RAMP = decltype(ramp_)::value;
     const int t0 = g * PG, ps = RAMP ? min(PG, nst - t0) : PG, p0 = t0 - prow;
-    ok = mbar_wait_bounded(&B.bars[stage], phase, lim);
+    if (!(ok = mbar_wait_warp(&B.bars[stage], phase, lim))) return;
     // the first row's inputs of these steps (columns t0 .. t0+PG-1 in sweep
     // order, produced RB-1 steps later by the previous band), and room in the
     // ring for the last row's outputs
-    if (IN == LU_RING && (!RAMP || t0 < ncol)) ok = wait_full(min(g + RB / PG, qlast)) && ok;
-    if (IN == LU_LINK && (!RAMP || t0 < ncol)) ok = lu_link_wait(&B.lbars[t0 / LU_LG], lim) && ok;
-    if (OUT == LU_RING && g + 1 >= (RB + LU_XB) / PG) ok = wait_empty(g + 1 - (RB + LU_XB) / PG) && ok;
-    ok = __all_sync(0xffffffffu, ok);
-    if (!ok) return;
+    if (IN == LU_RING && (!RAMP || t0 < ncol) && !(ok = wait_full(min(g + RB / PG, qlast)))) return;
+    if (IN == LU_LINK && (!RAMP || t0 < ncol) && !(ok = lu_link_wait(&B.lbars[t0 / LU_LG], lim))) return;
+    if (OUT == LU_RING && g + 1 >= (RB + LU_XB) / PG && !(ok = wait_empty(g + 1 - (RB + LU_XB) / PG))) return;
     const uint32_t st0 = B.stages + (uint32_t)stage * PG * CHB + (uint32_t)row * LS * sizeof(R);
     const uint32_t ch0 = FWD ? st0 : st0 + (uint32_t)(ps - 1) * CHB;
     const int k0 = PG == KS ? 0 : t0 & (KS - 1);
@@ -963,8 +973,8 @@ __device__ void lu_sweep_slice(const Slice<R>& S, int nwarp, int cs, int rank, i
   // gave up has not waited for is waited for (bounded) here
   if (cs > 1) {
     lu_cluster_sync();
-    if (linked && __syncthreads_or(gfail >= 0))
-      for (int i = threadIdx.x; i < (ncol + LU_LG - 1) / LU_LG; i += blockDim.x) lu_link_wait(&lbars[i], LU_POLL_DEFAULT);
+    if (linked && __syncthreads_or(gfail >= 0) && w == 0)
+      for (int i = 0; i < (ncol + LU_LG - 1) / LU_LG; ++i) lu_link_wait(&lbars[i], LU_POLL_DEFAULT);
   }
 }
 

@@ -112,16 +112,8 @@ size_t solve_bytes(const ot2d_params& p, int precision) {
 }
 
 bool batch_fits(int precision, bool precon, int kd_max, int jd_max) {
-  if (kd_max < 3 || jd_max < 3 || kd_max - 2 > 1024) return false;
-  // the mesh limit: in bands of 32 rows, the single-copy record ring (28 f32 /
-  // 26 FP64 elements per cell, 36 / 34 preconditioned), the cross-band ring
-  // and counters of every band, and one row of halo contributions, within
-  // one CTA's shared memory (the sweeps, spread over a cluster, need less)
-  const size_t es = precision == OT2D_FP32_MIXED ? sizeof(float) : sizeof(double);
-  const size_t ls = precision == OT2D_FP32_MIXED ? (precon ? 36 : 28) : (precon ? 34 : 26);
-  const size_t nb = (size_t)lu_nband(kd_max, 32);
-  const size_t lu = nb * (2 * 32 * ls * es + 16 + 128 * 4 * es + 4) + 16 + 4 * (size_t)jd_max * es;
-  return lu <= (size_t)SMEM_OPTIN_MAX && sizeof(double) * 3 * (size_t)jd_max <= (size_t)SMEM_OPTIN_MAX;
+  return precision == OT2D_FP32_MIXED ? lu_batch_fits<float>(precon, kd_max, jd_max)
+                                      : lu_batch_fits<double>(precon, kd_max, jd_max);
 }
 
 void solve_destroy(DevSolve& d) {

@@ -27,42 +27,10 @@
 #pragma once
 #include <type_traits>
 #include "dev_common.cuh"
+#include "lu_shape.h"
 
 namespace ot2d {
 
-// Lanes per cell and rows per band of the sweeps.  A sweep is a chain of
-// ncol + nrow steps, so its time is the time of one step.  Two lanes per cell
-// (both form the cell's correction, the even one its xi contribution, the odd
-// one its eta contribution) leave an f32 step 70 instructions instead of 127
-// and ~290 cycles; one lane per cell (bands of 32 rows) took 315.  FP64: the
-// pipe takes a warp instruction every 64 cycles per SM sub-partition whatever
-// the lanes do, so a step is the number of FP64 operations of a lane: 78 with
-// one lane per cell (5900 cycles a step), 47 with two, 21 with four, one per
-// variable (1930 cycles; the exchange between the lanes is the rest).  The
-// preconditioned FP64 operator, whose preconditioner couples the four
-// variables once more, stays at two.  Both sweeps and their records, 257x65
-// FP64: 1710 -> 755 us; 385x97: 2658 -> 1150; FP32-mixed 769x193: 485 -> 301.
-template <class R, bool PRE = false>
-struct LuSplit {
-  static constexpr int LP = (sizeof(R) == 8 && !PRE) ? 4 : 2;   // lanes per cell
-  static constexpr int RB = 32 / LP;                            // rows per band
-};
-
-// A (band, step) chunk holds the records of the band's RB cells one after
-// another (row-major): a cell's 24 fields are contiguous, so a lane reads
-// several consecutive fields with 16-byte shared loads.  The record stride LS
-// puts the rows of a load phase on disjoint banks: f32 24 elements (four rows
-// and both directions' groups of a 16-byte phase cover the 32 banks), FP64 28
-// (four rows x four 8-byte fields).  With Turkel preconditioning (PRE, the
-// preilu2d operator of lhs.f:2-467) a record carries 8 more fields: the
-// chk*qq products of both sweeps and the preconditioner factor.
-template <class R, bool PRE = false>
-struct LuLay {
-  static constexpr int NF = PRE ? 32 : 24;                                   // fields per record
-  static constexpr int LS = sizeof(R) == 4 ? (PRE ? 36 : 24) : (PRE ? 34 : 28);   // elements per cell record
-  static constexpr int RB = LuSplit<R, PRE>::RB;
-  static constexpr int CH = RB * LS;                                         // elements per chunk
-};
 // record fields; each group of four is one 16-byte (f32) access
 enum {
   LF_S = 0,    // 0..3: residual (forward input, then forward result)
@@ -79,20 +47,6 @@ enum {
 template <class R, bool PRE = false>
 __host__ __device__ __forceinline__ int lu_idx(int f, int r) {
   return r * LuLay<R, PRE>::LS + f;
-}
-
-__host__ __device__ __forceinline__ int lu_nrow(int kd) { return kd - 2; }
-__host__ __device__ __forceinline__ int lu_ncol(int jd) { return jd - 2; }
-// bands of rb rows and steps of a band
-__host__ __device__ __forceinline__ int lu_nband(int kd, int rb) { return (kd - 2 + rb - 1) / rb; }
-__host__ __device__ __forceinline__ int lu_nstep(int jd, int rb) { return jd - 2 + rb - 1; }
-// elements of one slice's record (element size esize bytes): chunks + 4
-// halo-contribution arrays, enough for the plain and the preconditioned
-// layout so that a slice can use either (36 / 34 elements per cell in bands
-// of 32 rows bound both)
-__host__ __device__ __forceinline__ int64_t lu_rec_elems(int jd, int kd, int esize) {
-  const int64_t ch = 32 * (esize == 4 ? 36 : 34);
-  return (int64_t)lu_nband(kd, 32) * lu_nstep(jd, 32) * ch + 8 * (int64_t)(lu_nrow(kd) + lu_ncol(jd)) + 64;
 }
 
 // fields f..f+3 of row l of a chunk (f a multiple of 4) as 16-byte accesses
@@ -461,50 +415,6 @@ __device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, u
   for (uint32_t it = 0; it < lim; ++it)
     if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
   return false;
-}
-
-// Cross-band ring: the last row of a band hands its outgoing (j,k-1)
-// contribution at its p-th column (in sweep order) to the next band through
-// slot p % LU_XB; the consumer's first row reads it at its own step p.
-constexpr int LU_XB = 64;         // a power of two; a band may run this many columns ahead of the next
-constexpr int LU_LG = 8;          // columns per barrier of a link between CTAs
-constexpr int LU_MAX_WARPS = 16;  // bands per CTA of a sweep
-constexpr int LU_MAX_CLUSTER = 8; // CTAs per slice
-
-// PG, the steps per group: a group's records arrive with one bulk copy, and
-// waits on the neighbouring bands are made and progress is published once per
-// group, so a band trails the one before it by RB + PG steps.  A group's
-// waits and bookkeeping cost about as much as two f32 steps: groups of 8 make
-// a step 215 cycles, groups of 4 294 (f32 sweeps of a 513x33 mesh, 147 and
-// 183 us), but hold twice the shared memory; in a batch whose sweeps share
-// their SMs with the turbulence solve the smaller groups are faster (64
-// 513x129 requests 1256 against 1402 us per iteration).  FP64 steps are an
-// order longer: groups of 2, which trail least.
-template <class R, bool WIDE>
-__host__ __device__ constexpr int lu_pg() { return sizeof(R) == 8 ? 2 : (WIDE ? 8 : 4); }
-// Exchange buffer of a warp, through which the lanes of a step pass values on
-// (a 16-byte store and load take the place of four shuffles).  A contribution
-// made at step t goes to slot (t+1) % lu_ks() of its lane; the slots of a lane
-// are 4 elements apart, as the columns of the cross-band ring are, so that a
-// cell takes its eta input at the same step stride from either.
-template <int PG>
-__host__ __device__ constexpr int lu_ks() { return PG < 4 ? 4 : PG; }
-template <class R, bool PRE, int PG>
-__host__ __device__ constexpr int lu_ex() {
-  return LuSplit<R, PRE>::LP == 2 ? 32 * 4 * (lu_ks<PG>() + 1) : 64 + 8 * 4 * (lu_ks<PG>() + 1);
-}
-
-// Shared memory of a sweep CTA: per warp D stages of a group's records with a
-// barrier each, its cross-band ring with a full and an empty barrier per
-// group of columns, and its exchange buffer; then one row of contributions
-// per column (at most maxcol): the halo's for the CTA with the first band in
-// sweep order, the previous CTA's last row for the others, with one barrier
-// per LU_LG columns.
-template <class R, bool PRE, int PG>
-__host__ __device__ __forceinline__ size_t lu_smem_bytes(int nwarp, int D, int maxcol) {
-  return (size_t)nwarp * (D * PG * LuLay<R, PRE>::CH + LU_XB * 4 + lu_ex<R, PRE, PG>()) * sizeof(R) +
-         (size_t)4 * maxcol * sizeof(R) + (size_t)nwarp * (D + 2 * (LU_XB / PG)) * sizeof(uint64_t) +
-         (size_t)((maxcol + LU_LG - 1) / LU_LG) * sizeof(uint64_t);
 }
 
 // address of a local shared-memory object in CTA `rank` of the cluster
@@ -891,17 +801,18 @@ __device__ void lu_sweep_slice(const Slice<R>& S, int nwarp, int cs, int rank, i
   const int band = base + w;
   R* stages = (R*)smem;
   R* xrings = stages + (size_t)nwarp * D * PG * CH;
-  R* exs = xrings + (size_t)nwarp * LU_XB * 4;
+  R* exs = xrings + (size_t)lu_nring(nwarp) * LU_XB * 4;
   R* rowbuf = exs + (size_t)nwarp * lu_ex<R, PRE, PG>();
   uint64_t* bars = (uint64_t*)(rowbuf + (size_t)4 * maxcol);
   uint64_t* xbars = bars + (size_t)nwarp * D;               // per warp: full[NS], empty[NS] of its ring
-  uint64_t* lbars = xbars + (size_t)nwarp * 2 * NS;
+  uint64_t* lbars = xbars + (size_t)lu_nring(nwarp) * 2 * NS;
   const bool wok = w < mine;
   // the CTA of the first band in sweep order takes the halo's contributions
   const bool first_cta = FWD ? rank == 0 : base + mine == nb;
   const bool linked = cs > 1 && mine > 0 && !first_cta;     // takes its row from the previous CTA
   for (int i = l; i < D; i += 32) mbar_init(&bars[(size_t)w * D + i], 1);
-  for (int i = l; i < 2 * NS; i += 32) mbar_init(&xbars[(size_t)w * 2 * NS + i], 1);
+  if (nwarp > 1)
+    for (int i = l; i < 2 * NS; i += 32) mbar_init(&xbars[(size_t)w * 2 * NS + i], 1);
   asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   for (int i = l; i < lu_ex<R, PRE, PG>(); i += 32) exs[(size_t)w * lu_ex<R, PRE, PG>() + i] = (R)0;
   if (linked) {

@@ -5,6 +5,7 @@
 #include <cstdint>
 #include <mutex>
 #include <cuda_runtime.h>
+#include "lu_shape.h"
 
 namespace ot2d {
 
@@ -62,9 +63,6 @@ struct DeviceOnce {
     return cudaSuccess;
   }
 };
-
-// Largest dynamic shared memory a CTA may opt in to on sm_103a (227 KB).
-constexpr int SMEM_OPTIN_MAX = 227 * 1024;
 
 struct Batch {
   int nslice = 0;          // slices in the batch

@@ -139,45 +139,12 @@ cudaError_t launch_lusgs_prep(const Slice<R>* d_sl, const Batch& b, int scale, c
   if (e == cudaSuccess && b.precon) e = launch_lusgs_prep_t<R, true>(d_sl, b, scale, st, only_lu, parts);
   return e;
 }
-// CTAs per slice of the sweeps (a cluster), for nb bands.  One warp per SM
-// sub-partition (4 bands per CTA) makes a step fastest, but takes SMs from
-// the residual and the turbulence solve of a large batch.  Measured per
-// iteration (us), one CTA against ceil(nb / 4): FP32-mixed RANS-SA 769x193
-// alone 760, 454; 8 per launch 1127, 869; 32 per launch 2715, 2786; 513x129
-// 16 per launch 557, 477 (wide groups), 32 per launch 1276, 1328.  FP64
-// 513x129 alone 3769, 1877; 8 per launch 7577, 6801; 16 per launch 12638,
-// 13024.  The same line separates the wide groups of the f32 sweeps (lu_pg).
-// Batches that run beside each other (halves, parts) share the SMs: in four
-// parts, 64 slices of 513x129 (512 bands) 1228, 1269, of 385x97 (384) 747,
-// 787, of 257x65 (256) 394, 383; 32 of 385x97 (192) 492, 483; FP64 257x65,
-// 64 slices (512) 4697, 4759, 32 (256) 2680, 2641.
-// More CTAs than that only where the bands or their shared memory do not fit.
-constexpr int LU_SPREAD_SLICES = 16, LU_SPREAD_BANDS = 256;
-template <class R, bool PRE, int PG>
-int lu_cluster(int nb, bool spread, int maxcol) {
-  const int want = spread ? std::min((nb + 3) / 4, LU_MAX_CLUSTER) : 1;
-  for (int cs = want; cs <= LU_MAX_CLUSTER; ++cs) {
-    const int nw = (nb + cs - 1) / cs;
-    if (nw <= LU_MAX_WARPS && lu_smem_bytes<R, PRE, PG>(nw, 2, maxcol) <= (size_t)SMEM_OPTIN_MAX) return cs;
-  }
-  return 0;
-}
 // ilu2d part 2: the forward and backward sweeps, launched at the device's
 // highest priority (they are the iteration's longest dependency chain and
 // run beside the turbulence branch)
 template <class R, bool PRE, int PG>
-cudaError_t launch_lusgs_sweeps_t(const Slice<R>* d_sl, const Batch& b, cudaStream_t st, int only_lu, bool spread) {
-  const int maxcol = b.max_wall;   // >= jd - 2 of every slice
-  const int nb = lu_nband(b.max_kd, LuSplit<R, PRE>::RB);
-  const int cs = lu_cluster<R, PRE, PG>(nb, spread, maxcol);
-  if (cs < 1) return cudaErrorInvalidConfiguration;
-  const int nw = (nb + cs - 1) / cs;
-  // records in flight per band: two groups, or lu_group chunks where that is
-  // more (FP64: 16 by default), within ~200 KB of shared memory
-  const int G = (b.lu_group == 1 || b.lu_group == 2 || b.lu_group == 4 || b.lu_group == 8) ? b.lu_group : 8;
-  int D = std::max(2, (sizeof(R) == 8 ? 2 : 1) * G / PG);
-  while (D > 2 && lu_smem_bytes<R, PRE, PG>(nw, D, maxcol) > 200 * 1024) --D;
-  const size_t smem = lu_smem_bytes<R, PRE, PG>(nw, D, maxcol);
+cudaError_t launch_lusgs_sweeps_t(const Slice<R>* d_sl, const Batch& b, cudaStream_t st, int only_lu,
+                                  const LuLaunch& L) {
   static DeviceOnce once;
   int prio = 0;
   cudaError_t ae = once.run(
@@ -197,27 +164,31 @@ cudaError_t launch_lusgs_sweeps_t(const Slice<R>* d_sl, const Batch& b, cudaStre
   at[0].id = cudaLaunchAttributePriority;
   at[0].val.priority = prio;
   at[1].id = cudaLaunchAttributeClusterDimension;
-  at[1].val.clusterDim.x = cs;
+  at[1].val.clusterDim.x = L.cs;
   at[1].val.clusterDim.y = 1;
   at[1].val.clusterDim.z = 1;
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(b.nslice * cs);
-  cfg.blockDim = dim3(32 * nw);
-  cfg.dynamicSmemBytes = smem;
+  cfg.gridDim = dim3(b.nslice * L.cs);
+  cfg.blockDim = dim3(32 * L.nw);
+  cfg.dynamicSmemBytes = L.smem;
   cfg.stream = st;
   cfg.attrs = at;
   cfg.numAttrs = 2;
-  cudaError_t e =
-      cudaLaunchKernelEx(&cfg, k_lu_sweep<R, true, PRE, PG>, d_sl, only_lu, b.poll_limit, b.lu_lag, cs, maxcol, D);
+  cudaError_t e = cudaLaunchKernelEx(&cfg, k_lu_sweep<R, true, PRE, PG>, d_sl, only_lu, b.poll_limit, b.lu_lag, L.cs,
+                                     b.max_wall, L.D);
   if (e != cudaSuccess) return e;
-  e = cudaLaunchKernelEx(&cfg, k_lu_sweep<R, false, PRE, PG>, d_sl, only_lu, b.poll_limit, b.lu_lag, cs, maxcol, D);
+  e = cudaLaunchKernelEx(&cfg, k_lu_sweep<R, false, PRE, PG>, d_sl, only_lu, b.poll_limit, b.lu_lag, L.cs, b.max_wall,
+                         L.D);
   if (e != cudaSuccess) return e;
   return cudaGetLastError();
 }
 template <class R, bool PRE>
 cudaError_t launch_lusgs_sweeps_p(const Slice<R>* d_sl, const Batch& b, cudaStream_t st, int only_lu) {
-  if (b.nslice <= LU_SPREAD_SLICES && b.shared_bands <= LU_SPREAD_BANDS) return launch_lusgs_sweeps_t<R, PRE, lu_pg<R, true>()>(d_sl, b, st, only_lu, true);
-  return launch_lusgs_sweeps_t<R, PRE, lu_pg<R, false>()>(d_sl, b, st, only_lu, false);
+  constexpr int W = lu_pg<R, true>(), N = lu_pg<R, false>();
+  const LuLaunch L = lu_launch<R, PRE>(b.max_kd, b.max_wall, lu_spread(b.nslice, b.shared_bands), b.lu_group);
+  if (!L.cs) return cudaErrorInvalidConfiguration;
+  return L.pg == W ? launch_lusgs_sweeps_t<R, PRE, W>(d_sl, b, st, only_lu, L)
+                   : launch_lusgs_sweeps_t<R, PRE, N>(d_sl, b, st, only_lu, L);
 }
 template <class R>
 cudaError_t launch_lusgs_sweeps(const Slice<R>* d_sl, const Batch& b, cudaStream_t st, int only_lu) {

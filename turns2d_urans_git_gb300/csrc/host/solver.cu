@@ -56,6 +56,17 @@ constexpr int FORCE_WIN = 8;
 // caller or from a restart file); returns an OT2D status.
 using InitFn = std::function<int(ot2d_solver*, Rec&)>;
 
+// The solver's device current for the time of a call that only reads, the
+// caller's afterwards.
+struct OnDevice {
+  int dev, prev = -1;
+  explicit OnDevice(int d) : dev(d) {
+    if (cudaGetDevice(&prev) != cudaSuccess) prev = -1;
+    cudaSetDevice(dev);
+  }
+  ~OnDevice() { if (prev >= 0 && prev != dev) cudaSetDevice(prev); }
+};
+
 // A submitted solve waiting for device memory.
 struct Pending {
   int id = -1;
@@ -961,6 +972,7 @@ int ot2d_solver_iterate(ot2d_solver* s, int32_t iters) {
 
 int ot2d_solver_sync(ot2d_solver* s) {
   if (!s) return OT2D_ERR_ARG;
+  OnDevice on(s->device);   // a check may allocate and launch (forces)
   return check(s);
 }
 
@@ -1025,7 +1037,11 @@ int ot2d_solver_get_q(ot2d_solver* s, int32_t id, double* q_out) {
   auto it = s->recs.find(id);
   if (it == s->recs.end()) return OT2D_ERR_ARG;
   Rec& r = it->second;
-  if (r.live) return copy_out(s, q_out, r.d.q64, r.d.n2 * r.d.nspec * r.d.P.nq * sizeof(double));
+  if (r.live) {
+    // the copy's events belong to the device of the solver's stream
+    OnDevice on(s->device);
+    return copy_out(s, q_out, r.d.q64, r.d.n2 * r.d.nspec * r.d.P.nq * sizeof(double));
+  }
   if (r.qkeep.empty()) return OT2D_ERR_ARG;
   std::memcpy(q_out, r.qkeep.data(), r.qkeep.size() * sizeof(double));
   return OT2D_OK;

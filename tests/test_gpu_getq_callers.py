@@ -1,8 +1,10 @@
-"""ot2d_solver_get_q for a thread whose current context is another one than
-the solver's device's.  Fresh buffers, whose copies go through the solver's
-pinned chunks."""
+"""ot2d_solver_get_q for callers other than one thread with the solver's
+device current: a thread whose current context is another one, and several
+threads that read states of one solver at once.  Fresh buffers, whose copies
+go through the solver's pinned chunks."""
 import ctypes as C
 import mmap
+import threading
 
 import numpy as np
 import pytest
@@ -47,3 +49,28 @@ def test_another_context_is_current():
         cu.cuCtxDestroy_v2(other)
     sv.close()
     sv2.close()
+
+
+def test_threads_read_at_once():
+    sv, ids, prm = _solver(8)
+    ref = [_fresh(p) for p in prm]
+    assert all(_get(sv, i, q) == 0 for i, q in zip(ids, ref))
+    assert not np.array_equal(ref[0], ref[1])
+    for _ in range(5):
+        out = [_fresh(p) for p in prm]
+        rc = [None] * len(ids)
+        start = threading.Barrier(len(ids))
+
+        def read(k):
+            start.wait()
+            rc[k] = _get(sv, ids[k], out[k])
+
+        ts = [threading.Thread(target=read, args=(k,)) for k in range(len(ids))]
+        for t in ts:
+            t.start()
+        for t in ts:
+            t.join()
+        assert rc == [0] * len(ids)
+        for a, b in zip(out, ref):
+            assert np.array_equal(a, b)
+    sv.close()

@@ -15,6 +15,7 @@
 #include <deque>
 #include <functional>
 #include <map>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -103,7 +104,8 @@ struct ot2d_solver {
   std::vector<cudaEvent_t> ev_d2h;        // per instance: its download finished
   cudaEvent_t ev_step = nullptr;          // the iteration's kernels finished
   static constexpr size_t OUT_CHUNK = (size_t)1 << 20;
-  char* h_out = nullptr;                  // two pinned chunks of copy_out
+  std::mutex mu_out;                      // one copy_out at a time uses
+  char* h_out = nullptr;                  // the two pinned chunks
   cudaEvent_t ev_out[2] = {};
   int cap = 0;
   double* d_red = nullptr; int32_t* d_ist = nullptr;
@@ -1009,8 +1011,10 @@ static int copy_out(ot2d_solver* s, void* dst, const void* src, size_t bytes) {
   cudaPointerAttributes a;
   const bool plain = cudaPointerGetAttributes(&a, dst) == cudaSuccess && a.type == cudaMemoryTypeUnregistered;
   if (!plain) cudaGetLastError();
-  if (plain && bytes && !host_resident(dst, bytes) &&
-      (s->h_out || cudaMallocHost(&s->h_out, 2 * CH) == cudaSuccess)) {
+  // (threads may read states of one solver at once: one at a time has the chunks)
+  std::unique_lock<std::mutex> chunks(s->mu_out, std::defer_lock);
+  if (plain && bytes && !host_resident(dst, bytes)) chunks.lock();
+  if (chunks.owns_lock() && (s->h_out || cudaMallocHost(&s->h_out, 2 * CH) == cudaSuccess)) {
     for (cudaEvent_t& e : s->ev_out)
       if (!e && cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess) return OT2D_ERR_CUDA;
     const size_t n = (bytes + CH - 1) / CH;

@@ -1128,10 +1128,17 @@ int iterate_host_parts(ot2d_solver* s, int32_t n, std::vector<Rec*>& rs, double*
   done = 0;
   int err = OT2D_OK;
   bool parts = true;
-  // uploads come after everything launched before
+  // uploads, and with them the parts, come after everything the solver stream
+  // has been given: what was launched before, the time step that a rebuild
+  // computes for the new batch
   if (!s->st_h2d && cudaStreamCreateWithFlags(&s->st_h2d, cudaStreamNonBlocking) != cudaSuccess) return OT2D_ERR_CUDA;
-  if (cudaEventRecord(s->ev_step, s->st) != cudaSuccess || cudaStreamWaitEvent(s->st_h2d, s->ev_step, 0) != cudaSuccess)
-    return OT2D_ERR_CUDA;
+  auto after_solver_stream = [&] {
+    return cudaEventRecord(s->ev_step, s->st) == cudaSuccess &&
+                   cudaStreamWaitEvent(s->st_h2d, s->ev_step, 0) == cudaSuccess
+               ? OT2D_OK
+               : OT2D_ERR_CUDA;
+  };
+  if ((err = after_solver_stream())) return err;
   for (int q = 0; q < s->np; ++q)
     if (cudaEventRecord(s->ev_pdown[q], s->pst[q]) != cudaSuccess) return OT2D_ERR_CUDA;
   for (int it = 0; it < iters && !err && parts; ++it) {
@@ -1180,6 +1187,7 @@ int iterate_host_parts(ot2d_solver* s, int32_t n, std::vector<Rec*>& rs, double*
         for (int i = 0; i < n; ++i)
           if (!rs[i]->live) { err = OT2D_ERR_ARG; break; }
         if (!err) err = rebuild(s);
+        if (!err) err = after_solver_stream();
         parts = s->parts;   // retirements took the batch below the parts' size
       }
     }

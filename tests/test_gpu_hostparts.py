@@ -51,3 +51,36 @@ def test_unlisted_requests_retire_during_the_call(precision, listed):
         sv.close()
     for a, b in zip(out["device"], out["host"]):
         assert np.array_equal(a, b)
+
+
+def test_resident_iterations_stay_as_they_were():
+    """A call of the host-buffer path leaves the device-resident iteration's
+    launches alone: its parts are its own.  The two paths in turn give the
+    bits of the device path alone.  A refused call changes nothing either."""
+    cases = _cases(20)
+    L = api.lib()
+    L.ot2d_solver_graph_kernels.argtypes = [C.c_void_p]
+
+    def run(host):
+        sv = api.Solver(OT2D_FP32_MIXED, check_every=100, keep_q=True)
+        ids = [sv.add(c[1], c[2], c[3], orders=0.0, max_iters=1000) for c in cases]
+        sv.iterate(3)
+        kernels = L.ot2d_solver_graph_kernels(sv._h)
+        if host:
+            q = [np.ascontiguousarray(sv.get_q(i, c[1])) for i, c in zip(ids, cases)]
+            assert _host_iterate(sv, [ids[0], 12345], q[:2], 1) != 0    # no such request
+            assert L.ot2d_solver_graph_kernels(sv._h) == kernels
+            assert _host_iterate(sv, ids, q, 2) == 0
+        else:
+            sv.iterate(2)
+        assert L.ot2d_solver_graph_kernels(sv._h) == kernels
+        sv.iterate(3)
+        sv.sync()
+        out = [sv.get_q(i, c[1]) for i, c in zip(ids, cases)]
+        sv.close()
+        return kernels, out
+
+    (ka, a), (kb, b) = run(False), run(True)
+    assert ka == kb
+    for x, y in zip(a, b):
+        assert np.array_equal(x, y)

@@ -138,18 +138,20 @@ struct ot2d_solver {
   cudaStream_t st2 = nullptr;
   cudaEvent_t ev_half[2] = {nullptr, nullptr};   // recorded in each half's graph after its rbc
   cudaEvent_t ev_join = nullptr;
-  // Host-buffer path: the batch in HP parts of about equal cells, a graph
-  // and a stream each, so that some parts' copies run while others iterate
-  // (built once that path is used)
+  // The batch in parts of about equal cells, a graph and a stream each: four
+  // for the device-resident iteration, eight (four below eight requests) for
+  // the host-buffer path, so that some parts' copies run while others iterate.
+  // Each set is built when its path first runs a batch.
   static constexpr int HP = 8, HP_MIN = 4;
-  int np = HP_MIN;                        // parts of this batch
-  bool want_parts = false;
-  bool parts = false;
-  DevBatch<double> p64[HP];
-  DevBatch<float> p32[HP];
-  cudaGraph_t pgraph[HP] = {};
-  cudaGraphExec_t pexec[HP] = {};
-  cudaStream_t pst[HP] = {};
+  struct Parts {
+    int n = 0;                            // 0: not built
+    DevBatch<double> b64[HP];
+    DevBatch<float> b32[HP];
+    cudaGraph_t graph[HP] = {};
+    cudaGraphExec_t exec[HP] = {};
+  } resident, host;
+  bool can_parts = false;                 // the batch is large enough for parts
+  cudaStream_t pst[HP] = {};              // both sets' streams (one set runs at a time)
   cudaEvent_t ev_pdone[HP] = {};
   cudaStream_t st_h2d = nullptr;          // the parts' uploads, one part after another
   cudaEvent_t ev_pup[HP] = {}, ev_pdown[HP] = {};   // a part's uploads / downloads finished
@@ -225,13 +227,18 @@ void drop_graph(ot2d_solver* s) {
   s->split = false;
   s->split4 = false;
   s->halves = false;
-  for (int q = 0; q < ot2d_solver::HP; ++q) {
-    if (s->pexec[q]) cudaGraphExecDestroy(s->pexec[q]);
-    if (s->pgraph[q]) cudaGraphDestroy(s->pgraph[q]);
-    s->pexec[q] = nullptr; s->pgraph[q] = nullptr;
+  for (ot2d_solver::Parts* P : {&s->resident, &s->host}) {
+    for (int q = 0; q < ot2d_solver::HP; ++q) {
+      if (P->exec[q]) cudaGraphExecDestroy(P->exec[q]);
+      if (P->graph[q]) cudaGraphDestroy(P->graph[q]);
+      P->exec[q] = nullptr; P->graph[q] = nullptr;
+    }
+    P->n = 0;
   }
-  s->parts = false;
+  s->can_parts = false;
 }
+
+int ensure_parts(ot2d_solver* s, ot2d_solver::Parts& P, int n);
 
 // batches of at least this many slices run in parts or as two pipelined halves
 constexpr int PIPE_MIN_SLICES = 16;
@@ -242,10 +249,11 @@ cudaError_t launch_graph_iteration(ot2d_solver* s) {
   if (s->split4) {
     // four independent parts, each on its own stream after what the solver
     // stream holds (uploads, a rebuild's time step)
+    if (ensure_parts(s, s->resident, ot2d_solver::HP_MIN)) return cudaErrorUnknown;
     cudaError_t e = cudaEventRecord(s->ev_step, s->st);
-    for (int q = 0; q < s->np && e == cudaSuccess; ++q) {
+    for (int q = 0; q < s->resident.n && e == cudaSuccess; ++q) {
       e = cudaStreamWaitEvent(s->pst[q], s->ev_step, 0);
-      if (e == cudaSuccess) e = cudaGraphLaunch(s->pexec[q], s->pst[q]);
+      if (e == cudaSuccess) e = cudaGraphLaunch(s->resident.exec[q], s->pst[q]);
     }
     return e;
   }
@@ -263,7 +271,7 @@ cudaError_t launch_graph_iteration(ot2d_solver* s) {
 cudaError_t join_halves(ot2d_solver* s) {
   if (s->split4) {
     cudaError_t e = cudaSuccess;
-    for (int q = 0; q < s->np && e == cudaSuccess; ++q) {
+    for (int q = 0; q < s->resident.n && e == cudaSuccess; ++q) {
       e = cudaEventRecord(s->ev_pdone[q], s->pst[q]);
       if (e == cudaSuccess) e = cudaStreamWaitEvent(s->st, s->ev_pdone[q], 0);
     }
@@ -277,17 +285,17 @@ cudaError_t join_halves(ot2d_solver* s) {
 template <class R> DevBatch<R>* halves_of(ot2d_solver* s);
 template <> DevBatch<double>* halves_of<double>(ot2d_solver* s) { return s->h64; }
 template <> DevBatch<float>* halves_of<float>(ot2d_solver* s) { return s->h32; }
-template <class R> DevBatch<R>* parts_of(ot2d_solver* s);
-template <> DevBatch<double>* parts_of<double>(ot2d_solver* s) { return s->p64; }
-template <> DevBatch<float>* parts_of<float>(ot2d_solver* s) { return s->p32; }
+template <class R> DevBatch<R>* parts_of(ot2d_solver::Parts& P);
+template <> DevBatch<double>* parts_of<double>(ot2d_solver::Parts& P) { return P.b64; }
+template <> DevBatch<float>* parts_of<float>(ot2d_solver::Parts& P) { return P.b32; }
 
-// The host-buffer path's parts: HP batches of about equal cells (a
-// request's time instances in one part), each captured as its own graph
-// on its own stream, with B's launch choices.
+// np batches of about equal cells (a request's time instances in one part),
+// each captured as its own graph on its own stream, with the launch choices
+// of the whole batch B.
 template <class R>
-int build_parts(ot2d_solver* s, const DevBatch<R>& B, int visc) {
+int build_parts(ot2d_solver* s, ot2d_solver::Parts& set, int np, const DevBatch<R>& B) {
   constexpr int HP = ot2d_solver::HP;
-  const int np = s->np;
+  const int visc = s->any_viscous ? 1 : 0;
   std::vector<int> ids = s->live;
   auto cells_of = [&](int id) { const ot2d_params& p = s->recs[id].d.P; return (size_t)p.jd * p.kd * p.nspec; };
   std::stable_sort(ids.begin(), ids.end(), [&](int a, int b) { return cells_of(a) > cells_of(b); });
@@ -299,9 +307,10 @@ int build_parts(ot2d_solver* s, const DevBatch<R>& B, int visc) {
       if (load[i] < load[q]) q = i;
     load[q] += cells_of(id);
     slices_of<R>(s, s->recs[id], slp[q]);
-    s->recs[id].part = q;
+    if (&set == &s->host) s->recs[id].part = q;
   }
-  DevBatch<R>* P = parts_of<R>(s);
+  if (!s->ev_step && cudaEventCreateWithFlags(&s->ev_step, cudaEventDisableTiming) != cudaSuccess) return OT2D_ERR_CUDA;
+  DevBatch<R>* P = parts_of<R>(set);
   for (int q = 0; q < np; ++q) {
     if (!s->pst[q] && cudaStreamCreateWithFlags(&s->pst[q], cudaStreamNonBlocking) != cudaSuccess) return OT2D_ERR_CUDA;
     for (cudaEvent_t* e : {&s->ev_pdone[q], &s->ev_pup[q], &s->ev_pdown[q]})
@@ -317,12 +326,27 @@ int build_parts(ot2d_solver* s, const DevBatch<R>& B, int visc) {
     cudaStream_t cs = s->pst[q];
     if (cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal) != cudaSuccess) return OT2D_ERR_CUDA;
     cudaError_t le = launch_iteration<R>(P[q].d_sl, P[q].b, visc, s->turb_bits, s->lhs_bits, cs);
-    cudaError_t ce = cudaStreamEndCapture(cs, &s->pgraph[q]);
+    cudaError_t ce = cudaStreamEndCapture(cs, &set.graph[q]);
     if (le != cudaSuccess || ce != cudaSuccess) return OT2D_ERR_CUDA;
-    if (cudaGraphInstantiate(&s->pexec[q], s->pgraph[q], 0) != cudaSuccess) return OT2D_ERR_CUDA;
+    if (cudaGraphInstantiate(&set.exec[q], set.graph[q], 0) != cudaSuccess) return OT2D_ERR_CUDA;
   }
-  s->parts = true;
+  set.n = np;
   return OT2D_OK;
+}
+
+// The parts of the current batch for one of the two paths, built when that
+// path first runs it.
+int ensure_parts(ot2d_solver* s, ot2d_solver::Parts& P, int n) {
+  if (P.n) return OT2D_OK;
+  return s->precision == OT2D_FP64 ? build_parts<double>(s, P, n, s->b64) : build_parts<float>(s, P, n, s->b32);
+}
+// Parts of the host-buffer path.  Two host iterations in 4, 6, 8 parts (us): 64
+// instances of 513x129 4155, 3825, 3847; 16 of them 1632, 1585, 1554; 64 of
+// 257x65 1523, 1416, 1395; 64 of 129x33 761, 748, 724.  (The device-resident
+// iteration keeps four: within 1 % of eight at large batches, faster at 16
+// slices.)
+int host_parts(const ot2d_solver* s) {
+  return s->live.size() >= (size_t)ot2d_solver::HP ? ot2d_solver::HP : ot2d_solver::HP_MIN;
 }
 
 // With the time step folded into the state update, the first iteration of a
@@ -391,32 +415,21 @@ int rebuild_t(ot2d_solver* s, DevBatch<R>& B) {
   if (branch_of_device(br) != cudaSuccess) return OT2D_ERR_CUDA;
   const int visc = s->any_viscous ? 1 : 0;
   const bool big = sl.size() >= (size_t)PIPE_MIN_SLICES;
-  const bool can_parts = big && s->live.size() >= (size_t)ot2d_solver::HP_MIN;
+  s->can_parts = big && s->live.size() >= (size_t)ot2d_solver::HP_MIN;
   // Unless the option says which: four independent parts where there are four
   // requests, else two halves.
   // Per iteration (us) in halves, in parts: five time instances of four
   // requests 257x65 250, 234; 16 pitching slices 257x65 261, 247; 24 slices
   // of five sizes 684, 668; 64 slices 513x129 1257, 1227, 129x33 188, 151.
-  const bool split4 = ch.pipeline >= 2 && can_parts;
+  const bool split4 = ch.pipeline >= 2 && s->can_parts;
   const bool split = (ch.pipeline & 1) && big && s->live.size() >= 2 && !split4;
-  if (split4 && !s->ev_step && cudaEventCreateWithFlags(&s->ev_step, cudaEventDisableTiming) != cudaSuccess)
-    return OT2D_ERR_CUDA;
   for (int id : s->live) { s->recs[id].half = -1; s->recs[id].part = -1; }
-  // the parts: for the device-resident iteration or once the host-buffer
-  // path has been used
-  const bool want_parts = (s->want_parts || split4) && can_parts;
-  // Eight parts once the host-buffer path has been used, four before.
-  // Two host iterations in 4, 6, 8 parts (us): 64 instances of 513x129 4155,
-  // 3825, 3847; 16 of them 1632, 1585, 1554; 64 of 257x65 1523, 1416, 1395;
-  // 64 of 129x33 761, 748, 724.
-  s->np = s->want_parts && s->live.size() >= (size_t)ot2d_solver::HP ? ot2d_solver::HP : ot2d_solver::HP_MIN;
   if (!split) {
     if (cudaStreamBeginCapture(s->st, cudaStreamCaptureModeThreadLocal) != cudaSuccess) return OT2D_ERR_CUDA;
     cudaError_t le = launch_iteration<R>(B.d_sl, B.b, visc, s->turb_bits, s->lhs_bits, s->st);
     cudaError_t ce = cudaStreamEndCapture(s->st, &s->graph);
     if (le != cudaSuccess || ce != cudaSuccess) return OT2D_ERR_CUDA;
     if (cudaGraphInstantiate(&s->gexec, s->graph, 0) != cudaSuccess) return OT2D_ERR_CUDA;
-    if (want_parts && (e = build_parts<R>(s, B, visc))) return e;
     s->split4 = split4;
     return time_step_now<R>(s, B);
   }
@@ -456,7 +469,6 @@ int rebuild_t(ot2d_solver* s, DevBatch<R>& B) {
   }
   s->halves = true;
   s->split = split;
-  if (want_parts && (e = build_parts<R>(s, B, visc))) return e;
   return time_step_now<R>(s, B);
 }
 
@@ -861,7 +873,7 @@ void ot2d_solver_destroy(ot2d_solver* s) {
   }
   if (s->ev_join) cudaEventDestroy(s->ev_join);
   for (int q = 0; q < ot2d_solver::HP; ++q) {
-    s->p64[q].release(); s->p32[q].release();
+    for (ot2d_solver::Parts* P : {&s->resident, &s->host}) { P->b64[q].release(); P->b32[q].release(); }
     for (cudaEvent_t e : {s->ev_pdone[q], s->ev_pup[q], s->ev_pdown[q]}) if (e) cudaEventDestroy(e);
     if (s->pst[q]) { cudaStreamSynchronize(s->pst[q]); cudaStreamDestroy(s->pst[q]); }
   }
@@ -1090,9 +1102,10 @@ int ot2d_solver_graph_kernels(ot2d_solver* s) {
   if (s->dirty) { int e = rebuild(s); if (e) return -e; }
   if (s->live.empty()) return 0;
   if (s->split4) {
-    int k = 0;
-    for (int q = 0; q < s->np; ++q) {
-      const int a = kernel_nodes(s->pgraph[q]);
+    int k = ensure_parts(s, s->resident, ot2d_solver::HP_MIN);
+    if (k) return -k;
+    for (int q = 0; q < s->resident.n; ++q) {
+      const int a = kernel_nodes(s->resident.graph[q]);
       if (a < 0) return a;
       k += a;
     }
@@ -1107,10 +1120,10 @@ int ot2d_solver_graph_kernels(ot2d_solver* s) {
 // when the batch folds it into the state update: after a host-buffer upload.
 cudaError_t host_time_step(ot2d_solver* s, int part, cudaStream_t st) {
   if (s->precision == OT2D_FP32_MIXED) {
-    DevBatch<float>& B = part < 0 ? s->b32 : s->p32[part];
+    DevBatch<float>& B = part < 0 ? s->b32 : s->host.b32[part];
     return B.b.ts_in_update ? launch_time_step<float>(B.d_sl, B.b, st) : cudaSuccess;
   }
-  DevBatch<double>& B = part < 0 ? s->b64 : s->p64[part];
+  DevBatch<double>& B = part < 0 ? s->b64 : s->host.b64[part];
   return B.b.ts_in_update ? launch_time_step<double>(B.d_sl, B.b, st) : cudaSuccess;
 }
 
@@ -1139,11 +1152,11 @@ int iterate_host_parts(ot2d_solver* s, int32_t n, std::vector<Rec*>& rs, double*
                : OT2D_ERR_CUDA;
   };
   if ((err = after_solver_stream())) return err;
-  for (int q = 0; q < s->np; ++q)
+  for (int q = 0; q < s->host.n; ++q)
     if (cudaEventRecord(s->ev_pdown[q], s->pst[q]) != cudaSuccess) return OT2D_ERR_CUDA;
   for (int it = 0; it < iters && !err && parts; ++it) {
     done = it + 1;
-    for (int q = 0; q < s->np && !err; ++q) {
+    for (int q = 0; q < s->host.n && !err; ++q) {
       cudaStream_t sq = s->pst[q];
       if (cudaStreamWaitEvent(s->st_h2d, s->ev_pdown[q], 0) != cudaSuccess) err = OT2D_ERR_CUDA;
       for (int i = 0; i < n && !err; ++i) {
@@ -1156,11 +1169,11 @@ int iterate_host_parts(ot2d_solver* s, int32_t n, std::vector<Rec*>& rs, double*
                    cudaStreamWaitEvent(sq, s->ev_pup[q], 0) != cudaSuccess))
         err = OT2D_ERR_CUDA;
       if (!err && s->precision == OT2D_FP32_MIXED &&
-          launch_shadow<float>(s->p32[q].d_sl, s->p32[q].b, sq) != cudaSuccess)
+          launch_shadow<float>(s->host.b32[q].d_sl, s->host.b32[q].b, sq) != cudaSuccess)
         err = OT2D_ERR_CUDA;
       // the uploaded state may differ from the one the last update saw
       if (!err && host_time_step(s, q, sq) != cudaSuccess) err = OT2D_ERR_CUDA;
-      if (!err && (cudaGraphLaunch(s->pexec[q], sq) != cudaSuccess ||
+      if (!err && (cudaGraphLaunch(s->host.exec[q], sq) != cudaSuccess ||
                    cudaEventRecord(s->ev_pdone[q], sq) != cudaSuccess ||
                    cudaStreamWaitEvent(s->st_d2h, s->ev_pdone[q], 0) != cudaSuccess))
         err = OT2D_ERR_CUDA;
@@ -1179,7 +1192,7 @@ int iterate_host_parts(ot2d_solver* s, int32_t n, std::vector<Rec*>& rs, double*
     }
     if (!err && (++s->since_check >= s->check_every || capped)) {
       // the status read sees every part done and no upload in flight
-      for (int q = 0; q < s->np && !err; ++q)
+      for (int q = 0; q < s->host.n && !err; ++q)
         if (cudaStreamWaitEvent(s->st, s->ev_pdone[q], 0) != cudaSuccess) err = OT2D_ERR_CUDA;
       if (!err && cudaStreamSynchronize(s->st_d2h) != cudaSuccess) err = OT2D_ERR_CUDA;
       if (!err) err = check(s);
@@ -1187,15 +1200,16 @@ int iterate_host_parts(ot2d_solver* s, int32_t n, std::vector<Rec*>& rs, double*
         for (int i = 0; i < n; ++i)
           if (!rs[i]->live) { err = OT2D_ERR_ARG; break; }
         if (!err) err = rebuild(s);
+        parts = s->can_parts;   // retirements took the batch below the parts' size
+        if (!err && parts) err = ensure_parts(s, s->host, host_parts(s));
         if (!err) err = after_solver_stream();
-        parts = s->parts;   // retirements took the batch below the parts' size
       }
     }
   }
   if (cudaStreamSynchronize(s->st_h2d) != cudaSuccess && !err) err = OT2D_ERR_CUDA;
   if (cudaStreamSynchronize(s->st_d2h) != cudaSuccess && !err) err = OT2D_ERR_CUDA;
-  for (int q = 0; q < s->np; ++q)
-    if (cudaStreamSynchronize(s->pst[q]) != cudaSuccess && !err) err = OT2D_ERR_CUDA;
+  for (int q = 0; q < ot2d_solver::HP; ++q)
+    if (s->pst[q] && cudaStreamSynchronize(s->pst[q]) != cudaSuccess && !err) err = OT2D_ERR_CUDA;
   if (cudaStreamSynchronize(s->st) != cudaSuccess && !err) err = OT2D_ERR_CUDA;
   return err;
 }
@@ -1203,9 +1217,6 @@ int iterate_host_parts(ot2d_solver* s, int32_t n, std::vector<Rec*>& rs, double*
 int ot2d_solver_iterate_host(ot2d_solver* s, int32_t n, const int32_t* ids, double* const* q_host, int32_t iters) {
   if (!s || n < 0 || (n && (!ids || !q_host)) || iters < 0) return OT2D_ERR_ARG;
   cudaSetDevice(s->device);
-  // A batch large enough for parts overlaps some parts' copies with the
-  // others' iterations.
-  if (!s->want_parts && s->live.size() >= (size_t)ot2d_solver::HP_MIN) s->want_parts = s->dirty = true;
   if (s->dirty) { int e = rebuild(s); if (e) return e; }
   std::vector<Rec*> rs;
   for (int i = 0; i < n; ++i) {
@@ -1225,9 +1236,11 @@ int ot2d_solver_iterate_host(ot2d_solver* s, int32_t n, const int32_t* ids, doub
   }
   int err = OT2D_OK;
   int32_t done = 0;
-  if (s->parts) {
-    // the rest (if retirements took the batch below the parts' size) in
-    // the single graph below
+  if (s->can_parts && iters > 0) {
+    // A batch large enough for parts overlaps some parts' copies with the
+    // others' iterations; the rest (if retirements took the batch below the
+    // parts' size) in the single graph below.
+    if ((err = ensure_parts(s, s->host, host_parts(s))) != OT2D_OK) return err;
     if ((err = iterate_host_parts(s, n, rs, q_host, iters, done)) != OT2D_OK || done == iters) return err;
   }
   for (int it = done; it < iters && !err; ++it) {

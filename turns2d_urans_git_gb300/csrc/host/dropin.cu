@@ -152,6 +152,16 @@ void host_store(double* p, const double* v, size_t n) {
   }
 }
 
+// This call's stream after the work that the default stream has been given.
+void after_default_stream(int& err) {
+  if (err || g_ctx.geo_waits) return;
+  if (!g_ctx.geo && cudaEventCreateWithFlags(&g_ctx.geo, cudaEventDisableTiming) != cudaSuccess) err = OT2D_ERR_CUDA;
+  if (!err && (cudaEventRecord(g_ctx.geo, cudaStreamLegacy) != cudaSuccess ||
+               cudaStreamWaitEvent(g_ctx.st, g_ctx.geo) != cudaSuccess))
+    err = OT2D_ERR_CUDA;
+  g_ctx.geo_waits = !err;
+}
+
 // A geometry array (centres, vertices, vertex speeds) on the device.  Device
 // memory is used in place, after the work that the default stream has been
 // given; host memory is copied as it stands, registered or not.
@@ -159,13 +169,7 @@ const double* geo_view(const double* p, size_t n, int& err) {
   if (!p || err) return nullptr;
   cudaPointerAttributes a;
   if (cudaPointerGetAttributes(&a, p) == cudaSuccess && (a.type == cudaMemoryTypeDevice || a.type == cudaMemoryTypeManaged)) {
-    if (!g_ctx.geo_waits) {
-      if (!g_ctx.geo && cudaEventCreateWithFlags(&g_ctx.geo, cudaEventDisableTiming) != cudaSuccess) err = OT2D_ERR_CUDA;
-      if (!err && (cudaEventRecord(g_ctx.geo, cudaStreamLegacy) != cudaSuccess ||
-                   cudaStreamWaitEvent(g_ctx.st, g_ctx.geo) != cudaSuccess))
-        err = OT2D_ERR_CUDA;
-      g_ctx.geo_waits = !err;
-    }
+    after_default_stream(err);
     return p;
   }
   cudaGetLastError();
@@ -267,9 +271,12 @@ int faces_upload(double* dst4, double* dst2, const double* xv, const double* yv,
 }
 
 // SA wall distance into dsn, formed on the device.  (A wall range outside the
-// mesh is left to the host's loop.)
+// mesh is left to the host's loop.)  The call's kernels follow the default
+// stream wherever the geometry lives: callers that fill q or turmu there, with
+// their mesh in host memory, never had to synchronise before vmu_sa or step.
 void wall_upload(double* dsn, const double* x, const double* y, const double* xv, const double* yv, int& err) {
   const ot2d_params& p = g_ctx.P;
+  after_default_stream(err);
   const size_t n2 = (size_t)p.jd * p.kd, nv = (size_t)p.jmax * p.kmax;
   if (p.jtail1 >= 2 && p.jtail1 <= p.jd && p.jtail2 <= p.jmax) {
     GeomArgs g{};

@@ -46,7 +46,14 @@ struct Ctx {
   cudaEvent_t geo = nullptr;
   bool geo_waits = false;                          // this call's stream waits for the caller's geometry
   std::vector<double> norms;
-  ~Ctx() { if (arena) cudaFree(arena); }
+  // a thread that ends gives back all that its calls kept (nothing runs: every
+  // call returns after its stream is done)
+  ~Ctx() {
+    for (void* d : {(void*)dP, (void*)dwork, (void*)dred, (void*)dist, (void*)arena}) if (d) cudaFree(d);
+    batch.release();
+    if (geo) cudaEventDestroy(geo);
+    if (st) cudaStreamDestroy(st);
+  }
 };
 // A call whose arguments need more staging than this allocates it and gives
 // it back (a cudaMalloc / cudaFree pair is a few microseconds per array,

@@ -273,8 +273,11 @@ typedef struct ot2d_result {
                                      was created) */
 #define OT2D_OPT_LU_LAG        7  /* LU-SGS schedule: steps each band trails the band it
                                      depends on beyond the minimum (default 0) */
-#define OT2D_OPT_LU_GROUP      8  /* LU-SGS record chunks in flight per band: 1, 2, 4 or 8
-                                     (default 0: 8, as the shared memory allows) */
+#define OT2D_OPT_LU_GROUP      8  /* FP64 LU-SGS sweeps: bulk copies of two record chunks
+                                     in flight per band, 1, 2, 4 or 8 (at least 2, as the
+                                     shared memory allows; default 0: 8).  The FP32-mixed
+                                     sweeps keep two copies of four or eight chunks in
+                                     flight whatever it says */
 #define OT2D_OPT_RT_SHAPE      9  /* residual tile: 0 16x16 (default in FP64), 1 32x8 (default in
                                      FP32-mixed), 2 8x32, 3 32x16 cells */
 #define OT2D_OPT_PIPELINE     10  /* 1: a batch of 16 or more time instances runs
@@ -302,16 +305,16 @@ int ot2d_solver_set_force_tol(ot2d_solver* s, double dcl, double dcd);
 /* Launch choices for batches of one mesh-size class, as an autotuner
  * measured them (turns2d_urans_git_gb300/tune.py).  When a batch is built,
  * the first entry whose kd_max / jd_max bound the batch's largest mesh (the
- * one with most cells) sets the residual tile shape, the LU-SGS copy group,
- * the LU-SGS band lag and whether a batch of 16 or more time instances runs
- * as two pipelined halves; without a matching entry the OT2D_OPT_* values
- * apply.  The choices change the launch geometry and schedule only: every
+ * one with most cells) sets the residual tile shape, the LU-SGS copies
+ * in flight (FP64), the LU-SGS band lag and whether a batch of 16 or more time
+ * instances runs as one graph, two pipelined halves or four parts; without a
+ * matching entry the OT2D_OPT_* values apply.  The choices change the launch geometry and schedule only: every
  * variant gives the same state bit for bit (the L2 norm is summed per
  * residual tile, so it agrees to rounding across tile shapes). */
 typedef struct ot2d_tuning {
   int32_t kd_max, jd_max;   /* class bound: kd <= kd_max and jd <= jd_max      */
-  int32_t rt_shape;         /* 0 16x16, 1 32x8, 2 8x32                          */
-  int32_t lu_group;         /* 0 (largest that fits), 1, 2, 4, 8                */
+  int32_t rt_shape;         /* 0 16x16, 1 32x8, 2 8x32, 3 32x16                 */
+  int32_t lu_group;         /* 0 (as 8), 1, 2, 4, 8: OT2D_OPT_LU_GROUP          */
   int32_t lu_lag;           /* 0..64                                            */
   int32_t pipeline;         /* 0 one graph, 1 two pipelined halves, 2 four parts (OT2D_OPT_PIPELINE) */
 } ot2d_tuning;

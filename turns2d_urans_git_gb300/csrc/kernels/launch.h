@@ -93,7 +93,7 @@ struct Batch {
   NormPart* d_part = nullptr;         // [max(cell_blocks, tile_blocks)] norm partials
   uint32_t poll_limit = 1u << 22;     // polls of a LU-SGS sweep wait before it gives up
   int lu_lag = 0;                     // extra steps each LU-SGS band trails its neighbour (schedule)
-  int lu_group = 0;                   // record chunks per bulk copy of the sweeps (0: largest that fits)
+  int lu_group = 0;                   // record copies in flight per band of the FP64 sweeps (0: 8)
 };
 
 // One full iteration of step.f for every slice of the batch:

@@ -134,16 +134,16 @@ inline bool lu_spread(int nslice, int shared_bands) {
 struct LuLaunch { int pg = 0, cs = 0, nw = 0, D = 0; size_t smem = 0; };
 
 // With groups of PG and at least mind stages.  More CTAs than the rule above
-// only where the bands or their shared memory do not fit; group: record
-// chunks in flight per band where that is more than mind groups (0: 8; FP64:
-// twice as many), within ~200 KB of shared memory.
+// only where the bands or their shared memory do not fit; group (0: as 8): in
+// FP64 the stages where that is more than mind, within ~200 KB of shared
+// memory.  (An f32 stage is four or eight steps: two are enough.)
 template <class R, bool PRE, int PG>
 inline LuLaunch lu_launch_pg(int nb, bool spread, int maxcol, int group, int mind) {
   const int want = spread ? std::min((nb + 3) / 4, LU_MAX_CLUSTER) : 1;
   for (int cs = want; cs <= LU_MAX_CLUSTER; ++cs) {
     const int nw = (nb + cs - 1) / cs;
     if (nw > LU_MAX_WARPS || lu_smem_bytes<R, PRE, PG>(cs, nw, mind, maxcol) > (size_t)SMEM_OPTIN_MAX) continue;
-    int D = std::max(mind, mind < 2 ? mind : (sizeof(R) == 8 ? 2 : 1) * (group ? group : 8) / PG);
+    int D = sizeof(R) == 8 && mind > 1 ? std::max(mind, group ? group : 8) : mind;
     while (D > mind && lu_smem_bytes<R, PRE, PG>(cs, nw, D, maxcol) > 200 * 1024) --D;
     return {PG, cs, nw, D, lu_smem_bytes<R, PRE, PG>(cs, nw, D, maxcol)};
   }

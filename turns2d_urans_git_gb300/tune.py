@@ -6,9 +6,11 @@ candidate choice and keeps the fastest:
   rt_shape   the fused residual's tile, 16x16, 32x8, 8x32 (256 threads) or
              32x16 (512 threads) interior cells per CTA (staged halo per
              cell against threads per face line)
-  lu_group   LU-SGS record chunks streamed per bulk copy (4 or 8)
-  lu_lag     LU-SGS hyperplane schedule: steps each 32-row band trails the
-             band it depends on beyond the minimum (0 or 4)
+  lu_group   FP64 LU-SGS sweeps: bulk copies of two record chunks in flight
+             per band (4 or 8); the FP32-mixed sweeps always keep two copies
+             in flight, so there the two candidates launch the same
+  lu_lag     LU-SGS hyperplane schedule: steps each band trails the band it
+             depends on beyond the minimum (0 or 4)
   pipeline   a batch of 16 or more time instances as one graph (0), as two
              halves on two streams with each half's residual beside the
              other half's sweeps (1), or as four independent parts on four

@@ -78,7 +78,7 @@ template <class R>
 struct DevBatch {
   Batch b;
   Slice<R>* d_sl = nullptr;
-  int32_t* d_idx = nullptr;   // first / jfirst / kfirst, 3*(n+1)
+  int32_t* d_idx = nullptr;   // six prefix tables of n+1 entries, behind the slices
   NormPart* d_part = nullptr;
   size_t cap_sl = 0, cap_part = 0;
   int rt_shape = 0;   // residual tile shape the next build lays out (rt_shape_dims)

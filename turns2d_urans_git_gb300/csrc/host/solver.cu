@@ -418,9 +418,14 @@ int rebuild_t(ot2d_solver* s, DevBatch<R>& B) {
   s->can_parts = big && s->live.size() >= (size_t)ot2d_solver::HP_MIN;
   // Unless the option says which: four independent parts where there are four
   // requests, else two halves.
-  // Per iteration (us) in halves, in parts: five time instances of four
-  // requests 257x65 250, 234; 16 pitching slices 257x65 261, 247; 24 slices
-  // of five sizes 684, 668; 64 slices 513x129 1257, 1227, 129x33 188, 151.
+  // Per iteration (us) in halves, in parts.  FP32-mixed: five time instances
+  // of four requests 257x65 250, 234; 16 pitching slices 257x65 261, 247; 24
+  // slices of five sizes 684, 668; 64 slices 513x129 1257, 1227, 129x33 188,
+  // 151.  FP64, 16, 24, 32, 64 slices: 513x129 4960, 5010; 7784, 7482; 9303,
+  // 9393; 17675, 17712; 385x97 3088, 3047; 4549, 4392; 5454, 5411; 10158,
+  // 10061; 257x65 1599, 1611; 2156, 2105; 2641, 2626; 4694, 4696; 129x33 729,
+  // 703; 816, 784; 849, 893; 1476, 1411 (one graph is slower than either but
+  // at 16 slices of 129x33, 698).
   const bool split4 = ch.pipeline >= 2 && s->can_parts;
   const bool split = (ch.pipeline & 1) && big && s->live.size() >= 2 && !split4;
   for (int id : s->live) { s->recs[id].half = -1; s->recs[id].part = -1; }

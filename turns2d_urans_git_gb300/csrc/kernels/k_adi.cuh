@@ -7,12 +7,14 @@
 // T_xi^-1, inverts a scalar pentadiagonal system per j-line and variable,
 // multiplies by N^-1, inverts per k-line, multiplies by T_eta and converts
 // q back.  Here q is never rewritten: the primitive values and every
-// per-cell factor are kept in scratch arrays (cell-parallel kernels), the
-// dissipation coefficients of the line systems are assembled per cell in
-// gather form, and each (line, variable) system is solved by one thread with
-// a sliding window over the reference's pentadag recurrences.  In FP64 the
-// conservative round trip of q (:853-860, :1047-1054) is applied at the end
-// so q leaves with the reference's bits.
+// per-cell factor are kept in scratch arrays (cell-parallel kernels) and the
+// rows of the line systems are assembled per cell in gather form
+// (adi_row_cell).  A line has three systems, since variables 1 and 2 share
+// one matrix; each is solved with pentadag's recurrences for its one or two
+// right-hand sides, 32 lines along j by a CTA through staged tiles
+// (k_lines.cuh), a line along k by one thread.  In FP64 the conservative round
+// trip of q (:853-860, :1047-1054) is applied at the end so q leaves with the
+// reference's bits.
 #pragma once
 #include "dev_common.cuh"
 #include "k_lines.cuh"

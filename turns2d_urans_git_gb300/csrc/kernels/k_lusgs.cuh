@@ -19,8 +19,8 @@
 //     the warps advance in a skewed lockstep; each warp streams its chunks
 //     into a shared-memory ring with cp.async.bulk (TMA) completing on
 //     mbarriers.  The lanes of a cell share its arithmetic (LuSplit), the
-//     contribution to the next row arrives by shuffle, across bands through a
-//     shared-memory ring and across the CTAs of the cluster through the next
+//     contribution to the next row passes through the warp's exchange buffer,
+//     across bands through a shared-memory ring and across the CTAs of the cluster through the next
 //     CTA's shared memory (st.async).  Every cell sees exactly the operands of
 //     the reference's hyperplane order, so the sweep equals the sequential
 //     one operation for operation.

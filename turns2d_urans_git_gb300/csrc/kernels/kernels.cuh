@@ -363,8 +363,8 @@ __global__ void k_rbc(const Slice<R>* __restrict__ sl) {
 // chunks of the band layout.  Row l of chunk (band, t) is cell (row RB band +
 // l, column t - l), so the chunks' rows walk the grid diagonally; thread i
 // computes row i / NC of chunk i % NC, which makes NC consecutive threads
-// read NC (32) consecutive cells of one row.  The records go to
-// the block's shared-memory copy of its chunks (chunk stride padded by 16
+// (32; 16 of the preconditioned FP64 records) read NC consecutive cells of one
+// row.  The records go to the block's shared-memory copy of its chunks (chunk stride padded by 16
 // bytes so the chunks of one row land in different banks), then each chunk
 // is stored with one bulk copy.  PRE: the preconditioned (preilu2d) records
 // of the slices with k_mp2 >= 0; each instantiation returns on the other

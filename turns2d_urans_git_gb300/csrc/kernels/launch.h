@@ -22,7 +22,7 @@ template <class R> constexpr int lu_prep_bs() { return sizeof(R) == 8 ? 256 : 51
 constexpr int BC_BS = 512;
 // threads of a CTA of one BC entry (several CTAs per slice)
 constexpr int BCE_BS = 128;
-// residual tile shapes (interior cells per CTA): 0 16x16, 1 32x8, 2 8x32
+// residual tile shapes (interior cells per CTA): 0 16x16, 1 32x8, 2 8x32, 3 32x16
 constexpr int RT_NSHAPE = 4;
 inline void rt_shape_dims(int shape, int& tj, int& tk) {
   tj = shape == 1 || shape == 3 ? 32 : (shape == 2 ? 8 : 16);
@@ -68,11 +68,11 @@ struct Batch {
   int nslice = 0;          // slices in the batch
   int moving = 0;          // some slice is time accurate on a pitching grid
   int precon = 0;          // some slice runs with Turkel preconditioning (k_mp2 >= 0)
+  int bands = 0;           // LU-SGS bands of the batch
+  int shared_bands = 0;    // and, where others run beside it, of all of them together
   // the solver's batches of steady requests with a first-order time step
   // factor: the local time step of the next iteration is computed by the
   // state update (k_update<R, true>), not by a kernel of its own
-  int bands = 0;           // LU-SGS bands of the batch
-  int shared_bands = 0;    // and, where others run beside it, of all of them together
   int ts_in_update = 0;
   int lim_mask = 0;        // reconstruction families of the slices: 1 central, 2 MUSCL, 4 WENO, 8 quad
   int rt_shape = 0;        // residual tile shape of the tile table (rt_shape_dims)
@@ -124,8 +124,6 @@ template <class R> cudaError_t launch_iter_begin(const Slice<R>* d_sl, const Bat
 template <class R> cudaError_t launch_time_step(const Slice<R>* d_sl, const Batch& b, cudaStream_t st);
 // pitch alone (the drop-in ot2d_pitch): slices with xc set and ist[4] == 1
 template <class R> cudaError_t launch_pitch(const Slice<R>* d_sl, const Batch& b, cudaStream_t st);
-// stqol over n elements of each of nv variables (stride qs): q of the
-// current step, the stored levels and the Newton target (time.f:110-175)
 // Geometry of one mesh (nhalo 1) from its vertices: the four face-normal
 // arrays (faces, ws apart) with, when speeds is not null, the two face-speed
 // arrays, and / or the SA wall distance sn of the centres (x, y).
@@ -135,6 +133,8 @@ struct GeomArgs {
   int64_t ws;
 };
 cudaError_t launch_geometry(const ot2d_params* d_p, int cells, const GeomArgs& g, cudaStream_t st);
+// stqol over n elements of each of nv variables (stride qs): q of the
+// current step, the stored levels and the Newton target (time.f:110-175)
 cudaError_t launch_stqol(const double* q, double* qtn, double* qtnm1, double* qnewt, int64_t qs, int nv, int ntac,
                          int istep, cudaStream_t st);
 // begin = 1 (mixed path): each slice's boundary CTA first applies the

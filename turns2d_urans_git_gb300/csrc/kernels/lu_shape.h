@@ -115,11 +115,13 @@ constexpr int SMEM_OPTIN_MAX = 227 * 1024;
 // CTAs per slice of the sweeps (a cluster), for nb bands.  One warp per SM
 // sub-partition (4 bands per CTA) makes a step fastest, but takes SMs from
 // the residual and the turbulence solve of a large batch.  Measured per
-// iteration (us), one CTA against ceil(nb / 4): FP32-mixed RANS-SA 769x193
-// alone 760, 454; 8 per launch 1127, 869; 32 per launch 2715, 2786; 513x129
-// 16 per launch 557, 477 (wide groups), 32 per launch 1276, 1328.  FP64
-// 513x129 alone 3769, 1877; 8 per launch 7577, 6801; 16 per launch 12638,
-// 13024.  The same line separates the wide groups of the f32 sweeps (lu_pg).
+// iteration (us), one CTA against ceil(nb / 4), RANS-SA in one launch.
+// FP32-mixed, with the groups that go with each form (lu_pg): 513x129 alone 364,
+// 275, 8 slices 454, 370, 16 slices 547, 474; 257x65 164, 151; 179, 164; 254,
+// 199; 129x33 103, 97; 105, 101; 110, 106; 32 slices of 513x129 1276, 1328 and
+// of 769x193 2715, 2786.  FP64: 513x129 alone 3675, 1771, 8 slices 4993, 3103,
+// 16 slices 6431, 5068; 385x97 2180, 1320; 2949, 2100; 3791, 3121; 257x65 1167,
+// 956; 1492, 1282; 1860, 1646; 129x33 the same (four bands: one CTA either way).
 // Batches that run beside each other (halves, parts) share the SMs: in four
 // parts, 64 slices of 513x129 (512 bands) 1228, 1269, of 385x97 (384) 747,
 // 787, of 257x65 (256) 394, 383; 32 of 385x97 (192) 492, 483; FP64 257x65,

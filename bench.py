@@ -52,7 +52,7 @@ PHASES = ["time_step", "bc", "residual", "rbc", "lusgs", "sa", "update"]
 # profiles/top_kernels_rans_sa_513x129_b8.md), scaled to the batch
 TRAFFIC_PER_CELL = {"residual": (40.496384e6 + 1.447168e6) / (8 * 65536),
                     # k_lu_prep + both sweeps (k_lu_edges, ~1 % of the phase, not captured)
-                    "lusgs": (35.18e6 + 53.31e6 + 52.36e6) / (8 * 65536),
+                    "lusgs": (35.25e6 + 53.37e6 + 52.37e6) / (8 * 65536),
                     # k_update as the phase timer runs it, without the folded time step
                     "update": (27.421952e6 + 0.079360e6) / (8 * 65536)}
 NPH = len(PHASES)

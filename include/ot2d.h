@@ -372,7 +372,8 @@ int ot2d_solver_live(const ot2d_solver* s);
 int ot2d_solver_queued(const ot2d_solver* s);
 /* copy the result of instance `id` (valid once retired, or a live snapshot) */
 int ot2d_solver_result(ot2d_solver* s, int32_t id, ot2d_result* out);
-/* download q (jd,kd,nspec,nq) of a live or retired-but-kept instance */
+/* download q (jd,kd,nspec,nq) of a live or retired-but-kept instance; several
+ * threads may read states of one solver at once (while none iterates it) */
 int ot2d_solver_get_q(ot2d_solver* s, int32_t id, double* q_out);
 /* total device bytes held by the live instances */
 size_t ot2d_solver_device_bytes(const ot2d_solver* s);
